@@ -336,7 +336,7 @@ class ForceEngine:
     # ---------------------------------------------------------------- the sweep
     @torch.no_grad()
     def energy_and_gradient(self, pos, species, src, dst, shifts, box, n_owned, dst_rowptr, plan=None, n_rows=None,
-                            pairs=None, row_mask=None):
+                            pairs=None, row_mask=None, src_csr=None):
         """pos [N_local,3] (owned rows first), species [N_local] (index), edges sorted by receiver with all
         receivers < n_owned, dst_rowptr [n_owned+1].  Returns (energy of owned atoms, dE/dpos [N_local,3],
         per-atom energies [n_owned]).  ``n_rows`` < N_local marks trailing rows of ``pos`` as padding: they may
@@ -345,7 +345,8 @@ class ForceEngine:
         optional fourth element is a device int64 scalar with the number of pair rows in use when U is a capacity.
         ``plan`` (an exchange plan of ``mace_ictc.domain``) refreshes the ghost rows between the interactions.
         ``row_mask`` [n_owned] (0 / 1) leaves padding rows among the owned rows out of the energy (and hence of
-        the gradient: a padding row has no edges)."""
+        the gradient: a padding row has no edges).  ``src_csr`` = (row offsets, edge ids) of the senders where the caller
+        has them."""
         self.refresh()
         m, c, lib, dev = self.model, self.c, self.lib, self.dev
         n_local, e = (pos.shape[0] if n_rows is None else int(n_rows)), int(src.numel())
@@ -363,7 +364,8 @@ class ForceEngine:
             _lib.check(lib.ictc_edge_geometry_forward(pos.data_ptr(), _lib.ptr(src), _lib.ptr(dst), _lib.ptr(shifts),
                                                       box_c, rmax, nb, pcut, e, _lib.ptr(sh), _lib.ptr(rb),
                                                       _lib.ptr(unit), _lib.ptr(length), st), "edge_geometry_forward")
-            src_csr = build_csr(src, n_local, assume_sorted=False)
+            if src_csr is None:
+                src_csr = build_csr(src, n_local, assume_sorted=False)
             grow = None if pairs is None else pairs[0]
             rep = None if pairs is None else pairs[1]               # the MLP kernels gather / scatter the pair rows
             live = pairs[3] if (pairs is not None and len(pairs) > 3) else None
@@ -373,7 +375,7 @@ class ForceEngine:
             # gate row of the edge at every position of the sender order (reverse sweep of the streamed mode)
             grow_by_pos = None
             if chunked:
-                grow_by_pos = src_csr[1] if grow is None else grow.index_select(0, src_csr[1])
+                grow_by_pos = src_csr[1][:e] if grow is None else grow.index_select(0, src_csr[1][:e])
             sp_owned = species[:n_owned]
             s_count = self.emb.shape[0]
             # ---- layer 0

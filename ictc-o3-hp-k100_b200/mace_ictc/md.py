@@ -50,6 +50,25 @@ def _arr(values, ctype):
     return (ctype * 3)(*[values[i] for i in range(3)])
 
 
+def _list_arguments(pos, lo, hi, box, periodic, cutoff):
+    """ctypes views of a neighbour call's geometry and its scratch buffer."""
+    lo_c, hi_c = _arr([float(x) for x in lo], C.c_double), _arr([float(x) for x in hi], C.c_double)
+    box_c, per_c = _arr([float(x) for x in box], C.c_double), _arr([int(x) for x in periodic], C.c_int)
+    nbytes = int(_lib.load().ictc_neighbor_scratch_bytes(pos.shape[0], lo_c, hi_c, float(cutoff)))
+    return lo_c, hi_c, box_c, per_c, torch.empty(nbytes, dtype=torch.uint8, device=pos.device)
+
+
+def count_edges(pos, num_centres, lo, hi, box, periodic, cutoff):
+    """Number of edges that ``neighbor_list`` finds, without building the list."""
+    lo_c, hi_c, box_c, per_c, scratch = _list_arguments(pos, lo, hi, box, periodic, cutoff)
+    counts = torch.empty(num_centres + 1, dtype=torch.int64, device=pos.device)
+    with _lib.on_device(pos.device):
+        _lib.check(_lib.load().ictc_neighbor_count(pos.data_ptr(), pos.shape[0], num_centres, lo_c, hi_c, box_c, per_c,
+                                                   float(cutoff), counts.data_ptr(), scratch.data_ptr(),
+                                                   _lib.stream(pos.device)), "ictc_neighbor_count")
+    return int(counts.sum().item())
+
+
 def neighbor_list(pos, num_centres, lo, hi, box, periodic, cutoff, return_keys=False):
     """Edges (src=j, dst=i) of the first ``num_centres`` rows, sorted by (dst, src, shift).
 
@@ -58,10 +77,7 @@ def neighbor_list(pos, num_centres, lo, hi, box, periodic, cutoff, return_keys=F
     """
     lib, dev = _lib.load(), pos.device
     n = pos.shape[0]
-    lo_c, hi_c = _arr([float(x) for x in lo], C.c_double), _arr([float(x) for x in hi], C.c_double)
-    box_c, per_c = _arr([float(x) for x in box], C.c_double), _arr([int(x) for x in periodic], C.c_int)
-    nbytes = int(lib.ictc_neighbor_scratch_bytes(n, lo_c, hi_c, float(cutoff)))
-    scratch = torch.empty(nbytes, dtype=torch.uint8, device=dev)
+    lo_c, hi_c, box_c, per_c, scratch = _list_arguments(pos, lo, hi, box, periodic, cutoff)
     rowptr = torch.empty(num_centres + 1, dtype=torch.int64, device=dev)
     scan = torch.empty(int(lib.ictc_scan_scratch_bytes(num_centres + 1)), dtype=torch.uint8, device=dev)
     pos = pos.contiguous()
@@ -119,54 +135,51 @@ class StaticNeighborList:
     every edge has its reverse in the list, more when senders can be ghosts)."""
 
     def __init__(self, num_atoms, box, cutoff, capacity, device, *, num_centres=None, lo=None, hi=None,
-                 periodic=(1, 1, 1), pair_fraction=0.5):
+                 periodic=(1, 1, 1), pair_fraction=0.5, dummy_row=True):
         self.n, self.cap, self.cutoff, self.dev = int(num_atoms), int(capacity), float(cutoff), device
         self.centres = self.n if num_centres is None else int(num_centres)
         lib = _lib.load()
         self.lo = _arr([0.0, 0.0, 0.0] if lo is None else [float(v) for v in lo], C.c_double)
         self.hi = _arr([float(b) for b in box] if hi is None else [float(v) for v in hi], C.c_double)
         self.box, self.per = _arr([float(b) for b in box], C.c_double), _arr([int(v) for v in periodic], C.c_int)
-        n1 = self.n + 1                                   # the position buffer carries one extra (dummy) row
-        self.scratch = torch.empty(int(lib.ictc_neighbor_scratch_bytes(n1, self.lo, self.hi, self.cutoff)),
+        # the position buffer of a recorded step carries one extra (dummy) row, the sender of the inert edges; a caller
+        # that reads the edge count and uses the live edges alone needs none
+        self.rows = self.n + (1 if dummy_row else 0)
+        self.pad_src = self.n if dummy_row else 0
+        self.scratch = torch.empty(int(lib.ictc_neighbor_scratch_bytes(self.rows, self.lo, self.hi, self.cutoff)),
                                    dtype=torch.uint8, device=device)
-        self.scan = torch.empty(int(lib.ictc_scan_scratch_bytes(self.centres + 1)), dtype=torch.uint8, device=device)
-        self.rowptr = torch.zeros(self.centres + 1, dtype=torch.int64, device=device)
+        # [row offsets | number of pairs | overflow flag] in one buffer, so that a host that wants all three copies once
+        self._rows = torch.zeros(self.centres + 3, dtype=torch.int64, device=device)
+        self.rowptr = self._rows[:self.centres + 1]
+        self.num_unique = self._rows[self.centres + 1:self.centres + 2]
+        self.overflow = self._rows[self.centres + 2:].view(torch.int32)[:1]
         self.src = torch.zeros(self.cap, dtype=torch.int64, device=device)
         self.dst = torch.zeros(self.cap, dtype=torch.int64, device=device)
         self.shifts = torch.zeros(self.cap, 3, dtype=torch.float32, device=device)
         self.keys = torch.zeros(self.cap, dtype=torch.int64, device=device)
-        self.overflow = torch.zeros(1, dtype=torch.int32, device=device)
         self.ucap = int(self.cap * pair_fraction) + 1024
         self.rev = torch.zeros(self.cap, dtype=torch.int64, device=device)
-        self.pscan = torch.zeros(self.cap, dtype=torch.int64, device=device)
         self.gate_row = torch.zeros(self.cap, dtype=torch.int64, device=device)
         self.rep = torch.zeros(self.ucap, dtype=torch.int64, device=device)
         self.other = torch.zeros(self.ucap, dtype=torch.int64, device=device)
-        self.num_unique = torch.zeros(1, dtype=torch.int64, device=device)
-        self.pscratch = torch.empty(int(lib.ictc_scan_scratch_bytes(self.cap)), dtype=torch.uint8, device=device)
 
-    def build(self, pos_ext):
-        """pos_ext [n+1, 3]: the atoms followed by the dummy row (far away from every atom)."""
-        lib, st = _lib.load(), _lib.stream(self.dev)
-        n, n1 = self.centres, self.n + 1
-        _lib.check(lib.ictc_neighbor_count(pos_ext.data_ptr(), n1, n, self.lo, self.hi, self.box, self.per,
-                                           self.cutoff, self.rowptr.data_ptr(), self.scratch.data_ptr(), st),
-                   "ictc_neighbor_count")
-        _lib.check(lib.ictc_inclusive_scan_i64(self.rowptr.data_ptr(), n + 1, self.scan.data_ptr(), st), "scan")
-        _lib.check(lib.ictc_neighbor_clamp(self.rowptr.data_ptr(), n, self.cap - 1, self.overflow.data_ptr(), st),
-                   "ictc_neighbor_clamp")       # cap - 1: the last slot always stays an inert edge
-        _lib.check(lib.ictc_neighbor_fill(pos_ext.data_ptr(), n1, n, self.lo, self.hi, self.box, self.per, self.cutoff,
-                                          self.rowptr.data_ptr(), self.cap, self.src.data_ptr(), self.dst.data_ptr(),
-                                          self.shifts.data_ptr(), self.keys.data_ptr(), self.scratch.data_ptr(), st),
-                   "ictc_neighbor_fill")
-        _lib.check(lib.ictc_neighbor_pad(self.rowptr.data_ptr() + 8 * n, self.cap, self.n, 0, self.src.data_ptr(),
-                                         self.dst.data_ptr(), self.shifts.data_ptr(), None, st),
-                   "ictc_neighbor_pad")
-        _lib.check(lib.ictc_neighbor_pairs(self.rowptr.data_ptr(), self.dst.data_ptr(), self.keys.data_ptr(), n,
-                                           self.cap, self.ucap, self.rowptr.data_ptr() + 8 * n, self.rev.data_ptr(),
-                                           self.pscan.data_ptr(), self.gate_row.data_ptr(), self.rep.data_ptr(),
-                                           self.other.data_ptr(), self.num_unique.data_ptr(),
-                                           self.pscratch.data_ptr(), st), "ictc_neighbor_pairs")
+    def build(self, pos):
+        """pos [rows, 3]: the atoms, followed by the dummy row (far away from every atom) if there is one."""
+        _lib.check(_lib.load().ictc_neighbor_build(
+            pos.data_ptr(), self.rows, self.centres, self.lo, self.hi, self.box, self.per, self.cutoff, self.cap,
+            self.ucap, self.pad_src, self.rowptr.data_ptr(), self.src.data_ptr(), self.dst.data_ptr(),
+            self.shifts.data_ptr(), self.keys.data_ptr(), self.rev.data_ptr(), self.gate_row.data_ptr(),
+            self.rep.data_ptr(), self.other.data_ptr(), self.num_unique.data_ptr(), self.overflow.data_ptr(),
+            self.scratch.data_ptr(), _lib.stream(self.dev)), "ictc_neighbor_build")
+
+    def counts(self):
+        """(edges, pairs, did a row not fit), read back in one copy."""
+        edges, unique, flag = self._rows[self.centres:].tolist()
+        return edges, unique, (flag & 0xffffffff) != 0
+
+    def sender_csr(self):
+        """Sender CSR of a list in which every edge has its reverse (all senders are centres)."""
+        return self.rowptr, self.rev
 
     def pairs(self):
         return self.gate_row, self.rep, self.other, self.num_unique
@@ -281,6 +294,7 @@ class MolecularDynamics:
         self.num_gate_rows = 0       # rows of the gate table of the last force call (edge pairs, or edges)
         self.graph = None
         self._static = None
+        self._eager_list = None      # neighbour-list buffers of steps that are launched one by one
         self._dist = None            # buffers of the decomposed step
         self.share_gates = bool(share_gates)     # evaluate the radial MLP once per (edge, reverse edge) pair
         self.graph_rebuilds = 0
@@ -308,16 +322,33 @@ class MolecularDynamics:
         self._forces_distributed()
         return self.forces
 
+    def _neighbors(self):
+        """This step's edge list in buffers that grow with the list: one build, one read-back."""
+        n, box = self.pos.shape[0], self.box.tolist()
+        while True:
+            if self._eager_list is None:
+                edges = count_edges(self.pos, n, [0, 0, 0], box, box, (1, 1, 1), self.cutoff)
+                self._eager_list = StaticNeighborList(n, box, self.cutoff, int(1.1 * edges) + 1024, self.device,
+                                                      dummy_row=False)
+            nl = self._eager_list
+            with _lib.on_device(self.device):
+                nl.build(self.pos)
+            edges, pairs, over = nl.counts()
+            if not over and pairs <= nl.ucap:
+                return nl, edges, pairs
+            self._eager_list = None         # the list outgrew its buffers
+
     def _forces_single(self):
         n = self.pos.shape[0]
         box = self.box.tolist()
-        src, dst, shifts, rowptr, keys = neighbor_list(self.pos, n, [0, 0, 0], box, box, (1, 1, 1), self.cutoff, True)
-        self.num_edges = int(src.numel())
+        nl, edges, num_pairs = self._neighbors()
+        src, dst, shifts, rowptr = nl.src[:edges], nl.dst[:edges], nl.shifts[:edges], nl.rowptr
+        self.num_edges = edges
         if self.engine is not None:
-            pairs = edge_pairs(rowptr, dst, keys, n) if self.share_gates else None
-            self.num_gate_rows = int(pairs[1].numel()) if pairs is not None else self.num_edges
+            pairs = (nl.gate_row[:edges], nl.rep[:num_pairs], nl.other[:num_pairs]) if self.share_gates else None
+            self.num_gate_rows = num_pairs if pairs is not None else edges
             energy, grad, _ = self.engine.energy_and_gradient(self.pos, self.species, src, dst, shifts, box, n, rowptr,
-                                                              pairs=pairs)
+                                                              pairs=pairs, src_csr=nl.sender_csr())
             if self._static is not None:            # keep the buffers the recorded graph reads and writes
                 self._static["energy"].copy_(energy.reshape(1))
                 self.forces.copy_(grad).neg_()
@@ -557,7 +588,8 @@ class MolecularDynamics:
         nl = st["nl"]
         energy, grad, _ = self.engine.energy_and_gradient(st["pos_ext"], st["species_ext"], nl.src, nl.dst, nl.shifts,
                                                           self.box.tolist(), n, nl.rowptr, n_rows=n,
-                                                          pairs=nl.pairs() if self.share_gates else None)
+                                                          pairs=nl.pairs() if self.share_gates else None,
+                                                          src_csr=nl.sender_csr())
         st["energy"].copy_(energy.reshape(1))
         self.forces.copy_(grad).neg_()
         self._kick(False)
@@ -674,6 +706,7 @@ class MolecularDynamics:
         if self.engine is None:
             raise RuntimeError("graph replay covers the engine path")
         dev = self.device
+        self._eager_list = None
         torch.cuda.empty_cache()        # the eager steps' cached blocks go back before the recording gets its own pool
         if self.world > 1:
             if self._dist is None:

@@ -207,6 +207,17 @@ int ictc_neighbor_clamp(int64_t* rowptr, int64_t num_centres, int64_t capacity, 
  * This lets a whole MD step run without the host ever learning the edge count (CUDA-graph replay). */
 int ictc_neighbor_pad(const int64_t* count, int64_t capacity, int64_t pad_src, int64_t pad_dst, int64_t* src,
                       int64_t* dst, float* shifts, int32_t* overflow, void* stream);
+/* Whole list in one call, for fixed-capacity buffers (recorded steps): atoms binned, rows counted and filled, offsets
+ * clamped to capacity - 1 (*overflow, sticky, is set when something did not fit), the tail filled with inert edges
+ * (sender pad_src, receiver 0), the pairing of ictc_neighbor_pairs, and rev[e] = edge id of the reverse of e (0 where
+ * there is none): with every sender a centre, rowptr and rev are the sender CSR of the list.  num_centres >= 1;
+ * capacities below 2^31; scratch as above. */
+int ictc_neighbor_build(const float* pos, int64_t num_atoms, int64_t num_centres, const double* host_lo,
+                        const double* host_hi, const double* host_box, const int* host_periodic, double cutoff,
+                        int64_t capacity, int64_t unique_capacity, int64_t pad_src, int64_t* rowptr, int64_t* src,
+                        int64_t* dst, float* shifts, int64_t* edge_keys, int64_t* rev, int64_t* gate_row,
+                        int64_t* rep_edge, int64_t* other_edge, int64_t* num_unique, int32_t* overflow, void* scratch,
+                        void* stream);
 /* Radial pairing of a neighbour list built by ictc_neighbor_fill (edge_keys = its work array, untouched
  * since): the edge (j -> i, S) and its reverse (i -> j, -S) have bitwise the same length, so length-only
  * quantities (radial basis, gate MLP) are evaluated once per pair.  Outputs: gate_row [capacity] = pair id
