@@ -9,13 +9,15 @@
 // so every operand is split into two TF32-representable parts, x = x_big + x_small, and a product is the sum of
 // the three tcgen05.mma passes big*big + big*small + small*big into one fp32 TMEM accumulator.
 //
-// One persistent CTA per SM works on tiles of 128 rows.  Warp roles:
-//   warp 0      streams pre-packed 64-unit weight chunks (32 KB: big and small part) into a 2-stage ring
-//               with cp.async.bulk, completing on mbarriers;
+// One persistent CTA per SM works on tiles of 128 rows.
+// A launch covers up to three matrices (segments): the three degree blocks of a channel linear, one launch instead of
+// three.  Warp roles:
+//   warp 0      streams pre-packed 64-unit weight chunks (32 KB: big and small part) into a 4-stage ring
+//               with cp.async.bulk, completing on mbarriers; a segment with a single chunk keeps it;
 //   warp 1      allocates TMEM and issues the MMAs (one thread), committing to mbarriers;
-//   warps 2-9   epilogue (forward: two groups taking alternate chunks; backward: warps 2-5 only):
+//   warps 2-9   (backward: 2-5) epilogue, in the forward kernel two groups taking alternate blocks:
 //               tcgen05.ld (thread = row), then coalesced row stores;
-//   warps 10-17 A-operand producers: global rows -> (activation | pair sum) -> split -> tcgen05.st into TMEM
+//   last eight  A-operand producers: global rows -> (activation | pair sum) -> split -> tcgen05.st into TMEM
 //               (the A operand is read from TMEM: lane = row, column = k; no shared memory for A at all).
 // Shared-memory layout of the B operand: element (n, k) of a [64 x 64] part lives at byte
 // (k / 4) * 1024 + n * 16 + (k % 4) * 4, i.e. 16-byte K chunks, each chunk row-contiguous (canonical K-major
@@ -23,41 +25,16 @@
 // matrices along n (SBO) 128 B, stride between the two K chunks of one K = 8 MMA (LBO) 1024 B.
 // Every mbarrier wait is bounded; a wait that runs out raises the library's status word and the CTA leaves
 // through the common exit (TMEM is always released).
-#include "tc05.cuh"
+#include "gate_gemm.cuh"
 
 namespace ictc {
 namespace gg {
 
 using namespace tc;
 
-constexpr int kThreads = 18 * 32;
-constexpr int kProducerWarp0 = 10, kProducerWarps = 8;   // warps 2-5 and 6-9: two epilogue groups
+constexpr int kFwdThreads = 18 * 32, kBwdThreads = 14 * 32;      // up to 16 warps leave 128 registers to a thread, 18 leave 96
+constexpr int kProducerWarps = 8, kFwdProducer0 = 10, kBwdProducer0 = 6;
 constexpr int kStagePitch = 272;                    // bytes per staged output row (256 + 16: conflict-free)
-
-struct Args {
-  const float* in;        // forward: z3 [rows, 64]; backward: dgates [*, nout]
-  const float* w;         // packed chunks, 8192 floats each
-  float* out;             // forward: gates [rows, nout]; backward: da3 [rows, 64]
-  const int64_t* pair_a;  // backward, optional
-  const int64_t* pair_b;
-  int64_t rows;
-  const int64_t* limit;   // optional device scalar: only min(rows, *limit) rows are processed (recorded graphs)
-  // Row windows (plain matrices only).  With `begin` (device scalar) the launch covers the window
-  // [*begin, min(*begin + rows, *limit)) of a longer row list: local row g = 0.. stands for list entry *begin + g.
-  const int64_t* begin;
-  const int64_t* in_index;   // forward: local row g reads in[in_index[*begin + g]] (null: in[*begin + g])
-  const int64_t* out_index;  // backward: local row g is written to out[out_index[*begin + g]] (null: out[*begin + g])
-  int nout;
-  int act;                // forward: apply the scaled SiLU to the input
-  int* status;
-  // Row addressing (units: floats).  Row g is sub-row g % mm of node g / mm; its 64-float block number b
-  // (the only block of the 64-wide side, chunk c * cs of the wide side) starts at
-  //   base + (g / mm) * ld + (b + g % mm) * 64.
-  // Plain matrices: mm = 1, ld = row length, cs = 1.  Per-degree feature blocks [node][path slot][m][C]:
-  // mm = 2l+1, ld = node stride, cs = mm (the slot-major layout is read and written in place).
-  int in_mm, out_mm, in_cs, out_cs;
-  int64_t in_ld, out_ld;
-};
 
 __device__ __forceinline__ int64_t row_offset(int64_t g, int mm, int64_t ld) {
   if (mm == 1) return g * ld;
@@ -66,13 +43,34 @@ __device__ __forceinline__ int64_t row_offset(int64_t g, int mm, int64_t ld) {
 }
 
 constexpr int kWStages = 4;      // weight ring
-constexpr int kAStagesBwd = 3;   // TMEM A ring of the backward kernel
+constexpr int kAStagesBwd = 3;   // A ring of the backward kernel
 
 struct Barriers {
   unsigned long long w_full[kWStages], w_empty[kWStages], a_full[4], a_empty[4], d_full[4], d_empty[4];
   unsigned tmem_base;
   volatile int failed;   // polled inside wait loops by other warps: every read must go to shared memory
-  volatile long long progress;   // backward: chunks finished by the first producer warp (read by the prefetch warps)
+};
+
+// The tiles of a launch, segment after segment, dealt out round robin over the CTAs.  Every warp role walks the same tiles
+// in the same order.
+struct Work {
+  int64_t base, rows0;       // first list entry and live rows of the first segment
+  int end0, end1, end2;      // running totals of tiles
+
+  __device__ Work(const Args& a) {
+    base = a.begin ? ldg(a.begin) : 0;
+    rows0 = a.limit ? ldg(a.limit) - base : a.seg[0].rows;
+    rows0 = rows0 < 0 ? 0 : (rows0 < a.seg[0].rows ? rows0 : a.seg[0].rows);
+    end0 = int((rows0 + kRows - 1) / kRows);
+    end1 = end0 + (a.segments > 1 ? int((a.seg[1].rows + kRows - 1) / kRows) : 0);
+    end2 = end1 + (a.segments > 2 ? int((a.seg[2].rows + kRows - 1) / kRows) : 0);
+  }
+  __device__ int64_t rows(const Args& a, int s) const { return s == 0 ? rows0 : a.seg[s].rows; }
+  __device__ int segment(int tile) const { return (tile >= end0) + (tile >= end1); }
+  __device__ int tiles() const { return end2; }
+  __device__ int64_t first_row(int tile, int s) const {
+    return int64_t(tile - (s == 0 ? 0 : s == 1 ? end0 : end1)) * kRows;
+  }
 };
 
 __device__ __forceinline__ void give_up(Barriers* b, int* status, int code) {
@@ -80,41 +78,44 @@ __device__ __forceinline__ void give_up(Barriers* b, int* status, int code) {
   if (status) atomicExch(status, code);
 }
 
-// ------------------------------------------------------------------------------------------------
-// forward.  Shared memory: W ring (4 x 32 KB) | output staging (2 x 34 KB) | barriers.
-// TMEM (512 columns): accumulator ring 4 x 64 | A operand of two tiles, each big (64) + small (64).
-constexpr int kFwdSmem = kWStages * kWStageBytes + 2 * kRows * kStagePitch + 256;
+// The weight stream of both kernels: chunk after chunk for every tile.  A segment with one chunk keeps it.
+__device__ __forceinline__ void stream_weights(const Args& a, const Work& work, Barriers* bar, unsigned char* w_buf, int code) {
+  int64_t it = 0;
+  int kept = -1;
+  for (int tile = blockIdx.x; tile < work.tiles() && !bar->failed; tile += gridDim.x) {
+    const int s = work.segment(tile);
+    const Segment& seg = a.seg[s];
+    if (s == kept) continue;
+    for (int c = 0; c < seg.chunks; ++c, ++it) {
+      const int slot = int(it % kWStages);
+      if (!mbar_wait(saddr(&bar->w_empty[slot]), unsigned((it / kWStages) & 1) ^ 1u)) { give_up(bar, a.status, code); return; }
+      mbar_expect_tx(saddr(&bar->w_full[slot]), kWStageBytes);
+      bulk_g2s(saddr(w_buf + slot * kWStageBytes), seg.w + int64_t(c) * (kWStageBytes / 4), kWStageBytes,
+               saddr(&bar->w_full[slot]));
+    }
+    kept = seg.chunks == 1 ? s : -1;
+  }
+}
 
-__global__ void __launch_bounds__(kThreads, 1) gate_gemm_forward_kernel(Args a) {
-  extern __shared__ __align__(128) unsigned char gg_smem[];
-  unsigned char* w_buf = gg_smem;
-  unsigned char* stage = w_buf + kWStages * kWStageBytes;
-  Barriers* bar = reinterpret_cast<Barriers*>(stage + 2 * kRows * kStagePitch);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int chunks = a.nout / kChunk;
-  const int64_t base = a.begin ? ldg(a.begin) : 0;
-  int64_t nrows = a.limit ? ldg(a.limit) - base : a.rows;
-  nrows = nrows < 0 ? 0 : (nrows < a.rows ? nrows : a.rows);
-  const int64_t tiles = (nrows + kRows - 1) / kRows;
-  const int64_t my_tiles = blockIdx.x < tiles ? (tiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
-
+// Barriers and all 512 TMEM columns; returns the TMEM base.
+__device__ __forceinline__ unsigned enter(Barriers* bar, int a_stages, int accumulators) {
   if (threadIdx.x == 0) {
     for (int i = 0; i < kWStages; ++i) {
       mbar_init(saddr(&bar->w_full[i]), 1);
       mbar_init(saddr(&bar->w_empty[i]), 1);
     }
-    for (int i = 0; i < 2; ++i) {
+    for (int i = 0; i < a_stages; ++i) {
       mbar_init(saddr(&bar->a_full[i]), kProducerWarps * 32);
       mbar_init(saddr(&bar->a_empty[i]), 1);
     }
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < accumulators; ++i) {
       mbar_init(saddr(&bar->d_full[i]), 1);
       mbar_init(saddr(&bar->d_empty[i]), 128);
     }
     bar->failed = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 1) {
+  if ((threadIdx.x >> 5) == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(saddr(&bar->tmem_base)),
                  "r"(512u)
                  : "memory");
@@ -123,71 +124,97 @@ __global__ void __launch_bounds__(kThreads, 1) gate_gemm_forward_kernel(Args a) 
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const unsigned tmem = bar->tmem_base;
+  return __shfl_sync(0xffffffffu, bar->tmem_base, 0);
+}
+
+__device__ __forceinline__ void leave(unsigned tmem) {
+  tc_fence_before();
+  __syncthreads();
+  if ((threadIdx.x >> 5) == 1) {
+    __syncwarp();
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+  }
+}
+
+// ------------------------------------------------------------------------------------------------
+// forward.  Shared memory: W ring (4 x 32 KB) | output staging (2 x 34 KB) | row offsets (2 x 1 KB) | barriers.
+// TMEM (512 columns): accumulator ring 4 x 64 | A operand of two tiles, each big (64) + small (64).
+// Two tiles per weight chunk (half the weight traffic from L2, two accumulators in the ring) was measured slower: 1 M rows
+// of 704 in 0.73 against 0.53 ms; the writes leave at 5.8 TB/s now (0.62 ms before the MMAs were issued by an elected lane).
+constexpr int kFwdSmem = kWStages * kWStageBytes + 2 * kRows * (kStagePitch + 8) + 256;
+
+__global__ void __launch_bounds__(kFwdThreads, 1) gate_gemm_forward_kernel(const __grid_constant__ Args a) {
+  extern __shared__ __align__(128) unsigned char gg_smem[];
+  unsigned char* w_buf = gg_smem;
+  unsigned char* stage = w_buf + kWStages * kWStageBytes;
+  int64_t* offsets = reinterpret_cast<int64_t*>(stage + 2 * kRows * kStagePitch);
+  Barriers* bar = reinterpret_cast<Barriers*>(offsets + 2 * kRows);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const Work work(a);
+  const unsigned tmem = enter(bar, 2, 4);
   const unsigned tmem_a = tmem + 4 * kChunk;       // A operands start after the accumulator ring
 
   if (warp == 0) {
-    // ---- weight chunk stream
-    if (lane == 0) {
-      int64_t it = 0;
-      for (int64_t t = 0; t < my_tiles && !bar->failed; ++t) {
-        for (int c = 0; c < chunks; ++c, ++it) {
-          const int s = int(it % kWStages);
-          if (!mbar_wait(saddr(&bar->w_empty[s]), unsigned((it / kWStages) & 1) ^ 1u)) { give_up(bar, a.status, 21); break; }
-          mbar_expect_tx(saddr(&bar->w_full[s]), kWStageBytes);
-          bulk_g2s(saddr(w_buf + s * kWStageBytes), a.w + int64_t(c) * (kWStageBytes / 4), kWStageBytes,
-                   saddr(&bar->w_full[s]));
-        }
-      }
-    }
+    if (lane == 0) stream_weights(a, work, bar, w_buf, 21);
   } else if (warp == 1) {
     // ---- MMA issue
-    if (lane == 0) {
-      int64_t it = 0;
-      for (int64_t t = 0; t < my_tiles && !bar->failed; ++t) {
-        const int ab = int(t & 1);
-        if (!mbar_wait(saddr(&bar->a_full[ab]), unsigned((t >> 1) & 1))) { give_up(bar, a.status, 22); break; }
-        tc_fence_after();
-        bool ok = true;
-        for (int c = 0; c < chunks; ++c, ++it) {
-          const int s = int(it % kWStages), d = int(it & 3);
-          if (!mbar_wait(saddr(&bar->w_full[s]), unsigned((it / kWStages) & 1)) ||
-              !mbar_wait(saddr(&bar->d_empty[d]), unsigned((it >> 2) & 1) ^ 1u)) {
-            give_up(bar, a.status, 23);
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          const unsigned w_big = saddr(w_buf + s * kWStageBytes), w_small = w_big + kWPartBytes;
-          issue_block(tmem + d * kChunk, tmem_a + ab * 2 * kK, w_big, w_small, true);
-          umma_commit(saddr(&bar->w_empty[s]));
-          umma_commit(saddr(&bar->d_full[d]));
+    int64_t it = 0, wit = 0;
+    int t = 0, kept = -1;
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < work.tiles() && ok && !bar->failed; tile += gridDim.x, ++t) {
+      const int s = work.segment(tile), chunks = a.seg[s].chunks;
+      const bool keep = chunks == 1 && tile + int(gridDim.x) < work.tiles() && work.segment(tile + gridDim.x) == s;
+      const int ab = t & 1;
+      if (!mbar_wait(saddr(&bar->a_full[ab]), unsigned((t >> 1) & 1))) { give_up(bar, a.status, 22); break; }
+      for (int c = 0; c < chunks; ++c, ++it) {
+        const int slot = int(wit % kWStages), d = int(it & 3);
+        if ((kept != s && !mbar_wait(saddr(&bar->w_full[slot]), unsigned((wit / kWStages) & 1))) ||
+            !mbar_wait(saddr(&bar->d_empty[d]), unsigned((it >> 2) & 1) ^ 1u)) {
+          give_up(bar, a.status, 23);
+          ok = false;
+          break;
         }
-        if (!ok) break;
-        umma_commit(saddr(&bar->a_empty[ab]));
+        tc_fence_after();
+        const unsigned w_big = saddr(w_buf + slot * kWStageBytes), w_small = w_big + kWPartBytes;
+        if (elect_one()) {
+          issue_block(tmem + d * kChunk, tmem_a + ab * 2 * kK, w_big, w_small, true);
+          if (!keep) umma_commit(saddr(&bar->w_empty[slot]));
+          umma_commit(saddr(&bar->d_full[d]));
+          if (c == chunks - 1) umma_commit(saddr(&bar->a_empty[ab]));
+        }
+        __syncwarp();
+        wit += !keep;
       }
+      kept = keep ? s : -1;
     }
-  } else if (warp < kProducerWarp0) {
+  } else if (warp < kFwdProducer0) {
     // ---- epilogue, two groups of four warps that take alternate chunks: tcgen05.ld gives thread = row; the
     // warp's 32 rows go through a padded staging buffer and leave as coalesced 256-byte row segments (two rows
     // per store instruction)
     const int q = warp & 3;                         // TMEM lane quarter this warp may read
     const int group = (warp - 2) >> 2;
     const int row = q * 32 + lane;
-    unsigned char* gstage = stage + group * (kRows * kStagePitch);
-    unsigned char* mine = gstage + row * kStagePitch;
-    const unsigned char* warp_rows = gstage + q * 32 * kStagePitch;
-    const int mm = a.out_mm;
+    unsigned char* mine = stage + (group * kRows + row) * kStagePitch;
+    // rows 2i + (lane >> 4) of this warp are stored by this lane, the 16 bytes lane & 15 of each
+    const unsigned char* from = stage + (group * kRows + q * 32 + (lane >> 4)) * kStagePitch + (lane & 15) * 16;
+    int64_t* my_offset = offsets + group * kRows + row;
+    const int64_t* offset = offsets + group * kRows + q * 32 + (lane >> 4);
     int64_t it = 0;
-    for (int64_t t = 0; t < my_tiles; ++t) {
-      const int64_t row0 = (blockIdx.x + t * gridDim.x) * kRows + q * 32;
-      // rows 2i + (lane >> 4) of this warp are stored by this lane: walk their offsets without dividing
-      const int64_t g0 = row0 + (lane >> 4);
-      const int64_t node0 = mm == 1 ? g0 : g0 / mm;
-      const int sub0 = mm == 1 ? 0 : int(g0 - node0 * mm);
-      const int64_t off0 = node0 * a.out_ld + sub0 * kK + (lane & 15) * 4;
-      bool ok = true;
-      for (int c = 0; c < chunks; ++c, ++it) {
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < work.tiles() && ok; tile += gridDim.x) {
+      const int s = work.segment(tile);
+      const Segment& seg = a.seg[s];
+      const int chunks = seg.chunks;
+      const int64_t g = work.first_row(tile, s) + row;
+      const bool valid = g < work.rows(a, s);
+      __syncwarp();
+      *my_offset = valid ? row_offset(g, seg.out_mm, seg.out_ld) : -1;
+      float* out = seg.out + (lane & 15) * 4;
+      const int64_t step = int64_t(seg.out_cs) * kChunk;
+      const float* add = (a.bias && s == 0 && valid && g < a.bias_nodes)
+                             ? a.bias + (a.bias_index ? ldg(a.bias_index + g) : g) * kK : nullptr;
+      for (int c = 0; c < chunks; ++c, ++it, out += step) {
         if (int(it & 1) != group) continue;
         const int d = int(it & 3);
         if (bar->failed || !mbar_wait(saddr(&bar->d_full[d]), unsigned((it >> 2) & 1))) {
@@ -202,6 +229,10 @@ __global__ void __launch_bounds__(kThreads, 1) gate_gemm_forward_kernel(Args a) 
         tmem_ld32(taddr + 32, v1);
         tc_fence_before();
         mbar_arrive(saddr(&bar->d_empty[d]));
+        if (add && c == 0) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) { v0[i] += __ldg(add + i); v1[i] += __ldg(add + 32 + i); }
+        }
         __syncwarp();                                // the previous chunk's read-back is complete
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
@@ -210,37 +241,29 @@ __global__ void __launch_bounds__(kThreads, 1) gate_gemm_forward_kernel(Args a) 
               make_float4(v1[4 * j], v1[4 * j + 1], v1[4 * j + 2], v1[4 * j + 3]);
         }
         __syncwarp();
-        float* base = a.out + int64_t(c) * a.out_cs * kChunk;
-        int64_t off = off0;
-        int sub = sub0;
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
-          const int r = 2 * i + (lane >> 4);
-          const float4 v = *reinterpret_cast<const float4*>(warp_rows + r * kStagePitch + (lane & 15) * 16);
-          if (row0 + r < nrows) __stcs(reinterpret_cast<float4*>(base + off), v);
-          if (mm == 1) {
-            off += 2 * a.out_ld;
-          } else {
-            sub += 2;
-            off += 2 * kK;
-            while (sub >= mm) { sub -= mm; off += a.out_ld - int64_t(mm) * kK; }
-          }
+          const int64_t off = offset[2 * i];
+          const float4 v = *reinterpret_cast<const float4*>(from + 2 * i * kStagePitch);
+          if (off >= 0) __stcs(reinterpret_cast<float4*>(out + off), v);
         }
       }
-      if (!ok) break;
     }
   } else {
     // ---- A producers: thread = (row, half of the 64 columns); z3 -> activation -> split -> TMEM
-    const int q = warp & 3, half = (warp - kProducerWarp0) >> 2;
+    const int q = warp & 3, half = (warp - kFwdProducer0) >> 2;
     const int row = q * 32 + lane;
-    for (int64_t t = 0; t < my_tiles; ++t) {
-      const int ab = int(t & 1);
-      const int64_t g = (blockIdx.x + t * gridDim.x) * kRows + row;
+    int t = 0;
+    for (int tile = blockIdx.x; tile < work.tiles(); tile += gridDim.x, ++t) {
+      const int s = work.segment(tile), ab = t & 1;
+      const Segment& seg = a.seg[s];
+      const int64_t g = work.first_row(tile, s) + row;
       float x[32];
-      if (g < nrows) {
-        const int64_t srow = a.in_index ? ldg(a.in_index + base + g) : base + g;
+      if (g < work.rows(a, s)) {
+        const int64_t srow = a.in_index ? ldg(a.in_index + work.base + g) : work.base + g;
+        const float* p = seg.in + row_offset(srow, seg.in_mm, seg.in_ld) + half * 32;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) ldg256(a.in + row_offset(srow, a.in_mm, a.in_ld) + half * 32 + j * 8, x + j * 8);
+        for (int j = 0; j < 4; ++j) ldg256(p + j * 8, x + j * 8);
       } else {
 #pragma unroll
         for (int i = 0; i < 32; ++i) x[i] = 0.f;
@@ -258,105 +281,71 @@ __global__ void __launch_bounds__(kThreads, 1) gate_gemm_forward_kernel(Args a) 
       mbar_arrive(saddr(&bar->a_full[ab]));
     }
   }
-  tc_fence_before();
-  __syncthreads();
-  if (warp == 1) {
-    __syncwarp();
-    tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
-  }
+  leave(tmem);
 }
 
 // ------------------------------------------------------------------------------------------------
-// backward.  Shared memory: W ring (4 x 32 KB) | barriers.  TMEM: two accumulators [128 x 64] that alternate
-// between tiles | A ring of three stages (big + small, 128 columns each); K runs over the nout / 64 chunks.
-constexpr int kBwdSmem = kWStages * kWStageBytes + 256;
+// backward.  Shared memory: W ring (4 x 32 KB) | raw input ring (3 x 32 KB) | barriers.  TMEM: two accumulators [128 x 64]
+// that alternate between tiles | A ring of three stages (big + small, 128 columns each); K runs over the chunks.
+// A producer warp fetches its 32 rows x 128 bytes of a stage with cp.async (whole lines, four rows per instruction) into a
+// private, swizzled buffer two stages ahead, so that neither the latency of the rows nor 32 different lines per load
+// instruction are on the path of a stage.  1 M rows of 704: 0.77 ms before (MMA issue 0.11, conversions 0.05, loads 0.06),
+// 0.56 now (5.5 TB/s).
+constexpr int kRawStages = 3;
+constexpr int kRawWarpBytes = 32 * 128;
+constexpr int kRawBytes = kRawStages * kProducerWarps * kRawWarpBytes;
+constexpr int kBwdSmem = kWStages * kWStageBytes + kRawBytes + 256;
 
-__global__ void __launch_bounds__(kThreads, 1) gate_gemm_backward_kernel(Args a) {
+__global__ void __launch_bounds__(kBwdThreads, 1) gate_gemm_backward_kernel(const __grid_constant__ Args a) {
   extern __shared__ __align__(128) unsigned char gg_smem[];
   unsigned char* w_buf = gg_smem;
-  Barriers* bar = reinterpret_cast<Barriers*>(w_buf + kWStages * kWStageBytes);
+  unsigned char* raw = w_buf + kWStages * kWStageBytes;
+  Barriers* bar = reinterpret_cast<Barriers*>(raw + kRawBytes);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int chunks = a.nout / kChunk;
-  const int64_t base = a.begin ? ldg(a.begin) : 0;
-  int64_t nrows = a.limit ? ldg(a.limit) - base : a.rows;
-  nrows = nrows < 0 ? 0 : (nrows < a.rows ? nrows : a.rows);
-  const int64_t tiles = (nrows + kRows - 1) / kRows;
-  const int64_t my_tiles = blockIdx.x < tiles ? (tiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
-
-  if (threadIdx.x == 0) {
-    for (int i = 0; i < kWStages; ++i) {
-      mbar_init(saddr(&bar->w_full[i]), 1);
-      mbar_init(saddr(&bar->w_empty[i]), 1);
-    }
-    for (int i = 0; i < kAStagesBwd; ++i) {
-      mbar_init(saddr(&bar->a_full[i]), kProducerWarps * 32);
-      mbar_init(saddr(&bar->a_empty[i]), 1);
-    }
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(saddr(&bar->d_full[i]), 1);
-      mbar_init(saddr(&bar->d_empty[i]), 128);
-    }
-    bar->failed = 0;
-    bar->progress = 0;
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(saddr(&bar->tmem_base)),
-                 "r"(512u)
-                 : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  const unsigned tmem = bar->tmem_base;
+  const Work work(a);
+  const unsigned tmem = enter(bar, kAStagesBwd, 2);
   const unsigned tmem_a = tmem + 2 * kChunk;
 
   if (warp == 0) {
-    if (lane == 0) {
-      int64_t it = 0;
-      for (int64_t t = 0; t < my_tiles && !bar->failed; ++t) {
-        for (int c = 0; c < chunks; ++c, ++it) {
-          const int s = int(it % kWStages);
-          if (!mbar_wait(saddr(&bar->w_empty[s]), unsigned((it / kWStages) & 1) ^ 1u)) { give_up(bar, a.status, 31); break; }
-          mbar_expect_tx(saddr(&bar->w_full[s]), kWStageBytes);
-          bulk_g2s(saddr(w_buf + s * kWStageBytes), a.w + int64_t(c) * (kWStageBytes / 4), kWStageBytes,
-                   saddr(&bar->w_full[s]));
-        }
-      }
-    }
+    if (lane == 0) stream_weights(a, work, bar, w_buf, 31);
   } else if (warp == 1) {
-    if (lane == 0) {
-      int64_t it = 0;
-      for (int64_t t = 0; t < my_tiles && !bar->failed; ++t) {
-        const int d = int(t & 1);
-        if (!mbar_wait(saddr(&bar->d_empty[d]), unsigned((t >> 1) & 1) ^ 1u)) { give_up(bar, a.status, 32); break; }
-        bool ok = true;
-        for (int c = 0; c < chunks; ++c, ++it) {
-          const int s = int(it % kWStages), sa = int(it % kAStagesBwd);
-          if (!mbar_wait(saddr(&bar->w_full[s]), unsigned((it / kWStages) & 1)) ||
-              !mbar_wait(saddr(&bar->a_full[sa]), unsigned((it / kAStagesBwd) & 1))) {
-            give_up(bar, a.status, 33);
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          const unsigned w_big = saddr(w_buf + s * kWStageBytes), w_small = w_big + kWPartBytes;
-          issue_block(tmem + d * kChunk, tmem_a + sa * 2 * kK, w_big, w_small, c == 0);
-          umma_commit(saddr(&bar->w_empty[s]));
-          umma_commit(saddr(&bar->a_empty[sa]));
+    int64_t it = 0, wit = 0;
+    int t = 0, kept = -1;
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < work.tiles() && ok && !bar->failed; tile += gridDim.x, ++t) {
+      const int s = work.segment(tile), chunks = a.seg[s].chunks;
+      const bool keep = chunks == 1 && tile + int(gridDim.x) < work.tiles() && work.segment(tile + gridDim.x) == s;
+      const int d = t & 1;
+      if (!mbar_wait(saddr(&bar->d_empty[d]), unsigned((t >> 1) & 1) ^ 1u)) { give_up(bar, a.status, 32); break; }
+      for (int c = 0; c < chunks; ++c, ++it) {
+        const int slot = int(wit % kWStages), sa = int(it % kAStagesBwd);
+        if ((kept != s && !mbar_wait(saddr(&bar->w_full[slot]), unsigned((wit / kWStages) & 1))) ||
+            !mbar_wait(saddr(&bar->a_full[sa]), unsigned((it / kAStagesBwd) & 1))) {
+          give_up(bar, a.status, 33);
+          ok = false;
+          break;
         }
-        if (!ok) break;
-        umma_commit(saddr(&bar->d_full[d]));
+        tc_fence_after();
+        const unsigned w_big = saddr(w_buf + slot * kWStageBytes), w_small = w_big + kWPartBytes;
+        if (elect_one()) {
+          issue_block(tmem + d * kChunk, tmem_a + sa * 2 * kK, w_big, w_small, c == 0);
+          if (!keep) umma_commit(saddr(&bar->w_empty[slot]));
+          umma_commit(saddr(&bar->a_empty[sa]));
+          if (c == chunks - 1) umma_commit(saddr(&bar->d_full[d]));
+        }
+        __syncwarp();
+        wit += !keep;
       }
+      kept = keep ? s : -1;
     }
-  } else if (warp < 6) {
+  } else if (warp < kBwdProducer0) {
     const int q = warp & 3;
     const int row = q * 32 + lane;
-    for (int64_t t = 0; t < my_tiles; ++t) {
-      const int d = int(t & 1);
-      const int64_t grow = (blockIdx.x + t * gridDim.x) * kRows + row;
+    int t = 0;
+    for (int tile = blockIdx.x; tile < work.tiles(); tile += gridDim.x, ++t) {
+      const int s = work.segment(tile), d = t & 1;
+      const Segment& seg = a.seg[s];
+      const int64_t g = work.first_row(tile, s) + row;
       if (bar->failed || !mbar_wait(saddr(&bar->d_full[d]), unsigned((t >> 1) & 1))) { give_up(bar, a.status, 34); break; }
       tc_fence_after();
       float v0[32], v1[32];
@@ -365,9 +354,9 @@ __global__ void __launch_bounds__(kThreads, 1) gate_gemm_backward_kernel(Args a)
       tmem_ld32(taddr + 32, v1);
       tc_fence_before();
       mbar_arrive(saddr(&bar->d_empty[d]));
-      if (grow < nrows) {
-        const int64_t orow = a.out_index ? ldg(a.out_index + base + grow) : base + grow;
-        float4* o = reinterpret_cast<float4*>(a.out + row_offset(orow, a.out_mm, a.out_ld));
+      if (g < work.rows(a, s)) {
+        const int64_t orow = a.out_index ? ldg(a.out_index + work.base + g) : work.base + g;
+        float4* o = reinterpret_cast<float4*>(seg.out + row_offset(orow, seg.out_mm, seg.out_ld));
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           o[j] = make_float4(v0[4 * j], v0[4 * j + 1], v0[4 * j + 2], v0[4 * j + 3]);
@@ -375,83 +364,78 @@ __global__ void __launch_bounds__(kThreads, 1) gate_gemm_backward_kernel(Args a)
         }
       }
     }
-  } else if (warp < kProducerWarp0) {
-    // ---- warps 6-9: L2 prefetch of the rows a few chunks ahead of the producers, across tile boundaries
-    // (thread = row).  They follow the producers through a progress counter and never wait when they are behind.
-    const int q = warp & 3;
-    const int row = q * 32 + lane;
-    constexpr int kAhead = 2;
-    const int64_t cstep = int64_t(a.in_cs) * kChunk;
-    int64_t pf_tile = 0;
-    int pf_chunk = 0;
-    const float* pa = nullptr;
-    const float* pb = nullptr;
+  } else {
+    // ---- A producers: thread = (row, half of a 64-column chunk); (dG[a] + dG[b]) -> split -> TMEM ring.
+    // `fetch` walks the stages (chunks of a tile, tile after tile) ahead of the loop that consumes them.  Lane l of the warp
+    // copies the 16-byte piece l & 7 of rows 4j + (l >> 3), j = 0..7; row r's piece p sits at position p ^ (r & 7).
+    const int pw = warp - kBwdProducer0, q = warp & 3, half = pw >> 2;
+    unsigned char* mine = raw + pw * kRawWarpBytes;
+    int f_tile = blockIdx.x, f_c = 0, f_chunks = 0, f_slot = 0;
+    int64_t f_step = 0;
+    const float* f_row[8];
     auto enter_tile = [&]() {
-      pa = pb = nullptr;
-      if (pf_tile >= my_tiles) return;
-      const int64_t g = (blockIdx.x + pf_tile * gridDim.x) * kRows + row;
-      if (g >= nrows) return;
-      const int64_t ra = a.pair_a ? __ldg(reinterpret_cast<const long long*>(a.pair_a + g)) : g;
-      const int64_t rb = a.pair_b ? __ldg(reinterpret_cast<const long long*>(a.pair_b + g)) : -1;
-      pa = a.in + row_offset(ra, a.in_mm, a.in_ld);
-      if (rb >= 0) pb = a.in + row_offset(rb, a.in_mm, a.in_ld);
+      if (f_tile >= work.tiles()) return;
+      const int s = work.segment(f_tile);
+      const Segment& seg = a.seg[s];
+      f_chunks = seg.chunks;
+      f_step = int64_t(seg.in_cs) * kChunk;
+      const int64_t nrows = work.rows(a, s), first = work.first_row(f_tile, s) + q * 32;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int64_t g = first + 4 * j + (lane >> 3);
+        const int64_t r = g < nrows ? (a.pair_a ? ldg(a.pair_a + g) : g) : -1;
+        f_row[j] = r < 0 ? nullptr : seg.in + row_offset(r, seg.in_mm, seg.in_ld) + half * 32 + (lane & 7) * 4;
+      }
     };
-    auto advance = [&]() {
-      if (pf_tile >= my_tiles) return;
-      if (pa) {
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(pa + pf_chunk * cstep));
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(pa + pf_chunk * cstep + 32));
+    auto fetch = [&]() {
+      if (f_tile < work.tiles()) {
+        unsigned char* slot = mine + f_slot * (kProducerWarps * kRawWarpBytes);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const int r = 4 * j + (lane >> 3);
+          const unsigned dst = saddr(slot + r * 128 + (((lane & 7) ^ (r & 7)) << 4));
+          const float* src = f_row[j] ? f_row[j] + f_c * f_step : a.seg[0].in;
+          cp_async16(dst, src, f_row[j] ? 16u : 0u);          // rows beyond the end are zeros
+        }
+        if (++f_slot == kRawStages) f_slot = 0;
+        if (++f_c == f_chunks) {
+          f_c = 0;
+          f_tile += gridDim.x;
+          enter_tile();
+        }
       }
-      if (pb) {
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(pb + pf_chunk * cstep));
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(pb + pf_chunk * cstep + 32));
-      }
-      if (++pf_chunk == chunks) {
-        pf_chunk = 0;
-        ++pf_tile;
-        enter_tile();
-      }
+      cp_async_commit();
     };
     enter_tile();
-    for (int k = 0; k < kAhead; ++k) advance();
-    const int64_t total = my_tiles * chunks;
-    for (int64_t it = 0; it < total; ++it) {
-      advance();
-      const long long start = clock64();
-      bool ok = true;
-      while (bar->progress <= it && !bar->failed) {
-        if (clock64() - start > kWaitCycles) { ok = false; break; }
-        __nanosleep(64);
-      }
-      if (!ok || bar->failed) break;
-    }
-  } else {
-    // ---- A producers: thread = (row, half of a 64-column chunk); (dG[a] + dG[b]) -> split -> TMEM ring
-    const int q = warp & 3, half = (warp - kProducerWarp0) >> 2;
-    const int row = q * 32 + lane;
+#pragma unroll
+    for (int k = 0; k < kRawStages - 1; ++k) fetch();
     int64_t it = 0;
-    for (int64_t t = 0; t < my_tiles; ++t) {
-      const int64_t g = (blockIdx.x + t * gridDim.x) * kRows + row;
-      const int64_t ra = g < nrows ? (a.pair_a ? __ldg(reinterpret_cast<const long long*>(a.pair_a + g)) : g) : -1;
-      const int64_t rb = (g < nrows && a.pair_b) ? __ldg(reinterpret_cast<const long long*>(a.pair_b + g)) : -1;
-      const float* pa = a.in + row_offset(ra >= 0 ? ra : 0, a.in_mm, a.in_ld) + half * 32;
-      const float* pb = a.in + row_offset(rb >= 0 ? rb : 0, a.in_mm, a.in_ld) + half * 32;
-      const int64_t cstep = int64_t(a.in_cs) * kChunk;
-      bool ok = true;
+    int slot = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < work.tiles() && ok; tile += gridDim.x) {
+      const int s = work.segment(tile), chunks = a.seg[s].chunks;
+      const Segment& seg = a.seg[s];
+      const int64_t g = work.first_row(tile, s) + q * 32 + lane;
+      const int64_t rb = (a.pair_b && g < work.rows(a, s)) ? ldg(a.pair_b + g) : -1;
       for (int c = 0; c < chunks; ++c, ++it) {
         const int sa = int(it % kAStagesBwd);
+        fetch();
+        cp_async_wait<kRawStages - 1>();
+        __syncwarp();
         float x[32];
-        if (ra >= 0) {
+        const unsigned char* rows = mine + slot * (kProducerWarps * kRawWarpBytes) + lane * 128;
 #pragma unroll
-          for (int j = 0; j < 4; ++j) ldg256(pa + c * cstep + j * 8, x + j * 8);
-        } else {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) x[i] = 0.f;
+        for (int p = 0; p < 8; ++p) {
+          const float4 v = *reinterpret_cast<const float4*>(rows + ((p ^ (lane & 7)) << 4));
+          x[4 * p] = v.x; x[4 * p + 1] = v.y; x[4 * p + 2] = v.z; x[4 * p + 3] = v.w;
         }
+        __syncwarp();                          // the slot may be filled again
+        if (++slot == kRawStages) slot = 0;
         if (rb >= 0) {
+          const float* pb = seg.in + row_offset(rb, seg.in_mm, seg.in_ld) + half * 32 + c * (int64_t(seg.in_cs) * kChunk);
           float y[32];
 #pragma unroll
-          for (int j = 0; j < 4; ++j) ldg256(pb + c * cstep + j * 8, y + j * 8);
+          for (int j = 0; j < 4; ++j) ldg256(pb + j * 8, y + j * 8);
 #pragma unroll
           for (int i = 0; i < 32; ++i) x[i] += y[i];
         }
@@ -465,18 +449,11 @@ __global__ void __launch_bounds__(kThreads, 1) gate_gemm_backward_kernel(Args a)
         store_split_tmem(t_big, t_big + kK, x);
         tc_fence_before();
         mbar_arrive(saddr(&bar->a_full[sa]));
-        if (warp == kProducerWarp0 && lane == 0) bar->progress = it + 1;
       }
-      if (!ok) break;
     }
+    cp_async_wait<0>();          // no copy may be in flight when the block leaves
   }
-  tc_fence_before();
-  __syncthreads();
-  if (warp == 1) {
-    __syncwarp();
-    tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
-  }
+  leave(tmem);
 }
 
 // Packs W3 [nout, 64] into 64-unit chunks in the shared-memory operand layout, big part then small part.
@@ -493,11 +470,32 @@ __global__ void gate_pack_kernel(int nout, const float* __restrict__ w, int tran
   out[c * (2 * kChunk * kK) + kChunk * kK + off] = small;
 }
 
-static int grid_size(int64_t rows) {
+// One persistent CTA per SM
+static int prepare(Args& a) {
   int dev = 0, sms = 148;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int64_t tiles = (rows + kRows - 1) / kRows;
+  int64_t tiles = 0;
+  for (int s = 0; s < a.segments; ++s) tiles += (a.seg[s].rows + kRows - 1) / kRows;
+  a.status = kernel_status_word();
   return int(tiles < sms ? tiles : sms);
+}
+
+int launch_forward(Args a, cudaStream_t st) {
+  static const cudaError_t attr =
+      cudaFuncSetAttribute(gate_gemm_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFwdSmem);
+  if (attr != cudaSuccess) { set_error("gate gemm smem: %s", cudaGetErrorString(attr)); return ICTC_ERR_LAUNCH; }
+  const int grid = prepare(a);
+  gate_gemm_forward_kernel<<<grid, kFwdThreads, kFwdSmem, st>>>(a);
+  return finish_launch("gate_gemm_forward");
+}
+
+int launch_backward(Args a, cudaStream_t st) {
+  static const cudaError_t attr =
+      cudaFuncSetAttribute(gate_gemm_backward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kBwdSmem);
+  if (attr != cudaSuccess) { set_error("gate gemm smem: %s", cudaGetErrorString(attr)); return ICTC_ERR_LAUNCH; }
+  const int grid = prepare(a);
+  gate_gemm_backward_kernel<<<grid, kBwdThreads, kBwdSmem, st>>>(a);
+  return finish_launch("gate_gemm_backward");
 }
 
 static int check_common(int64_t rows, int nout) {
@@ -532,15 +530,11 @@ int ictc_gate_gemm_forward(int64_t num_rows, int num_out, const float* z3, const
     set_error("gate gemm forward: buffers must be 32-byte aligned");
     return ICTC_ERR_BAD_ARG;
   }
-  static const cudaError_t attr = cudaFuncSetAttribute(gg::gate_gemm_forward_kernel,
-                                                       cudaFuncAttributeMaxDynamicSharedMemorySize, gg::kFwdSmem);
-  if (attr != cudaSuccess) { set_error("gate gemm smem: %s", cudaGetErrorString(attr)); return ICTC_ERR_LAUNCH; }
   gg::Args a{};
-  a.in = z3; a.w = w_packed; a.out = gates; a.rows = num_rows; a.limit = row_limit; a.nout = num_out; a.act = apply_silu ? 1 : 0;
-  a.in_mm = a.out_mm = a.in_cs = a.out_cs = 1; a.in_ld = gg::kK; a.out_ld = num_out;
-  a.status = kernel_status_word();
-  gg::gate_gemm_forward_kernel<<<gg::grid_size(num_rows), gg::kThreads, gg::kFwdSmem, (cudaStream_t)stream>>>(a);
-  return finish_launch("gate_gemm_forward");
+  a.segments = 1;
+  a.seg[0] = gg::segment(z3, w_packed, gates, num_rows, num_out / gg::kChunk, 1, gg::kK, 1, num_out);
+  a.limit = row_limit; a.act = apply_silu ? 1 : 0;
+  return gg::launch_forward(a, (cudaStream_t)stream);
 }
 
 int ictc_gate_gemm_backward(int64_t num_rows, int num_out, const float* dgates, const int64_t* pair_a,
@@ -553,15 +547,11 @@ int ictc_gate_gemm_backward(int64_t num_rows, int num_out, const float* dgates, 
     set_error("gate gemm backward: buffers must be 32-byte aligned");
     return ICTC_ERR_BAD_ARG;
   }
-  static const cudaError_t attr = cudaFuncSetAttribute(gg::gate_gemm_backward_kernel,
-                                                       cudaFuncAttributeMaxDynamicSharedMemorySize, gg::kBwdSmem);
-  if (attr != cudaSuccess) { set_error("gate gemm smem: %s", cudaGetErrorString(attr)); return ICTC_ERR_LAUNCH; }
   gg::Args a{};
-  a.in = dgates; a.w = w_packed_t; a.out = da3; a.pair_a = pair_a; a.pair_b = pair_b; a.rows = num_rows; a.limit = row_limit; a.nout = num_out;
-  a.in_mm = a.out_mm = a.in_cs = a.out_cs = 1; a.in_ld = num_out; a.out_ld = gg::kK;
-  a.status = kernel_status_word();
-  gg::gate_gemm_backward_kernel<<<gg::grid_size(num_rows), gg::kThreads, gg::kBwdSmem, (cudaStream_t)stream>>>(a);
-  return finish_launch("gate_gemm_backward");
+  a.segments = 1;
+  a.seg[0] = gg::segment(dgates, w_packed_t, da3, num_rows, num_out / gg::kChunk, 1, num_out, 1, gg::kK);
+  a.pair_a = pair_a; a.pair_b = pair_b; a.limit = row_limit;
+  return gg::launch_backward(a, (cudaStream_t)stream);
 }
 
 
@@ -575,16 +565,11 @@ int ictc_gate_gemm_forward_rows(int64_t capacity, int num_out, const float* z3, 
     set_error("gate gemm forward rows: buffers must be 32-byte aligned");
     return ICTC_ERR_BAD_ARG;
   }
-  static const cudaError_t attr = cudaFuncSetAttribute(gg::gate_gemm_forward_kernel,
-                                                       cudaFuncAttributeMaxDynamicSharedMemorySize, gg::kFwdSmem);
-  if (attr != cudaSuccess) { set_error("gate gemm smem: %s", cudaGetErrorString(attr)); return ICTC_ERR_LAUNCH; }
   gg::Args a{};
-  a.in = z3; a.w = w_packed; a.out = gates; a.rows = capacity; a.limit = row_end; a.begin = row_begin; a.in_index = row_index;
-  a.nout = num_out; a.act = apply_silu ? 1 : 0;
-  a.in_mm = a.out_mm = a.in_cs = a.out_cs = 1; a.in_ld = gg::kK; a.out_ld = num_out;
-  a.status = kernel_status_word();
-  gg::gate_gemm_forward_kernel<<<gg::grid_size(capacity), gg::kThreads, gg::kFwdSmem, (cudaStream_t)stream>>>(a);
-  return finish_launch("gate_gemm_forward_rows");
+  a.segments = 1;
+  a.seg[0] = gg::segment(z3, w_packed, gates, capacity, num_out / gg::kChunk, 1, gg::kK, 1, num_out);
+  a.limit = row_end; a.begin = row_begin; a.in_index = row_index; a.act = apply_silu ? 1 : 0;
+  return gg::launch_forward(a, (cudaStream_t)stream);
 }
 
 int ictc_gate_gemm_backward_rows(int64_t capacity, int num_out, const float* dgates, const int64_t* row_begin,
@@ -597,16 +582,11 @@ int ictc_gate_gemm_backward_rows(int64_t capacity, int num_out, const float* dga
     set_error("gate gemm backward rows: buffers must be 32-byte aligned");
     return ICTC_ERR_BAD_ARG;
   }
-  static const cudaError_t attr = cudaFuncSetAttribute(gg::gate_gemm_backward_kernel,
-                                                       cudaFuncAttributeMaxDynamicSharedMemorySize, gg::kBwdSmem);
-  if (attr != cudaSuccess) { set_error("gate gemm smem: %s", cudaGetErrorString(attr)); return ICTC_ERR_LAUNCH; }
   gg::Args a{};
-  a.in = dgates; a.w = w_packed_t; a.out = da3; a.rows = capacity; a.limit = row_end; a.begin = row_begin; a.out_index = out_index;
-  a.nout = num_out;
-  a.in_mm = a.out_mm = a.in_cs = a.out_cs = 1; a.in_ld = num_out; a.out_ld = gg::kK;
-  a.status = kernel_status_word();
-  gg::gate_gemm_backward_kernel<<<gg::grid_size(capacity), gg::kThreads, gg::kBwdSmem, (cudaStream_t)stream>>>(a);
-  return finish_launch("gate_gemm_backward_rows");
+  a.segments = 1;
+  a.seg[0] = gg::segment(dgates, w_packed_t, da3, capacity, num_out / gg::kChunk, 1, num_out, 1, gg::kK);
+  a.limit = row_end; a.begin = row_begin; a.out_index = out_index;
+  return gg::launch_backward(a, (cudaStream_t)stream);
 }
 
 
@@ -626,23 +606,9 @@ int ictc_channel_linear_tc(int64_t num_rows, int k_chunks, int n_chunks, const f
     return ICTC_ERR_BAD_ARG;
   }
   gg::Args a{};
-  a.in = in; a.w = w_packed; a.out = out; a.rows = num_rows; a.status = kernel_status_word();
-  a.in_mm = in_mm; a.out_mm = out_mm; a.in_ld = in_ld; a.out_ld = out_ld;
-  a.in_cs = in_mm; a.out_cs = out_mm;
-  if (k_chunks == 1) {
-    static const cudaError_t attr = cudaFuncSetAttribute(gg::gate_gemm_forward_kernel,
-                                                         cudaFuncAttributeMaxDynamicSharedMemorySize, gg::kFwdSmem);
-    if (attr != cudaSuccess) { set_error("channel linear smem: %s", cudaGetErrorString(attr)); return ICTC_ERR_LAUNCH; }
-    a.nout = n_chunks * gg::kChunk;
-    gg::gate_gemm_forward_kernel<<<gg::grid_size(num_rows), gg::kThreads, gg::kFwdSmem, (cudaStream_t)stream>>>(a);
-  } else {
-    static const cudaError_t attr = cudaFuncSetAttribute(gg::gate_gemm_backward_kernel,
-                                                         cudaFuncAttributeMaxDynamicSharedMemorySize, gg::kBwdSmem);
-    if (attr != cudaSuccess) { set_error("channel linear smem: %s", cudaGetErrorString(attr)); return ICTC_ERR_LAUNCH; }
-    a.nout = k_chunks * gg::kChunk;
-    gg::gate_gemm_backward_kernel<<<gg::grid_size(num_rows), gg::kThreads, gg::kBwdSmem, (cudaStream_t)stream>>>(a);
-  }
-  return finish_launch("channel_linear_tc");
+  a.segments = 1;
+  a.seg[0] = gg::segment(in, w_packed, out, num_rows, k_chunks * n_chunks, in_mm, in_ld, out_mm, out_ld);
+  return k_chunks == 1 ? gg::launch_forward(a, (cudaStream_t)stream) : gg::launch_backward(a, (cudaStream_t)stream);
 }
 
 }  // extern "C"

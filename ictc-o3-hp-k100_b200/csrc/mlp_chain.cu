@@ -97,7 +97,7 @@ __device__ __forceinline__ unsigned setup(const Args& a, unsigned char* smem, Ba
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  return bar->tmem_base;
+  return __shfl_sync(0xffffffffu, bar->tmem_base, 0);
 }
 
 __device__ __forceinline__ void teardown(unsigned tmem) {
@@ -124,8 +124,11 @@ __device__ __forceinline__ void mma_loop(const Args& a, Barriers* bar, unsigned 
         ++phase[s];
         tc_fence_after();
         const unsigned base = tmem + s * kSlotCols;
-        issue_block(base + 2 * kK, base, w_big, w_small, true);
-        umma_commit(saddr(&bar->h_full[s]));
+        if (elect_one()) {
+          issue_block(base + 2 * kK, base, w_big, w_small, true);
+          umma_commit(saddr(&bar->h_full[s]));
+        }
+        __syncwarp();
       }
     }
   }
@@ -143,7 +146,7 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_chain_forward_kernel(Args a) 
   const unsigned tmem = setup(a, chain_smem, bar, w0s);
 
   if (warp == 1) {
-    if (lane == 0) mma_loop(a, bar, chain_smem, tmem, my_tiles);
+    mma_loop(a, bar, chain_smem, tmem, my_tiles);
   } else if (warp >= 2) {
     const int s = (warp - 2) / kSlotWarps, q = warp & 3, half = ((warp - 2) % kSlotWarps) >> 2;
     const int row = q * 32 + lane;
@@ -216,7 +219,7 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_chain_backward_kernel(Args a)
   const unsigned tmem = setup(a, chain_smem, bar, w0s);
 
   if (warp == 1) {
-    if (lane == 0) mma_loop(a, bar, chain_smem, tmem, my_tiles);
+    mma_loop(a, bar, chain_smem, tmem, my_tiles);
   } else if (warp >= 2) {
     const int s = (warp - 2) / kSlotWarps, q = warp & 3, half = ((warp - 2) % kSlotWarps) >> 2;
     const int row = q * 32 + lane;

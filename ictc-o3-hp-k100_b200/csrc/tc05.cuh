@@ -55,6 +55,14 @@ __device__ __forceinline__ void bulk_g2s(unsigned dst, const void* src, unsigned
                "l"(src), "r"(bytes), "r"(bar)
                : "memory");
 }
+// 16 bytes global -> shared, the part beyond `bytes` filled with zeros
+__device__ __forceinline__ void cp_async16(unsigned dst, const void* src, unsigned bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_async_wait() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
@@ -130,15 +138,30 @@ __device__ __forceinline__ void ldg256(const float* p, float* v) {
                : "l"(p));
 }
 
+// One lane of a converged warp.  MMAs are issued under it and not under `lane == 0`: the compiler then knows that their
+// operands are uniform and an MMA costs 31 issue cycles instead of 52 (at N = 64, where the tensor core needs 32).
+__device__ __forceinline__ bool elect_one() {
+  unsigned p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
+}
+
+// x = big + small with 11 significant bits each, both rounded to nearest: the big part with integer arithmetic, the small
+// part with Veltkamp's splitting (a NaN, which the integer sum may turn into a number, comes through the small part).
+// The conversion instruction runs at a sixteenth of the rate of these: 64 of them per thread and 64-wide block were what
+// the GEMM kernels waited for (backward, 1 M rows of 704: 0.66 ms, 0.56 with this).
+__device__ __forceinline__ void split_tf32(float x, unsigned& big, unsigned& small) {
+  big = (__float_as_uint(x) + 0x1000u) & 0xffffe000u;
+  const float rest = x - __uint_as_float(big);
+  const float c = rest * 8193.f;
+  small = __float_as_uint(__fsub_rn(c, __fsub_rn(c, rest)));
+}
+
 // Splits 32 values of one row and writes the two parts into the TMEM A operand (lane = row, column = k).
 __device__ __forceinline__ void store_split_tmem(unsigned t_big, unsigned t_small, const float (&x)[32]) {
   unsigned b[32], sm[32];
 #pragma unroll
-  for (int i = 0; i < 32; ++i) {
-    const float big = to_tf32(x[i]);
-    b[i] = __float_as_uint(big);
-    sm[i] = __float_as_uint(to_tf32(x[i] - big));
-  }
+  for (int i = 0; i < 32; ++i) split_tf32(x[i], b[i], sm[i]);
   tmem_st32(t_big, b);
   tmem_st32(t_small, sm);
   tmem_st_wait();

@@ -18,7 +18,7 @@
 //     index r): element (f, k) of an operand with F feature rows lives at byte (k / 4) * F * 16 + f * 16 + (k % 4) * 4,
 //     i.e. one thread writes one 16-byte chunk = four consecutive rows of one feature.  fence.proxy.async orders
 //     these generic writes before the MMA's reads;
-//   * one thread of warp 0 issues, per K = 8 step and 128-feature tile, the three MMAs small*big + big*small +
+//   * one lane of warp 0 issues, per K = 8 step and 128-feature tile, the three MMAs small*big + big*small +
 //     big*big (fp32-level accuracy, the reference forbids plain TF32: ictc_o3/backends/k100/fp32_policy.py:6-11)
 //     and commits the operand stage back to the transform warps.
 // At the end four warps read the accumulators (thread = feature row) and store the CTA's partial result; a second
@@ -113,20 +113,20 @@ __global__ void __launch_bounds__(kThreads, 1) weight_grad_kernel(Args a) {
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const unsigned tmem = bar->tmem_base;
+  const unsigned tmem = __shfl_sync(0xffffffffu, bar->tmem_base, 0);
 
   if (warp == 0) {
     // ---- MMA issue: per operand stage ks_n K = 8 steps, three products per feature tile
-    if (lane == 0) {
-      bool ok = true;
-      for (int64_t it = 0; it < mine && !bar->failed; ++it) {
-        const int s = int(it % kOpStages);
-        if (!mbar_wait(saddr(&bar->op_full[s]), unsigned((it / kOpStages) & 1))) {
-          give_up(bar, a.status, 41);
-          ok = false;
-          break;
-        }
-        tc_fence_after();
+    bool ok = true;
+    for (int64_t it = 0; it < mine && !bar->failed; ++it) {
+      const int s = int(it % kOpStages);
+      if (!mbar_wait(saddr(&bar->op_full[s]), unsigned((it / kOpStages) & 1))) {
+        give_up(bar, a.status, 41);
+        ok = false;
+        break;
+      }
+      tc_fence_after();
+      if (elect_one()) {
         for (int ks = 0; ks < ks_n; ++ks) {
           const unsigned base = saddr(ops + s * op_b + ks * ks_b);
           const unsigned b_big = base + tiles * 2 * kAPart;
@@ -142,8 +142,10 @@ __global__ void __launch_bounds__(kThreads, 1) weight_grad_kernel(Args a) {
         }
         umma_commit(saddr(&bar->op_empty[s]));
       }
-      if (ok && mine > 0 && !bar->failed) umma_commit(saddr(&bar->done));
+      __syncwarp();
     }
+    if (ok && mine > 0 && !bar->failed && elect_one()) umma_commit(saddr(&bar->done));
+    __syncwarp();
   } else if (warp == 1) {
     // ---- row stream: lane r copies rows r, r + 32, ... of the stage (one bulk copy per row and operand)
     for (int64_t it = 0; it < mine && !bar->failed; ++it) {
@@ -212,13 +214,13 @@ __global__ void __launch_bounds__(kThreads, 1) weight_grad_kernel(Args a) {
 #pragma unroll
         for (int j = 0; j < 4; ++j)
           v[j] = (src_off[i] >= 0 && row0[i] + j < valid) ? *reinterpret_cast<const float*>(in + src_off[i] + j * src_step[i]) : 0.f;
-        float4 big, small;
-        big.x = to_tf32(v[0]); small.x = to_tf32(v[0] - big.x);
-        big.y = to_tf32(v[1]); small.y = to_tf32(v[1] - big.y);
-        big.z = to_tf32(v[2]); small.z = to_tf32(v[2] - big.z);
-        big.w = to_tf32(v[3]); small.w = to_tf32(v[3] - big.w);
-        *reinterpret_cast<float4*>(out + dst_off[i]) = big;
-        *reinterpret_cast<float4*>(out + dst_off[i] + part[i]) = small;
+        uint4 big, small;
+        split_tf32(v[0], big.x, small.x);
+        split_tf32(v[1], big.y, small.y);
+        split_tf32(v[2], big.z, small.z);
+        split_tf32(v[3], big.w, small.w);
+        *reinterpret_cast<uint4*>(out + dst_off[i]) = big;
+        *reinterpret_cast<uint4*>(out + dst_off[i] + part[i]) = small;
       }
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // generic writes -> visible to the MMA's reads
       __syncwarp();
@@ -265,16 +267,21 @@ __global__ void __launch_bounds__(kThreads, 1) weight_grad_kernel(Args a) {
   }
 }
 
-// dW[o, i] = sum over the CTAs' partial results, in CTA order.
-__global__ void weight_grad_reduce_kernel(const float* __restrict__ partial, int parts, int tiles, int NO, float* dw,
-                                          int64_t dw_ld) {
-  const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= NO * kK) return;
-  const int o = idx / kK, i = idx % kK;
+// dW[o, i] = sum over the CTAs' partial results, in a fixed order.
+// 64 values per block; four groups of threads take a quarter of the partial results each.
+__global__ void __launch_bounds__(256) weight_grad_reduce_kernel(const float* __restrict__ partial, int parts, int tiles,
+                                                                 float* dw, int64_t dw_ld) {
+  __shared__ float quarter[4][kK];
+  const int i = threadIdx.x & (kK - 1), k = threadIdx.x >> 6;
   const int64_t pitch = int64_t(tiles) * kRows * kK;
+  const float* p = partial + int64_t(blockIdx.x) * kK + i;
+  const int per = (parts + 3) / 4, last = min(parts, (k + 1) * per);
   float s = 0.f;
-  for (int b = 0; b < parts; ++b) s += partial[b * pitch + idx];
-  dw[o * dw_ld + i] = s;
+#pragma unroll 8
+  for (int b = k * per; b < last; ++b) s += p[b * pitch];
+  quarter[k][i] = s;
+  __syncthreads();
+  if (k == 0) dw[blockIdx.x * dw_ld + i] = (quarter[0][i] + quarter[1][i]) + (quarter[2][i] + quarter[3][i]);
 }
 
 static int grid_size(int64_t rows) {
@@ -325,9 +332,7 @@ int ictc_weight_grad_tc(int64_t num_rows, int num_out, const float* grad, int64_
   a.NO = num_out; a.status = kernel_status_word();
   wg::weight_grad_kernel<<<grid, wg::kThreads, smem, (cudaStream_t)stream>>>(a);
   if (int rc = finish_launch("weight_grad")) return rc;
-  const int n = num_out * tc::kK;
-  wg::weight_grad_reduce_kernel<<<(n + 255) / 256, 256, 0, (cudaStream_t)stream>>>(workspace, grid, tiles, num_out,
-                                                                                 dweight, dweight_ld);
+  wg::weight_grad_reduce_kernel<<<num_out, 256, 0, (cudaStream_t)stream>>>(workspace, grid, tiles, dweight, dweight_ld);
   return finish_launch("weight_grad_reduce");
 }
 
