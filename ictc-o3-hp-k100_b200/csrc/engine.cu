@@ -5,13 +5,9 @@
 // Bessel basis with polynomial envelope (mace_ictc/models/radial_basis.py:11-92), the direction
 // harmonics (ictc_o3/basis/ictd_irreps.py:1153-1208), SiLU * 1.679 (mace_ictc/models/mace/layers.py:307-314)
 // and the position gradient scatter of autograd.  One kernel each way instead of ~30 launches.
-#include "ictc_common.cuh"
-#include "generated/harmonics_tables.cuh"
+#include "geometry.cuh"
 
 namespace ictc {
-
-template <int A> __device__ __forceinline__ float ipw(float x) { return A == 0 ? 1.f : (A == 1 ? x : x * x); }
-template <int A> __device__ __forceinline__ float dpw(float x) { return A == 0 ? 0.f : (A == 1 ? 1.f : 2.f * x); }
 
 constexpr int kRadialMax = 16;
 
@@ -33,16 +29,6 @@ struct GeomArgs {
   float* dvec;               // [E,3]
 };
 
-__device__ __forceinline__ void envelope(float r, float r_max, int p, float& env, float& denv) {
-  const float u = r / r_max;
-  if (!(r < r_max)) { env = 0.f; denv = 0.f; return; }
-  const float pf = float(p);
-  const float up = powf(u, float(p - 1));   // u^(p-1)
-  const float a = (pf + 1.f) * (pf + 2.f) * 0.5f, b = pf * (pf + 2.f), c = pf * (pf + 1.f) * 0.5f;
-  env = 1.f - a * up * u + b * up * u * u - c * up * u * u * u;
-  denv = (-a * pf * up + b * (pf + 1.f) * up * u - c * (pf + 2.f) * up * u * u) / r_max;
-}
-
 __global__ void geom_forward_kernel(GeomArgs a) {
   const int64_t e = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   if (e >= a.E) return;
@@ -61,11 +47,7 @@ __global__ void geom_forward_kernel(GeomArgs a) {
   a.unit[3 * e + 2] = z;
   a.length[e] = r;
   float val[9];
-#pragma unroll
-  for (int h = 0; h < 9; ++h) val[h] = 0.f;
-#define ICTC_T(h, aa, bb, cc, cf) val[h] = fmaf(cf, ipw<aa>(x) * ipw<bb>(y) * ipw<cc>(z), val[h]);
-  ICTC_HARM_TERMS(ICTC_T)
-#undef ICTC_T
+  harmonics_value(x, y, z, val);
 #pragma unroll
   for (int h = 0; h < 9; ++h) a.sh[9 * e + h] = val[h];
   float env, denv;
@@ -80,37 +62,13 @@ __global__ void geom_backward_kernel(GeomArgs a) {
   if (e >= a.E) return;
   const float x = a.unit[3 * e], y = a.unit[3 * e + 1], z = a.unit[3 * e + 2];
   const float r = a.length[e];
-  const float rc = fmaxf(r, 1e-8f);
-  // harmonics: du = J^T dsh
   float g[9];
 #pragma unroll
   for (int h = 0; h < 9; ++h) g[h] = a.dsh[9 * e + h];
-  float d0 = 0.f, d1 = 0.f, d2 = 0.f;
-#define ICTC_T(h, aa, bb, cc, cf)                                        \
-  d0 = fmaf(g[h] * (cf), dpw<aa>(x) * ipw<bb>(y) * ipw<cc>(z), d0);       \
-  d1 = fmaf(g[h] * (cf), ipw<aa>(x) * dpw<bb>(y) * ipw<cc>(z), d1);       \
-  d2 = fmaf(g[h] * (cf), ipw<aa>(x) * ipw<bb>(y) * dpw<cc>(z), d2);
-  ICTC_HARM_TERMS(ICTC_T)
-#undef ICTC_T
-  // radial basis: dr = sum_k drb_k * d(rb_k)/dr
-  float env, denv;
-  envelope(r, a.r_max, a.p, env, denv);
-  const float rs = fmaxf(r, 1e-12f);
-  const float pref = sqrtf(2.f / a.r_max);
-  const float w = 3.14159265358979323846f / a.r_max;
-  float dr = 0.f;
-  for (int k = 0; k < a.num_basis; ++k) {
-    const float wk = w * float(k + 1);
-    float s, c;
-    sincosf(r * wk, &s, &c);
-    const float f = pref * s / rs;                      // bessel value
-    const float df = pref * (wk * c / rs - s / (rs * rs));
-    dr = fmaf(a.drb[e * a.num_basis + k], df * env + f * denv, dr);
-  }
-  const float dot = x * d0 + y * d1 + z * d2;
-  a.dvec[3 * e + 0] = dr * x + (d0 - dot * x) / rc;
-  a.dvec[3 * e + 1] = dr * y + (d1 - dot * y) / rc;
-  a.dvec[3 * e + 2] = dr * z + (d2 - dot * z) / rc;
+  const float3 v = edge_vector_gradient(x, y, z, r, g, a.drb + e * a.num_basis, a.num_basis, a.p, a.r_max);
+  a.dvec[3 * e + 0] = v.x;
+  a.dvec[3 * e + 1] = v.y;
+  a.dvec[3 * e + 2] = v.z;
 }
 
 // grad[i] = sum_{e: dst(e)=i} dvec[e] - sum_{e: src(e)=i} dvec[e]; fixed CSR order, no atomics.

@@ -54,18 +54,18 @@ struct Barriers {
 // The tiles of a launch, segment after segment, dealt out round robin over the CTAs.  Every warp role walks the same tiles
 // in the same order.
 struct Work {
-  int64_t base, rows0;       // first list entry and live rows of the first segment
+  int64_t base, live;        // first list entry, bound of the live rows
   int end0, end1, end2;      // running totals of tiles
 
   __device__ Work(const Args& a) {
     base = a.begin ? ldg(a.begin) : 0;
-    rows0 = a.limit ? ldg(a.limit) - base : a.seg[0].rows;
-    rows0 = rows0 < 0 ? 0 : (rows0 < a.seg[0].rows ? rows0 : a.seg[0].rows);
-    end0 = int((rows0 + kRows - 1) / kRows);
-    end1 = end0 + (a.segments > 1 ? int((a.seg[1].rows + kRows - 1) / kRows) : 0);
-    end2 = end1 + (a.segments > 2 ? int((a.seg[2].rows + kRows - 1) / kRows) : 0);
+    live = a.limit ? ldg(a.limit) - base : a.seg[0].rows + a.seg[1].rows + a.seg[2].rows;
+    if (live < 0) live = 0;
+    end0 = int((rows(a, 0) + kRows - 1) / kRows);
+    end1 = end0 + (a.segments > 1 ? int((rows(a, 1) + kRows - 1) / kRows) : 0);
+    end2 = end1 + (a.segments > 2 ? int((rows(a, 2) + kRows - 1) / kRows) : 0);
   }
-  __device__ int64_t rows(const Args& a, int s) const { return s == 0 ? rows0 : a.seg[s].rows; }
+  __device__ int64_t rows(const Args& a, int s) const { return live < a.seg[s].rows ? live : a.seg[s].rows; }
   __device__ int segment(int tile) const { return (tile >= end0) + (tile >= end1); }
   __device__ int tiles() const { return end2; }
   __device__ int64_t first_row(int tile, int s) const {

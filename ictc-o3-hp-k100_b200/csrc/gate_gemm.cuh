@@ -27,7 +27,7 @@ struct Args {
   int segments;
   const int64_t* pair_a;  // backward, optional: row g is in[pair_a[g]] + in[pair_b[g]] (one segment)
   const int64_t* pair_b;
-  const int64_t* limit;   // optional device scalar: only min(rows, *limit) rows of the first segment are processed
+  const int64_t* limit;   // optional device scalar: only min(rows, *limit) rows of every segment are processed
   // Row windows (one segment, plain matrices).  With `begin` (device scalar) the launch covers the window
   // [*begin, min(*begin + rows, *limit)) of a longer row list: local row g = 0.. stands for list entry *begin + g.
   const int64_t* begin;

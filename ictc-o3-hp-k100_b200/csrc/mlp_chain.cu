@@ -15,7 +15,7 @@
 // TMEM per slot (192 columns): A big [0,64) | A small [64,128) | accumulator [128,192).
 // The weights of the two 64 x 64 layers stay in shared memory in the B-operand layout (64 KB), the narrow layer's
 // as a plain [64][8] table.  Every mbarrier wait is bounded and reports through the library's status word.
-#include "tc05.cuh"
+#include "mlp_chain.cuh"
 
 namespace ictc {
 namespace chain {
@@ -30,23 +30,12 @@ constexpr int kXchgBytes = 2 * kRows * 8 * 4;       // partial drb rows of both 
 constexpr int kBarOffset = 2 * kWStageBytes + kTableBytes + kXchgBytes;
 constexpr int kSmem = kBarOffset + 256;            // W(a) | W(b) | W0 table | drb exchange | barriers
 
-struct Args {
-  const float* in;     // forward: rb [E, nb]; backward: da3 [E, 64]
-  const float* w0;     // [64, nb] (forward: W0; backward: W0 as well, used as dz1 @ W0)
-  const float* wa;     // packed 64 x 64 operand of the first MMA layer (forward: W1, backward: W2 transposed use)
-  const float* wb;     // packed operand of the second MMA layer (forward: W2, backward: W1 transposed use)
-  float* z1;           // forward outputs / backward inputs [E, 64]
-  float* z2;
-  float* z3;
-  float* drb;          // backward output [E, nb]
-  const int64_t* rows; // optional row index: forward reads rb[rows[r]], backward writes / adds to drb[rows[r]]
-  const int64_t* in_a; // backward, optional: row r starts from in[in_a[r]] + in[in_b[r]] (in_b[r] < 0: first term only)
-  const int64_t* in_b;
-  int accumulate;      // backward: drb[...] += instead of =
-  const int64_t* limit; // optional device scalar: only min(E, *limit) rows are processed (recorded graphs)
-  int64_t E;
-  int nb;
-  int* status;
+// Two stacks share the CTAs half and half (the rows of both are the same, so is their work).
+struct Share {
+  int stack, first, step;
+  __device__ Share(const Args& a)
+      : stack(a.stacks == 2 ? int(blockIdx.x & 1) : 0), first(a.stacks == 2 ? blockIdx.x >> 1 : blockIdx.x),
+        step(a.stacks == 2 ? gridDim.x >> 1 : gridDim.x) {}
 };
 
 struct Barriers {
@@ -66,7 +55,7 @@ __device__ __forceinline__ void stg256(float* p, const float* v) {
 }
 
 // Common prologue: barriers, TMEM, weights.  Returns the TMEM base address.
-__device__ __forceinline__ unsigned setup(const Args& a, unsigned char* smem, Barriers* bar, float* w0s) {
+__device__ __forceinline__ unsigned setup(const Args& a, const Stack& k, unsigned char* smem, Barriers* bar, float* w0s) {
   const int warp = threadIdx.x >> 5;
   if (threadIdx.x == 0) {
     for (int i = 0; i < 2; ++i) {
@@ -81,12 +70,12 @@ __device__ __forceinline__ unsigned setup(const Args& a, unsigned char* smem, Ba
     bar->failed = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     mbar_expect_tx(saddr(&bar->w_full), 2 * kWStageBytes);
-    bulk_g2s(saddr(smem), a.wa, kWStageBytes, saddr(&bar->w_full));
-    bulk_g2s(saddr(smem + kWStageBytes), a.wb, kWStageBytes, saddr(&bar->w_full));
+    bulk_g2s(saddr(smem), k.wa, kWStageBytes, saddr(&bar->w_full));
+    bulk_g2s(saddr(smem + kWStageBytes), k.wb, kWStageBytes, saddr(&bar->w_full));
   }
   for (int i = threadIdx.x; i < 64 * 8; i += blockDim.x) {
-    const int n = i >> 3, k = i & 7;
-    w0s[i] = k < a.nb ? a.w0[n * a.nb + k] : 0.f;
+    const int n = i >> 3, b = i & 7;
+    w0s[i] = b < a.nb ? k.w0[n * a.nb + b] : 0.f;
   }
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(saddr(&bar->tmem_base)),
@@ -135,15 +124,17 @@ __device__ __forceinline__ void mma_loop(const Args& a, Barriers* bar, unsigned 
 }
 
 // ------------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(kThreads, 1) mlp_chain_forward_kernel(Args a) {
+__global__ void __launch_bounds__(kThreads, 1) mlp_chain_forward_kernel(const __grid_constant__ Args a) {
   extern __shared__ __align__(128) unsigned char chain_smem[];
   float* w0s = reinterpret_cast<float*>(chain_smem + 2 * kWStageBytes);
   Barriers* bar = reinterpret_cast<Barriers*>(chain_smem + kBarOffset);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t nrows = a.limit ? (ldg(a.limit) < a.E ? ldg(a.limit) : a.E) : a.E;
   const int64_t tiles = (nrows + kRows - 1) / kRows;
-  const int64_t my_tiles = blockIdx.x < tiles ? (tiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
-  const unsigned tmem = setup(a, chain_smem, bar, w0s);
+  const Share share(a);
+  const Stack& stack = a.stack[share.stack];
+  const int64_t my_tiles = share.first < tiles ? (tiles - share.first + share.step - 1) / share.step : 0;
+  const unsigned tmem = setup(a, stack, chain_smem, bar, w0s);
 
   if (warp == 1) {
     mma_loop(a, bar, chain_smem, tmem, my_tiles);
@@ -154,14 +145,14 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_chain_forward_kernel(Args a) 
     const unsigned t_big = lane_base + half * 32, t_acc = lane_base + 2 * kK + half * 32;
     unsigned phase = 0;
     for (int64_t i = s; i < my_tiles; i += 2) {
-      const int64_t g = (blockIdx.x + i * gridDim.x) * kRows + row;
+      const int64_t g = (share.first + i * share.step) * kRows + row;
       const bool valid = g < nrows;
       // ---- layer 0 in fp32: z1[n] = sum_k rb[k] W0[n][k] for this thread's 32 units
       float rb[8];
 #pragma unroll
       const int64_t src_row = (valid && a.rows) ? __ldg(reinterpret_cast<const long long*>(a.rows + g)) : g;
 #pragma unroll
-      for (int k = 0; k < 8; ++k) rb[k] = (valid && k < a.nb) ? __ldg(a.in + src_row * a.nb + k) : 0.f;
+      for (int k = 0; k < 8; ++k) rb[k] = (valid && k < a.nb) ? __ldg(stack.in + src_row * a.nb + k) : 0.f;
       float x[32];
 #pragma unroll
       for (int n = 0; n < 32; ++n) {
@@ -186,7 +177,7 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_chain_forward_kernel(Args a) 
           tmem_ld32(t_acc, x);
         }
         if (valid) {
-          float* z = (layer == 0 ? a.z1 : layer == 1 ? a.z2 : a.z3) + g * kK + half * 32;
+          float* z = (layer == 0 ? stack.z1 : layer == 1 ? stack.z2 : stack.z3) + g * kK + half * 32;
 #pragma unroll
           for (int j = 0; j < 4; ++j) stg256(z + j * 8, x + j * 8);
         }
@@ -207,7 +198,7 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_chain_forward_kernel(Args a) 
 // ------------------------------------------------------------------------------------------------
 // backward: t3 = da3 * silu'(z3);  da2 = t3 @ W2;  t2 = da2 * silu'(z2);  da1 = t2 @ W1;  t1 = da1 * silu'(z1);
 // drb = t1 @ W0.  (wa = W2 packed for x @ W2, wb = W1 packed for x @ W1.)
-__global__ void __launch_bounds__(kThreads, 1) mlp_chain_backward_kernel(Args a) {
+__global__ void __launch_bounds__(kThreads, 1) mlp_chain_backward_kernel(const __grid_constant__ Args a) {
   extern __shared__ __align__(128) unsigned char chain_smem[];
   float* w0s = reinterpret_cast<float*>(chain_smem + 2 * kWStageBytes);
   float* xchg = w0s + 64 * 8;                                         // [128][8] partial drb of the upper half
@@ -215,8 +206,10 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_chain_backward_kernel(Args a)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t nrows = a.limit ? (ldg(a.limit) < a.E ? ldg(a.limit) : a.E) : a.E;
   const int64_t tiles = (nrows + kRows - 1) / kRows;
-  const int64_t my_tiles = blockIdx.x < tiles ? (tiles - blockIdx.x + gridDim.x - 1) / gridDim.x : 0;
-  const unsigned tmem = setup(a, chain_smem, bar, w0s);
+  const Share share(a);
+  const Stack& stack = a.stack[share.stack];
+  const int64_t my_tiles = share.first < tiles ? (tiles - share.first + share.step - 1) / share.step : 0;
+  const unsigned tmem = setup(a, stack, chain_smem, bar, w0s);
 
   if (warp == 1) {
     mma_loop(a, bar, chain_smem, tmem, my_tiles);
@@ -230,7 +223,7 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_chain_backward_kernel(Args a)
     float* slot_x = xchg + (s * kRows + row) * 8;
     unsigned phase = 0, xphase = 0;
     for (int64_t i = s; i < my_tiles; i += 2) {
-      const int64_t g = (blockIdx.x + i * gridDim.x) * kRows + row;
+      const int64_t g = (share.first + i * share.step) * kRows + row;
       const bool valid = g < nrows;
       float x[32], z[32];
       bool ok = true;
@@ -240,7 +233,7 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_chain_backward_kernel(Args a)
         if (valid) {
 #pragma unroll
           for (int j = 0; j < 4; ++j)
-            ldg256((layer == 0 ? a.z3 : layer == 1 ? a.z2 : a.z1) + g * kK + half * 32 + j * 8, z + j * 8);
+            ldg256((layer == 0 ? stack.z3 : layer == 1 ? stack.z2 : stack.z1) + g * kK + half * 32 + j * 8, z + j * 8);
         } else {
 #pragma unroll
           for (int n = 0; n < 32; ++n) z[n] = 0.f;
@@ -249,12 +242,12 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_chain_backward_kernel(Args a)
           if (valid) {
             const int64_t ra = a.in_a ? ldg(a.in_a + g) : g;
 #pragma unroll
-            for (int j = 0; j < 4; ++j) ldg256(a.in + ra * kK + half * 32 + j * 8, x + j * 8);
+            for (int j = 0; j < 4; ++j) ldg256(stack.in + ra * kK + half * 32 + j * 8, x + j * 8);
             const int64_t rb = a.in_b ? ldg(a.in_b + g) : -1;
             if (rb >= 0) {
               float y[32];
 #pragma unroll
-              for (int j = 0; j < 4; ++j) ldg256(a.in + rb * kK + half * 32 + j * 8, y + j * 8);
+              for (int j = 0; j < 4; ++j) ldg256(stack.in + rb * kK + half * 32 + j * 8, y + j * 8);
 #pragma unroll
               for (int n = 0; n < 32; ++n) x[n] += y[n];
             }
@@ -306,7 +299,7 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_chain_backward_kernel(Args a)
         p[0] += lo.x; p[1] += lo.y; p[2] += lo.z; p[3] += lo.w;
         p[4] += hi.x; p[5] += hi.y; p[6] += hi.z; p[7] += hi.w;
         if (valid) {
-          float* o = a.drb + (a.rows ? __ldg(reinterpret_cast<const long long*>(a.rows + g)) : g) * a.nb;
+          float* o = stack.drb + (a.rows ? __ldg(reinterpret_cast<const long long*>(a.rows + g)) : g) * a.nb;
 #pragma unroll
           for (int k = 0; k < 8; ++k)
             if (k < a.nb) o[k] = a.accumulate ? o[k] + p[k] : p[k];
@@ -318,11 +311,30 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_chain_backward_kernel(Args a)
   teardown(tmem);
 }
 
-static int grid_size(int64_t rows) {
+static int grid_size(const Args& a) {
   int dev = 0, sms = 148;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const int64_t tiles = (rows + kRows - 1) / kRows;
-  return int(tiles < sms ? tiles : sms);
+  const int64_t tiles = (a.E + kRows - 1) / kRows;
+  const int per = sms / a.stacks;
+  return a.stacks * int(tiles < per ? tiles : per);
+}
+
+int launch_forward(Args a, cudaStream_t st) {
+  static const cudaError_t attr =
+      cudaFuncSetAttribute(mlp_chain_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+  if (attr != cudaSuccess) { set_error("mlp chain smem: %s", cudaGetErrorString(attr)); return ICTC_ERR_LAUNCH; }
+  a.status = kernel_status_word();
+  mlp_chain_forward_kernel<<<grid_size(a), kThreads, kSmem, st>>>(a);
+  return finish_launch("mlp_chain_forward");
+}
+
+int launch_backward(Args a, cudaStream_t st) {
+  static const cudaError_t attr =
+      cudaFuncSetAttribute(mlp_chain_backward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
+  if (attr != cudaSuccess) { set_error("mlp chain smem: %s", cudaGetErrorString(attr)); return ICTC_ERR_LAUNCH; }
+  a.status = kernel_status_word();
+  mlp_chain_backward_kernel<<<grid_size(a), kThreads, kSmem, st>>>(a);
+  return finish_launch("mlp_chain_backward");
 }
 
 }  // namespace chain
@@ -346,14 +358,11 @@ int ictc_mlp_chain_forward(int64_t num_edges, int num_basis, const float* rb, co
     set_error("mlp chain forward: buffers must be 32-byte aligned");
     return ICTC_ERR_BAD_ARG;
   }
-  static const cudaError_t attr = cudaFuncSetAttribute(chain::mlp_chain_forward_kernel,
-                                                       cudaFuncAttributeMaxDynamicSharedMemorySize, chain::kSmem);
-  if (attr != cudaSuccess) { set_error("mlp chain smem: %s", cudaGetErrorString(attr)); return ICTC_ERR_LAUNCH; }
   chain::Args a{};
-  a.in = rb; a.rows = rb_rows; a.limit = row_limit; a.w0 = w0; a.wa = w1_packed; a.wb = w2_packed; a.z1 = z1; a.z2 = z2; a.z3 = z3; a.E = num_edges; a.nb = num_basis;
-  a.status = kernel_status_word();
-  chain::mlp_chain_forward_kernel<<<chain::grid_size(num_edges), chain::kThreads, chain::kSmem, (cudaStream_t)stream>>>(a);
-  return finish_launch("mlp_chain_forward");
+  a.stacks = 1;
+  a.stack[0] = chain::Stack{rb, w0, w1_packed, w2_packed, z1, z2, z3, nullptr};
+  a.rows = rb_rows; a.limit = row_limit; a.E = num_edges; a.nb = num_basis;
+  return chain::launch_forward(a, (cudaStream_t)stream);
 }
 
 int ictc_mlp_chain_backward(int64_t num_edges, int num_basis, const float* da3, const float* w0, const float* w1t_packed,
@@ -379,15 +388,13 @@ int ictc_mlp_chain_backward_paired(int64_t num_edges, int num_basis, const float
     set_error("mlp chain backward: buffers must be 32-byte aligned");
     return ICTC_ERR_BAD_ARG;
   }
-  static const cudaError_t attr = cudaFuncSetAttribute(chain::mlp_chain_backward_kernel,
-                                                       cudaFuncAttributeMaxDynamicSharedMemorySize, chain::kSmem);
-  if (attr != cudaSuccess) { set_error("mlp chain smem: %s", cudaGetErrorString(attr)); return ICTC_ERR_LAUNCH; }
   chain::Args a{};
-  a.in = da3; a.w0 = w0; a.wa = w2t_packed; a.wb = w1t_packed; a.z1 = const_cast<float*>(z1); a.z2 = const_cast<float*>(z2);
-  a.z3 = const_cast<float*>(z3); a.drb = drb; a.in_a = pair_a; a.in_b = pair_b; a.rows = drb_rows; a.limit = row_limit; a.accumulate = accumulate ? 1 : 0; a.E = num_edges; a.nb = num_basis;
-  a.status = kernel_status_word();
-  chain::mlp_chain_backward_kernel<<<chain::grid_size(num_edges), chain::kThreads, chain::kSmem, (cudaStream_t)stream>>>(a);
-  return finish_launch("mlp_chain_backward");
+  a.stacks = 1;
+  a.stack[0] = chain::Stack{da3, w0, w2t_packed, w1t_packed, const_cast<float*>(z1), const_cast<float*>(z2),
+                            const_cast<float*>(z3), drb};
+  a.in_a = pair_a; a.in_b = pair_b; a.rows = drb_rows; a.limit = row_limit; a.accumulate = accumulate ? 1 : 0;
+  a.E = num_edges; a.nb = num_basis;
+  return chain::launch_backward(a, (cudaStream_t)stream);
 }
 
 }  // extern "C"

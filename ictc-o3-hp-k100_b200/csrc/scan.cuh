@@ -36,9 +36,10 @@ __global__ void __launch_bounds__(kPrefixThreads) tile_sum_kernel(int64_t n, LOA
     if (i < n) v += load(i);
   }
   v = block_sum(v, warp_tot);
-  if (threadIdx.x == 0) sums[blockIdx.x] = v;
+  if (threadIdx.x == 0) sums[blockIdx.y * gridDim.x + blockIdx.x] = v;
 }
 
+// blockIdx.y numbers independent inputs of the same length; the functors look it up themselves.
 // store(i, sum of the values before i, value i) for every i < n.  `sums`: totals of the tiles, or null: the values
 // before the tile are read again (then `load` must not read what `store` writes).
 template <class T, class LOAD, class STORE>
@@ -47,7 +48,7 @@ __global__ void __launch_bounds__(kPrefixThreads) prefix_kernel(int64_t n, LOAD 
   const int64_t base = int64_t(blockIdx.x) * kPrefixTile;
   T before = 0;
   if (sums) {
-    for (int64_t i = threadIdx.x; i < blockIdx.x; i += kPrefixThreads) before += sums[i];
+    for (int64_t i = threadIdx.x; i < blockIdx.x; i += kPrefixThreads) before += sums[blockIdx.y * gridDim.x + i];
   } else {
     for (int64_t i = threadIdx.x; i < base; i += kPrefixThreads) before += load(i);
   }
@@ -80,15 +81,15 @@ __global__ void __launch_bounds__(kPrefixThreads) prefix_kernel(int64_t n, LOAD 
 
 inline int64_t prefix_tiles(int64_t n) { return n > 0 ? (n + kPrefixTile - 1) / kPrefixTile : 0; }
 
-// `in_place`: store() writes where load() reads; `sums`: prefix_tiles(n) values of scratch.  Returns the launches made.
+// `in_place`: store() writes where load() reads; `sums`: inputs * prefix_tiles(n) values of scratch.
 template <class T, class LOAD, class STORE>
-int prefix_sum(int64_t n, LOAD load, STORE store, T* sums, bool in_place, cudaStream_t st) {
+void prefix_sum(int64_t n, LOAD load, STORE store, T* sums, bool in_place, cudaStream_t st, int inputs = 1) {
   const int64_t tiles = prefix_tiles(n);
-  if (tiles == 0) return 0;
+  if (tiles == 0) return;
   const bool two = tiles > kPrefixDirect || (in_place && tiles > 1);
-  if (two) tile_sum_kernel<T><<<(unsigned)tiles, kPrefixThreads, 0, st>>>(n, load, sums);
-  prefix_kernel<T><<<(unsigned)tiles, kPrefixThreads, 0, st>>>(n, load, store, two ? (const T*)sums : (const T*)nullptr);
-  return two ? 2 : 1;
+  const dim3 grid((unsigned)tiles, (unsigned)inputs);
+  if (two) tile_sum_kernel<T><<<grid, kPrefixThreads, 0, st>>>(n, load, sums);
+  prefix_kernel<T><<<grid, kPrefixThreads, 0, st>>>(n, load, store, two ? (const T*)sums : (const T*)nullptr);
 }
 
 }  // namespace ictc

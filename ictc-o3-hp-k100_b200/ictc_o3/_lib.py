@@ -70,12 +70,39 @@ SIGNATURES = {
     "ictc_harmonics_forward": (_I, [_I, _L, _P, _P, _P]),
     "ictc_harmonics_vjp": (_I, [_I, _L, _P, _P, _P, _P]),
     "ictc_harmonics_second": (_I, [_I, _L, _P, _P, _P, _P, _P, _P]),
+    "ictc_sweep_workspace": (_L, [_P]),
+    "ictc_sweep_run": (_I, [_P, _I, _P]),
+    "ictc_sweep_struct_bytes": (_L, []),
     "ictc_sc_num_weights": (_I, [_I, _I]),
     "ictc_sc_scratch_bytes": (_L, [_I, _I, _I, _L, _I]),
     "ictc_sc_forward": (_I, [_I, _I, _I, _L, _I, _I, _P, _P, _P, _P, _P]),
     "ictc_sc_adjoint": (_I, [_I, _I, _I, _L, _I, _I, _P, _P, _P, _P, _P, _P, _P, _P]),
     "ictc_sc_second": (_I, [_I, _I, _I, _L, _I, _I, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P]),
 }
+
+
+class SweepLayer(C.Structure):
+    """Mirror of ``ictc_sweep_layer``."""
+    _fields_ = [("w0", _P), ("hid", _P * 2), ("hid_t", _P * 2), ("w3", _P), ("w3t", _P), ("path_weight", _P),
+                ("up", _P * 3), ("up_b", _P * 3), ("ml", _P * 3), ("ml_b", _P * 3), ("pl", _P * 3), ("pl_b", _P * 3),
+                ("bank", _P), ("num_gates", _L), ("slots", _L * 3)]
+
+
+class Sweep(C.Structure):
+    """Mirror of ``ictc_sweep`` (field order and types are checked against the header's size by a test)."""
+    _fields_ = ([(n, _L) for n in ("n_local", "n_owned", "edges", "pair_rows", "num_species", "graphs", "chunk_rows",
+                                   "chunk_capacity_dst", "chunk_capacity_src", "stream_gates", "num_basis", "poly_p",
+                                   "hidden", "mask_atomic")]
+                + [("r_max", C.c_double), ("box", C.c_double * 3), ("gradient_sign", C.c_double)]
+                + [(n, _P) for n in ("pos", "src", "dst", "shifts", "cells", "batch", "numbers", "species_table")]
+                + [("species_table_size", _L)]
+                + [(n, _P) for n in ("species", "dst_rowptr", "dst_order", "src_rowptr", "src_order", "gate_row", "rep",
+                                     "other", "live", "row_mask", "features", "feature_grad", "energy", "atomic", "gradient",
+                                     "host_status", "host_status_event", "status", "up0_table", "sc0_table", "readout_rp",
+                                     "readout_rs", "readout_w2", "readout_ro0")]
+                + [("layer", SweepLayer * 2), ("work", _P), ("work_bytes", _L), ("host_marks", _P),
+                   ("host_marks_capacity", _L), ("host_mark_labels", _P), ("host_counts", _P)])
+
 
 _lib = None
 
@@ -92,6 +119,8 @@ def load():
         for name, (res, args) in SIGNATURES.items():
             fn = getattr(lib, name)
             fn.restype, fn.argtypes = res, args
+        if lib.ictc_sweep_struct_bytes() != C.sizeof(Sweep):
+            raise ImportError(f"{LIB_PATH} was built from another version of include/ictc_b200.h: build it again")
         _lib = lib
     return _lib
 

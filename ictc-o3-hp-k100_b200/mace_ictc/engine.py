@@ -3,8 +3,9 @@ sweep over the B200 kernels, without the autograd tape.
 
 Same arithmetic as ``MaceIctcModel.forward`` followed by ``autograd.grad(E, pos)``
 (reference: mace_ictc/hp/runtime.py:82-111 over mace_ictc/models/mace/backbone.py:860-1246), specialised to
-what an MD step needs: frozen weights, gradient with respect to positions only.  Every adjoint below is
-the hand-written reverse of the line that produced the value; tests compare it with the autograd path.
+what an MD step and an energy-and-forces call need: frozen weights, gradient with respect to positions only.  The
+launch sequence is native (``csrc/sweep.cu``); this module lays the weights out for it, sizes the workspace and
+calls it, once, or stage by stage where ghost rows are exchanged in between.  Tests compare it with the autograd path.
 Node features live in ir_mul rows ([rows, 9C], degree blocks [2l+1, C]) from end to end, so channel
 linears are GEMMs over contiguous rows and no mul_ir <-> ir_mul conversion is made.
 
@@ -21,15 +22,24 @@ from __future__ import annotations
 
 import ctypes as C
 import math
+import threading
 
 import torch
 
 from ictc_o3 import _lib
 from ictc_o3.ops.topology import build_csr
-from ictc_o3.symmetric_contraction import _ScCall
-from .model import SILU_SCALE, MaceIctcModel
+from .model import MaceIctcModel
 
-_DEGREES = ((0, 1), (1, 3), (4, 5))        # (first component, number of components) of the degree blocks
+_ALL, _STAGES = 31, (1, 2, 4, 8, 16)
+_LABELS = ("radial_mlp_hidden_forward_{nout}", "gate_gemm_forward_{nout}", "graph_forward_l{layer}",
+           "graph_adjoint_l{layer}", "gate_gemm_backward_{nout}", "radial_mlp_hidden_backward_{nout}",
+           "channel_linear_tc", "symmetric_contraction_l{layer}")
+_MARKS = 1024            # timed launches of one sweep (eager steps of a benchmark)
+_local = threading.local()
+
+
+class _Weights:
+    """The sweep's view of one state of the parameters: packed operands and the struct that points at them."""
 
 
 class ForceEngine:
@@ -49,8 +59,8 @@ class ForceEngine:
         self.c = model.channels
         self.dev = next(model.parameters()).device
         self.lib = _lib.load()
-        self._versions = None
-        self._spec = {0: _lib.tp_spec(0, 2, 2), 1: _lib.tp_spec(2, 2, 2)}
+        self._weights = None
+        self._watched = None
         self.chunk_rows = None if chunk_rows is None else int(chunk_rows)
         self.chunk_margin = float(chunk_margin)
         # with chunks: True = the gates are streamed too (produced per chunk in the forward sweep, recomputed per chunk
@@ -64,59 +74,94 @@ class ForceEngine:
         self.refresh()
 
     # ---------------------------------------------------------------- weights
+    def _watch(self):
+        """Every module and parameter slot of the model with what it holds now: a replaced one is noticed by identity."""
+        slots, modules = [], list(self.model.modules())
+        for module in modules:
+            for table in (module._modules, module._parameters):
+                slots.extend((table, key, value) for key, value in table.items())
+        params = list(self.model.parameters())
+        inter = list(self.model.interactions)
+        return slots, modules, params, inter
+
+    def _state(self):
+        _, _, params, inter = self._watched
+        m = self.model
+        return ([(p._version, p.data_ptr()) for p in params], [i.avg_num_neighbors for i in inter], m.max_radius,
+                m.polynomial_cutoff_p, m.number_of_basis)
+
+    def hooked(self):
+        """Does any module carry a forward hook (which the sweep would not call)?"""
+        self.refresh()
+        return any(m._forward_hooks or m._forward_pre_hooks for m in self._watched[1])
+
     def refresh(self):
         """(Re)build the GEMM-ready weight views when a parameter changed."""
-        versions = tuple(p._version for p in self.model.parameters())
-        if versions == self._versions:
-            return
-        m, c = self.model, self.c
+        if self._watched is None or any(table.get(key) is not value for table, key, value in self._watched[0]):
+            self._watched, self._weights = self._watch(), None
+        state = self._state()
+        if self._weights is not None and self._weights.state == state:
+            return self._weights
+        w = self._layout()
+        w.state = state
+        self._weights = w
+        return w
+
+    def _layout(self):
+        m, c, w = self.model, self.c, _Weights()
+        if any(p.dtype != torch.float32 or p.device != self.dev for p in self._watched[2]):
+            raise ValueError("the force engine needs float32 parameters on one CUDA device")
+        w.keep, w.struct = [], _lib.Sweep()
+
+        def hold(t):
+            w.keep.append(t)
+            return t.data_ptr()
+
         with torch.no_grad():
-            self.emb = m.node_embedding.weight.t().contiguous()                         # [S, C]
-            self.layers = []
-            for inter, prod in zip(m.interactions, m.products):
-                lin = inter.input_lmax
+            emb = m.node_embedding.weight.t()                                            # [S, C]
+            w.nout = []
+            for k, (inter, prod) in enumerate(zip(m.interactions, m.products)):
                 fc = [mod.weight.contiguous() for mod in inter.fc if isinstance(mod, torch.nn.Linear)]
                 if not (len(fc) == 4 and fc[0].shape[0] == 64 and fc[0].shape[1] <= 8 and tuple(fc[1].shape) == (64, 64)
                         and tuple(fc[2].shape) == (64, 64) and fc[3].shape[1] == 64 and fc[3].shape[0] % 64 == 0):
                     raise ValueError("the force engine needs the radial MLP num_basis (<= 8) -> 64 -> 64 -> 64 -> P*C")
-                L = {
-                    "up": [inter.linear_up.adapters[str(l)].weight.contiguous() for l in range(lin + 1)],
-                    "fc0": fc[0], "nout": fc[3].shape[0],
-                    "ml": [(inter.message_linear.weights[str(l)] / max(inter.avg_num_neighbors, 1e-8)).contiguous()
-                           for l in range(3)],
-                    "counts": [inter.tp.path_counts_by_l[l] for l in range(3)],
-                    "tpw": None if bool(torch.all(inter.tp.weight == 1)) else inter.tp.weight.contiguous(),
-                    "w3": self._pack(fc[3], 0), "w3t": self._pack(fc[3], 1),
-                    "hid": [self._pack(fc[1], 0), self._pack(fc[2], 0)],
-                    "hid_t": [self._pack(fc[1], 1), self._pack(fc[2], 1)],
-                }
-                wsc = inter.self_connection.weights["0"]                                 # [S, C(out), C(in)]
-                s = wsc.shape[0]
-                L["sc_fwd"] = wsc.permute(2, 0, 1).reshape(c, s * c).contiguous()          # x @ -> [n, S*C(out)]
-                L["sc_bwd"] = wsc.permute(1, 0, 2).reshape(c, s * c).contiguous()          # dout @ -> [n, S*C(in)]
-                L["bank"] = prod.symmetric_contractions.weight_bank()
-                L["target"] = prod.target_lmax
-                pl = [(prod.linear[str(l)] / math.sqrt(c)).contiguous() for l in range(prod.target_lmax + 1)]
-                L["pl0"], L["pl0_t"] = pl[0], pl[0].t().contiguous()
-                # operand-layout copies for the tensor-core channel linears: key -> (packed, k_chunks, n_chunks)
-                P = {}
-                for l in range(lin + 1):
-                    up = L["up"][l]
-                    P["up", l] = self._pack_lin(up, up.t().contiguous())                  # x @ up^T
-                    P["up_b", l] = self._pack_lin(up.t().contiguous(), up)                # x @ up
-                for l in range(3):
-                    ml = L["ml"][l]
-                    P["ml", l] = self._pack_lin(ml, ml.t().contiguous())                  # x @ ml^T
-                    P["ml_b", l] = self._pack_lin(ml.t().contiguous(), ml)                # x @ ml
-                for l in range(prod.target_lmax + 1):
-                    P["pl", l] = self._pack_lin(pl[l].t().contiguous(), pl[l])            # x @ pl
-                    P["pl_b", l] = self._pack_lin(pl[l], pl[l].t().contiguous())          # x @ pl^T
-                L["packed"] = P
-                self.layers.append(L)
-            self.ro0 = m.layer_energy_readouts[0].readout.weight.reshape(-1).contiguous()  # [C]
-            self.ro1_w1 = m.last_layer_energy_readout.linear_1.weight.contiguous()          # [16, C]
-            self.ro1_w2 = m.last_layer_energy_readout.linear_2.weight.reshape(-1).contiguous()  # [16]
-        self._versions = versions
+                L = w.struct.layer[k]
+                L.w0 = hold(fc[0])
+                L.hid = (hold(self._pack(fc[1], 0)), hold(self._pack(fc[2], 0)))
+                L.hid_t = (hold(self._pack(fc[1], 1)), hold(self._pack(fc[2], 1)))
+                L.w3, L.w3t = hold(self._pack(fc[3], 0)), hold(self._pack(fc[3], 1))
+                L.num_gates = fc[3].shape[0]
+                w.nout.append(fc[3].shape[0])
+                L.path_weight = None if bool(torch.all(inter.tp.weight == 1)) else hold(inter.tp.weight.contiguous())
+                L.slots = tuple(inter.tp.path_counts_by_l[l] for l in range(3))
+                L.bank = hold(prod.symmetric_contractions.weight_bank())
+                ml = [inter.message_linear.weights[str(l)] / max(inter.avg_num_neighbors, 1e-8) for l in range(3)]
+                L.ml = tuple(hold(self._pack_lin(v, v.t())) for v in ml)                 # x @ ml^T
+                L.ml_b = tuple(hold(self._pack_lin(v.t(), v)) for v in ml)               # x @ ml
+                if k == 0:
+                    pl = [prod.linear[str(l)] / math.sqrt(c) for l in range(3)]
+                    L.pl = tuple(hold(self._pack_lin(v.t(), v)) for v in pl)             # x @ pl
+                    L.pl_b = tuple(hold(self._pack_lin(v, v.t())) for v in pl)           # x @ pl^T
+                else:
+                    up = [inter.linear_up.adapters[str(l)].weight for l in range(3)]
+                    L.up = tuple(hold(self._pack_lin(v, v.t())) for v in up)             # x @ up^T
+                    L.up_b = tuple(hold(self._pack_lin(v.t(), v)) for v in up)           # x @ up
+            # products of weights alone; in double precision, rounded once
+            d = lambda t: t.double()                                                     # noqa: E731
+            first, last = m.interactions
+            s = w.struct
+            s.up0_table = hold((d(emb) @ d(first.linear_up.adapters["0"].weight).t()).float().contiguous())
+            s.sc0_table = hold(torch.einsum("si,soi->so", d(emb), d(first.self_connection.weights["0"])).float().contiguous())
+            ro = m.last_layer_energy_readout
+            w1 = d(ro.linear_1.weight)                                                   # [H, C]
+            s.readout_rp = hold((w1 @ d(m.products[1].linear["0"]).t() / math.sqrt(c)).float().contiguous())
+            s.readout_rs = hold(torch.einsum("ho,soi->shi", w1, d(last.self_connection.weights["0"])).float().contiguous())
+            s.readout_w2 = hold(ro.linear_2.weight.reshape(-1).contiguous())
+            s.readout_ro0 = hold(m.layer_energy_readouts[0].readout.weight.reshape(-1).contiguous())
+            s.hidden, s.num_species = w1.shape[0], m.num_elements
+            s.num_basis, s.poly_p, s.r_max = m.number_of_basis, m.polynomial_cutoff_p, m.max_radius
+            s.species_table, s.species_table_size = hold(m.atomic_number_to_index), m.atomic_number_to_index.numel()
+        return w
 
     def _pack(self, w, transpose):
         """A [rows, 64] matrix in the shared-memory operand layout of the tcgen05 kernels."""
@@ -130,33 +175,10 @@ class ForceEngine:
         """Operand copy for out = x @ w_in_major, where w_in_major is [K, N] and w_out_major its transpose."""
         k, n = w_in_major.shape
         if k == 64:
-            return self._pack(w_out_major.contiguous(), 0), 1, n // 64
+            return self._pack(w_out_major.contiguous(), 0)
         if n != 64:
             raise ValueError("tensor-core channel linear needs a 64-wide side")
-        return self._pack(w_in_major.contiguous(), 1), k // 64, 1
-
-    def _lin(self, L, key, rows, in_t, in_off, in_mm, in_ld, out_t, out_off, out_mm, out_ld):
-        """out rows = in rows @ W on the tensor cores, reading / writing per-degree blocks in place."""
-        packed, kc, nc = L["packed"][key]
-        t0 = self._mark()
-        _lib.check(self.lib.ictc_channel_linear_tc(rows, kc, nc, in_t.data_ptr() + 4 * in_off, in_mm, in_ld,
-                                                   packed.data_ptr(), out_t.data_ptr() + 4 * out_off, out_mm, out_ld,
-                                                   self._st()), "channel_linear_tc")
-        self._done("channel_linear_tc", t0)
-
-    def _lin_blocks(self, L, key, rows, in_t, out_t, in_wide=None, out_wide=None, degrees=3):
-        """One channel linear per degree block of [rows, 9C] buffers; ``in_wide`` / ``out_wide`` = path-slot counts
-        per degree when that side is the [rows, 35C]-style slot-major tensor-product layout."""
-        c = self.c
-        in_off = out_off = 0
-        for l, (off, mm) in enumerate(_DEGREES[:degrees]):
-            i_off, i_ld = (in_off, in_t.shape[1]) if in_wide else (off * c, in_t.shape[1])
-            o_off, o_ld = (out_off, out_t.shape[1]) if out_wide else (off * c, out_t.shape[1])
-            self._lin(L, (key, l), rows * mm, in_t, i_off, mm, i_ld, out_t, o_off, mm, o_ld)
-            if in_wide:
-                in_off += in_wide[l] * mm * c
-            if out_wide:
-                out_off += out_wide[l] * mm * c
+        return self._pack(w_in_major.contiguous(), 1)
 
     # ---------------------------------------------------------------- buffers
     @staticmethod
@@ -170,173 +192,74 @@ class ForceEngine:
         g = 1 << (rows.bit_length() - 5)
         return (rows + g - 1) // g * g
 
-    def _rows(self, rows, *cols, zero=False):
-        make = torch.zeros if zero else torch.empty
-        return make(self.bucket(rows), *cols, dtype=torch.float32, device=self.dev)[:rows]
-
-    # ---------------------------------------------------------------- small launch helpers
-    def _st(self):
-        return _lib.stream(self.dev)
-
-    def _silu(self, x):
-        y = torch.empty_like(x)
-        _lib.check(self.lib.ictc_silu_forward(x.numel(), SILU_SCALE, x.data_ptr(), y.data_ptr(), self._st()), "silu")
-        return y
-
-    def _silu_bwd(self, x, dy):
-        dx = torch.empty_like(x)
-        _lib.check(self.lib.ictc_silu_backward(x.numel(), SILU_SCALE, x.data_ptr(), dy.data_ptr(), dx.data_ptr(),
-                                               self._st()), "silu_backward")
-        return dx
-
-    def _species_linear(self, x, species, w, s):
-        full = torch.mm(x, w).view(x.shape[0], s, self.c)
-        return full.gather(1, species.view(-1, 1, 1).expand(-1, 1, self.c)).squeeze(1)
-
-    def _mark(self):
-        if self.profile is None:
-            return None
-        ev = torch.cuda.Event(enable_timing=True)
-        ev.record(torch.cuda.current_stream(self.dev))
-        return ev
-
-    def _done(self, name, start):
-        if start is not None:
-            self.profile.append((name, start, self._mark()))
-
-    # ---------------------------------------------------------------- radial MLP
-    def _hidden(self, rb, L, rows, count, limit):
-        """Hidden layers of the radial MLP: pre-activations z1..z3 [count, 64]; row r reads rb[rows[r]] (rows None:
-        rb[r]); ``limit`` = device scalar with the number of rows in use when ``count`` is a capacity."""
-        pre = [self._rows(count, 64) for _ in range(3)]
-        t0 = self._mark()
-        _lib.check(self.lib.ictc_mlp_chain_forward(count, rb.shape[1], _lib.ptr(rb), _lib.ptr(rows), L["fc0"].data_ptr(),
-                                                   L["hid"][0].data_ptr(), L["hid"][1].data_ptr(), _lib.ptr(pre[0]),
-                                                   _lib.ptr(pre[1]), _lib.ptr(pre[2]), _lib.ptr(limit), self._st()),
-                   "mlp_chain_forward")
-        self._done(f"radial_mlp_hidden_forward_{L['nout']}", t0)
-        return pre
-
-    def _gate_table(self, z3, L, limit):
-        """Gates of every row of z3 (one row per edge pair, or per edge without pairing)."""
-        count, nout = z3.shape[0], L["nout"]
-        gates = self._rows(count, nout)
-        t0 = self._mark()
-        _lib.check(self.lib.ictc_gate_gemm_forward(count, nout, _lib.ptr(z3), L["w3"].data_ptr(), _lib.ptr(gates), 1,
-                                                   _lib.ptr(limit), self._st()), "gate_gemm_forward")
-        self._done(f"gate_gemm_forward_{nout}", t0)
-        return gates
-
-    def _gate_chunk(self, z3, L, buf, index, begin_ptr, end_ptr):
-        """Gates of the list entries [*begin, *end) into ``buf``: row r = act(z3[index[*begin + r]]) @ W3^T."""
-        t0 = self._mark()
-        _lib.check(self.lib.ictc_gate_gemm_forward_rows(buf.shape[0], L["nout"], _lib.ptr(z3), _lib.ptr(index), begin_ptr,
-                                                        end_ptr, L["w3"].data_ptr(), buf.data_ptr(), 1, self._st()),
-                   "gate_gemm_forward_rows")
-        self._done(f"gate_gemm_forward_{L['nout']}", t0)
-
     def _streaming(self, table_rows):
         """Are the gates streamed per chunk (True) or is the table of ``table_rows`` rows kept for both sweeps?"""
         if self.stream_gates is not None:
             return bool(self.stream_gates)
         total = torch.cuda.get_device_properties(self.dev).total_memory
-        return 4 * table_rows * sum(L["nout"] for L in self.layers) > 0.4 * total
+        return 4 * table_rows * sum(self.refresh().nout) > 0.4 * total
 
-    def _chunks(self, rows, rowptr, edges):
-        """[(first row, end row)] of the owner-row chunks and the edge capacity of a chunk buffer; also raises the
-        device-side overflow flag when a chunk holds more edges than the buffer."""
+    def _chunk_capacity(self, rows, rowptr, edges):
+        """Edge capacity of a chunk buffer of a sweep over ``rows`` owner rows (0: one pass over everything); also raises
+        the device-side overflow flag when a chunk holds more edges than the buffer."""
         if self.chunk_rows is None or self.chunk_rows >= rows:
-            return [(0, rows)], None
+            return 0
         step = self.chunk_rows
         key = (rows, step)
         if key not in self._bounds:        # built outside any stream capture: the first call is a warm-up step
             bounds = list(range(0, rows, step)) + [rows]
-            self._bounds[key] = (bounds, torch.tensor(bounds, dtype=torch.int64, device=self.dev))
-        bounds, idx = self._bounds[key]
+            self._bounds[key] = torch.tensor(bounds, dtype=torch.int64, device=self.dev)
         cap = self.bucket(int(step * (edges / max(rows, 1)) * self.chunk_margin) + 1024)
-        cuts = rowptr.index_select(0, idx)
+        cuts = rowptr.index_select(0, self._bounds[key])
         self.overflow.logical_or_(((cuts[1:] - cuts[:-1]) > cap).any())
-        return list(zip(bounds[:-1], bounds[1:])), cap
-
-    # ---------------------------------------------------------------- tensor-product sweeps
-    def _tp_forward(self, layer, L, x, sh, z3, src, rowptr, rows, e, grow, limit):
-        """Receiver-row sweep of one interaction: gates from z3 (pair rows through ``grow``), message rows out."""
-        c, lib = self.c, self.lib
-        width = (9 if layer == 0 else 35) * c
-        out = self._rows(rows, width)
-        chunks, cap = self._chunks(rows, rowptr, e)
-        if cap is None or not self._streaming(z3.shape[0]):
-            gates = self._gate_table(z3, L, limit)
-            t0 = self._mark()
-            _lib.check(lib.ictc_tp_graph_forward_shared(self._spec[layer], c, rows, e, x.data_ptr(), sh.data_ptr(),
-                                                        _lib.ptr(L["tpw"]), gates.data_ptr(), _lib.ptr(grow),
-                                                        src.data_ptr(), rowptr.data_ptr(), None, None, out.data_ptr(),
-                                                        self._st()), "tp_graph_forward")
-            self._done(f"graph_forward_l{layer}", t0)
-            return out, gates
-        buf = torch.empty(cap, L["nout"], dtype=torch.float32, device=self.dev)
-        for r0, r1 in chunks:
-            b, en = rowptr.data_ptr() + 8 * r0, rowptr.data_ptr() + 8 * r1
-            self._gate_chunk(z3, L, buf, grow, b, en)
-            t0 = self._mark()
-            _lib.check(lib.ictc_tp_graph_forward_chunk(self._spec[layer], c, r1 - r0, x.data_ptr(), sh.data_ptr(),
-                                                       _lib.ptr(L["tpw"]), buf.data_ptr(), None, b, cap, src.data_ptr(),
-                                                       b, None, None, out.data_ptr() + 4 * r0 * width, self._st()),
-                       "tp_graph_forward_chunk")
-            self._done(f"graph_forward_l{layer}", t0)
-        return out, None
-
-    def _tp_adjoint(self, layer, L, x, sh, z3, gates, dst, src_csr, v, n_rows, e, grow, grow_by_pos, need_x):
-        """Sender-row sweep: dx [n_rows, .] (optional), dsh [E, 9] and the gradient of silu(z3) per EDGE
-        (da3e [E, 64], row = edge id).  The gate gradients exist per chunk only."""
-        c, lib = self.c, self.lib
-        rowptr, order = src_csr
-        nout = L["nout"]
-        xw = x.shape[1]
-        dx = self._rows(n_rows, xw) if need_x else None
-        dsh = self._rows(e, 9)
-        da3e = self._rows(e, 64)
-        chunks, cap = self._chunks(n_rows, rowptr, e)
-        if cap is None:
-            cap = self.bucket(max(e, 1))
-        table = gates is not None            # the pair table of the forward sweep is still there
-        dg = torch.empty(cap, nout, dtype=torch.float32, device=self.dev)
-        gbuf = None if table else torch.empty(cap, nout, dtype=torch.float32, device=self.dev)
-        for s0, s1 in chunks:
-            b, en = rowptr.data_ptr() + 8 * s0, rowptr.data_ptr() + 8 * s1
-            if not table:      # the chunk's gates are recomputed for the reverse sweep
-                self._gate_chunk(z3, L, gbuf, grow_by_pos, b, en)
-            t0 = self._mark()
-            _lib.check(lib.ictc_tp_graph_adjoint_chunk(
-                self._spec[layer], c, s1 - s0, x.data_ptr() + 4 * s0 * xw, sh.data_ptr(), _lib.ptr(L["tpw"]),
-                (gates if table else gbuf).data_ptr(), _lib.ptr(grow) if table else None, 0 if table else 1,
-                None if table else b, 0 if table else cap, dst.data_ptr(), b, _lib.ptr(order), None, v.data_ptr(),
-                None if dx is None else dx.data_ptr() + 4 * s0 * xw, dsh.data_ptr(), dg.data_ptr(), b, cap, self._st()),
-                "tp_graph_adjoint_chunk")
-            self._done(f"graph_adjoint_l{layer}", t0)
-            t0 = self._mark()
-            _lib.check(lib.ictc_gate_gemm_backward_rows(cap, nout, dg.data_ptr(), b, en, _lib.ptr(order),
-                                                        L["w3t"].data_ptr(), da3e.data_ptr(), self._st()),
-                       "gate_gemm_backward_rows")
-            self._done(f"gate_gemm_backward_{nout}", t0)
-        return dx, dsh, da3e
-
-    def _hidden_bwd(self, da3e, pre, L, pairs, drb, accumulate, limit):
-        """Input gradient of the hidden layers: row u starts from da3e[rep[u]] + da3e[other[u]] (the two edges of a
-        pair) and adds / writes its result to drb[rep[u]]; without pairing row = edge."""
-        count = pre[0].shape[0]
-        pa, pb = (None, None) if pairs is None else (pairs[1], pairs[2])
-        t0 = self._mark()
-        _lib.check(self.lib.ictc_mlp_chain_backward_paired(
-            count, L["fc0"].shape[1], _lib.ptr(da3e), _lib.ptr(pa), _lib.ptr(pb), L["fc0"].data_ptr(),
-            L["hid_t"][0].data_ptr(), L["hid_t"][1].data_ptr(), _lib.ptr(pre[0]), _lib.ptr(pre[1]), _lib.ptr(pre[2]),
-            _lib.ptr(drb), _lib.ptr(pa), int(accumulate), _lib.ptr(limit), self._st()), "mlp_chain_backward")
-        self._done(f"radial_mlp_hidden_backward_{L['nout']}", t0)
+        return cap
 
     # ---------------------------------------------------------------- the sweep
+    def _run(self, s, w, plan):
+        """Workspace, then the launch sequence: at once, or stage by stage around the exchanges of ``plan``."""
+        need = int(self.lib.ictc_sweep_workspace(C.byref(s)))
+        if need < 0:
+            raise RuntimeError(f"ictc_sweep_workspace: {_lib.last_error()}")
+        if not torch.cuda.is_current_stream_capturing():
+            need = self.bucket(need >> 8) << 8
+        work = torch.empty(need, dtype=torch.uint8, device=self.dev)
+        s.work, s.work_bytes = work.data_ptr(), need
+        counts = (C.c_int64 * 2)()
+        s.host_counts = C.addressof(counts)
+        if self.profile is not None:
+            events = [torch.cuda.Event(enable_timing=True) for _ in range(2 * _MARKS)]
+            for e in events:
+                e.record()
+            handles = (C.c_void_p * (2 * _MARKS))(*[e.cuda_event for e in events])
+            labels = (C.c_int64 * _MARKS)()
+            s.host_marks, s.host_marks_capacity, s.host_mark_labels = C.addressof(handles), _MARKS, C.addressof(labels)
+        st = _lib.stream(self.dev)
+
+        def stages(mask):
+            _lib.check(self.lib.ictc_sweep_run(C.byref(s), mask, st), "ictc_sweep_run")
+
+        if plan is None:
+            stages(_ALL)
+        else:
+            n, feats, grads = s.n_owned, plan.features, plan.feature_grad
+            stages(_STAGES[0])
+            halo = plan.exchange.forward_async(feats[:n])         # the ghost rows travel while the hidden state is computed
+            stages(_STAGES[1])
+            feats[n:] = halo()
+            stages(_STAGES[2])
+            halo = plan.exchange.adjoint_async(grads[n:].contiguous())      # and back while the radial MLP is differentiated
+            stages(_STAGES[3])
+            grads[:n] += halo()
+            stages(_STAGES[4])
+        _lib.CALLS += int(counts[0])
+        if self.profile is not None:
+            for k in range(int(counts[1])):
+                kind, layer = divmod(int(labels[k]), 2)
+                self.profile.append((_LABELS[kind].format(layer=layer, nout=w.nout[layer]), events[2 * k], events[2 * k + 1]))
+
     @torch.no_grad()
     def energy_and_gradient(self, pos, species, src, dst, shifts, box, n_owned, dst_rowptr, plan=None, n_rows=None,
-                            pairs=None, row_mask=None, src_csr=None):
+                            pairs=None, row_mask=None, src_csr=None, out=None, sign=1.0):
         """pos [N_local,3] (owned rows first), species [N_local] (index), edges sorted by receiver with all
         receivers < n_owned, dst_rowptr [n_owned+1].  Returns (energy of owned atoms, dE/dpos [N_local,3],
         per-atom energies [n_owned]).  ``n_rows`` < N_local marks trailing rows of ``pos`` as padding: they may
@@ -346,119 +269,90 @@ class ForceEngine:
         ``plan`` (an exchange plan of ``mace_ictc.domain``) refreshes the ghost rows between the interactions.
         ``row_mask`` [n_owned] (0 / 1) leaves padding rows among the owned rows out of the energy (and hence of
         the gradient: a padding row has no edges).  ``src_csr`` = (row offsets, edge ids) of the senders where the caller
-        has them."""
-        self.refresh()
-        m, c, lib, dev = self.model, self.c, self.lib, self.dev
+        has them.  ``out`` = (energy [1], gradient [N_local,3]) receives the results, the gradient times ``sign``."""
+        w, dev = self.refresh(), self.dev
         n_local, e = (pos.shape[0] if n_rows is None else int(n_rows)), int(src.numel())
-        species = species[:n_local]
-        st = self._st()
-        L0, L1 = self.layers
-        nb, pcut, rmax = m.number_of_basis, m.polynomial_cutoff_p, m.max_radius
         with _lib.on_device(dev):
-            # ---- edge geometry
-            sh = self._rows(e, 9)
-            rb = self._rows(e, nb)
-            unit = self._rows(e, 3)
-            length = self._rows(e)
-            box_c = (C.c_float * 3)(*[float(b) for b in box])
-            _lib.check(lib.ictc_edge_geometry_forward(pos.data_ptr(), _lib.ptr(src), _lib.ptr(dst), _lib.ptr(shifts),
-                                                      box_c, rmax, nb, pcut, e, _lib.ptr(sh), _lib.ptr(rb),
-                                                      _lib.ptr(unit), _lib.ptr(length), st), "edge_geometry_forward")
             if src_csr is None:
                 src_csr = build_csr(src, n_local, assume_sorted=False)
-            grow = None if pairs is None else pairs[0]
-            rep = None if pairs is None else pairs[1]               # the MLP kernels gather / scatter the pair rows
-            live = pairs[3] if (pairs is not None and len(pairs) > 3) else None
-            count = e if pairs is None else int(rep.numel())
-            chunked = (self.chunk_rows is not None and self.chunk_rows < max(n_owned, n_local)
-                       and self._streaming(count))
-            # gate row of the edge at every position of the sender order (reverse sweep of the streamed mode)
-            grow_by_pos = None
-            if chunked:
-                grow_by_pos = src_csr[1][:e] if grow is None else grow.index_select(0, src_csr[1][:e])
-            sp_owned = species[:n_owned]
-            s_count = self.emb.shape[0]
-            # ---- layer 0
-            x0 = self.emb.index_select(0, species)                               # [N_local, C]
-            u0 = self._rows(n_local, c)
-            self._lin(L0, ("up", 0), n_local, x0, 0, 1, c, u0, 0, 1, c)
-            pre0 = self._hidden(rb, L0, rep, count, live)
-            M0, g0 = self._tp_forward(0, L0, u0, sh, pre0[2], src, dst_rowptr, n_owned, e, grow, live)   # [n, 9C]
-            m0 = self._rows(n_owned, 9 * c)
-            self._lin_blocks(L0, "ml", n_owned, M0, m0)
-            sc0 = self._species_linear(x0[:n_owned], sp_owned, L0["sc_fwd"], s_count)
-            call0 = _ScCall(c, 2, s_count, sp_owned, True)
-            y0 = call0.forward(m0, L0["bank"])                                    # [n, 9C]
-            h1 = self._rows(n_owned, 9 * c)
-            self._lin_blocks(L0, "pl", n_owned, y0, h1)
-            h1[:, :c] += sc0
-            e0 = torch.mv(h1[:, :c], self.ro0)
-            # ---- halo: the ghost rows travel while the layer-1 hidden state (which needs only the radial basis) is computed
-            halo = None if plan is None else plan.forward_async(h1)
-            pre1 = self._hidden(rb, L1, rep, count, live)
-            h1_full = h1 if plan is None else torch.cat((h1, halo()), 0)
-            # ---- layer 1
-            u1 = self._rows(n_local, 9 * c)
-            self._lin_blocks(L1, "up", n_local, h1_full, u1)
-            M1, g1 = self._tp_forward(1, L1, u1, sh, pre1[2], src, dst_rowptr, n_owned, e, grow, live)   # [n, 35C]
-            m1 = self._rows(n_owned, 9 * c)
-            self._lin_blocks(L1, "ml", n_owned, M1, m1, in_wide=L1["counts"])     # slot-major block contracted in place
-            del M1
-            sc1 = self._species_linear(h1[:, :c].contiguous(), sp_owned, L1["sc_fwd"], s_count)
-            call1 = _ScCall(c, 0, s_count, sp_owned, True)
-            y1 = call1.forward(m1, L1["bank"])                                    # [n, C]
-            h2 = torch.mm(y1, L1["pl0"]) + sc1
-            z = torch.mm(h2, self.ro1_w1.t())
-            a = self._silu(z)
-            e1 = torch.mv(a, self.ro1_w2)
-            atomic = e0 + e1
-            if row_mask is not None:
-                atomic = atomic * row_mask
-            energy = atomic.sum()
-
-            # ================= reverse sweep (dE = 1 for every owned atom) =================
-            da = self.ro1_w2.unsqueeze(0).expand(n_owned, -1).contiguous()
-            if row_mask is not None:
-                da = da * row_mask.unsqueeze(1)
-            dz = self._silu_bwd(z, da)
-            dh2 = torch.mm(dz, self.ro1_w1)                                        # [n, C]
-            dy1 = torch.mm(dh2, L1["pl0_t"])
-            dm1, _ = call1.adjoint(m1, L1["bank"], dy1, (True, False))             # [n, 9C]
-            v1 = self._rows(n_owned, 35 * c)
-            self._lin_blocks(L1, "ml_b", n_owned, dm1, v1, out_wide=L1["counts"])
-            du1, dsh1, da3e = self._tp_adjoint(1, L1, u1, sh, pre1[2], g1, dst, src_csr, v1, n_local, e, grow,
-                                               grow_by_pos, True)
-            del v1, g1
-            dh1_full = self._rows(n_local, 9 * c)
-            self._lin_blocks(L1, "up_b", n_local, du1, dh1_full)
-            # the ghost rows' cotangents travel back while the layer-1 MLP is differentiated
-            halo = None if plan is None else plan.adjoint_async(dh1_full[n_owned:].contiguous())
-            drb = self._rows(e, nb, zero=True)
-            self._hidden_bwd(da3e, pre1, L1, pairs, drb, False, live)
-            del pre1
-            dh1 = dh1_full[:n_owned]
+            energy, grad = out if out is not None else (torch.empty(1, dtype=torch.float32, device=dev),
+                                                        torch.empty(n_local, 3, dtype=torch.float32, device=dev))
+            atomic = torch.empty(n_owned, dtype=torch.float32, device=dev)
+            status = torch.empty(3, dtype=torch.int32, device=dev)
+            s = _lib.Sweep.from_buffer_copy(w.struct)
+            s.n_local, s.n_owned, s.edges, s.graphs, s.mask_atomic, s.gradient_sign = n_local, n_owned, e, 1, 1, sign
+            s.box = tuple(float(b) for b in box)
+            s.pos, s.src, s.dst, s.shifts = pos.data_ptr(), src.data_ptr(), dst.data_ptr(), _lib.ptr(shifts)
+            s.species, s.status = species.data_ptr(), status.data_ptr()
+            s.dst_rowptr, s.src_rowptr, s.src_order = dst_rowptr.data_ptr(), src_csr[0].data_ptr(), _lib.ptr(src_csr[1])
+            rows = e
+            if pairs is not None:
+                s.gate_row, s.rep, s.other = (t.data_ptr() for t in pairs[:3])
+                s.live = pairs[3].data_ptr() if len(pairs) > 3 else None
+                rows = int(pairs[1].numel())
+            s.pair_rows = rows
+            s.row_mask = _lib.ptr(row_mask)
+            if self.chunk_rows is not None and self.chunk_rows < max(n_owned, n_local):
+                s.chunk_rows, s.stream_gates = self.chunk_rows, int(self._streaming(rows))
+                s.chunk_capacity_dst = self._chunk_capacity(n_owned, dst_rowptr, e) or self.bucket(max(e, 1))
+                s.chunk_capacity_src = self._chunk_capacity(n_local, src_csr[0], e) or self.bucket(max(e, 1))
+            s.energy, s.atomic, s.gradient = energy.data_ptr(), atomic.data_ptr(), grad.data_ptr()
+            halo = None
             if plan is not None:
-                dh1 = dh1 + halo()
-            else:
-                dh1 = dh1.clone()
-            full = torch.mm(dh2, L1["sc_bwd"]).view(n_owned, s_count, c)
-            dh1[:, :c] += full.gather(1, sp_owned.view(-1, 1, 1).expand(-1, 1, c)).squeeze(1)
-            dh1[:, :c] += self.ro0 if row_mask is None else self.ro0.unsqueeze(0) * row_mask.unsqueeze(1)
-            dy0 = self._rows(n_owned, 9 * c)
-            self._lin_blocks(L0, "pl_b", n_owned, dh1, dy0)
-            dm0, _ = call0.adjoint(m0, L0["bank"], dy0, (True, False))
-            v0 = self._rows(n_owned, 9 * c)
-            self._lin_blocks(L0, "ml_b", n_owned, dm0, v0)
-            _, dsh0, da3e = self._tp_adjoint(0, L0, u0, sh, pre0[2], g0, dst, src_csr, v0, n_local, e, grow,
-                                             grow_by_pos, False)
-            self._hidden_bwd(da3e, pre0, L0, pairs, drb, True, live)
-            dsh1 += dsh0
-            dvec = self._rows(e, 3)
-            _lib.check(lib.ictc_edge_geometry_backward(_lib.ptr(unit), _lib.ptr(length), rmax, nb, pcut, e,
-                                                       _lib.ptr(dsh1), _lib.ptr(drb), _lib.ptr(dvec), st),
-                       "edge_geometry_backward")
-            grad = self._rows(n_local, 3)
-            _lib.check(lib.ictc_position_gradient(n_local, n_owned, dst_rowptr.data_ptr(), src_csr[0].data_ptr(),
-                                                  _lib.ptr(src_csr[1]), _lib.ptr(dvec), grad.data_ptr(), st),
-                       "position_gradient")
-        return energy, grad, atomic
+                halo = _Halo(plan, n_local, 9 * self.c, dev)
+                s.features, s.feature_grad = halo.features.data_ptr(), halo.feature_grad.data_ptr()
+            self._run(s, w, halo)
+        return energy[0], grad, atomic
+
+    @torch.no_grad()
+    def energy_and_forces(self, pos, numbers, batch, src, dst, shifts, cell, row_mask, check):
+        """(energy per graph, forces, per-atom energies) of a graph whose edges the caller has built, in any order.
+        ``check`` raises ValueError on an atomic number outside the model or an edge index outside the graph."""
+        w, dev = self.refresh(), self.dev
+        n, graphs = pos.shape[0], cell.shape[0]
+        with _lib.on_device(dev):
+            energy = torch.empty(graphs, dtype=torch.float32, device=dev)
+            forces = torch.empty(n, 3, dtype=torch.float32, device=dev)
+            atomic = torch.empty(n, dtype=torch.float32, device=dev)
+            species = torch.empty(n, dtype=torch.int64, device=dev)
+            status = torch.zeros(3, dtype=torch.int32, device=dev)
+            s = _lib.Sweep.from_buffer_copy(w.struct)
+            s.n_local = s.n_owned = n
+            s.edges = s.pair_rows = src.numel()
+            s.graphs, s.gradient_sign = graphs, -1.0
+            s.pos, s.src, s.dst, s.shifts = pos.data_ptr(), src.data_ptr(), dst.data_ptr(), shifts.data_ptr()
+            s.cells, s.batch, s.numbers = cell.data_ptr(), batch.data_ptr(), numbers.data_ptr()
+            s.species, s.status, s.row_mask = species.data_ptr(), status.data_ptr(), _lib.ptr(row_mask)
+            s.energy, s.atomic, s.gradient = energy.data_ptr(), atomic.data_ptr(), forces.data_ptr()
+            if check:
+                flags, event = _status_mailbox(dev)
+                s.host_status, s.host_status_event = flags.data_ptr(), event.cuda_event
+            self._run(s, w, None)
+            if check:
+                event.synchronize()
+                unknown, by_dst, by_src = flags.tolist()
+                if unknown:
+                    raise ValueError(f"Encountered atomic numbers outside {self.model.atomic_numbers}")
+                if by_dst < 0 or by_src < 0:
+                    raise ValueError("edge index outside [0, num_nodes)")
+        return energy, forces, atomic
+
+
+class _Halo:
+    """Exchange plan and the two feature buffers whose ghost rows it fills."""
+
+    def __init__(self, exchange, rows, width, device):
+        self.exchange = exchange
+        self.features = torch.empty(rows, width, dtype=torch.float32, device=device)
+        self.feature_grad = torch.empty(rows, width, dtype=torch.float32, device=device)
+
+
+def _status_mailbox(device):
+    """Pinned words and an event of this thread and device: a sweep's status is copied early and read when the sweep has
+    been queued, so that the host does not wait for the sweep itself."""
+    boxes = _local.__dict__.setdefault("boxes", {})
+    if device not in boxes:
+        event = torch.cuda.Event()
+        event.record()
+        boxes[device] = (torch.zeros(3, dtype=torch.int32, pin_memory=True), event)
+    return boxes[device]

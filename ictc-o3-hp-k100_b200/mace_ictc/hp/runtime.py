@@ -47,6 +47,27 @@ def create_model(*, channels=64, lmax=3, edge_lmax=None, num_interactions=2, cor
     return model.to(device=device, dtype=dtype)
 
 
+def _force_engine(model, tensors):
+    """The tape-free engine for an inference call, or None where the autograd route has to answer: other widths or
+    depths, forward hooks, tensors of another type or device, tracing and autocast (which that route refuses)."""
+    if type(model) is not MaceIctcModel or model.channels != 64 or len(model.interactions) != 2:
+        return None
+    positions = tensors[0]
+    if (not all(t.is_cuda and t.device == positions.device for t in tensors) or positions.dtype != torch.float32
+            or tensors[3].numel() == 0 or positions.shape[0] == 0 or model.node_embedding.weight.dtype != torch.float32
+            or torch.is_autocast_enabled("cuda") or torch._C._are_functorch_transforms_active()
+            or torch.compiler.is_compiling() or any(type(t) is not torch.Tensor for t in tensors[1:])):
+        return None
+    engine = model.__dict__.get("_force_engine")
+    if engine is None or engine.dev != positions.device:
+        from ..engine import ForceEngine
+        if model.node_embedding.weight.device != positions.device:
+            return None
+        engine = ForceEngine(model)
+        model.__dict__["_force_engine"] = engine
+    return None if engine.hooked() else engine
+
+
 def energy_and_forces(model, positions, atomic_numbers, batch, edge_src, edge_dst, edge_shifts, cell, *,
                       training=False, owned_mask=None):
     """Energies per graph [B], forces [N, 3] = -dE/dpositions and per-atom energies [N] of a graph whose edges
@@ -70,6 +91,16 @@ def energy_and_forces(model, positions, atomic_numbers, batch, edge_src, edge_ds
     if owned_mask is not None:
         if tuple(owned_mask.shape) != (count,) or owned_mask.requires_grad:
             raise ValueError(f"owned_mask: expected a constant tensor of shape [{count}]")
+    if not training:
+        engine = _force_engine(model, (positions, atomic_numbers, batch, edge_src, edge_dst, edge_shifts, cell))
+        if engine is not None:
+            dtype = torch.float32
+            mask = None if owned_mask is None else owned_mask.to(dtype).contiguous()
+            energy, forces, per_atom = engine.energy_and_forces(
+                positions.detach().contiguous(), atomic_numbers.long().contiguous(), batch.long().contiguous(),
+                edge_src.long().contiguous(), edge_dst.long().contiguous(), edge_shifts.detach().to(dtype).contiguous(),
+                cell.detach().to(dtype).contiguous(), mask, not model.skip_input_validation)
+            return {"energy": energy, "forces": forces, "atomic_energy": per_atom}
     with torch.enable_grad():
         coords = positions if positions.requires_grad else positions.detach().requires_grad_(True)
         per_atom = model(coords, atomic_numbers, batch, edge_src, edge_dst, edge_shifts, cell)

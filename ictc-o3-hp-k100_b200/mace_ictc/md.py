@@ -347,14 +347,12 @@ class MolecularDynamics:
         if self.engine is not None:
             pairs = (nl.gate_row[:edges], nl.rep[:num_pairs], nl.other[:num_pairs]) if self.share_gates else None
             self.num_gate_rows = num_pairs if pairs is not None else edges
-            energy, grad, _ = self.engine.energy_and_gradient(self.pos, self.species, src, dst, shifts, box, n, rowptr,
-                                                              pairs=pairs, src_csr=nl.sender_csr())
-            if self._static is not None:            # keep the buffers the recorded graph reads and writes
-                self._static["energy"].copy_(energy.reshape(1))
-                self.forces.copy_(grad).neg_()
-            else:
-                self.energy = energy
-                self.forces = (-grad).contiguous()
+            # a recorded graph reads and writes fixed buffers: an eager step in between keeps to them
+            out = (self._static["energy"], self.forces) if self._static is not None else None
+            energy, forces, _ = self.engine.energy_and_gradient(self.pos, self.species, src, dst, shifts, box, n, rowptr,
+                                                                pairs=pairs, src_csr=nl.sender_csr(), out=out, sign=-1.0)
+            if out is None:
+                self.energy, self.forces = energy, forces
             return self.forces
         topo = Topology(src, dst, n, dst_sorted=True)
         topo._by_dst = (rowptr, None)
@@ -586,12 +584,9 @@ class MolecularDynamics:
         st["pos_ext"][:n].copy_(self.pos)
         st["nl"].build(st["pos_ext"])
         nl = st["nl"]
-        energy, grad, _ = self.engine.energy_and_gradient(st["pos_ext"], st["species_ext"], nl.src, nl.dst, nl.shifts,
-                                                          self.box.tolist(), n, nl.rowptr, n_rows=n,
-                                                          pairs=nl.pairs() if self.share_gates else None,
-                                                          src_csr=nl.sender_csr())
-        st["energy"].copy_(energy.reshape(1))
-        self.forces.copy_(grad).neg_()
+        self.engine.energy_and_gradient(st["pos_ext"], st["species_ext"], nl.src, nl.dst, nl.shifts, self.box.tolist(), n,
+                                        nl.rowptr, n_rows=n, pairs=nl.pairs() if self.share_gates else None,
+                                        src_csr=nl.sender_csr(), out=(st["energy"], self.forces), sign=-1.0)
         self._kick(False)
 
     def run(self, steps, check_every=25, margin=1.10, on_step=None):

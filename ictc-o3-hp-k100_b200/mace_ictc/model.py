@@ -267,6 +267,11 @@ class MaceIctcModel(nn.Module):
         self.assume_edges_within_radius = False
         self.skip_input_validation = False
 
+    def __getstate__(self):
+        state = self.__dict__.copy()
+        state.pop("_force_engine", None)       # laid-out weights of the inference route: rebuilt on the first call
+        return state
+
     def species_index(self, atomic_numbers):
         idx = self.atomic_number_to_index[atomic_numbers.long()]
         if not self.skip_input_validation and bool(torch.any(idx < 0)):

@@ -390,6 +390,79 @@ int ictc_sc_second(int lmax, int target_lmax, int channels, int64_t num_nodes, i
                    const float* x, const int64_t* species, const float* w, const float* gy, const float* hx,
                    const float* hw, float* dgy, float* dx, float* dw, void* scratch, void* stream);
 
+/* ------------------------------------------------------------------ force sweep
+ * Energy and position gradient of the two-interaction C64 / lmax 2 model as one launch sequence (the force path of
+ * mace_ictc/hp/runtime.py:82-111).  All pointers are device pointers; edges need not be sorted when dst_order is given or
+ * when both row-offset pointers are NULL (the sweep then builds both CSRs).  Weight matrices marked "packed" come from
+ * ictc_gate_pack_weights. */
+typedef struct {
+  const float* w0;              /* first radial layer [64, num_basis] */
+  const float* hid[2];          /* packed hidden layers, forward and (hid_t) transposed use */
+  const float* hid_t[2];
+  const float* w3;              /* packed last layer, forward and transposed use */
+  const float* w3t;
+  const float* path_weight;     /* [P, 64] or NULL (all one) */
+  const float* up[3];           /* packed linear_up per degree (second interaction), and its transposed use */
+  const float* up_b[3];
+  const float* ml[3];           /* packed message linear */
+  const float* ml_b[3];
+  const float* pl[3];           /* packed product linear (first interaction) */
+  const float* pl_b[3];
+  const float* bank;            /* symmetric-contraction weights [S, NW, 64] */
+  int64_t num_gates;            /* P * 64 */
+  int64_t slots[3];             /* path slots per output degree */
+} ictc_sweep_layer;
+
+typedef struct {
+  int64_t n_local, n_owned, edges, pair_rows, num_species, graphs;
+  int64_t chunk_rows, chunk_capacity_dst, chunk_capacity_src, stream_gates;   /* chunk_rows 0: whole tables */
+  int64_t num_basis, poly_p, hidden, mask_atomic;
+  double r_max, box[3], gradient_sign;
+  const float* pos;             /* [>= n_local, 3] */
+  const int64_t *src, *dst;     /* [edges] */
+  const float* shifts;          /* [edges, 3] lattice units, or NULL */
+  const float* cells;           /* [graphs, 3, 3], or NULL: box */
+  const int64_t* batch;         /* graph of an atom, or NULL: one graph */
+  const int64_t* numbers;       /* atomic numbers [n_local], or NULL: species holds the indices */
+  const int64_t* species_table;
+  int64_t species_table_size;
+  int64_t* species;             /* [n_local], output when numbers is given */
+  const int64_t *dst_rowptr, *dst_order, *src_rowptr, *src_order;
+  const int64_t *gate_row, *rep, *other, *live;      /* radial pairing, or NULL; live: pair rows in use, or NULL */
+  const float* row_mask;        /* [n_owned] or NULL */
+  float* features;              /* [n_local, 576]: output of the first interaction, owned rows first (NULL: internal) */
+  float* feature_grad;          /* [n_local, 576]: its gradient (NULL: internal) */
+  float* energy;                /* [graphs] */
+  float* atomic;                /* [n_owned] */
+  float* gradient;              /* [n_local, 3], times gradient_sign */
+  int32_t* host_status;         /* host (pinned), or NULL: the three status words are copied here early ... */
+  void* host_status_event;      /* ... and this cudaEvent_t is recorded behind the copy */
+  int32_t* status;              /* bit 0: atomic number outside the model; word 1, 2: CSR flags (-1: edge index outside) */
+  const float* up0_table;       /* [S, 64] embedding x linear_up of the first interaction */
+  const float* sc0_table;       /* [S, 64] embedding x self connection */
+  const float *readout_rp, *readout_rs, *readout_w2, *readout_ro0;
+  ictc_sweep_layer layer[2];
+  void* work;
+  int64_t work_bytes;
+  void** host_marks;            /* host array of cudaEvent_t pairs around the heavy launches, or NULL */
+  int64_t host_marks_capacity;  /* pairs */
+  int64_t* host_mark_labels;    /* host: label of every pair used */
+  int64_t* host_counts;         /* host: [0] launches, [1] pairs used (added to) */
+} ictc_sweep;
+
+/* Bytes of workspace the sweep needs for these sizes. */
+int64_t ictc_sweep_workspace(const ictc_sweep* host_args);
+/* Stages (bits of `stages`), to be run in this order; a host that exchanges ghost rows does so between them:
+ *   1  species, geometry, first interaction up to `features` of the owned rows
+ *   2  hidden radial layers of the second interaction          (ghost rows of `features` due afterwards)
+ *   4  second interaction, readouts, their adjoint up to `feature_grad` (all rows)
+ *   8  radial adjoint of the second interaction                (ghost contributions to `feature_grad` due afterwards)
+ *   16 adjoint of the first interaction, position gradient
+ * Running all five at once (31) merges launches of the two interactions. */
+int ictc_sweep_run(const ictc_sweep* host_args, int stages, void* stream);
+/* sizeof(ictc_sweep), for bindings that mirror the struct. */
+int64_t ictc_sweep_struct_bytes(void);
+
 #ifdef __cplusplus
 }
 #endif

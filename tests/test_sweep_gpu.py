@@ -1,0 +1,140 @@
+"""The native force sweep behind ``energy_and_forces`` and the MD drivers: against the autograd route (every edge order,
+general cells, batches of graphs, masks, sizes around the kernels' blocks), stage by stage around an exchange of ghost
+rows, after parameter updates, and its error cases."""
+import copy
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+TOL = 1e-5          # fp32 against fp32 over two layers: the two routes each hold 1e-5 against the float64 oracle
+ELEMENTS = (1, 6, 8)
+
+
+def _model(seed=1):
+    from mace_ictc.hp import create_model
+    torch.manual_seed(seed)
+    model = create_model(channels=64, lmax=2, cutoff=4.5, avg_num_neighbors=32.0)
+    with torch.no_grad():
+        for name, p in model.named_parameters():
+            if "linear_up" in name or "self_connection" in name:
+                p.add_(0.05 * torch.randn_like(p))
+    return model
+
+
+def _autograd(model, graph, mask=None):
+    """The tape route (what training uses)."""
+    from mace_ictc.hp import energy_and_forces
+    return {k: v.detach() for k, v in energy_and_forces(model, *graph, training=True, owned_mask=mask).items()}
+
+
+def _close(got, want, tol=TOL):
+    for key in want:
+        err = float((got[key] - want[key]).abs().max()) / float(want[key].abs().max())
+        assert err < tol, (key, err)
+
+
+def _graph(rng, sizes, skewed):
+    """Random gases, one cell each (skewed or rectangular), every edge within 5 A: some lie beyond the cutoff."""
+    pos, z, batch, src, dst, shifts, cells = [], [], [], [], [], [], []
+    first = 0
+    for g, n in enumerate(sizes):
+        side = max(10.0, (n / 0.05) ** (1.0 / 3.0))
+        cell = np.diag([side, side * 1.1, side * 0.95])
+        if skewed:
+            cell += rng.normal(0.0, 0.6, (3, 3))
+        p = rng.random((n, 3)) @ cell
+        images = np.stack(np.meshgrid(*[[-1, 0, 1]] * 3, indexing="ij"), -1).reshape(-1, 3)
+        for image in images:
+            vec = p[None, :, :] - p[:, None, :] + image @ cell           # [src, dst]
+            near = (np.linalg.norm(vec, axis=-1) < 5.0) & (np.linalg.norm(vec, axis=-1) > 0.7)
+            j, i = np.nonzero(near)
+            src.append(j + first)
+            dst.append(i + first)
+            shifts.append(np.repeat(image[None], len(j), 0))
+        pos.append(p)
+        z.append(rng.choice(ELEMENTS, n))
+        batch.append(np.full(n, g))
+        cells.append(cell)
+        first += n
+    src, dst, shifts = np.concatenate(src), np.concatenate(dst), np.concatenate(shifts)
+    order = rng.permutation(len(src))
+    t = lambda a, d: torch.as_tensor(np.asarray(a), dtype=d, device="cuda")       # noqa: E731
+    return [t(np.concatenate(pos), torch.float32), t(np.concatenate(z), torch.int64), t(np.concatenate(batch), torch.int64),
+            t(src[order], torch.int64), t(dst[order], torch.int64), t(shifts[order], torch.int64), t(cells, torch.float32)]
+
+
+@pytest.mark.parametrize("sizes,skewed", [((2,), False), ((33,), True), ((70, 1, 40), True), ((129,) * 3, False), ((700,), True)])
+def test_against_the_autograd_route(sizes, skewed):
+    from mace_ictc.hp import energy_and_forces
+    model = _model()
+    graph = _graph(np.random.default_rng(sum(sizes)), sizes, skewed)
+    _close(energy_and_forces(model, *graph), _autograd(model, graph))
+    order = torch.argsort(graph[4], stable=True)
+    for k in (3, 4, 5):
+        graph[k] = graph[k][order]
+    model.preserve_edge_order = True
+    model.skip_input_validation = True
+    mask = (torch.arange(sum(sizes), device="cuda") % 3 != 1).float()
+    want = _autograd(model, graph, mask)
+    got = energy_and_forces(model, *graph, owned_mask=mask)
+    _close(got, want)
+    assert torch.equal(got["forces"], energy_and_forces(model, *graph, owned_mask=mask)["forces"])
+
+
+def test_parameter_updates_replacement_copies_and_hooks():
+    from mace_ictc.hp import energy_and_forces
+    model = _model()
+    graph = _graph(np.random.default_rng(3), (50,), False)
+    before = energy_and_forces(model, *graph)
+    twin = copy.deepcopy(model)
+    with torch.no_grad():
+        model.products[0].linear["1"].mul_(1.5)
+    _close(energy_and_forces(model, *graph), _autograd(model, graph))
+    model.interactions[1].fc[0].weight = torch.nn.Parameter(model.interactions[1].fc[0].weight * 0.9)
+    _close(energy_and_forces(model, *graph), _autograd(model, graph))
+    model.interactions[0].avg_num_neighbors = 20.0
+    after = energy_and_forces(model, *graph)
+    _close(after, _autograd(model, graph))
+    assert float((after["forces"] - before["forces"]).abs().max()) > 1e-3 * float(before["forces"].abs().max())
+    assert torch.equal(energy_and_forces(twin, *graph)["forces"], before["forces"])
+    seen = []
+    handle = model.products[1].register_forward_hook(lambda *_: seen.append(1))
+    energy_and_forces(model, *graph)
+    assert seen == [1]
+    handle.remove()
+
+
+def test_unknown_atoms_and_bad_edges_raise_and_the_next_call_works():
+    from mace_ictc.hp import energy_and_forces
+    model = _model()
+    graph = _graph(np.random.default_rng(4), (40,), False)
+    good = energy_and_forces(model, *graph)
+    for index, value in ((1, 7), (1, 500), (3, 40), (4, -1)):
+        bad = list(graph)
+        bad[index] = bad[index].clone()
+        bad[index][5] = value
+        with pytest.raises(ValueError):
+            energy_and_forces(model, *bad)
+    assert torch.equal(energy_and_forces(model, *graph)["forces"], good["forces"])
+
+
+@pytest.mark.parametrize("chunk_rows", [None, 300])
+def test_stages_around_a_ghost_exchange(chunk_rows):
+    """One rank that owns the whole box and sees its periodic images as ghost rows: same forces as the periodic list."""
+    from mace_ictc import synthetic as S
+    from mace_ictc.md import MolecularDynamics
+    model = _model()
+    pos, box, species = S.jittered_lattice(8, 9, 7, 2.15, 0.1, 3)
+    z = np.array(ELEMENTS)[species]
+    whole = MolecularDynamics(model, pos, z, box, seed=2)
+    want = whole.gather(whole.compute_forces())
+    split = MolecularDynamics(model, pos, z, box, seed=2, skin=1.0, chunk_rows=chunk_rows, stream_gates=True)
+    split.engine.chunk_margin = 12.0         # ghost rows have few edges, so a chunk of owned rows is far above the mean
+    split._setup_distributed()
+    split._forces_distributed()
+    got = split.gather(split.forces)
+    assert float((got - want).abs().max()) < TOL * float(want.abs().max())
+    assert abs(float(split._dist["energy"]) - float(whole.energy)) < 1e-6 * abs(float(whole.energy))
+    assert int(split.engine.overflow.item()) == 0
