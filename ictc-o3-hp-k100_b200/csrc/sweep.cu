@@ -9,6 +9,7 @@
 //   * the hidden radial layers of both interactions share a launch in each direction (mlp_chain.cu);
 //   * products of weight matrices that no input depends on (embedding x linear_up, embedding x self connection,
 //     readout x product linear) are formed when the weights are laid out, not per atom.
+#include <exception>
 #include <vector>
 #include "csr.cuh"
 #include "gate_gemm.cuh"
@@ -32,7 +33,8 @@ struct EmbedArgs {
   float* u0;                   // [n, 64]
   double* energy;              // [graphs], cleared here
   int64_t graphs, n;
-  int* status;                 // 1: an atomic number outside the model
+  const int64_t* batch;        // or null
+  int* status;                 // bit 0: an atomic number outside the model, bit 1: a graph index outside [0, graphs)
 };
 
 __global__ void embed_kernel(EmbedArgs a) {
@@ -52,7 +54,35 @@ __global__ void embed_kernel(EmbedArgs a) {
   } else {
     s = a.species[row];
   }
+  if (a.batch && (i & 15) == 1) {
+    const int64_t b = ldg(a.batch + row);
+    if (b < 0 || b >= a.graphs) atomicOr(a.status, 2);
+  }
   reinterpret_cast<float4*>(a.u0)[i] = __ldg(reinterpret_cast<const float4*>(a.up + s * kC) + (i & 15));
+}
+
+// Are the parameters still what the weights were laid out from?  A version counter does not see a write through
+// `parameter.data`, so every word is compared (0.25 M words: 3 us, hidden behind the host's next launches).
+constexpr int kWatchWords = 2048, kWatchThreads = 256;
+
+__global__ void __launch_bounds__(kWatchThreads) watch_kernel(const int64_t* __restrict__ tiles, const int* __restrict__ copy,
+                                                              int* status) {
+  const int64_t t = blockIdx.x;
+  const int* now = reinterpret_cast<const int*>(ldg(tiles + 2 * t));
+  const int words = int(ldg(tiles + 2 * t + 1));
+  bool differ = false;
+#pragma unroll
+  for (int k = 0; k < kWatchWords / kWatchThreads; ++k) {
+    const int i = threadIdx.x + k * kWatchThreads;
+    if (i < words) differ |= now[i] != copy[t * kWatchWords + i];
+  }
+  if (__syncthreads_or(differ) && threadIdx.x == 0) atomicOr(status, 4);
+}
+
+// Graph of an atom; an index outside the batch is flagged by embed_kernel and read as graph 0.
+__device__ __forceinline__ int64_t graph_of(const int64_t* batch, int64_t atom, int64_t graphs) {
+  const int64_t b = ldg(batch + atom);
+  return b >= 0 && b < graphs ? b : 0;
 }
 
 // ------------------------------------------------------------------------------------------------ geometry
@@ -64,6 +94,7 @@ struct GeoArgs {
   float box[3];
   const float* cells;          // [graphs, 3, 3] or null: `box`
   const int64_t* batch;        // graph of an atom (null: graph 0)
+  int64_t graphs;
   float r_max;
   int num_basis, p;
   int64_t E;
@@ -117,7 +148,7 @@ __global__ void __launch_bounds__(kGeoThreads) geometry_kernel(GeoArgs a) {
     if (a.shifts) {
       const float s0 = a.shifts[3 * e], s1 = a.shifts[3 * e + 1], s2 = a.shifts[3 * e + 2];
       if (a.cells) {
-        const float* cell = a.cells + 9 * (a.batch ? ldg(a.batch + j) : 0);
+        const float* cell = a.cells + 9 * (a.batch ? graph_of(a.batch, j, a.graphs) : 0);
 #pragma unroll
         for (int k = 0; k < 3; ++k) v[k] += s0 * ldg(cell + k) + s1 * ldg(cell + 3 + k) + s2 * ldg(cell + 6 + k);
       } else {
@@ -252,6 +283,7 @@ struct TailArgs {
   int H;
   const float* mask;           // [n] or null
   const int64_t* batch;        // or null
+  int64_t graphs;
   int mask_atomic;
   float* atomic;               // [n]
   double* energy;              // [graphs]
@@ -313,7 +345,7 @@ __global__ void __launch_bounds__(kTailWarps * 32) tail_kernel(TailArgs a) {
     if (lane == 0) {
       a.atomic[n] = a.mask_atomic ? e * m : e;
       if (a.batch) {
-        const int64_t b = ldg(a.batch + n);
+        const int64_t b = graph_of(a.batch, n, a.graphs);
         if (b != graph && graph >= 0) {
           atomicAdd(a.energy + graph, sum);
           sum = 0.0;
@@ -479,11 +511,16 @@ int Runner::run() {
   double* energy = buffer<double>(p.graphs);
   float* u0 = buffer(N * kC);
   call(1, -1, 1, [&] {
-    EmbedArgs a{p.numbers, p.species_table, p.species_table_size, p.species, p.up0_table, u0, energy, p.graphs, N, p.status};
+    EmbedArgs a{p.numbers, p.species_table, p.species_table_size, p.species, p.up0_table, u0, energy, p.graphs, N, p.batch, p.status};
     const int64_t threads = 16 * N > p.graphs ? 16 * N : p.graphs;
     if (threads > 0) embed_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(a);
     return finish_launch("sweep_embed");
   });
+  if (p.watch_count > 0)
+    call(1, -1, 1, [&] {
+      watch_kernel<<<(unsigned)p.watch_count, kWatchThreads, 0, st>>>(p.watch_tiles, p.watch_copy, p.status);
+      return finish_launch("sweep_watch");
+    });
   const int64_t *dst_rowptr = p.dst_rowptr, *dst_order = p.dst_order, *src_rowptr = p.src_rowptr, *src_order = p.src_order;
   if (!dst_rowptr || !src_rowptr) {
     CsrPair pair{};
@@ -514,6 +551,7 @@ int Runner::run() {
   }
   GeoArgs geo{};
   geo.pos = p.pos; geo.src = p.src; geo.dst = p.dst; geo.shifts = p.shifts; geo.cells = p.cells; geo.batch = p.batch;
+  geo.graphs = p.graphs;
   for (int k = 0; k < 3; ++k) geo.box[k] = float(p.box[k]);
   geo.r_max = float(p.r_max); geo.num_basis = int(p.num_basis); geo.p = int(p.poly_p); geo.E = E;
   geo.gate_row = paired ? p.gate_row : nullptr; geo.rep = p.rep;
@@ -610,7 +648,7 @@ int Runner::run() {
   contraction(4, 1, m1, y1);
   call(4, -1, 1, [&] {
     TailArgs a{y1, features, W0, p.species, p.readout_rp, p.readout_rs, p.readout_w2, p.readout_ro0, int(p.hidden),
-               p.row_mask, p.batch, int(p.mask_atomic), p.atomic, energy, dy1, dh, n};
+               p.row_mask, p.batch, p.graphs, int(p.mask_atomic), p.atomic, energy, dy1, dh, n};
     if (n > 0) tail_kernel<<<(unsigned)((n + kTailWarps * kTailNodes - 1) / (kTailWarps * kTailNodes)), kTailWarps * 32, 0, st>>>(a);
     return finish_launch("sweep_tail");
   });
@@ -728,7 +766,7 @@ int Runner::run() {
 static int check(const ictc_sweep* p) {
   if (!p || p->n_local < 0 || p->n_owned < 0 || p->n_owned > p->n_local || p->edges < 0 || p->edges > 2147483647LL ||
       p->pair_rows < 0 || p->graphs < 1 || p->num_species < 1 || p->num_basis < 1 || p->num_basis > 8 || p->poly_p < 2 ||
-      p->hidden < 1 || !(p->r_max > 0) || p->chunk_rows < 0) {
+      p->hidden < 1 || !(p->r_max > 0) || p->chunk_rows < 0 || p->watch_count < 0 || p->watch_count > 2147483647LL) {
     set_error("sweep: sizes");
     return ICTC_ERR_BAD_ARG;
   }
@@ -755,8 +793,13 @@ static int64_t sweep_bytes(const ictc_sweep& p, int stages) {
 int64_t ictc_sweep_workspace(const ictc_sweep* p) {
   if (sweep::check(p)) return -1;
   // with all stages the interactions share launches and buffers live longer: the larger of both placements
-  const int64_t one = sweep_bytes(*p, 1), all = sweep_bytes(*p, 31);
-  return one > all ? one : all;
+  try {
+    const int64_t one = sweep_bytes(*p, 1), all = sweep_bytes(*p, 31);
+    return one > all ? one : all;
+  } catch (const std::exception& e) {          // the placement's lists: host memory is exhausted
+    set_error("sweep: %s", e.what());
+    return -1;
+  }
 }
 
 int ictc_sweep_run(const ictc_sweep* p, int stages, void* stream) {
@@ -770,12 +813,17 @@ int ictc_sweep_run(const ictc_sweep* p, int stages, void* stream) {
     set_error("sweep: features and feature_grad are needed when the stages run one by one");
     return ICTC_ERR_BAD_ARG;
   }
-  if (p->work_bytes < sweep_bytes(*p, stages & 31)) {
-    set_error("sweep: workspace of %lld bytes is too small", (long long)p->work_bytes);
+  try {
+    if (p->work_bytes < sweep_bytes(*p, stages & 31)) {
+      set_error("sweep: workspace of %lld bytes is too small", (long long)p->work_bytes);
+      return ICTC_ERR_BAD_ARG;
+    }
+    sweep::Runner r(*p, stages & 31, (cudaStream_t)stream, false);
+    return r.run();
+  } catch (const std::exception& e) {
+    set_error("sweep: %s", e.what());
     return ICTC_ERR_BAD_ARG;
   }
-  sweep::Runner r(*p, stages & 31, (cudaStream_t)stream, false);
-  return r.run();
 }
 
 }  // extern "C"

@@ -101,7 +101,8 @@ class Sweep(C.Structure):
                                      "host_status", "host_status_event", "status", "up0_table", "sc0_table", "readout_rp",
                                      "readout_rs", "readout_w2", "readout_ro0")]
                 + [("layer", SweepLayer * 2), ("work", _P), ("work_bytes", _L), ("host_marks", _P),
-                   ("host_marks_capacity", _L), ("host_mark_labels", _P), ("host_counts", _P)])
+                   ("host_marks_capacity", _L), ("host_mark_labels", _P), ("host_counts", _P), ("watch_tiles", _P),
+                   ("watch_copy", _P), ("watch_count", _L)])
 
 
 _lib = None

@@ -27,14 +27,25 @@ import threading
 import torch
 
 from ictc_o3 import _lib
+from ictc_o3.basis.ictd_irreps import EdgeWeightedPathPreservingTensorProduct
 from ictc_o3.ops.topology import build_csr
-from .model import MaceIctcModel
+from ictc_o3.symmetric_contraction import ICTDBridgeUSymmetricContractionSO3, _Contraction, _Contractions
+from .model import (ElementConditionedLinearSO3, EquivariantChannelLinearSO3, InteractionBlock, MaceIctcModel, MLPReadout,
+                    Normalize2MomSiLU, PathPreservingLinearSO3, ProductBlock, ScalarReadout)
 
 _ALL, _STAGES = 31, (1, 2, 4, 8, 16)
 _LABELS = ("radial_mlp_hidden_forward_{nout}", "gate_gemm_forward_{nout}", "graph_forward_l{layer}",
            "graph_adjoint_l{layer}", "gate_gemm_backward_{nout}", "radial_mlp_hidden_backward_{nout}",
            "channel_linear_tc", "symmetric_contraction_l{layer}")
 _MARKS = 1024            # timed launches of one sweep (eager steps of a benchmark)
+_WATCH_WORDS = 2048      # words of a parameter that one block of the sweep compares
+_KNOWN = frozenset((ElementConditionedLinearSO3, EquivariantChannelLinearSO3, InteractionBlock, MaceIctcModel, MLPReadout,
+                    Normalize2MomSiLU, PathPreservingLinearSO3, ProductBlock, ScalarReadout, torch.nn.Linear,
+                    torch.nn.ModuleDict, torch.nn.ModuleList, torch.nn.ParameterDict, torch.nn.ParameterList,
+                    torch.nn.Sequential, EdgeWeightedPathPreservingTensorProduct, ICTDBridgeUSymmetricContractionSO3,
+                    _Contraction, _Contractions))
+_HOOKS = ("_forward_hooks", "_forward_pre_hooks", "_backward_hooks", "_backward_pre_hooks")
+_GLOBAL_HOOKS = ("_global_forward_hooks", "_global_forward_pre_hooks", "_global_backward_hooks", "_global_backward_pre_hooks")
 _local = threading.local()
 
 
@@ -49,7 +60,7 @@ class ForceEngine:
     bounds.  ``stream_gates``: see the attribute."""
 
     def __init__(self, model: MaceIctcModel, chunk_rows: int | None = None, chunk_margin: float = 1.3,
-                 stream_gates: bool | None = None):
+                 stream_gates: bool | None = None, lay_out: bool = True):
         if len(model.interactions) != 2:
             raise ValueError("the force engine covers the two-interaction model")
         if model.channels != 64:
@@ -71,14 +82,15 @@ class ForceEngine:
         self.overflow = torch.zeros(1, dtype=torch.int32, device=self.dev)   # sticky: a chunk buffer was too small
         self.profile = None      # list of (kernel name, start event, end event) when enabled by a benchmark
         self._bounds = {}
-        self.refresh()
+        if lay_out:
+            self.refresh()
 
     # ---------------------------------------------------------------- weights
     def _watch(self):
         """Every module and parameter slot of the model with what it holds now: a replaced one is noticed by identity."""
         slots, modules = [], list(self.model.modules())
         for module in modules:
-            for table in (module._modules, module._parameters):
+            for table in (module._modules, module._parameters, module._buffers):
                 slots.extend((table, key, value) for key, value in table.items())
         params = list(self.model.parameters())
         inter = list(self.model.interactions)
@@ -90,21 +102,55 @@ class ForceEngine:
         return ([(p._version, p.data_ptr()) for p in params], [i.avg_num_neighbors for i in inter], m.max_radius,
                 m.polynomial_cutoff_p, m.number_of_basis)
 
-    def hooked(self):
-        """Does any module carry a forward hook (which the sweep would not call)?"""
-        self.refresh()
-        return any(m._forward_hooks or m._forward_pre_hooks for m in self._watched[1])
+    def stands_for(self):
+        """Does the sweep compute what the model's own ``forward`` would?  Not with hooks, with modules of other types or
+        with a replaced ``forward``, with base coefficients that still require grad, or with other widths."""
+        if self._watched is None or self._replaced():
+            self._watched, self._weights = self._watch(), None
+        modules, inter = self._watched[1], self._watched[3]
+        table = torch.nn.modules.module
+        if any(getattr(table, name) for name in _GLOBAL_HOOKS):
+            return False
+        for m in modules:
+            own = m.__dict__
+            if type(m) not in _KNOWN or "forward" in own or any(own[name] for name in _HOOKS):
+                return False
+        return not any(i.tp.weight.requires_grad for i in inter) and self._sizes_fit()
+
+    def _sizes_fit(self):
+        m = self.model
+        if m.channels != 64 or len(m.interactions) != 2 or not 1 <= m.number_of_basis <= 8 or m.polynomial_cutoff_p < 2:
+            return False
+        if not m.max_radius > 0 or any(p.dtype != torch.float32 or p.device != self.dev for p in self._watched[2]):
+            return False
+        for inter in m.interactions:
+            shapes = [tuple(x.weight.shape) if type(x) is torch.nn.Linear and x.bias is None else None for x in inter.fc]
+            if shapes != [(64, m.number_of_basis), None, (64, 64), None, (64, 64), None, (inter.tp.num_paths * 64, 64)]:
+                return False
+        return True
+
+    def _replaced(self):
+        return any(table.get(key) is not value for table, key, value in self._watched[0])
 
     def refresh(self):
         """(Re)build the GEMM-ready weight views when a parameter changed."""
-        if self._watched is None or any(table.get(key) is not value for table, key, value in self._watched[0]):
+        if self._watched is None or self._replaced():
             self._watched, self._weights = self._watch(), None
         state = self._state()
-        if self._weights is not None and self._weights.state == state:
-            return self._weights
-        w = self._layout()
-        w.state = state
-        self._weights = w
+        w, stream = self._weights, torch.cuda.current_stream(self.dev)
+        if w is None or w.state != state:
+            with _lib.on_device(self.dev):
+                w = self._layout()
+                w.event = torch.cuda.Event()
+                w.event.record(stream)
+            w.state, w.streams = state, {stream.cuda_stream}
+            self._weights = w
+        elif stream.cuda_stream not in w.streams and not torch.cuda.is_current_stream_capturing():
+            # laid out on another stream: wait for that, and keep the memory until this stream is done with it
+            stream.wait_event(w.event)
+            for t in w.keep:
+                t.record_stream(stream)
+            w.streams.add(stream.cuda_stream)
         return w
 
     def _layout(self):
@@ -160,8 +206,25 @@ class ForceEngine:
             s.readout_ro0 = hold(m.layer_energy_readouts[0].readout.weight.reshape(-1).contiguous())
             s.hidden, s.num_species = w1.shape[0], m.num_elements
             s.num_basis, s.poly_p, s.r_max = m.number_of_basis, m.polynomial_cutoff_p, m.max_radius
+            w.tiles, w.copy = self._snapshot(w.keep)
             s.species_table, s.species_table_size = hold(m.atomic_number_to_index), m.atomic_number_to_index.numel()
         return w
+
+    def _snapshot(self, keep):
+        """The parameters' words as they are now, in pieces, and where each piece stands: the sweep of a call with the
+        caller's own graph compares them, since a write through ``parameter.data`` changes neither address nor version."""
+        table, flat = [], []
+        for p in self._watched[2]:
+            if not p.is_contiguous():
+                return None, None                     # laid out anew on every call
+            words = p.detach().reshape(-1)
+            pieces = (words.numel() + _WATCH_WORDS - 1) // _WATCH_WORDS
+            table += [(p.data_ptr() + 4 * _WATCH_WORDS * k, min(_WATCH_WORDS, words.numel() - _WATCH_WORDS * k))
+                      for k in range(pieces)]
+            flat.append(torch.nn.functional.pad(words, (0, pieces * _WATCH_WORDS - words.numel())))
+        tiles, copy = torch.tensor(table, dtype=torch.int64, device=self.dev), torch.cat(flat)
+        keep += [tiles, copy]
+        return tiles, copy
 
     def _pack(self, w, transpose):
         """A [rows, 64] matrix in the shared-memory operand layout of the tcgen05 kernels."""
@@ -307,7 +370,10 @@ class ForceEngine:
     @torch.no_grad()
     def energy_and_forces(self, pos, numbers, batch, src, dst, shifts, cell, row_mask, check):
         """(energy per graph, forces, per-atom energies) of a graph whose edges the caller has built, in any order.
-        ``check`` raises ValueError on an atomic number outside the model or an edge index outside the graph."""
+        ``check`` raises ValueError on an atomic number outside the model; a graph or edge index outside its range always
+        does."""
+        if self._weights is not None and self._weights.tiles is None:
+            self._weights = None
         w, dev = self.refresh(), self.dev
         n, graphs = pos.shape[0], cell.shape[0]
         with _lib.on_device(dev):
@@ -324,17 +390,22 @@ class ForceEngine:
             s.cells, s.batch, s.numbers = cell.data_ptr(), batch.data_ptr(), numbers.data_ptr()
             s.species, s.status, s.row_mask = species.data_ptr(), status.data_ptr(), _lib.ptr(row_mask)
             s.energy, s.atomic, s.gradient = energy.data_ptr(), atomic.data_ptr(), forces.data_ptr()
-            if check:
-                flags, event = _status_mailbox(dev)
-                s.host_status, s.host_status_event = flags.data_ptr(), event.cuda_event
+            if w.tiles is not None:
+                s.watch_tiles, s.watch_copy, s.watch_count = w.tiles.data_ptr(), w.copy.data_ptr(), w.tiles.shape[0]
+            flags, event = _status_mailbox(dev)
+            s.host_status, s.host_status_event = flags.data_ptr(), event.cuda_event
             self._run(s, w, None)
-            if check:
-                event.synchronize()
-                unknown, by_dst, by_src = flags.tolist()
-                if unknown:
-                    raise ValueError(f"Encountered atomic numbers outside {self.model.atomic_numbers}")
-                if by_dst < 0 or by_src < 0:
-                    raise ValueError("edge index outside [0, num_nodes)")
+            event.synchronize()
+            bits, by_dst, by_src = flags.tolist()
+        if bits & 4:                     # a parameter was written behind its version counter
+            self._weights = None
+            return self.energy_and_forces(pos, numbers, batch, src, dst, shifts, cell, row_mask, check)
+        if bits & 1 and check:
+            raise ValueError(f"Encountered atomic numbers outside {self.model.atomic_numbers}")
+        if bits & 2:
+            raise ValueError(f"batch: graph index outside [0, {graphs})")
+        if by_dst < 0 or by_src < 0:
+            raise ValueError("edge index outside [0, num_nodes)")
         return energy, forces, atomic
 
 

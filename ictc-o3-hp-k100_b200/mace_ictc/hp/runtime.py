@@ -6,7 +6,7 @@ import torch
 from ..model import MaceIctcModel
 
 
-from ictc_o3.operators import _need_degree, _need_positive
+from ictc_o3.operators import _need_degree, _need_positive, strict_fp32
 
 
 def create_model(*, channels=64, lmax=3, edge_lmax=None, num_interactions=2, correlation=3, use_reduced_cg=False,
@@ -47,25 +47,35 @@ def create_model(*, channels=64, lmax=3, edge_lmax=None, num_interactions=2, cor
     return model.to(device=device, dtype=dtype)
 
 
-def _force_engine(model, tensors):
+def _force_engine(model, tensors, mask):
     """The tape-free engine for an inference call, or None where the autograd route has to answer: other widths or
-    depths, forward hooks, tensors of another type or device, tracing and autocast (which that route refuses)."""
+    depths, hooks, tensors of another type, shape or device, stream capture (a recorded call reads the parameters at each
+    replay), forward-mode and functorch tracing, and autocast (which that route refuses)."""
     if type(model) is not MaceIctcModel or model.channels != 64 or len(model.interactions) != 2:
         return None
-    positions = tensors[0]
-    if (not all(t.is_cuda and t.device == positions.device for t in tensors) or positions.dtype != torch.float32
-            or tensors[3].numel() == 0 or positions.shape[0] == 0 or model.node_embedding.weight.dtype != torch.float32
+    positions, numbers, batch, src, dst, shifts, cell = tensors
+    dev, edges = positions.device, src.shape
+    if (positions.dtype != torch.float32 or type(positions) not in (torch.Tensor, torch.nn.Parameter)
+            or any(type(t) is not torch.Tensor for t in tensors[1:])
+            or not all(t.is_cuda and t.device == dev and t.layout == torch.strided for t in tensors)
+            or any(t.dtype != torch.int64 for t in (batch, src, dst))
+            or numbers.dtype.is_floating_point or numbers.dtype.is_complex
+            or shifts.dtype.is_complex or cell.dtype.is_complex
+            or len(edges) != 1 or dst.shape != edges or tuple(shifts.shape) != (edges[0], 3)
+            or edges[0] == 0 or positions.shape[0] == 0 or cell.shape[0] == 0
+            or mask is not None and (type(mask) is not torch.Tensor or mask.device != dev)
             or torch.is_autocast_enabled("cuda") or torch._C._are_functorch_transforms_active()
-            or torch.compiler.is_compiling() or any(type(t) is not torch.Tensor for t in tensors[1:])):
+            or torch.autograd.forward_ad._current_level >= 0 or torch.compiler.is_compiling()
+            or torch.cuda.is_current_stream_capturing()):
         return None
     engine = model.__dict__.get("_force_engine")
-    if engine is None or engine.dev != positions.device:
+    if engine is None or engine.dev != dev:
         from ..engine import ForceEngine
-        if model.node_embedding.weight.device != positions.device:
+        if model.node_embedding.weight.device != dev:
             return None
-        engine = ForceEngine(model)
+        engine = ForceEngine(model, lay_out=False)
         model.__dict__["_force_engine"] = engine
-    return None if engine.hooked() else engine
+    return engine if engine.stands_for() else None
 
 
 def energy_and_forces(model, positions, atomic_numbers, batch, edge_src, edge_dst, edge_shifts, cell, *,
@@ -88,12 +98,17 @@ def energy_and_forces(model, positions, atomic_numbers, batch, edge_src, edge_ds
     for name, value in (("atomic_numbers", atomic_numbers), ("batch", batch)):
         if tuple(value.shape) != (count,):
             raise ValueError(f"{name}: expected shape [{count}], got {tuple(value.shape)}")
+    for name, value in (("edge_src", edge_src), ("edge_shifts", edge_shifts)):
+        # rows are picked by the receivers' sort order: a shorter table would be indexed outside its rows on the device
+        if value.ndim == 0 or edge_dst.ndim == 0 or value.shape[0] < edge_dst.shape[0]:
+            raise ValueError(f"{name}: expected a row for each of the {edge_dst.numel()} receivers, got {tuple(value.shape)}")
     if owned_mask is not None:
         if tuple(owned_mask.shape) != (count,) or owned_mask.requires_grad:
             raise ValueError(f"owned_mask: expected a constant tensor of shape [{count}]")
     if not training:
-        engine = _force_engine(model, (positions, atomic_numbers, batch, edge_src, edge_dst, edge_shifts, cell))
+        engine = _force_engine(model, (positions, atomic_numbers, batch, edge_src, edge_dst, edge_shifts, cell), owned_mask)
         if engine is not None:
+            strict_fp32()
             dtype = torch.float32
             mask = None if owned_mask is None else owned_mask.to(dtype).contiguous()
             energy, forces, per_atom = engine.energy_and_forces(

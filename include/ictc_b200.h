@@ -437,7 +437,8 @@ typedef struct {
   float* gradient;              /* [n_local, 3], times gradient_sign */
   int32_t* host_status;         /* host (pinned), or NULL: the three status words are copied here early ... */
   void* host_status_event;      /* ... and this cudaEvent_t is recorded behind the copy */
-  int32_t* status;              /* bit 0: atomic number outside the model; word 1, 2: CSR flags (-1: edge index outside) */
+  int32_t* status;              /* word 0: bit 0 atomic number outside the model, bit 1 graph index outside [0, graphs),
+                                 * bit 2 watched weights differ; word 1, 2: CSR flags (-1: edge index outside) */
   const float* up0_table;       /* [S, 64] embedding x linear_up of the first interaction */
   const float* sc0_table;       /* [S, 64] embedding x self connection */
   const float *readout_rp, *readout_rs, *readout_w2, *readout_ro0;
@@ -448,6 +449,9 @@ typedef struct {
   int64_t host_marks_capacity;  /* pairs */
   int64_t* host_mark_labels;    /* host: label of every pair used */
   int64_t* host_counts;         /* host: [0] launches, [1] pairs used (added to) */
+  const int64_t* watch_tiles;   /* [watch_count][2]: address and words (<= 2048) of a piece of a parameter, or NULL */
+  const int32_t* watch_copy;    /* [watch_count][2048]: what stood there when the weights were laid out */
+  int64_t watch_count;
 } ictc_sweep;
 
 /* Bytes of workspace the sweep needs for these sizes. */

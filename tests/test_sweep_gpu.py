@@ -104,6 +104,28 @@ def test_parameter_updates_replacement_copies_and_hooks():
     energy_and_forces(model, *graph)
     assert seen == [1]
     handle.remove()
+    model.products[0].linear["2"].data.mul_(0.7)              # no version counter moves
+    model.last_layer_energy_readout.linear_2.weight.data.copy_(torch.randn(1, 16, device="cuda"))
+    _close(energy_and_forces(model, *graph), _autograd(model, graph))
+    model.interactions[1].fc[1] = torch.nn.Tanh()             # a module that the sweep does not know
+    _close(energy_and_forces(model, *graph), _autograd(model, graph))
+
+
+def test_weights_laid_out_on_another_stream():
+    from mace_ictc.hp import energy_and_forces
+    model = _model()
+    graph = _graph(np.random.default_rng(5), (60,), False)
+    want = _autograd(model, graph)
+    for _ in range(3):
+        side = torch.cuda.Stream()
+        side.wait_stream(torch.cuda.current_stream())
+        with torch.no_grad():
+            model.products[0].linear["1"].mul_(1.0)           # laid out again, here on the current stream
+        energy_and_forces(model, *graph)
+        with torch.cuda.stream(side):
+            got = energy_and_forces(model, *graph)
+        torch.cuda.current_stream().wait_stream(side)
+        _close(got, want)
 
 
 def test_unknown_atoms_and_bad_edges_raise_and_the_next_call_works():
@@ -111,12 +133,19 @@ def test_unknown_atoms_and_bad_edges_raise_and_the_next_call_works():
     model = _model()
     graph = _graph(np.random.default_rng(4), (40,), False)
     good = energy_and_forces(model, *graph)
-    for index, value in ((1, 7), (1, 500), (3, 40), (4, -1)):
+    for index, value in ((1, 7), (1, 500), (2, 1), (2, -1), (3, 40), (4, -1)):
         bad = list(graph)
         bad[index] = bad[index].clone()
         bad[index][5] = value
         with pytest.raises(ValueError):
             energy_and_forces(model, *bad)
+    for index in (3, 5):                                      # one row short: refused before anything is launched
+        bad = list(graph)
+        bad[index] = bad[index][:-1]
+        with pytest.raises(ValueError):
+            energy_and_forces(model, *bad)
+    with pytest.raises((ValueError, RuntimeError)):
+        energy_and_forces(model, *graph, owned_mask=torch.ones(40))
     assert torch.equal(energy_and_forces(model, *graph)["forces"], good["forces"])
 
 
