@@ -122,6 +122,82 @@ struct LayoutArgs {
   int count[kLayoutBlocks], m[kLayoutBlocks], off[kLayoutBlocks + 1];
 };
 
+// Rows of 2l+1 = 1, 3, 5 or 7 components and channels in fours (the network's own layouts), 16-byte aligned buffers.
+// A thread turns one quad, 4 channels x M components, in registers: its 4M floats are M consecutive 16-byte pieces of the
+// mul_ir row and one piece in each of the M component rows on the ir_mul side.  The ir_mul side is accessed in global
+// memory (neighbouring quads are neighbouring pieces); the mul_ir side, where a thread's pieces lie M apart, through
+// a tile of whole rows in shared memory that moves in consecutive pieces (M is odd, so 16-byte accesses M apart hit
+// different banks).  Bound by memory: one read and one write of the rows.  The tile is small enough for eight blocks per
+// SM, which hide each other's barriers.  20,011 rows of 576 and of
+// 2,240 floats, both ways: 568 -> 218 us, 4.1 TB/s.
+constexpr int kTileThreads = 256, kTileBytes = 24 * 1024;
+struct LayoutTile {
+  int rows;                    // rows of a tile
+  int quads;                   // quads of a row
+  int first[kLayoutBlocks + 1];      // first quad of a block
+};
+
+template <int M> __device__ __forceinline__ void turn_quad(float4* mul_ir, float4* ir_mul, int pitch, bool to_ir_mul) {
+  float4 q[M];
+  if (to_ir_mul) {
+    float v[4 * M];
+#pragma unroll
+    for (int k = 0; k < M; ++k) q[k] = mul_ir[k];
+#pragma unroll
+    for (int k = 0; k < M; ++k) { v[4 * k] = q[k].x; v[4 * k + 1] = q[k].y; v[4 * k + 2] = q[k].z; v[4 * k + 3] = q[k].w; }
+#pragma unroll
+    for (int k = 0; k < M; ++k) ir_mul[k * pitch] = make_float4(v[k], v[M + k], v[2 * M + k], v[3 * M + k]);
+  } else {
+    float v[4 * M];
+#pragma unroll
+    for (int k = 0; k < M; ++k) q[k] = __ldg(ir_mul + k * pitch);
+#pragma unroll
+    for (int k = 0; k < M; ++k) { v[k] = q[k].x; v[M + k] = q[k].y; v[2 * M + k] = q[k].z; v[3 * M + k] = q[k].w; }
+#pragma unroll
+    for (int k = 0; k < M; ++k) mul_ir[k] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+  }
+}
+
+__global__ void __launch_bounds__(kTileThreads) layout_tile_kernel(LayoutArgs a, LayoutTile t, const float* __restrict__ in,
+                                                                   float* __restrict__ out, int to_ir_mul) {
+  extern __shared__ __align__(16) float4 layout_tile[];
+  const int row_pieces = a.width / 4, pitch = a.C / 4;
+  for (int64_t r0 = int64_t(blockIdx.x) * t.rows; r0 < a.rows; r0 += int64_t(gridDim.x) * t.rows) {
+    const int rows = int(min(int64_t(t.rows), a.rows - r0)), pieces = rows * row_pieces;
+    const float4* from = reinterpret_cast<const float4*>(in) + r0 * row_pieces;
+    float4* to = reinterpret_cast<float4*>(out) + r0 * row_pieces;
+    if (to_ir_mul) {
+      for (int i = threadIdx.x; i < pieces; i += kTileThreads)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(unsigned(__cvta_generic_to_shared(layout_tile + i))),
+                     "l"(from + i)
+                     : "memory");
+      asm volatile("cp.async.wait_all;" ::: "memory");
+      __syncthreads();
+    }
+    for (int item = threadIdx.x; item < rows * t.quads; item += kTileThreads) {
+      const int row = item / t.quads, q = item - row * t.quads;
+      int b = 0;
+      while (b + 1 < a.nblocks && q >= t.first[b + 1]) ++b;
+      const int m = a.m[b], rel = q - t.first[b], slot = rel / pitch, c = rel - slot * pitch;
+      const int block = row * row_pieces + a.off[b] / 4 + slot * pitch * m;
+      float4* tile = layout_tile + block + c * m;
+      float4* global = (to_ir_mul ? to : const_cast<float4*>(from)) + block + c;
+      switch (m) {
+        case 1: turn_quad<1>(tile, global, pitch, to_ir_mul); break;
+        case 3: turn_quad<3>(tile, global, pitch, to_ir_mul); break;
+        case 5: turn_quad<5>(tile, global, pitch, to_ir_mul); break;
+        default: turn_quad<7>(tile, global, pitch, to_ir_mul); break;
+      }
+    }
+    __syncthreads();
+    if (!to_ir_mul) {
+      for (int i = threadIdx.x; i < pieces; i += kTileThreads) to[i] = layout_tile[i];
+      __syncthreads();
+    }
+  }
+}
+
+// Other component counts, channel counts and alignments.
 // One block per group of rows: a row is read as it lies in memory (coalesced) into shared memory, and written in the
 // other order from there (the transposed reads hit shared memory with odd strides 2l+1, or stride C across the
 // 2l+1 <= 5 components: no bank conflicts worth mentioning), so both global accesses are contiguous.
@@ -234,6 +310,23 @@ int ictc_layout_copy(int64_t rows, int channels, int num_blocks, const int* host
   const int64_t total = rows * int64_t(off);
   if (total == 0) return ICTC_OK;
   if (!in || !out) { set_error("layout copy: NULL buffer"); return ICTC_ERR_BAD_ARG; }
+  bool quads = channels % 4 == 0 && off <= kTileBytes / 4 &&
+               ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
+  LayoutTile t{};
+  for (int b = 0; b < num_blocks; ++b) {
+    quads = quads && (a.m[b] == 1 || a.m[b] == 3 || a.m[b] == 5 || a.m[b] == 7);
+    t.first[b] = t.quads;
+    t.quads += a.count[b] * (channels / 4);
+  }
+  t.first[num_blocks] = t.quads;
+  if (quads) {
+    const int64_t spread = (rows + 148 * 8 - 1) / (148 * 8);        // few rows: one block each before tiles grow
+    t.rows = int(spread < kTileBytes / (4 * off) ? spread : kTileBytes / (4 * off));
+    const int64_t tiles = (rows + t.rows - 1) / t.rows;
+    const unsigned blocks = unsigned(tiles < 148 * 8 ? tiles : 148 * 8);
+    layout_tile_kernel<<<blocks, kTileThreads, size_t(t.rows) * off * 4, (cudaStream_t)stream>>>(a, t, in, out, to_ir_mul);
+    return finish_launch("layout_tile");
+  }
   const size_t smem = size_t(off) * sizeof(float);
   if (smem > 200 * 1024) { set_error("layout copy: rows of %d floats do not fit shared memory", off); return ICTC_ERR_TOO_LARGE; }
   if (smem > 48 * 1024) {
