@@ -16,6 +16,7 @@
 #include "geometry.cuh"
 #include "mlp_chain.cuh"
 #include "scan.cuh"
+#include "tp_chunk.cuh"
 
 namespace ictc {
 namespace sweep {
@@ -604,7 +605,7 @@ int Runner::run() {
       const int64_t r1 = r0 + chunk_rows(n) < n ? r0 + chunk_rows(n) : n;
       gates(stage, layer, pre[layer][2], buf, p.chunk_capacity_dst, geo.gate_row, dst_rowptr + r0, dst_rowptr + r1);
       call(stage, label(kGraphFwd, layer), 1, [&] {
-        return ictc_tp_graph_forward_chunk(spec[layer], kC, r1 - r0, x, geo.sh, L.path_weight, buf, nullptr, dst_rowptr + r0,
+        return tp_graph_forward_chunk(n, spec[layer], kC, r1 - r0, x, geo.sh, L.path_weight, buf, nullptr, dst_rowptr + r0,
                                            p.chunk_capacity_dst, src, dst_rowptr + r0, nullptr, nullptr, out + r0 * width,
                                            st);
       });
@@ -676,7 +677,7 @@ int Runner::run() {
       const int64_t *b = src_rowptr + s0, *en = src_rowptr + s1;
       if (!table) gates(stage, layer, pre[layer][2], gbuf, cap, gates_by_position, b, en);
       call(stage, label(kGraphAdj, layer), 1, [&] {
-        return ictc_tp_graph_adjoint_chunk(spec[layer], kC, s1 - s0, x + s0 * xw, geo.sh, L.path_weight, g,
+        return tp_graph_adjoint_chunk(N, spec[layer], kC, s1 - s0, x + s0 * xw, geo.sh, L.path_weight, g,
                                            table ? geo.gate_row : nullptr, table ? 0 : 1, table ? nullptr : b,
                                            table ? 0 : cap, dst, b, src_order, nullptr, cot, dx ? dx + s0 * xw : nullptr,
                                            dsh, dg, b, cap, st);

@@ -1,6 +1,7 @@
 // C-ABI entry points of the tensor product / graph message kernels and library-wide helpers.
 #include <stdarg.h>
 #include <string.h>
+#include "tp_chunk.cuh"
 #include "tp_tma_kernels.cuh"
 
 namespace ictc {
@@ -69,6 +70,45 @@ __global__ void bounded_wait_selftest_kernel(long long limit_cycles, int* status
 static bool check(bool ok, const char* what) {
   if (!ok) set_error("invalid argument: %s", what);
   return ok;
+}
+
+int tp_graph_forward_chunk(int64_t sweep_rows, int spec, int channels, int64_t num_rows, const float* x, const float* sh,
+                                const float* w, const float* g, const int64_t* gate_row, const int64_t* g_base,
+                                int64_t g_capacity, const int64_t* src, const int64_t* dst_rowptr,
+                                const int64_t* dst_order, const float* mask, float* out, void* stream) {
+  const TpOps* o = find_ops(spec);
+  if (!o) return ICTC_ERR_BAD_SPEC;
+  if (!check(channels > 0 && num_rows >= 0 && g_capacity >= 0, "sizes")) return ICTC_ERR_BAD_ARG;
+  if (num_rows == 0) return ICTC_OK;
+  if (!check(out && dst_rowptr && x && sh && g && src, "x, sh, g, src, dst_rowptr, out must not be NULL")) return ICTC_ERR_BAD_ARG;
+  if (!check(!g_base || g_capacity > 0, "g_capacity must be positive when g_base is given")) return ICTC_ERR_BAD_ARG;
+  TpArgs a{};
+  a.x = x; a.sh = sh; a.w = w; a.g = g; a.mask = mask; a.out = out; a.nbr = src; a.rowptr = dst_rowptr;
+  a.grow = gate_row; a.order = dst_order; a.E = 1; a.N = num_rows; a.C = channels; a.status = kernel_status_word();
+  a.g_base = g_base; a.g_cap = g_capacity; a.sweep_rows = sweep_rows;
+  return o->graph_forward(a, (cudaStream_t)stream);
+}
+
+int tp_graph_adjoint_chunk(int64_t sweep_rows, int spec, int channels, int64_t num_rows, const float* x, const float* sh,
+                                const float* w, const float* g, const int64_t* gate_row, int g_by_position,
+                                const int64_t* g_base, int64_t g_capacity, const int64_t* dst,
+                                const int64_t* src_rowptr, const int64_t* src_order, const float* mask, const float* v,
+                                float* dx, float* dsh, float* dg, const int64_t* dg_base, int64_t dg_capacity,
+                                void* stream) {
+  const TpOps* o = find_ops(spec);
+  if (!o) return ICTC_ERR_BAD_SPEC;
+  if (!check(channels > 0 && num_rows >= 0 && g_capacity >= 0 && dg_capacity >= 0, "sizes")) return ICTC_ERR_BAD_ARG;
+  if (num_rows == 0 || (!dx && !dsh && !dg)) return ICTC_OK;
+  if (!check(src_rowptr && x && sh && g && dst && v, "x, sh, g, dst, v, src_rowptr must not be NULL")) return ICTC_ERR_BAD_ARG;
+  if (!check(!g_base || g_capacity > 0, "g_capacity must be positive when g_base is given")) return ICTC_ERR_BAD_ARG;
+  if (!check(!(dg && dg_base) || dg_capacity > 0, "dg_capacity must be positive when dg_base is given")) return ICTC_ERR_BAD_ARG;
+  TpArgs a{};
+  a.x = x; a.sh = sh; a.w = w; a.g = g; a.mask = mask; a.v = v; a.dx = dx; a.dsh = dsh; a.dg = dg; a.nbr = dst;
+  a.grow = gate_row; a.rowptr = src_rowptr; a.order = src_order; a.E = 1; a.N = num_rows; a.C = channels;
+  a.status = kernel_status_word();
+  a.g_base = g_base; a.g_cap = g_capacity; a.sweep_rows = sweep_rows; a.g_by_pos = g_by_position ? 1 : 0;
+  a.dg_base = dg ? dg_base : nullptr; a.dg_cap = dg_capacity;
+  return o->adjoint(a, true, (cudaStream_t)stream);
 }
 
 }  // namespace ictc
@@ -204,17 +244,8 @@ int ictc_tp_graph_forward_chunk(int spec, int channels, int64_t num_rows, const 
                                 const float* w, const float* g, const int64_t* gate_row, const int64_t* g_base,
                                 int64_t g_capacity, const int64_t* src, const int64_t* dst_rowptr,
                                 const int64_t* dst_order, const float* mask, float* out, void* stream) {
-  const TpOps* o = find_ops(spec);
-  if (!o) return ICTC_ERR_BAD_SPEC;
-  if (!check(channels > 0 && num_rows >= 0 && g_capacity >= 0, "sizes")) return ICTC_ERR_BAD_ARG;
-  if (num_rows == 0) return ICTC_OK;
-  if (!check(out && dst_rowptr && x && sh && g && src, "x, sh, g, src, dst_rowptr, out must not be NULL")) return ICTC_ERR_BAD_ARG;
-  if (!check(!g_base || g_capacity > 0, "g_capacity must be positive when g_base is given")) return ICTC_ERR_BAD_ARG;
-  TpArgs a{};
-  a.x = x; a.sh = sh; a.w = w; a.g = g; a.mask = mask; a.out = out; a.nbr = src; a.rowptr = dst_rowptr;
-  a.grow = gate_row; a.order = dst_order; a.E = 1; a.N = num_rows; a.C = channels; a.status = kernel_status_word();
-  a.g_base = g_base; a.g_cap = g_capacity;
-  return o->graph_forward(a, (cudaStream_t)stream);
+  return tp_graph_forward_chunk(INT64_MAX, spec, channels, num_rows, x, sh, w, g, gate_row, g_base, g_capacity, src,
+                                dst_rowptr, dst_order, mask, out, stream);
 }
 
 int ictc_tp_graph_adjoint_chunk(int spec, int channels, int64_t num_rows, const float* x, const float* sh,
@@ -223,20 +254,8 @@ int ictc_tp_graph_adjoint_chunk(int spec, int channels, int64_t num_rows, const 
                                 const int64_t* src_rowptr, const int64_t* src_order, const float* mask, const float* v,
                                 float* dx, float* dsh, float* dg, const int64_t* dg_base, int64_t dg_capacity,
                                 void* stream) {
-  const TpOps* o = find_ops(spec);
-  if (!o) return ICTC_ERR_BAD_SPEC;
-  if (!check(channels > 0 && num_rows >= 0 && g_capacity >= 0 && dg_capacity >= 0, "sizes")) return ICTC_ERR_BAD_ARG;
-  if (num_rows == 0 || (!dx && !dsh && !dg)) return ICTC_OK;
-  if (!check(src_rowptr && x && sh && g && dst && v, "x, sh, g, dst, v, src_rowptr must not be NULL")) return ICTC_ERR_BAD_ARG;
-  if (!check(!g_base || g_capacity > 0, "g_capacity must be positive when g_base is given")) return ICTC_ERR_BAD_ARG;
-  if (!check(!(dg && dg_base) || dg_capacity > 0, "dg_capacity must be positive when dg_base is given")) return ICTC_ERR_BAD_ARG;
-  TpArgs a{};
-  a.x = x; a.sh = sh; a.w = w; a.g = g; a.mask = mask; a.v = v; a.dx = dx; a.dsh = dsh; a.dg = dg; a.nbr = dst;
-  a.grow = gate_row; a.rowptr = src_rowptr; a.order = src_order; a.E = 1; a.N = num_rows; a.C = channels;
-  a.status = kernel_status_word();
-  a.g_base = g_base; a.g_cap = g_capacity; a.g_by_pos = g_by_position ? 1 : 0;
-  a.dg_base = dg ? dg_base : nullptr; a.dg_cap = dg_capacity;
-  return o->adjoint(a, true, (cudaStream_t)stream);
+  return tp_graph_adjoint_chunk(INT64_MAX, spec, channels, num_rows, x, sh, w, g, gate_row, g_by_position, g_base,
+                                g_capacity, dst, src_rowptr, src_order, mask, v, dx, dsh, dg, dg_base, dg_capacity, stream);
 }
 
 int ictc_selftest_bounded_wait(int64_t limit_cycles, int code, void* stream) {

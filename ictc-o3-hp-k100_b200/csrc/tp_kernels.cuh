@@ -91,6 +91,7 @@ struct TpArgs {
   const int64_t* dg_base;  // device scalar: the gate gradient of the edge at CSR position q goes to row q - *dg_base
                            // (rows outside [0, dg_cap) are not stored); null: row = edge id
   int64_t g_cap, dg_cap;
+  int64_t sweep_rows;      // owner rows of the whole sweep that this launch is a chunk of (0: N)
   int g_by_pos;            // gate row = CSR position of the edge instead of grow[e] / e
 };
 

@@ -77,7 +77,6 @@ constexpr bool kStageRows = false;
 // Warps (= owner rows) per block and the resident warps per SM the kernels are compiled for (12 warps of 32 lanes cap
 // the registers at 168 per thread).  One warp per block: a block ends with its row, no warp waits for a longer row.
 constexpr int kTmaWarps = ICTC_TMA_WARPS;
-constexpr int kTmaMinBlocks = ICTC_TMA_MIN_WARPS / ICTC_TMA_WARPS;
 #ifndef ICTC_TMA_MIN_WARPS_ADJ
 #define ICTC_TMA_MIN_WARPS_ADJ 12
 #endif
@@ -98,18 +97,53 @@ template <class S, class F, int CPL, int STAGES, bool ADJ> struct TmaLayout {
   static constexpr unsigned RED_OFF = GEO_OFF + GEO_BYTES;
   static constexpr unsigned RED_BYTES = ADJ ? RED_EDGES * S::NH * RED_PITCH * 4 : 0;
   static constexpr unsigned WARP_BYTES = ((RED_OFF + RED_BYTES + 127) / 128) * 128;
-  static constexpr unsigned BLOCK_BYTES = WARP_BYTES * kTmaWarps;
 };
 
 // ------------------------------------------------------------------------------------------------
-template <class S, class F, int CPL, int STAGES>
-__global__ void __launch_bounds__(kTmaWarps * 32, kTmaMinBlocks) tp_graph_forward_tma_kernel(TpArgs a) {
+// Few rows leave most of the chip's warp slots empty while every warp walks its row's edges one after the other.  With
+// SPLIT > 1 a block of SPLIT warps shares a row, each warp takes a consecutive part of its edges, and the parts' sums are
+// added in shared memory in a fixed order.  Measured in us, one warp against four (64 channels, 33 edges per row):
+//   rows                216          1,000        1,501        3,000        6,000
+//   222 forward      33 -> 14     46 -> 37     55 -> 50     94 -> 87    162 -> 160
+//   222 adjoint      64 -> 27     83 -> 68    104 -> 92    190 -> 181   393 -> 399
+//   022 forward      25 -> 10     28 -> 16     27 -> 18     35 -> 31     61 -> 58
+//   022 adjoint      33 -> 14     37 -> 24     45 -> 30     76 -> 55    115 -> 106
+// With 8 edges per row the lines cross earlier: forward at 1,501 rows (20.5 -> 20.6), adjoint at 4,000 (79.5 -> 79.8); with
+// 32 channels the forward's at 1,000 (12.4 -> 12.4; 1,501: 14.4 -> 16.1), the adjoint's beyond 4,000 (48.6 -> 48.8).  So the
+// forward splits while one warp per row would not fill the chip once (half of that with 32 channels), the adjoint
+// up to twice that.  The rule looks at the rows of the whole sweep: a sweep in chunks of rows adds up in the same order.
+constexpr int kSplit = 4;
+constexpr int64_t kResidentRows = 148 * ICTC_TMA_MIN_WARPS;
+constexpr int64_t split_limit_forward(int cpl) { return kResidentRows * cpl / 2; }
+constexpr int64_t split_limit_adjoint() { return 2 * kResidentRows; }
+__host__ __device__ constexpr int split_warps(int split) { return split > 1 ? split : kTmaWarps; }
+
+// Sum of the warps' partial rows (`count` vectors per lane, parked at the start of every warp's slot memory), added
+// in warp order; warp w finishes the vectors w, w + SPLIT, ...
+template <int SPLIT, int COUNT, unsigned WARP_BYTES, class V, class Put>
+__device__ __forceinline__ void add_parts(unsigned char* smem, const V (&mine)[COUNT], int warp, int lane, Put put) {
+  V* part = reinterpret_cast<V*>(smem + warp * WARP_BYTES) + lane;
+#pragma unroll
+  for (int k = 0; k < COUNT; ++k) part[k * 32] = mine[k];
+  __syncthreads();
+  for (int k = warp; k < COUNT; k += SPLIT) {
+    V sum = reinterpret_cast<const V*>(smem)[k * 32 + lane];
+#pragma unroll
+    for (int w = 1; w < SPLIT; ++w)
+      sum = vfma(reinterpret_cast<const V*>(smem + w * WARP_BYTES)[k * 32 + lane], V::dup(1.f), sum);
+    put(k, sum);
+  }
+}
+
+template <class S, class F, int CPL, int STAGES, int SPLIT>
+__global__ void __launch_bounds__(split_warps(SPLIT) * 32, ICTC_TMA_MIN_WARPS / split_warps(SPLIT))
+tp_graph_forward_tma_kernel(TpArgs a) {
   using V = Vec<CPL>;
   using L = TmaLayout<S, F, CPL, STAGES, false>;
   constexpr int C = L::C;
   extern __shared__ __align__(128) unsigned char tma_smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t n = int64_t(blockIdx.x) * kTmaWarps + warp;
+  const int64_t n = SPLIT > 1 ? int64_t(blockIdx.x) : int64_t(blockIdx.x) * kTmaWarps + warp;
   if (n >= a.N) return;
   unsigned char* mine = tma_smem + warp * L::WARP_BYTES;
   const unsigned bars = smem_addr(mine + L::BAR_OFF);
@@ -126,7 +160,12 @@ __global__ void __launch_bounds__(kTmaWarps * 32, kTmaMinBlocks) tp_graph_forwar
   V acc[S::NO];
 #pragma unroll
   for (int k = 0; k < S::NO; ++k) acc[k] = V::dup(0.f);
-  const int64_t begin = ldg(a.rowptr + n), end = ldg(a.rowptr + n + 1);
+  int64_t begin = ldg(a.rowptr + n), end = ldg(a.rowptr + n + 1);
+  if (SPLIT > 1) {
+    const int64_t len = end - begin;
+    end = begin + len * (warp + 1) / SPLIT;
+    begin += len * warp / SPLIT;
+  }
   // edge ids and row numbers fit 32 bits (checked by the launcher): 32 x 32 -> 64-bit multiplies form the addresses
   auto edge_at = [&](int64_t it) -> int { return int(a.order ? ldg(a.order + it) : it); };
   auto row_at = [&](int e) -> int { return int(ldg(a.nbr + e)); };
@@ -190,6 +229,7 @@ __global__ void __launch_bounds__(kTmaWarps * 32, kTmaMinBlocks) tp_graph_forwar
         const int64_t owner = it - slot + s + (refilled ? STAGES : 0);
         if (owner < end) mbar_wait(bars + s * 8, refilled ? parity ^ 1u : parity);
       }
+      if (SPLIT > 1) break;       // the row's other warps wait for this one at the block's barrier
       return;
     }
     const unsigned char* base = mine + slot * L::SLOT_BYTES + lane * (CPL * 4);
@@ -219,20 +259,26 @@ __global__ void __launch_bounds__(kTmaWarps * 32, kTmaMinBlocks) tp_graph_forwar
     }
   }
   float* op = a.out + n * (S::NO * C) + lane * CPL;
+  if constexpr (SPLIT > 1) {
+    static_assert(S::NO <= STAGES * S::NP, "the partial row has to fit the slots");
+    __syncwarp();
+    add_parts<SPLIT, S::NO, L::WARP_BYTES>(tma_smem, acc, warp, lane, [&](int k, V v) { v.store(op + k * C); });
+    return;
+  }
 #pragma unroll
   for (int k = 0; k < S::NO; ++k) acc[k].store(op + k * C);
 }
 
 // ------------------------------------------------------------------------------------------------
 // PLAIN: no edge mask and no path weights (decided on the host), so the per-path scaling code is not compiled in.
-template <class S, class F, int CPL, int STAGES, bool GRAPH, bool NEEDX, bool NEEDH, bool NEEDG, bool PLAIN>
-__global__ void __launch_bounds__(kTmaWarps * 32, kTmaMinWarpsAdj / kTmaWarps) tp_adjoint_tma_kernel(TpArgs a) {
+template <class S, class F, int CPL, int STAGES, bool GRAPH, bool NEEDX, bool NEEDH, bool NEEDG, bool PLAIN, int SPLIT>
+__global__ void __launch_bounds__(split_warps(SPLIT) * 32, kTmaMinWarpsAdj / split_warps(SPLIT)) tp_adjoint_tma_kernel(TpArgs a) {
   using V = Vec<CPL>;
   using L = TmaLayout<S, F, CPL, STAGES, true>;
   constexpr int C = L::C;
   extern __shared__ __align__(128) unsigned char tma_smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t owner = int64_t(blockIdx.x) * kTmaWarps + warp;
+  const int64_t owner = SPLIT > 1 ? int64_t(blockIdx.x) : int64_t(blockIdx.x) * kTmaWarps + warp;
   if (owner >= (GRAPH ? a.N : a.E)) return;
   unsigned char* mine = tma_smem + warp * L::WARP_BYTES;
   const unsigned bars = smem_addr(mine + L::BAR_OFF);
@@ -259,6 +305,11 @@ __global__ void __launch_bounds__(kTmaWarps * 32, kTmaMinWarpsAdj / kTmaWarps) t
   if (GRAPH) {
     begin = ldg(a.rowptr + owner);
     end = ldg(a.rowptr + owner + 1);
+  }
+  if (SPLIT > 1) {
+    const int64_t len = end - begin;
+    end = begin + len * (warp + 1) / SPLIT;
+    begin += len * warp / SPLIT;
   }
   auto edge_at = [&](int64_t it) -> int { return int((GRAPH && a.order) ? ldg(a.order + it) : it); };
   auto row_of = [&](int e) -> int { return GRAPH ? int(ldg(a.nbr + e)) : e; };
@@ -315,6 +366,7 @@ __global__ void __launch_bounds__(kTmaWarps * 32, kTmaMinWarpsAdj / kTmaWarps) t
         const int64_t owner = it - slot + s + (refilled ? STAGES : 0);
         if (owner < end) mbar_wait(bars + s * 8, refilled ? parity ^ 1u : parity);
       }
+      if (SPLIT > 1) break;
       return;
     }
     const unsigned char* base = mine + slot * L::SLOT_BYTES + lane * (CPL * 4);
@@ -385,6 +437,12 @@ __global__ void __launch_bounds__(kTmaWarps * 32, kTmaMinWarpsAdj / kTmaWarps) t
   }
   if (NEEDX) {
     float* dxp = a.dx + owner * (S::NX * C) + lane * CPL;
+    if constexpr (SPLIT > 1) {
+      static_assert(S::NX <= STAGES * S::NP, "the partial row has to fit the slots");
+      __syncwarp();
+      add_parts<SPLIT, S::NX, L::WARP_BYTES>(tma_smem, dx, warp, lane, [&](int i, V v) { v.store(dxp + i * C); });
+      return;
+    }
 #pragma unroll
     for (int i = 0; i < S::NX; ++i) dx[i].store(dxp + i * C);
   }
@@ -404,33 +462,42 @@ template <class K> int set_smem(K kernel, unsigned bytes) {
 
 constexpr int kFwdStages = 4, kAdjStages = 4;
 
-template <class S, class F, int CPL> int launch_graph_forward_tma(const TpArgs& a, cudaStream_t st) {
+inline bool split_rows(const TpArgs& a, int64_t limit) { return (a.sweep_rows > 0 ? a.sweep_rows : a.N) <= limit; }
+
+template <class S, class F, int CPL, int SPLIT> int launch_graph_forward_tma(const TpArgs& a, cudaStream_t st) {
   using L = TmaLayout<S, F, CPL, kFwdStages, false>;
-  auto kernel = tp_graph_forward_tma_kernel<S, F, CPL, kFwdStages>;
-  static const int attr = set_smem(kernel, L::BLOCK_BYTES);
+  constexpr int warps = split_warps(SPLIT);
+  auto kernel = tp_graph_forward_tma_kernel<S, F, CPL, kFwdStages, SPLIT>;
+  static const int attr = set_smem(kernel, L::WARP_BYTES * warps);
   if (attr != ICTC_OK) return attr;
-  const int64_t blocks = (a.N + kTmaWarps - 1) / kTmaWarps;
-  kernel<<<(unsigned)blocks, kTmaWarps * 32, L::BLOCK_BYTES, st>>>(a);
+  const int64_t blocks = SPLIT > 1 ? a.N : (a.N + kTmaWarps - 1) / kTmaWarps;
+  kernel<<<(unsigned)blocks, warps * 32, L::WARP_BYTES * warps, st>>>(a);
   return finish_launch("tp_graph_forward_tma");
 }
 
-template <class S, class F, int CPL, bool GRAPH, bool NX_, bool NH_, bool NG_, bool PLAIN>
+template <class S, class F, int CPL, bool GRAPH, bool NX_, bool NH_, bool NG_, bool PLAIN, int SPLIT>
 int launch_adjoint_tma_plain(const TpArgs& a, cudaStream_t st) {
   using L = TmaLayout<S, F, CPL, kAdjStages, true>;
-  auto kernel = tp_adjoint_tma_kernel<S, F, CPL, kAdjStages, GRAPH, NX_, NH_, NG_, PLAIN>;
-  static const int attr = set_smem(kernel, L::BLOCK_BYTES);
+  constexpr int warps = split_warps(SPLIT);
+  auto kernel = tp_adjoint_tma_kernel<S, F, CPL, kAdjStages, GRAPH, NX_, NH_, NG_, PLAIN, SPLIT>;
+  static const int attr = set_smem(kernel, L::WARP_BYTES * warps);
   if (attr != ICTC_OK) return attr;
   const int64_t owners = GRAPH ? a.N : a.E;
-  const int64_t blocks = (owners + kTmaWarps - 1) / kTmaWarps;
-  kernel<<<(unsigned)blocks, kTmaWarps * 32, L::BLOCK_BYTES, st>>>(a);
+  const int64_t blocks = SPLIT > 1 ? owners : (owners + kTmaWarps - 1) / kTmaWarps;
+  kernel<<<(unsigned)blocks, warps * 32, L::WARP_BYTES * warps, st>>>(a);
   return finish_launch("tp_adjoint_tma");
 }
 
 template <class S, class F, int CPL, bool GRAPH, bool NX_, bool NH_, bool NG_>
 int launch_adjoint_tma_one(const TpArgs& a, cudaStream_t st) {
   // the unscaled sender-row sweep is the molecular-dynamics case and gets its own instantiation
-  if (GRAPH && !a.mask && !a.w) return launch_adjoint_tma_plain<S, F, CPL, GRAPH, NX_, NH_, NG_, GRAPH>(a, st);
-  return launch_adjoint_tma_plain<S, F, CPL, GRAPH, NX_, NH_, NG_, false>(a, st);
+  const bool plain = GRAPH && !a.mask && !a.w;
+  if (GRAPH && split_rows(a, split_limit_adjoint())) {
+    if (plain) return launch_adjoint_tma_plain<S, F, CPL, GRAPH, NX_, NH_, NG_, GRAPH, GRAPH ? kSplit : 1>(a, st);
+    return launch_adjoint_tma_plain<S, F, CPL, GRAPH, NX_, NH_, NG_, false, GRAPH ? kSplit : 1>(a, st);
+  }
+  if (plain) return launch_adjoint_tma_plain<S, F, CPL, GRAPH, NX_, NH_, NG_, GRAPH, 1>(a, st);
+  return launch_adjoint_tma_plain<S, F, CPL, GRAPH, NX_, NH_, NG_, false, 1>(a, st);
 }
 
 template <class S, class F, int CPL, bool GRAPH> int launch_adjoint_tma_g(const TpArgs& a, cudaStream_t st) {
@@ -450,8 +517,12 @@ template <class S, class F, int CPL, bool GRAPH> int launch_adjoint_tma_g(const 
 template <class S, int ID> int graph_forward_dispatch_tma(const TpArgs& a, cudaStream_t st) {
   if (a.N > 0 && a.E > 0 && a.E <= 2147483647LL && (a.C == 32 || a.C == 64) && a.N <= 2147483647LL &&
       aligned16(a.x) && aligned16(a.g) && aligned8(a.out) && (!a.w || aligned8(a.w))) {
-    if (a.C == 64) return launch_graph_forward_tma<S, TpFast<ID, 2>, 2>(a, st);
-    return launch_graph_forward_tma<S, TpFast<ID, 1>, 1>(a, st);
+    if (split_rows(a, split_limit_forward(a.C / 32))) {
+      if (a.C == 64) return launch_graph_forward_tma<S, TpFast<ID, 2>, 2, kSplit>(a, st);
+      return launch_graph_forward_tma<S, TpFast<ID, 1>, 1, kSplit>(a, st);
+    }
+    if (a.C == 64) return launch_graph_forward_tma<S, TpFast<ID, 2>, 2, 1>(a, st);
+    return launch_graph_forward_tma<S, TpFast<ID, 1>, 1, 1>(a, st);
   }
   return graph_forward_dispatch<S, ID>(a, st);
 }
