@@ -530,6 +530,9 @@ def normalized_silu(features, scale=1.0):
     """SiLU followed by a constant factor (ictc_o3/operators.py:631-636)."""
     if isinstance(scale, bool) or not isinstance(scale, (int, float)):
         raise TypeError(f"scale: expected a plain number, got {type(scale).__name__}")
+    from .ops.activation import kernel_takes, scaled_silu
+    if kernel_takes(features):
+        return scaled_silu(features, float(scale))
     return float(scale) * torch.nn.functional.silu(features)
 
 

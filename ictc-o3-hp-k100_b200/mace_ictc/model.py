@@ -22,7 +22,7 @@ from torch import nn
 
 from ictc_o3.basis.ictd_irreps import EdgeWeightedPathPreservingTensorProduct
 from ictc_o3.operators import (PackedGraphMessage, _RowsTimesWeight, _tc_eligible, channel_linear, convert_layout,
-                               direction_harmonics, strict_fp32)
+                               direction_harmonics, normalized_silu, strict_fp32)
 from ictc_o3.symmetric_contraction import ICTDBridgeUSymmetricContractionSO3
 
 SILU_SCALE = 1.6791767923989418
@@ -43,7 +43,7 @@ def merge_irreps(blocks: Dict[int, torch.Tensor], channels: int, lmax: int) -> t
 
 class Normalize2MomSiLU(nn.Module):
     def forward(self, x):
-        return torch.nn.functional.silu(x) * SILU_SCALE
+        return normalized_silu(x, SILU_SCALE)
 
 
 def bessel_embedding(r: torch.Tensor, r_max: float, num_basis: int, p: int) -> torch.Tensor:

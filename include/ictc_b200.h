@@ -258,6 +258,10 @@ int ictc_position_gradient(int64_t num_rows, int64_t num_dst_rows, const int64_t
  * ictc_o3/backends/k100/hip_activation.py:27-38. */
 int ictc_silu_forward(int64_t n, float scale, const float* x, float* y, void* stream);
 int ictc_silu_backward(int64_t n, float scale, const float* x, const float* dy, float* dx, void* stream);
+/* Adjoint of ictc_silu_backward with cotangent h: gx = h dy scale silu''(x), gdy = h scale silu'(x); either may be NULL
+ * (mode 2 of the same reference kernel). */
+int ictc_silu_second(int64_t n, float scale, const float* x, const float* dy, const float* h, float* gx, float* gdy,
+                     void* stream);
 /* Whole-row conversion between the model-native mul_ir layout (every block [C, 2l+1], channel outer) and the
  * kernel-native ir_mul layout (every block [2l+1, C], channel contiguous) in one launch.  A row is a sequence of
  * num_blocks degree blocks; block b holds host_counts[b] path slots of host_ms[b] components each (HOST int
