@@ -258,6 +258,37 @@ int ictc_tp_graph_adjoint_chunk(int spec, int channels, int64_t num_rows, const 
                                 g_capacity, dst, src_rowptr, src_order, mask, v, dx, dsh, dg, dg_base, dg_capacity, stream);
 }
 
+int ictc_tp_graph_second_covers(int channels, int64_t num_nodes, int64_t num_edges) {
+  return (channels == 32 || channels == 64) && num_nodes > 0 && num_nodes <= 2147483647LL && num_edges > 0 &&
+         num_edges <= 2147483647LL;
+}
+
+int ictc_tp_graph_second(int spec, int channels, int64_t num_nodes, int64_t num_edges, const float* x, const float* sh,
+                         const float* w, const float* g, const float* hx, const float* hs, const float* hg,
+                         const int64_t* src, const int64_t* dst, const int64_t* dst_rowptr, const int64_t* dst_order,
+                         const int64_t* src_rowptr, const int64_t* src_order, const float* mask, const float* v,
+                         float* gx, float* gsh, float* gg, float* gv, void* stream) {
+  const TpOps* o = find_ops(spec);
+  if (!o) return ICTC_ERR_BAD_SPEC;
+  if (!check(ictc_tp_graph_second_covers(channels, num_nodes, num_edges), "sizes")) return ICTC_ERR_BAD_ARG;
+  if (!check(x && sh && g && hx && hs && hg && src && dst && dst_rowptr && src_rowptr && v && gx && gsh && gg,
+             "buffers must not be NULL")) return ICTC_ERR_BAD_ARG;
+  uintptr_t bits = 0;
+  for (const float* p : {x, hx, v, (const float*)gx, (const float*)gg, (const float*)gv, w})
+    bits |= reinterpret_cast<uintptr_t>(p) & 7;
+  if (!check(bits == 0 && aligned16(g) && aligned16(hg), "rows must be 8-byte aligned, gate rows 16-byte aligned"))
+    return ICTC_ERR_BAD_ARG;
+  TpArgs a{};
+  a.x = x; a.sh = sh; a.w = w; a.g = g; a.mask = mask; a.v = v; a.dx = gx; a.dsh = gsh; a.dg = gg; a.nbr = dst;
+  a.rowptr = src_rowptr; a.order = src_order; a.E = num_edges; a.N = num_nodes; a.C = channels;
+  a.status = kernel_status_word();
+  const TpTangents t{hx, hs, hg};
+  if (int rc = o->second(a, t, false, (cudaStream_t)stream)) return rc;
+  if (!gv) return ICTC_OK;
+  a.nbr = src; a.rowptr = dst_rowptr; a.order = dst_order; a.out = gv;
+  return o->second(a, t, true, (cudaStream_t)stream);
+}
+
 int ictc_selftest_bounded_wait(int64_t limit_cycles, int code, void* stream) {
   if (limit_cycles < 1 || limit_cycles > 200000000LL || code == 0) {
     set_error("selftest: limit must be 1..2e8 cycles and the code non-zero");

@@ -105,6 +105,27 @@ template <int ID, int CPL> struct TpConst;
 #define ICTC_M_P_DA(i, k) s = vfma(x[i], vg[k], s);
 #define ICTC_M_P_DE(t, j) dsh[j] = vfma(s, Vec<CPL>{K::c[t]}, dsh[j]); }
 #define ICTC_M_P_PE(p) if (NEEDG) store_dg(p, dgp);
+// the same programs over two geometries (second derivatives, tp_second_kernels.cuh)
+#define ICTC_GETH(e) (hh.template get<(e) % Chunk<CPL>::PER>())
+#define ICTC_LDB2(e) if ((e) % Chunk<CPL>::PER == 0) { ch.load(sb, (e)); hh.load(sbh, (e)); }
+#define ICTC_M_S_PB(p)                                                    \
+  gp = gate(p); hp = hgate(p); dgp = V::dup(0.f);                         \
+  _Pragma("unroll") for (int i = 0; i < Base::NX; ++i) xg[i] = vfma(x[i], hp, vmul(hx[i], gp));
+#define ICTC_M_S_ZF(e, k) ICTC_LDB2(e) z = vmul(ICTC_GETB(e), v[k]); y = vmul(ICTC_GETH(e), v[k]);
+#define ICTC_M_S_ZA(e, k) ICTC_LDB2(e) z = vfma(ICTC_GETB(e), v[k], z); y = vfma(ICTC_GETH(e), v[k], y);
+#define ICTC_M_S_Q(i, p)                                                  \
+  dx[i] = vfma(y, gp, vfma(z, hp, dx[i]));                                \
+  dgp = vfma(hx[i], z, vfma(x[i], y, dgp));
+#define ICTC_M_S_VG(k, p)
+#define ICTC_M_S_DF(i, k) { V s = vmul(xg[i], v[k]);
+#define ICTC_M_S_DA(i, k) s = vfma(xg[i], v[k], s);
+#define ICTC_M_S_DE(t, j) dsh[j] = vfma(s, V{K::c[t]}, dsh[j]); }
+#define ICTC_M_S_PE(p) store_dg(p, dgp);
+#define ICTC_M_SF_F(e, i) ICTC_LDB2(e) z = vmul(x[i], ICTC_GETB(e)); y = vfma(hx[i], ICTC_GETB(e), vmul(x[i], ICTC_GETH(e)));
+#define ICTC_M_SF_A(e, i)                                                 \
+  ICTC_LDB2(e) z = vfma(x[i], ICTC_GETB(e), z);                           \
+  y = vfma(hx[i], ICTC_GETB(e), vfma(x[i], ICTC_GETH(e), y));
+#define ICTC_M_SF_K(k, p) acc[k] = vfma(z, hge[p], vfma(y, ge[p], acc[k]));
 #define ICTC_M_DSHT_F(t, i, j, k, p) dsh[j] = vmul(vmul(x[i], vg[k]), Vec<CPL>{K::c[t]});
 #define ICTC_M_DSHT_A(t, i, j, k, p) dsh[j] = vfma(vmul(x[i], vg[k]), Vec<CPL>{K::c[t]}, dsh[j]);
 
@@ -150,6 +171,24 @@ template <int ID, int CPL> struct TpConst;
       V v[Base::NO], vg[Base::NO];                                                                      \
       ICTC_TP_##S##_ADJP(ICTC_M_P_PB, ICTC_M_P_VL, ICTC_M_P_ZF, ICTC_M_P_ZA, ICTC_M_P_Q, ICTC_M_P_VG,   \
                          ICTC_M_P_DF, ICTC_M_P_DA, ICTC_M_P_DE, ICTC_M_P_PE)                            \
+    }                                                                                                   \
+    template <class CotF, class GateF, class HGateF, class StoreF>                                      \
+    static __device__ __forceinline__ void second_fused(const V (&x)[Base::NX], const V (&hx)[Base::NX], \
+                                                        CotF cot, GateF gate, HGateF hgate, const V* sb, \
+                                                        const V* sbh, V (&dx)[Base::NX],                \
+                                                        V (&dsh)[Base::NH], StoreF store_dg) {          \
+      Chunk<CPL> ch, hh;                                                                                \
+      V z, y, gp, hp, dgp;                                                                              \
+      V v[Base::NO], xg[Base::NX];                                                                      \
+      ICTC_TP_##S##_ADJP(ICTC_M_S_PB, ICTC_M_P_VL, ICTC_M_S_ZF, ICTC_M_S_ZA, ICTC_M_S_Q, ICTC_M_S_VG,   \
+                         ICTC_M_S_DF, ICTC_M_S_DA, ICTC_M_S_DE, ICTC_M_S_PE)                            \
+    }                                                                                                   \
+    static __device__ __forceinline__ void second_forward(const V (&x)[Base::NX], const V (&hx)[Base::NX], \
+                                                          const V (&ge)[Base::NP], const V (&hge)[Base::NP], \
+                                                          const V* sb, const V* sbh, V (&acc)[Base::NO]) { \
+      Chunk<CPL> ch, hh;                                                                                \
+      V z, y;                                                                                           \
+      ICTC_TP_##S##_FB(ICTC_M_SF_F, ICTC_M_SF_A, ICTC_M_SF_K)                                           \
     }                                                                                                   \
     static __device__ __forceinline__ void dharm(const V (&x)[Base::NX], const V (&v)[Base::NO],        \
                                                  const V (&ge)[Base::NP], V (&dsh)[Base::NH]) {         \

@@ -95,6 +95,11 @@ struct TpArgs {
   int g_by_pos;            // gate row = CSR position of the edge instead of grow[e] / e
 };
 
+// Cotangents of the adjoint's three outputs (second derivatives).
+struct TpTangents {
+  const float *hx, *hs, *hg;
+};
+
 // Row of edge e, found at position `pos` of the owner's CSR walk, in the gate table.
 __device__ __forceinline__ int64_t gate_row_of(const TpArgs& a, int64_t e, int64_t pos) {
   int64_t r = a.g_by_pos ? pos : (a.grow ? ldg(a.grow + e) : e);
@@ -281,6 +286,7 @@ struct TpOps {
   int (*edge_forward)(const TpArgs&, cudaStream_t);
   int (*graph_forward)(const TpArgs&, cudaStream_t);
   int (*adjoint)(const TpArgs&, bool graph, cudaStream_t);
+  int (*second)(const TpArgs&, const TpTangents&, bool forward, cudaStream_t) = nullptr;
 };
 
 template <class S> int launch_edge_forward(const TpArgs& a, cudaStream_t st) {

@@ -1,5 +1,5 @@
 // One translation unit per tensor-product spec: compile with -DICTC_SPEC=L222 (etc.).
-#include "tp_tma_kernels.cuh"
+#include "tp_second_kernels.cuh"
 
 #ifndef ICTC_SPEC
 #error "compile with -DICTC_SPEC=<spec name from generated/tp_spec_tables.cuh>"

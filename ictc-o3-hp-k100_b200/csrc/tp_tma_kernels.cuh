@@ -542,9 +542,4 @@ template <class S, int ID> int adjoint_dispatch_tma(const TpArgs& a, bool graph,
   return adjoint_dispatch<S, ID>(a, graph, st);
 }
 
-template <class S, int ID> TpOps make_ops_tma() {
-  return TpOps{S::NX, S::NH, S::NP, S::NO, S::NNZ, &launch_edge_forward<S>, &graph_forward_dispatch_tma<S, ID>,
-               &adjoint_dispatch_tma<S, ID>};
-}
-
 }  // namespace ictc

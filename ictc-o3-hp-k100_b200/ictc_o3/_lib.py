@@ -33,6 +33,8 @@ SIGNATURES = {
     "ictc_tp_graph_forward_chunk": (_I, [_I, _I, _L, _P, _P, _P, _P, _P, _P, _L, _P, _P, _P, _P, _P, _P]),
     "ictc_tp_graph_adjoint_chunk": (_I, [_I, _I, _L, _P, _P, _P, _P, _P, _I, _P, _L, _P, _P, _P, _P, _P, _P, _P, _P, _P,
                                          _L, _P]),
+    "ictc_tp_graph_second_covers": (_I, [_I, _L, _L]),
+    "ictc_tp_graph_second": (_I, [_I, _I, _L, _L] + [_P] * 20),
     "ictc_gate_gemm_forward_rows": (_I, [_L, _I, _P, _P, _P, _P, _P, _P, _I, _P]),
     "ictc_gate_gemm_backward_rows": (_I, [_L, _I, _P, _P, _P, _P, _P, _P, _P]),
     "ictc_mlp_chain_backward_paired": (_I, [_L, _I, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _P, _I, _P, _P]),

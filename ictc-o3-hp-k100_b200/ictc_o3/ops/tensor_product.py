@@ -97,6 +97,26 @@ class TpCall:
         return dx, dsh, dg
 
 
+    def second(self, x, sh, g, v, hx, hs, hg, need_v):
+        """Gradients of <hx, dx> + <hs, dsh> + <hg, dg> with respect to x, sh, g and (``need_v``) v in two launches, or None
+        where the kernels do not apply: edge-owned rows, other channel counts, misaligned rows."""
+        lib, dev, c, topo = _lib.load(), x.device, self.channels, self.topology
+        if topo is None or not lib.ictc_tp_graph_second_covers(c, topo.num_nodes, topo.num_edges):
+            return None
+        weight = [] if self.weight is None else [self.weight]
+        if any(t.data_ptr() % 8 for t in (x, hx, v, *weight)) or any(t.data_ptr() % 16 for t in (g, hg)):
+            return None
+        (dst_rowptr, dst_order), (src_rowptr, src_order) = topo.by_dst(), topo.by_src()
+        gx, gsh, gg = torch.empty_like(x), torch.empty_like(sh), torch.empty_like(g)
+        gv = torch.empty_like(v) if need_v else None
+        with _lib.on_device(dev), _Timed("graph_second", dev):
+            _lib.check(lib.ictc_tp_graph_second(
+                self.spec, c, topo.num_nodes, topo.num_edges, *(_lib.ptr(t) for t in (
+                    x, sh, self.weight, g, hx, hs, hg, topo.src, topo.dst, dst_rowptr, dst_order, src_rowptr, src_order,
+                    self.mask, v, gx, gsh, gg, gv)), _lib.stream(dev)), "ictc_tp_graph_second")
+        return gx, gsh, gg, gv
+
+
 def _add(a, b):
     if a is None:
         return b
@@ -154,6 +174,11 @@ class _TpAdjoint(torch.autograd.Function):
 
         def fwd(xa, sa, ga):
             return _TpForward.apply(xa, sa, ga, call) if record else call.forward(xa, sa, ga)
+
+        if not record and need_x and need_s and need_g and not (hx is None or hs is None or hg is None):
+            fused = call.second(x, sh, g, v, hx, hs, hg, need_v)
+            if fused is not None:
+                return (*fused, None, None)
 
         big_x = big_s = big_g = big_v = None
         # L = <hx, dx> + <hs, dsh> + <hg, dg> = <v, F(hx,sh,g) + F(x,hs,g) + F(x,sh,hg)>

@@ -138,6 +138,16 @@ int ictc_tp_graph_adjoint_chunk(int spec, int channels, int64_t num_rows, const 
                                 float* dx, float* dsh, float* dg, const int64_t* dg_base, int64_t dg_capacity,
                                 void* stream);
 
+/* Mixed second derivatives of the graph message: gradients of <v, F(hx,sh,g) + F(x,hs,g) + F(x,sh,hg)> with respect to x, sh, g
+ * (all needed) and v (gv, or NULL); replaces the reference's second-derivative launches (ictc_o3/operators.py:57-158).
+ * Both CSRs of the edge list; ictc_tp_graph_second_covers tells the sizes (1 = yes); rows 8-byte, g and hg 16-byte aligned. */
+int ictc_tp_graph_second_covers(int channels, int64_t num_nodes, int64_t num_edges);
+int ictc_tp_graph_second(int spec, int channels, int64_t num_nodes, int64_t num_edges, const float* x, const float* sh,
+                         const float* w, const float* g, const float* hx, const float* hs, const float* hg,
+                         const int64_t* src, const int64_t* dst, const int64_t* dst_rowptr, const int64_t* dst_order,
+                         const int64_t* src_rowptr, const int64_t* src_order, const float* mask, const float* v,
+                         float* gx, float* gsh, float* gg, float* gv, void* stream);
+
 /* ------------------------------------------------------------------ CSR topology
  * Counting sort of edges by an int64 key in [0, num_nodes): rowptr [N+1], order [E] (edge ids,
  * ascending inside a row, i.e. a stable sort), *sorted_flag (device int32) = 1 when the keys were
