@@ -16,7 +16,7 @@ namespace ictc {
 
 __global__ void csr_init_kernel(CsrPair p, int64_t N) {
   const CsrSet& c = p.set[blockIdx.y];
-  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x + pdl_enter();
   if (i < N) c.counts[i] = 0;
   if (i == 0) {
     *c.flag = 1;
@@ -27,7 +27,7 @@ __global__ void csr_init_kernel(CsrPair p, int64_t N) {
 // `place` = how many edges of the row came earlier
 __global__ void csr_count_kernel(CsrPair p, int64_t E, int64_t N) {
   const CsrSet& c = p.set[blockIdx.y];
-  const int64_t e = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  const int64_t e = int64_t(blockIdx.x) * blockDim.x + threadIdx.x + pdl_enter();
   if (e >= E) return;
   const int64_t k = c.keys[e];
   if (k < 0 || k >= N) {
@@ -49,7 +49,7 @@ struct CsrStore {
 
 __global__ void csr_fill_kernel(CsrPair p, int64_t E, int64_t N) {
   const CsrSet& c = p.set[blockIdx.y];
-  const int64_t e = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  const int64_t e = int64_t(blockIdx.x) * blockDim.x + threadIdx.x + pdl_enter();
   if (e >= E) return;
   if (*c.flag == 1) {
     c.order[e] = e;
@@ -72,10 +72,11 @@ constexpr int kRankRows = 8;
 
 __global__ void __launch_bounds__(kRankRows * 32) csr_rank_kernel(CsrPair p, int64_t N) {
   __shared__ bool is_long[kRankRows];
+  const int zero = pdl_enter();
   const CsrSet& c = p.set[blockIdx.y];
   if (*c.flag == 1) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t first = int64_t(blockIdx.x) * kRankRows, row = first + warp;
+  const int64_t first = int64_t(blockIdx.x) * kRankRows + zero, row = first + warp;
   const int64_t begin = row < N ? c.rowptr[row] : 0, end = row < N ? c.rowptr[row + 1] : 0;
   if (lane == 0) is_long[warp] = end - begin > kLongRow;
   if (end - begin <= kLongRow) {
@@ -117,13 +118,13 @@ CsrSet csr_set(const int64_t* keys, int64_t N, int64_t E, int64_t* rowptr, int64
 }
 
 int csr_build(const CsrPair& p, int sets, int64_t N, int64_t E, int64_t* sums, cudaStream_t st) {
-  csr_init_kernel<<<dim3((unsigned)(N / 256 + 1), sets), 256, 0, st>>>(p, N);
-  if (E > 0) csr_count_kernel<<<dim3((unsigned)((E + 255) / 256), sets), 256, 0, st>>>(p, E, N);
+  launch_after(csr_init_kernel, dim3((unsigned)(N / 256 + 1), sets), 256, 0, st, p, N);
+  if (E > 0) launch_after(csr_count_kernel, dim3((unsigned)((E + 255) / 256), sets), 256, 0, st, p, E, N);
   prefix_sum<int64_t>(N, CsrLoad{p}, CsrStore{p}, sums, false, st, sets);
   if (E > 0) {
-    csr_fill_kernel<<<dim3((unsigned)((E + 255) / 256), sets), 256, 0, st>>>(p, E, N);
+    launch_after(csr_fill_kernel, dim3((unsigned)((E + 255) / 256), sets), 256, 0, st, p, E, N);
     if (N > 0)
-      csr_rank_kernel<<<dim3((unsigned)((N + kRankRows - 1) / kRankRows), sets), kRankRows * 32, 0, st>>>(p, N);
+      launch_after(csr_rank_kernel, dim3((unsigned)((N + kRankRows - 1) / kRankRows), sets), kRankRows * 32, 0, st, p, N);
   }
   return finish_launch("csr_build");
 }

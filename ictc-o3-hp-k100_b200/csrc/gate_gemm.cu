@@ -57,9 +57,9 @@ struct Work {
   int64_t base, live;        // first list entry, bound of the live rows
   int end0, end1, end2;      // running totals of tiles
 
-  __device__ Work(const Args& a) {
-    base = a.begin ? ldg(a.begin) : 0;
-    live = a.limit ? ldg(a.limit) - base : a.seg[0].rows + a.seg[1].rows + a.seg[2].rows;
+  __device__ Work(const Args& a, int zero) {
+    base = a.begin ? ldg(a.begin + zero) : zero;
+    live = a.limit ? ldg(a.limit + zero) - base : a.seg[0].rows + a.seg[1].rows + a.seg[2].rows;
     if (live < 0) live = 0;
     end0 = int((rows(a, 0) + kRows - 1) / kRows);
     end1 = end0 + (a.segments > 1 ? int((rows(a, 1) + kRows - 1) / kRows) : 0);
@@ -151,8 +151,8 @@ __global__ void __launch_bounds__(kFwdThreads, 1) gate_gemm_forward_kernel(const
   int64_t* offsets = reinterpret_cast<int64_t*>(stage + 2 * kRows * kStagePitch);
   Barriers* bar = reinterpret_cast<Barriers*>(offsets + 2 * kRows);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const Work work(a);
   const unsigned tmem = enter(bar, 2, 4);
+  const Work work(a, pdl_enter());
   const unsigned tmem_a = tmem + 4 * kChunk;       // A operands start after the accumulator ring
 
   if (warp == 0) {
@@ -302,8 +302,8 @@ __global__ void __launch_bounds__(kBwdThreads, 1) gate_gemm_backward_kernel(cons
   unsigned char* raw = w_buf + kWStages * kWStageBytes;
   Barriers* bar = reinterpret_cast<Barriers*>(raw + kRawBytes);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const Work work(a);
   const unsigned tmem = enter(bar, kAStagesBwd, 2);
+  const Work work(a, pdl_enter());
   const unsigned tmem_a = tmem + 2 * kChunk;
 
   if (warp == 0) {
@@ -471,12 +471,13 @@ __global__ void gate_pack_kernel(int nout, const float* __restrict__ w, int tran
 }
 
 // One persistent CTA per SM
-static int prepare(Args& a) {
+static int prepare(Args& a, bool& one_wave) {
   int dev = 0, sms = 148;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   int64_t tiles = 0;
   for (int s = 0; s < a.segments; ++s) tiles += (a.seg[s].rows + kRows - 1) / kRows;
   a.status = kernel_status_word();
+  one_wave = tiles <= sms;
   return int(tiles < sms ? tiles : sms);
 }
 
@@ -484,8 +485,9 @@ int launch_forward(Args a, cudaStream_t st) {
   static const cudaError_t attr =
       cudaFuncSetAttribute(gate_gemm_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kFwdSmem);
   if (attr != cudaSuccess) { set_error("gate gemm smem: %s", cudaGetErrorString(attr)); return ICTC_ERR_LAUNCH; }
-  const int grid = prepare(a);
-  gate_gemm_forward_kernel<<<grid, kFwdThreads, kFwdSmem, st>>>(a);
+  bool one_wave;
+  const int grid = prepare(a, one_wave);
+  launch_if(one_wave, gate_gemm_forward_kernel, grid, kFwdThreads, kFwdSmem, st, a);
   return finish_launch("gate_gemm_forward");
 }
 
@@ -493,8 +495,9 @@ int launch_backward(Args a, cudaStream_t st) {
   static const cudaError_t attr =
       cudaFuncSetAttribute(gate_gemm_backward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kBwdSmem);
   if (attr != cudaSuccess) { set_error("gate gemm smem: %s", cudaGetErrorString(attr)); return ICTC_ERR_LAUNCH; }
-  const int grid = prepare(a);
-  gate_gemm_backward_kernel<<<grid, kBwdThreads, kBwdSmem, st>>>(a);
+  bool one_wave;
+  const int grid = prepare(a, one_wave);
+  launch_if(one_wave, gate_gemm_backward_kernel, grid, kBwdThreads, kBwdSmem, st, a);
   return finish_launch("gate_gemm_backward");
 }
 

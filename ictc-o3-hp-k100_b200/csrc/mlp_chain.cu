@@ -69,19 +69,23 @@ __device__ __forceinline__ unsigned setup(const Args& a, const Stack& k, unsigne
     }
     bar->failed = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    mbar_expect_tx(saddr(&bar->w_full), 2 * kWStageBytes);
-    bulk_g2s(saddr(smem), k.wa, kWStageBytes, saddr(&bar->w_full));
-    bulk_g2s(saddr(smem + kWStageBytes), k.wb, kWStageBytes, saddr(&bar->w_full));
-  }
-  for (int i = threadIdx.x; i < 64 * 8; i += blockDim.x) {
-    const int n = i >> 3, b = i & 7;
-    w0s[i] = b < a.nb ? k.w0[n * a.nb + b] : 0.f;
   }
   if (warp == 1) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(saddr(&bar->tmem_base)),
                  "r"(512u)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  __syncthreads();
+  const int zero = pdl_enter();
+  if (threadIdx.x == 0) {
+    mbar_expect_tx(saddr(&bar->w_full), 2 * kWStageBytes);
+    bulk_g2s(saddr(smem), k.wa, kWStageBytes, saddr(&bar->w_full));
+    bulk_g2s(saddr(smem + kWStageBytes), k.wb, kWStageBytes, saddr(&bar->w_full));
+  }
+  for (int i = threadIdx.x + zero; i < 64 * 8; i += blockDim.x) {
+    const int n = i >> 3, b = i & 7;
+    w0s[i] = b < a.nb ? k.w0[n * a.nb + b] : 0.f;
   }
   tc_fence_before();
   __syncthreads();
@@ -129,12 +133,12 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_chain_forward_kernel(const __
   float* w0s = reinterpret_cast<float*>(chain_smem + 2 * kWStageBytes);
   Barriers* bar = reinterpret_cast<Barriers*>(chain_smem + kBarOffset);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t nrows = a.limit ? (ldg(a.limit) < a.E ? ldg(a.limit) : a.E) : a.E;
-  const int64_t tiles = (nrows + kRows - 1) / kRows;
   const Share share(a);
   const Stack& stack = a.stack[share.stack];
-  const int64_t my_tiles = share.first < tiles ? (tiles - share.first + share.step - 1) / share.step : 0;
   const unsigned tmem = setup(a, stack, chain_smem, bar, w0s);
+  const int64_t nrows = a.limit ? (ldg(a.limit) < a.E ? ldg(a.limit) : a.E) : a.E;
+  const int64_t tiles = (nrows + kRows - 1) / kRows;
+  const int64_t my_tiles = share.first < tiles ? (tiles - share.first + share.step - 1) / share.step : 0;
 
   if (warp == 1) {
     mma_loop(a, bar, chain_smem, tmem, my_tiles);
@@ -204,12 +208,12 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_chain_backward_kernel(const _
   float* xchg = w0s + 64 * 8;                                         // [128][8] partial drb of the upper half
   Barriers* bar = reinterpret_cast<Barriers*>(chain_smem + kBarOffset);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t nrows = a.limit ? (ldg(a.limit) < a.E ? ldg(a.limit) : a.E) : a.E;
-  const int64_t tiles = (nrows + kRows - 1) / kRows;
   const Share share(a);
   const Stack& stack = a.stack[share.stack];
-  const int64_t my_tiles = share.first < tiles ? (tiles - share.first + share.step - 1) / share.step : 0;
   const unsigned tmem = setup(a, stack, chain_smem, bar, w0s);
+  const int64_t nrows = a.limit ? (ldg(a.limit) < a.E ? ldg(a.limit) : a.E) : a.E;
+  const int64_t tiles = (nrows + kRows - 1) / kRows;
+  const int64_t my_tiles = share.first < tiles ? (tiles - share.first + share.step - 1) / share.step : 0;
 
   if (warp == 1) {
     mma_loop(a, bar, chain_smem, tmem, my_tiles);
@@ -319,12 +323,14 @@ static int grid_size(const Args& a) {
   return a.stacks * int(tiles < per ? tiles : per);
 }
 
+static bool one_wave(const Args& a) { return a.stacks * ((a.E + kRows - 1) / kRows) <= 148; }
+
 int launch_forward(Args a, cudaStream_t st) {
   static const cudaError_t attr =
       cudaFuncSetAttribute(mlp_chain_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
   if (attr != cudaSuccess) { set_error("mlp chain smem: %s", cudaGetErrorString(attr)); return ICTC_ERR_LAUNCH; }
   a.status = kernel_status_word();
-  mlp_chain_forward_kernel<<<grid_size(a), kThreads, kSmem, st>>>(a);
+  launch_if(one_wave(a), mlp_chain_forward_kernel, grid_size(a), kThreads, kSmem, st, a);
   return finish_launch("mlp_chain_forward");
 }
 
@@ -333,7 +339,7 @@ int launch_backward(Args a, cudaStream_t st) {
       cudaFuncSetAttribute(mlp_chain_backward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmem);
   if (attr != cudaSuccess) { set_error("mlp chain smem: %s", cudaGetErrorString(attr)); return ICTC_ERR_LAUNCH; }
   a.status = kernel_status_word();
-  mlp_chain_backward_kernel<<<grid_size(a), kThreads, kSmem, st>>>(a);
+  launch_if(one_wave(a), mlp_chain_backward_kernel, grid_size(a), kThreads, kSmem, st, a);
   return finish_launch("mlp_chain_backward");
 }
 

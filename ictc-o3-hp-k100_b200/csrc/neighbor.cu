@@ -35,7 +35,7 @@ __device__ __forceinline__ void cell_of(const NbGrid& g, const float* p, int (&c
 // Counting sort by cell: the histogram's atomic hands every atom its place inside the cell, so that the fill needs no
 // atomics.  The order inside a cell is arbitrary; the edge list does not depend on it (rows are sorted by key).
 __global__ void nb_bin_count_kernel(NbGrid g, const float* __restrict__ pos, int64_t n, int* count, int2* where) {
-  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x + pdl_enter();
   if (i >= n) return;
   int c[3];
   cell_of(g, pos + 3 * i, c);
@@ -46,7 +46,7 @@ __global__ void nb_bin_count_kernel(NbGrid g, const float* __restrict__ pos, int
 // atoms[] = (x, y, z, index) grouped by cell: a candidate costs one 16-byte load, contiguous over the lanes
 __global__ void nb_bin_fill_kernel(const float* __restrict__ pos, int64_t n, const int* __restrict__ cell_start,
                                    const int2* __restrict__ where, float4* atoms) {
-  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x + pdl_enter();
   if (i >= n) return;
   const int2 w = where[i];
   atoms[cell_start[w.x] + w.y] = make_float4(pos[3 * i], pos[3 * i + 1], pos[3 * i + 2], __int_as_float(int(i)));
@@ -148,7 +148,7 @@ __global__ void __launch_bounds__(kNbWarps * 32) nb_count_kernel(NbGrid g, const
                                                                  int64_t* rowptr, uint2* packed) {
   __shared__ NbCells cells[kNbWarps];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t i = int64_t(blockIdx.x) * kNbWarps + warp;
+  const int64_t i = int64_t(blockIdx.x) * kNbWarps + warp + pdl_enter();
   if (i >= centres) return;
   unsigned n = 0, self = 0, above = 0;
   nb_visit(g, pos, cell_start, atoms, i, lane, cells[warp], [&](bool hit, int64_t key) {
@@ -180,7 +180,7 @@ __global__ void __launch_bounds__(kNbWarps * 32) nb_fill_kernel(NbGrid g, const 
   __shared__ NbCells cells[kNbWarps];
   __shared__ int64_t stage[kNbWarps][kNbStage];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t i = int64_t(blockIdx.x) * kNbWarps + warp;
+  const int64_t i = int64_t(blockIdx.x) * kNbWarps + warp + pdl_enter();
   if (i >= centres) return;
   const int64_t begin = rowptr[i], end = rowptr[i + 1];
   if (end > capacity || begin > end) return;   // offsets must have been clamped to the capacity
@@ -307,8 +307,9 @@ __global__ void nb_pair_kernel(const int64_t* __restrict__ rowptr, const int* __
                                const int64_t* __restrict__ keys, int64_t centres, int64_t capacity,
                                int64_t unique_capacity, int64_t pad_src, int64_t* src, int64_t* dst, float* shifts,
                                int64_t* rev, int64_t* gate_row, int64_t* rep_edge, int64_t* other_edge) {
-  const int64_t e = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
-  const int64_t count = rowptr[centres], total = u_row[centres];
+  const int zero = pdl_enter();
+  const int64_t e = int64_t(blockIdx.x) * blockDim.x + threadIdx.x + zero;
+  const int64_t count = rowptr[centres + zero], total = u_row[centres + zero];
   if (e < capacity) {
     if (e < count) {
       const int64_t key = keys[e], j = key / 27, i = dst[e];
@@ -362,7 +363,7 @@ constexpr float kAccel = 9.64853321e-3f;   // 1 eV/(A amu) in A/fs^2
 __global__ void md_kick_drift_kernel(int64_t n, float dt, const float* __restrict__ force,
                                      const float* __restrict__ inv_mass, float* vel, float* pos, const float* box,
                                      int drift) {
-  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x + pdl_enter();
   if (i >= n) return;
   const float s = 0.5f * dt * kAccel * inv_mass[i];
 #pragma unroll
@@ -502,9 +503,9 @@ struct StoreRows {
 
 static void nb_bin(const NbGrid& g, const float* pos, int64_t N, int64_t cells, const NbScratch& s, cudaStream_t st) {
   cudaMemsetAsync(s.cell_count, 0, 4 * cells, st);
-  if (N > 0) nb_bin_count_kernel<<<(unsigned)((N + 255) / 256), 256, 0, st>>>(g, pos, N, s.cell_count, s.where);
+  if (N > 0) launch_after(nb_bin_count_kernel, (unsigned)((N + 255) / 256), 256, 0, st, g, pos, N, s.cell_count, s.where);
   prefix_sum<int>(cells, LoadInt{s.cell_count}, StoreCellStart{s.cell_start}, reinterpret_cast<int*>(s.sums), false, st);
-  if (N > 0) nb_bin_fill_kernel<<<(unsigned)((N + 255) / 256), 256, 0, st>>>(pos, N, s.cell_start, s.where, s.atoms);
+  if (N > 0) launch_after(nb_bin_fill_kernel, (unsigned)((N + 255) / 256), 256, 0, st, pos, N, s.cell_start, s.where, s.atoms);
 }
 
 int ictc_neighbor_count(const float* pos, int64_t num_atoms, int64_t num_centres, const double* host_lo,
@@ -522,7 +523,7 @@ int ictc_neighbor_count(const float* pos, int64_t num_atoms, int64_t num_centres
   nb_carve(scratch, num_atoms, cells, &s);
   nb_bin(g, pos, num_atoms, cells, s, st);
   if (num_centres > 0)
-    nb_count_kernel<<<(unsigned)((num_centres + kNbWarps - 1) / kNbWarps), kNbWarps * 32, 0, st>>>(
+    launch_after(nb_count_kernel, (unsigned)((num_centres + kNbWarps - 1) / kNbWarps), kNbWarps * 32, 0, st,
         g, pos, s.cell_start, s.atoms, num_centres, rowptr, nullptr);
   else
     cudaMemsetAsync(rowptr, 0, 8, st);
@@ -543,7 +544,7 @@ int ictc_neighbor_fill(const float* pos, int64_t num_atoms, int64_t num_centres,
   }
   NbScratch s;
   nb_carve(scratch, num_atoms, cells, &s);
-  nb_fill_kernel<<<(unsigned)((num_centres + kNbWarps - 1) / kNbWarps), kNbWarps * 32, 0, (cudaStream_t)stream>>>(
+  launch_after(nb_fill_kernel, (unsigned)((num_centres + kNbWarps - 1) / kNbWarps), kNbWarps * 32, 0, (cudaStream_t)stream,
       g, pos, s.cell_start, s.atoms, num_centres, rowptr, capacity, src, dst, shifts, edge_keys);
   return finish_launch("neighbor_fill");
 }
@@ -572,15 +573,15 @@ int ictc_neighbor_build(const float* pos, int64_t num_atoms, int64_t num_centres
   nb_carve(scratch, num_atoms, cells, &s);
   nb_bin(g, pos, num_atoms, cells, s, st);
   const unsigned blocks = (unsigned)((num_centres + kNbWarps - 1) / kNbWarps);
-  nb_count_kernel<<<blocks, kNbWarps * 32, 0, st>>>(g, pos, s.cell_start, s.atoms, num_centres, nullptr, s.packed);
+  launch_after(nb_count_kernel, blocks, kNbWarps * 32, 0, st, g, pos, s.cell_start, s.atoms, num_centres, nullptr, s.packed);
   // capacity - 1: the last slot always stays an inert edge
   prefix_sum<unsigned long long>(num_centres, LoadPacked{s.packed},
                                  StoreRows{rowptr, s.u_row, num_centres, capacity - 1, num_unique, overflow}, s.sums,
                                  false, st);
-  nb_fill_kernel<<<blocks, kNbWarps * 32, 0, st>>>(g, pos, s.cell_start, s.atoms, num_centres, rowptr, capacity, src,
+  launch_after(nb_fill_kernel, blocks, kNbWarps * 32, 0, st, g, pos, s.cell_start, s.atoms, num_centres, rowptr, capacity, src,
                                                   dst, shifts, edge_keys);
   const int64_t span = capacity > unique_capacity ? capacity : unique_capacity;
-  nb_pair_kernel<<<(unsigned)((span + 255) / 256), 256, 0, st>>>(rowptr, s.u_row, edge_keys, num_centres, capacity,
+  launch_after(nb_pair_kernel, (unsigned)((span + 255) / 256), 256, 0, st, rowptr, s.u_row, edge_keys, num_centres, capacity,
                                                                 unique_capacity, pad_src, src, dst, shifts, rev,
                                                                 gate_row, rep_edge, other_edge);
   return finish_launch("neighbor_build");
@@ -644,7 +645,7 @@ int ictc_md_kick(int64_t num_atoms, float dt, const float* force, const float* i
     return ICTC_ERR_BAD_ARG;
   }
   if (num_atoms == 0) return ICTC_OK;
-  md_kick_drift_kernel<<<(unsigned)((num_atoms + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
+  launch_after(md_kick_drift_kernel, (unsigned)((num_atoms + 255) / 256), 256, 0, (cudaStream_t)stream,
       num_atoms, dt, force, inv_mass, vel, pos, box, drift);
   return finish_launch("md_kick");
 }

@@ -88,7 +88,7 @@ template <class T> struct WeightLoader {
 template <class T, int LT, int MODE>
 __global__ void __launch_bounds__(128) sc_node_kernel(ScArgs a) {
   constexpr int NY = (LT + 1) * (LT + 1);
-  const int64_t idx = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  const int64_t idx = int64_t(blockIdx.x) * blockDim.x + threadIdx.x + pdl_enter();
   if (idx >= a.N * a.C) return;
   const int64_t n = idx / a.C;
   const int c = int(idx % a.C);
@@ -179,8 +179,8 @@ static int sc_check(int lmax, int target_lmax, int C, int64_t N, int S) {
 
 template <class T, int MODE> static int launch_node(int target_lmax, const ScArgs& a, cudaStream_t st) {
   const unsigned blocks = unsigned((a.N * a.C + 127) / 128);
-  if (target_lmax == 0) sc_node_kernel<T, 0, MODE><<<blocks, 128, 0, st>>>(a);
-  else sc_node_kernel<T, 2, MODE><<<blocks, 128, 0, st>>>(a);
+  if (target_lmax == 0) launch_after(sc_node_kernel<T, 0, MODE>, blocks, 128, 0, st, a);
+  else launch_after(sc_node_kernel<T, 2, MODE>, blocks, 128, 0, st, a);
   return finish_launch("sc_node_kernel");
 }
 

@@ -28,7 +28,7 @@ template <class T> __device__ __forceinline__ T block_sum(T v, T* warp_tot) {
 template <class T, class LOAD>
 __global__ void __launch_bounds__(kPrefixThreads) tile_sum_kernel(int64_t n, LOAD load, T* sums) {
   __shared__ T warp_tot[kPrefixThreads / 32];
-  const int64_t base = int64_t(blockIdx.x) * kPrefixTile;
+  const int64_t base = int64_t(blockIdx.x) * kPrefixTile + pdl_enter();
   T v = 0;
 #pragma unroll
   for (int k = 0; k < kPrefixItems; ++k) {
@@ -45,7 +45,7 @@ __global__ void __launch_bounds__(kPrefixThreads) tile_sum_kernel(int64_t n, LOA
 template <class T, class LOAD, class STORE>
 __global__ void __launch_bounds__(kPrefixThreads) prefix_kernel(int64_t n, LOAD load, STORE store, const T* sums) {
   __shared__ T warp_tot[kPrefixThreads / 32];
-  const int64_t base = int64_t(blockIdx.x) * kPrefixTile;
+  const int64_t base = int64_t(blockIdx.x) * kPrefixTile + pdl_enter();
   T before = 0;
   if (sums) {
     for (int64_t i = threadIdx.x; i < blockIdx.x; i += kPrefixThreads) before += sums[blockIdx.y * gridDim.x + i];
@@ -88,8 +88,8 @@ void prefix_sum(int64_t n, LOAD load, STORE store, T* sums, bool in_place, cudaS
   if (tiles == 0) return;
   const bool two = tiles > kPrefixDirect || (in_place && tiles > 1);
   const dim3 grid((unsigned)tiles, (unsigned)inputs);
-  if (two) tile_sum_kernel<T><<<grid, kPrefixThreads, 0, st>>>(n, load, sums);
-  prefix_kernel<T><<<grid, kPrefixThreads, 0, st>>>(n, load, store, two ? (const T*)sums : (const T*)nullptr);
+  if (two) launch_after(tile_sum_kernel<T, LOAD>, grid, kPrefixThreads, 0, st, n, load, sums);
+  launch_after(prefix_kernel<T, LOAD, STORE>, grid, kPrefixThreads, 0, st, n, load, store, two ? (const T*)sums : (const T*)nullptr);
 }
 
 }  // namespace ictc

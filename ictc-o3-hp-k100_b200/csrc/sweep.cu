@@ -39,7 +39,7 @@ struct EmbedArgs {
 };
 
 __global__ void embed_kernel(EmbedArgs a) {
-  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x + pdl_enter();
   if (i < a.graphs) a.energy[i] = 0.0;
   const int64_t row = i >> 4;
   if (row >= a.n) return;
@@ -68,7 +68,7 @@ constexpr int kWatchWords = 2048, kWatchThreads = 256;
 
 __global__ void __launch_bounds__(kWatchThreads) watch_kernel(const int64_t* __restrict__ tiles, const int* __restrict__ copy,
                                                               int* status) {
-  const int64_t t = blockIdx.x;
+  const int64_t t = blockIdx.x + pdl_enter();
   const int* now = reinterpret_cast<const int*>(ldg(tiles + 2 * t));
   const int words = int(ldg(tiles + 2 * t + 1));
   bool differ = false;
@@ -134,7 +134,7 @@ template <bool STORE> __device__ __forceinline__ void block_rows9(float* global,
 
 __global__ void __launch_bounds__(kGeoThreads) geometry_kernel(GeoArgs a) {
   __shared__ __align__(16) float rows[kGeoThreads * 9];
-  const int64_t first = int64_t(blockIdx.x) * kGeoThreads, e = first + threadIdx.x;
+  const int64_t first = int64_t(blockIdx.x) * kGeoThreads + pdl_enter(), e = first + threadIdx.x;
   if (e < a.E) {
     int64_t i = ldg(a.dst + e), j = ldg(a.src + e);
     if (a.safe_src) {
@@ -190,7 +190,7 @@ __global__ void __launch_bounds__(kGeoThreads) geometry_kernel(GeoArgs a) {
 
 __global__ void __launch_bounds__(kGeoThreads) geometry_backward_kernel(GeoArgs a) {
   __shared__ __align__(16) float rows[2][kGeoThreads * 9];
-  const int64_t first = int64_t(blockIdx.x) * kGeoThreads, e = first + threadIdx.x;
+  const int64_t first = int64_t(blockIdx.x) * kGeoThreads + pdl_enter(), e = first + threadIdx.x;
   block_rows9<false>(const_cast<float*>(a.dsh[0]), rows[0], first, a.E);
   block_rows9<false>(const_cast<float*>(a.dsh[1]), rows[1], first, a.E);
   __syncthreads();
@@ -222,7 +222,7 @@ struct GradArgs {
 };
 
 __global__ void position_gradient8_kernel(GradArgs a) {
-  const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x + pdl_enter();
   if (t < a.graphs) a.energy[t] = float(a.energy_sum[t]);
   const int64_t i = t >> 3;
   const int sub = int(t & 7);
@@ -257,13 +257,13 @@ __global__ void position_gradient8_kernel(GradArgs a) {
 // out[i] = table[index[i]]; a sender order is not filled behind its last row (inert edges have no sender), so what stands
 // there is not an index.
 __global__ void gather_index_kernel(const int64_t* __restrict__ table, const int64_t* __restrict__ index, int64_t n, int64_t* out) {
-  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
+  const int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x + pdl_enter();
   if (i >= n) return;
   const int64_t k = index[i];
   out[i] = k >= 0 && k < n ? table[k] : 0;
 }
 static int gather_index(const int64_t* table, const int64_t* index, int64_t n, int64_t* out, cudaStream_t st) {
-  if (n > 0) gather_index_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(table, index, n, out);
+  if (n > 0) launch_after(gather_index_kernel, (unsigned)((n + 255) / 256), 256, 0, st, table, index, n, out);
   return finish_launch("sweep_gather_index");
 }
 
@@ -298,7 +298,7 @@ constexpr int kTailWarps = 8, kTailNodes = 4;      // atoms per warp
 __global__ void __launch_bounds__(kTailWarps * 32) tail_kernel(TailArgs a) {
   __shared__ double block_energy[kTailWarps];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t first = (int64_t(blockIdx.x) * kTailWarps + warp) * kTailNodes;
+  const int64_t first = (int64_t(blockIdx.x) * kTailWarps + warp) * kTailNodes + pdl_enter();
   const float2 ro = __ldg(reinterpret_cast<const float2*>(a.ro0) + lane);
   double sum = 0.0;
   int64_t graph = -1;
@@ -514,12 +514,12 @@ int Runner::run() {
   call(1, -1, 1, [&] {
     EmbedArgs a{p.numbers, p.species_table, p.species_table_size, p.species, p.up0_table, u0, energy, p.graphs, N, p.batch, p.status};
     const int64_t threads = 16 * N > p.graphs ? 16 * N : p.graphs;
-    if (threads > 0) embed_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(a);
+    if (threads > 0) launch_after(embed_kernel, (unsigned)((threads + 255) / 256), 256, 0, st, a);
     return finish_launch("sweep_embed");
   });
   if (p.watch_count > 0)
     call(1, -1, 1, [&] {
-      watch_kernel<<<(unsigned)p.watch_count, kWatchThreads, 0, st>>>(p.watch_tiles, p.watch_copy, p.status);
+      launch_after(watch_kernel, (unsigned)p.watch_count, kWatchThreads, 0, st, p.watch_tiles, p.watch_copy, p.status);
       return finish_launch("sweep_watch");
     });
   const int64_t *dst_rowptr = p.dst_rowptr, *dst_order = p.dst_order, *src_rowptr = p.src_rowptr, *src_order = p.src_order;
@@ -567,7 +567,7 @@ int Runner::run() {
   geo.rb = buffer(U * p.num_basis);
   const unsigned geo_blocks = (unsigned)((E + kGeoThreads - 1) / kGeoThreads);
   call(1, -1, 1, [&] {
-    if (E > 0) geometry_kernel<<<geo_blocks, kGeoThreads, 0, st>>>(geo);
+    if (E > 0) launch_after(geometry_kernel, geo_blocks, kGeoThreads, 0, st, geo);
     return finish_launch("sweep_geometry");
   });
   float* pre[2][3];
@@ -650,7 +650,7 @@ int Runner::run() {
   call(4, -1, 1, [&] {
     TailArgs a{y1, features, W0, p.species, p.readout_rp, p.readout_rs, p.readout_w2, p.readout_ro0, int(p.hidden),
                p.row_mask, p.batch, p.graphs, int(p.mask_atomic), p.atomic, energy, dy1, dh, n};
-    if (n > 0) tail_kernel<<<(unsigned)((n + kTailWarps * kTailNodes - 1) / (kTailWarps * kTailNodes)), kTailWarps * 32, 0, st>>>(a);
+    if (n > 0) launch_after(tail_kernel, (unsigned)((n + kTailWarps * kTailNodes - 1) / (kTailWarps * kTailNodes)), kTailWarps * 32, 0, st, a);
     return finish_launch("sweep_tail");
   });
   float* dm = buffer(n * W0);
@@ -751,14 +751,14 @@ int Runner::run() {
   }
   geo.dvec = dvec;
   call(16, -1, 1, [&] {
-    if (E > 0) geometry_backward_kernel<<<geo_blocks, kGeoThreads, 0, st>>>(geo);
+    if (E > 0) launch_after(geometry_backward_kernel, geo_blocks, kGeoThreads, 0, st, geo);
     return finish_launch("sweep_geometry_backward");
   });
   call(16, -1, 1, [&] {
     GradArgs a{N, n, dst_rowptr, dst_order, src_rowptr, src_order, dvec, float(p.gradient_sign), p.gradient, energy,
                p.energy, p.graphs};
     const int64_t threads = 8 * N > p.graphs ? 8 * N : p.graphs;
-    if (threads > 0) position_gradient8_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, st>>>(a);
+    if (threads > 0) launch_after(position_gradient8_kernel, (unsigned)((threads + 255) / 256), 256, 0, st, a);
     return finish_launch("sweep_position_gradient");
   });
   return rc;

@@ -143,7 +143,7 @@ tp_graph_forward_tma_kernel(TpArgs a) {
   constexpr int C = L::C;
   extern __shared__ __align__(128) unsigned char tma_smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t n = SPLIT > 1 ? int64_t(blockIdx.x) : int64_t(blockIdx.x) * kTmaWarps + warp;
+  int64_t n = SPLIT > 1 ? int64_t(blockIdx.x) : int64_t(blockIdx.x) * kTmaWarps + warp;
   if (n >= a.N) return;
   unsigned char* mine = tma_smem + warp * L::WARP_BYTES;
   const unsigned bars = smem_addr(mine + L::BAR_OFF);
@@ -160,6 +160,7 @@ tp_graph_forward_tma_kernel(TpArgs a) {
   V acc[S::NO];
 #pragma unroll
   for (int k = 0; k < S::NO; ++k) acc[k] = V::dup(0.f);
+  n += pdl_enter();
   int64_t begin = ldg(a.rowptr + n), end = ldg(a.rowptr + n + 1);
   if (SPLIT > 1) {
     const int64_t len = end - begin;
@@ -278,7 +279,7 @@ __global__ void __launch_bounds__(split_warps(SPLIT) * 32, kTmaMinWarpsAdj / spl
   constexpr int C = L::C;
   extern __shared__ __align__(128) unsigned char tma_smem[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t owner = SPLIT > 1 ? int64_t(blockIdx.x) : int64_t(blockIdx.x) * kTmaWarps + warp;
+  int64_t owner = SPLIT > 1 ? int64_t(blockIdx.x) : int64_t(blockIdx.x) * kTmaWarps + warp;
   if (owner >= (GRAPH ? a.N : a.E)) return;
   unsigned char* mine = tma_smem + warp * L::WARP_BYTES;
   const unsigned bars = smem_addr(mine + L::BAR_OFF);
@@ -292,6 +293,7 @@ __global__ void __launch_bounds__(split_warps(SPLIT) * 32, kTmaMinWarpsAdj / spl
   BTerm bt[L::R];
 #pragma unroll
   for (int r = 0; r < L::R; ++r) bt[r] = (r * 32 + lane < F::NB) ? F::ap(r * 32 + lane) : BTerm{0, 0.f, 0, 0.f};
+  owner += pdl_enter();
   V x[S::NX], dx[S::NX];
   {
     const float* xp = a.x + owner * (S::NX * C) + lane * CPL;
@@ -471,7 +473,7 @@ template <class S, class F, int CPL, int SPLIT> int launch_graph_forward_tma(con
   static const int attr = set_smem(kernel, L::WARP_BYTES * warps);
   if (attr != ICTC_OK) return attr;
   const int64_t blocks = SPLIT > 1 ? a.N : (a.N + kTmaWarps - 1) / kTmaWarps;
-  kernel<<<(unsigned)blocks, warps * 32, L::WARP_BYTES * warps, st>>>(a);
+  launch_after(kernel, (unsigned)blocks, warps * 32, L::WARP_BYTES * warps, st, a);
   return finish_launch("tp_graph_forward_tma");
 }
 
@@ -484,7 +486,7 @@ int launch_adjoint_tma_plain(const TpArgs& a, cudaStream_t st) {
   if (attr != ICTC_OK) return attr;
   const int64_t owners = GRAPH ? a.N : a.E;
   const int64_t blocks = SPLIT > 1 ? owners : (owners + kTmaWarps - 1) / kTmaWarps;
-  kernel<<<(unsigned)blocks, warps * 32, L::WARP_BYTES * warps, st>>>(a);
+  launch_after(kernel, (unsigned)blocks, warps * 32, L::WARP_BYTES * warps, st, a);
   return finish_launch("tp_adjoint_tma");
 }
 
