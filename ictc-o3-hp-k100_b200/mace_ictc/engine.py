@@ -72,6 +72,7 @@ class ForceEngine:
         self.lib = _lib.load()
         self._weights = None
         self._watched = None
+        self._fit = None         # (state of the model, do its sizes fit the sweep?)
         self.chunk_rows = None if chunk_rows is None else int(chunk_rows)
         self.chunk_margin = float(chunk_margin)
         # with chunks: True = the gates are streamed too (produced per chunk in the forward sweep, recomputed per chunk
@@ -94,28 +95,31 @@ class ForceEngine:
                 slots.extend((table, key, value) for key, value in table.items())
         params = list(self.model.parameters())
         inter = list(self.model.interactions)
-        return slots, modules, params, inter
+        own = [module.__dict__ for module in modules]
+        hooks = [d[name] for d in own for name in _HOOKS]
+        return slots, modules, params, inter, all(type(module) in _KNOWN for module in modules), own, hooks
 
     def _state(self):
-        _, _, params, inter = self._watched
+        params, inter = self._watched[2:4]
         m = self.model
         return ([(p._version, p.data_ptr()) for p in params], [i.avg_num_neighbors for i in inter], m.max_radius,
                 m.polynomial_cutoff_p, m.number_of_basis)
 
     def stands_for(self):
         """Does the sweep compute what the model's own ``forward`` would?  Not with hooks, with modules of other types or
-        with a replaced ``forward``, with base coefficients that still require grad, or with other widths."""
+        with a replaced ``forward``, with base coefficients that still require grad, or with other widths.  Returns the state of
+        the model for ``energy_and_forces``, or None."""
         if self._watched is None or self._replaced():
-            self._watched, self._weights = self._watch(), None
-        modules, inter = self._watched[1], self._watched[3]
+            self._watched, self._weights, self._fit = self._watch(), None, None
+        _, modules, _, inter, known, own, hooks = self._watched
         table = torch.nn.modules.module
-        if any(getattr(table, name) for name in _GLOBAL_HOOKS):
-            return False
-        for m in modules:
-            own = m.__dict__
-            if type(m) not in _KNOWN or "forward" in own or any(own[name] for name in _HOOKS):
-                return False
-        return not any(i.tp.weight.requires_grad for i in inter) and self._sizes_fit()
+        if (not known or any(getattr(table, name) for name in _GLOBAL_HOOKS) or any(hooks)
+                or any("forward" in d for d in own) or any(i.tp.weight.requires_grad for i in inter)):
+            return None
+        state, fit = self._state(), self._fit
+        if fit is None or fit[0] != state:
+            fit = self._fit = state, self._sizes_fit()
+        return state if fit[1] else None
 
     def _sizes_fit(self):
         m = self.model
@@ -132,11 +136,12 @@ class ForceEngine:
     def _replaced(self):
         return any(table.get(key) is not value for table, key, value in self._watched[0])
 
-    def refresh(self):
-        """(Re)build the GEMM-ready weight views when a parameter changed."""
-        if self._watched is None or self._replaced():
-            self._watched, self._weights = self._watch(), None
-        state = self._state()
+    def refresh(self, state=None):
+        """(Re)build the GEMM-ready weight views when a parameter changed.  ``state``: what ``stands_for`` has just found."""
+        if state is None:
+            if self._watched is None or self._replaced():
+                self._watched, self._weights, self._fit = self._watch(), None, None
+            state = self._state()
         w, stream = self._weights, torch.cuda.current_stream(self.dev)
         if w is None or w.state != state:
             with _lib.on_device(self.dev):
@@ -368,13 +373,13 @@ class ForceEngine:
         return energy[0], grad, atomic
 
     @torch.no_grad()
-    def energy_and_forces(self, pos, numbers, batch, src, dst, shifts, cell, row_mask, check):
+    def energy_and_forces(self, pos, numbers, batch, src, dst, shifts, cell, row_mask, check, state=None):
         """(energy per graph, forces, per-atom energies) of a graph whose edges the caller has built, in any order.
         ``check`` raises ValueError on an atomic number outside the model; a graph or edge index outside its range always
         does."""
         if self._weights is not None and self._weights.tiles is None:
             self._weights = None
-        w, dev = self.refresh(), self.dev
+        w, dev = self.refresh(state), self.dev
         n, graphs = pos.shape[0], cell.shape[0]
         with _lib.on_device(dev):
             energy = torch.empty(graphs, dtype=torch.float32, device=dev)

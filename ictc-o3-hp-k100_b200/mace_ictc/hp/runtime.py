@@ -75,7 +75,8 @@ def _force_engine(model, tensors, mask):
             return None
         engine = ForceEngine(model, lay_out=False)
         model.__dict__["_force_engine"] = engine
-    return engine if engine.stands_for() else None
+    state = engine.stands_for()
+    return None if state is None else (engine, state)
 
 
 def energy_and_forces(model, positions, atomic_numbers, batch, edge_src, edge_dst, edge_shifts, cell, *,
@@ -106,15 +107,16 @@ def energy_and_forces(model, positions, atomic_numbers, batch, edge_src, edge_ds
         if tuple(owned_mask.shape) != (count,) or owned_mask.requires_grad:
             raise ValueError(f"owned_mask: expected a constant tensor of shape [{count}]")
     if not training:
-        engine = _force_engine(model, (positions, atomic_numbers, batch, edge_src, edge_dst, edge_shifts, cell), owned_mask)
-        if engine is not None:
+        found = _force_engine(model, (positions, atomic_numbers, batch, edge_src, edge_dst, edge_shifts, cell), owned_mask)
+        if found is not None:
             strict_fp32()
+            engine, state = found
             dtype = torch.float32
             mask = None if owned_mask is None else owned_mask.to(dtype).contiguous()
             energy, forces, per_atom = engine.energy_and_forces(
                 positions.detach().contiguous(), atomic_numbers.long().contiguous(), batch.long().contiguous(),
                 edge_src.long().contiguous(), edge_dst.long().contiguous(), edge_shifts.detach().to(dtype).contiguous(),
-                cell.detach().to(dtype).contiguous(), mask, not model.skip_input_validation)
+                cell.detach().to(dtype).contiguous(), mask, not model.skip_input_validation, state)
             return {"energy": energy, "forces": forces, "atomic_energy": per_atom}
     with torch.enable_grad():
         coords = positions if positions.requires_grad else positions.detach().requires_grad_(True)
