@@ -69,6 +69,10 @@ SIGNATURES = {
     "ictc_silu_forward": (_I, [_L, C.c_float, _P, _P, _P]),
     "ictc_silu_backward": (_I, [_L, C.c_float, _P, _P, _P, _P]),
     "ictc_silu_second": (_I, [_L, C.c_float, _P, _P, _P, _P, _P, _P]),
+    "ictc_narrow_linear_forward": (_I, [_L, _P, _P, _P, _P]),
+    "ictc_narrow_linear_input_grad": (_I, [_L, _P, _P, _P, _P]),
+    "ictc_narrow_linear_workspace": (_L, [_L]),
+    "ictc_narrow_linear_weight_grad": (_I, [_L, _P, _P, _P, _P, _P]),
     "ictc_layout_copy": (_I, [_L, _I, _I, C.POINTER(C.c_int), C.POINTER(C.c_int), _P, _P, _I, _P]),
     "ictc_harmonics_forward": (_I, [_I, _L, _P, _P, _P]),
     "ictc_harmonics_vjp": (_I, [_I, _L, _P, _P, _P, _P]),

@@ -23,6 +23,7 @@ from torch import nn
 from ictc_o3.basis.ictd_irreps import EdgeWeightedPathPreservingTensorProduct
 from ictc_o3.operators import (PackedGraphMessage, _RowsTimesWeight, _tc_eligible, channel_linear, convert_layout,
                                direction_harmonics, normalized_silu, strict_fp32)
+from ictc_o3.ops.narrow_linear import NarrowLinear, narrow_takes
 from ictc_o3.symmetric_contraction import ICTDBridgeUSymmetricContractionSO3
 
 SILU_SCALE = 1.6791767923989418
@@ -153,11 +154,14 @@ class InteractionBlock(nn.Module):
 
     def radial_gates(self, edge_feats):
         """The gate MLP; layers whose sides are multiples of 64 (the hidden layers and the wide last one) run on
-        the tcgen05 channel-linear kernel, the narrow first layer on the library GEMM."""
+        the tcgen05 channel-linear kernel, the narrow first layer (8 radial functions) on kernels of its own."""
         h = edge_feats
         for mod in self.fc:
             if isinstance(mod, nn.Linear) and _tc_eligible(h, mod.weight):
                 h = _RowsTimesWeight.apply(h, mod.weight)
+            elif (type(mod) is nn.Linear and mod.bias is None and narrow_takes(h, mod.weight)
+                  and not (mod._forward_hooks or mod._forward_pre_hooks or mod._backward_hooks or mod._backward_pre_hooks)):
+                h = NarrowLinear.apply(h, mod.weight)
             else:
                 h = mod(h)
         return h

@@ -272,6 +272,13 @@ int ictc_silu_backward(int64_t n, float scale, const float* x, const float* dy, 
  * (mode 2 of the same reference kernel). */
 int ictc_silu_second(int64_t n, float scale, const float* x, const float* dy, const float* h, float* gx, float* gdy,
                      void* stream);
+/* Linear map from 8 to 64 columns, y = x w^T over rows, with its input gradient g w and its weight gradient g^T x (fixed
+ * summation order; workspace of ictc_narrow_linear_workspace(rows) bytes).  16-byte aligned buffers.  The first layer of the
+ * radial stack (mace_ictc/models/mace/layers.py:825-835). */
+int ictc_narrow_linear_forward(int64_t rows, const float* x, const float* w, float* y, void* stream);
+int ictc_narrow_linear_input_grad(int64_t rows, const float* g, const float* w, float* dx, void* stream);
+int64_t ictc_narrow_linear_workspace(int64_t rows);
+int ictc_narrow_linear_weight_grad(int64_t rows, const float* g, const float* x, float* dw, float* workspace, void* stream);
 /* Whole-row conversion between the model-native mul_ir layout (every block [C, 2l+1], channel outer) and the
  * kernel-native ir_mul layout (every block [2l+1, C], channel contiguous) in one launch.  A row is a sequence of
  * num_blocks degree blocks; block b holds host_counts[b] path slots of host_ms[b] components each (HOST int

@@ -1,0 +1,30 @@
+"""The 8 -> 64 linear map and its first and second derivatives against float64, around its blocks and on shifted buffers."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+EPS = 2.0 ** -24
+
+
+@pytest.mark.parametrize("rows,shift", [(1, 0), (15, 1), (17, 0), (129, 0), (18945, 0), (100003, 0)])
+def test_value_and_derivatives(rows, shift):
+    from ictc_o3.ops.narrow_linear import NarrowLinear, narrow_takes
+    gen = torch.Generator("cuda").manual_seed(rows)
+    make = lambda *s: torch.randn(s[0] * s[1] + shift, device="cuda", generator=gen)[shift:].reshape(s)     # noqa: E731
+    x, w, g, hx, hw = make(rows, 8), make(64, 8), make(rows, 64), make(rows, 8), make(64, 8)
+    assert narrow_takes(x, w)
+
+    def chain(f, x, w, g, hx, hw):
+        x, w, g = (t.clone() if t.dtype == torch.float64 else t for t in (x, w, g))
+        x, w, g = (t.detach().requires_grad_(True) for t in (x, w, g))
+        y = f(x, w)
+        first = torch.autograd.grad(y, [x, w], g, create_graph=True)
+        return [y.detach(), *(t.detach() for t in first), *torch.autograd.grad(first, [x, w, g], [hx, hw])]
+
+    got = chain(NarrowLinear.apply, x, w, g, hx, hw)
+    d = [t.double() for t in (x, w, g, hx, hw)]
+    want = chain(lambda a, b: a @ b.t(), *d)
+    size = chain(lambda a, b: a @ b.t(), *[t.abs() for t in d])          # sums of the terms' magnitudes
+    # a sum of n terms in 32 bits is off by at most n half-units of that; random signs leave far less: 8 + sqrt(rows)
+    for a, b, s in zip(got, want, size):
+        assert float(((a.double() - b).abs() - (16 + rows ** 0.5) * EPS * s).max()) <= 0.0
