@@ -41,6 +41,10 @@ __device__ __forceinline__ int pdl_enter() {
 constexpr int64_t kEarlyBlocks = 148 * 8;
 template <class... P, class... A>
 inline void launch_if(bool early, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+  if (!early) {
+    kernel<<<grid, block, smem, st>>>(P(args)...);
+    return;
+  }
   cudaLaunchAttribute attr{};
   attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr.val.programmaticStreamSerializationAllowed = 1;
@@ -50,7 +54,7 @@ inline void launch_if(bool early, void (*kernel)(P...), dim3 grid, dim3 block, s
   cfg.dynamicSmemBytes = smem;
   cfg.stream = st;
   cfg.attrs = &attr;
-  cfg.numAttrs = early ? 1 : 0;
+  cfg.numAttrs = 1;
   cudaLaunchKernelEx(&cfg, kernel, P(args)...);
 }
 template <class... P, class... A>
