@@ -26,8 +26,9 @@ import threading
 
 import torch
 
-from ictc_o3 import _lib
+from ictc_o3 import _lib, tables
 from ictc_o3.basis.ictd_irreps import EdgeWeightedPathPreservingTensorProduct
+from ictc_o3.operators import EdgeTensorProduct, PackedGraphMessage
 from ictc_o3.ops.topology import build_csr
 from ictc_o3.symmetric_contraction import ICTDBridgeUSymmetricContractionSO3, _Contraction, _Contractions
 from .model import (ElementConditionedLinearSO3, EquivariantChannelLinearSO3, InteractionBlock, MaceIctcModel, MLPReadout,
@@ -39,14 +40,69 @@ _LABELS = ("radial_mlp_hidden_forward_{nout}", "gate_gemm_forward_{nout}", "grap
            "channel_linear_tc", "symmetric_contraction_l{layer}")
 _MARKS = 1024            # timed launches of one sweep (eager steps of a benchmark)
 _WATCH_WORDS = 2048      # words of a parameter that one block of the sweep compares
-_KNOWN = frozenset((ElementConditionedLinearSO3, EquivariantChannelLinearSO3, InteractionBlock, MaceIctcModel, MLPReadout,
-                    Normalize2MomSiLU, PathPreservingLinearSO3, ProductBlock, ScalarReadout, torch.nn.Linear,
-                    torch.nn.ModuleDict, torch.nn.ModuleList, torch.nn.ParameterDict, torch.nn.ParameterList,
-                    torch.nn.Sequential, EdgeWeightedPathPreservingTensorProduct, ICTDBridgeUSymmetricContractionSO3,
-                    _Contraction, _Contractions))
 _HOOKS = ("_forward_hooks", "_forward_pre_hooks", "_backward_hooks", "_backward_pre_hooks")
 _GLOBAL_HOOKS = ("_global_forward_hooks", "_global_forward_pre_hooks", "_global_backward_hooks", "_global_backward_pre_hooks")
 _local = threading.local()
+
+
+def _linear(module, rows, cols, bias=False):
+    """A Linear of this shape (rows None: any) and nothing else; without a bias where the bias would count."""
+    return (type(module) is torch.nn.Linear and (bias or module.bias is None) and module.weight.shape[1] == cols
+            and (rows is None or module.weight.shape[0] == rows))
+
+
+def _table(params, degrees, shape_of):
+    return type(params) is torch.nn.ParameterDict and all(
+        str(l) in params and tuple(params[str(l)].shape) == shape_of(l) for l in degrees)
+
+
+def _has(module, kind, **attributes):
+    return type(module) is kind and all(getattr(module, k, None) == v for k, v in attributes.items())
+
+
+def covers(m):
+    """Is every module at its place the one whose forward the sweep reproduces, with the shapes that the layout reads and
+    nothing (a bias, another activation, a further output) that it does not read?"""
+    c, species = 64, getattr(m, "num_elements", None)
+    if not (_has(m, MaceIctcModel, channels=c, lmax=2, num_interaction=2) and _linear(m.node_embedding, c, species, bias=True)
+            and all(_has(x, torch.nn.ModuleList) for x in (m.interactions, m.products, m.layer_energy_readouts))
+            and len(m.interactions) == len(m.products) == 2 and len(m.layer_energy_readouts) >= 1):
+        return False
+    first, last = m.layer_energy_readouts[0], m.last_layer_energy_readout
+    if not (_has(first, ScalarReadout, channels=c) and _linear(first.readout, 1, c)
+            and _has(last, MLPReadout) and _linear(last.linear_1, None, c) and _has(last.activation, Normalize2MomSiLU)
+            and _linear(last.linear_2, 1, last.linear_1.weight.shape[0])):
+        return False
+    for inter, prod, l_in, l_out in zip(m.interactions, m.products, (0, 2), (2, 0)):
+        if not (_has(inter, InteractionBlock, channels=c, lmax=2, input_lmax=l_in, sc_lmax=0)
+                and _has(inter.tp, EdgeWeightedPathPreservingTensorProduct, channels=c, internal_compute_dtype=torch.float32)
+                and [tuple(path) for path in inter.tp.paths] == tables.natural_paths(l_in, 2, 2)
+                and tuple(inter.tp.weight.shape) == (len(inter.tp.paths), c)):
+            return False
+        op = inter._message                    # made by the first forward of the model
+        if op is not None and not (type(op) is PackedGraphMessage and type(op.edge) is EdgeTensorProduct and op.tp is inter.tp):
+            return False
+        if not (_has(inter.fc, torch.nn.Sequential) and len(inter.fc) == 7
+                and all(_has(inter.fc[k], Normalize2MomSiLU) for k in (1, 3, 5))
+                and all(_linear(inter.fc[k], *shape) for k, shape in
+                        ((0, (64, m.number_of_basis)), (2, (64, 64)), (4, (64, 64)), (6, (inter.tp.num_paths * c, 64))))):
+            return False
+        up, ml, sc = inter.linear_up, inter.message_linear, inter.self_connection
+        if not (_has(up, EquivariantChannelLinearSO3, channels=c, lmax=l_in) and _has(up.adapters, torch.nn.ModuleDict)
+                and all(str(l) in up.adapters and _linear(up.adapters[str(l)], c, c, bias=True) for l in range(l_in + 1))
+                and _has(ml, PathPreservingLinearSO3, out_channels=c, lmax=2)
+                and _table(ml.weights, range(3), lambda l: (c, c * inter.tp.path_counts_by_l[l]))
+                and _has(sc, ElementConditionedLinearSO3, channels=c, lmax=0, num_elements=species)
+                and _table(sc.weights, (0,), lambda l: (species, c, c))):
+            return False
+        con = prod.symmetric_contractions if _has(prod, ProductBlock, channels=c, lmax=2, target_lmax=l_out) else None
+        if not (_has(con, ICTDBridgeUSymmetricContractionSO3, channels=c, lmax=2, target_lmax=l_out, num_elements=species,
+                     ir_mul=False)
+                and _has(con.symmetric_contractions, _Contractions)
+                and all(_has(x, _Contraction) for x in con.symmetric_contractions.contractions)
+                and _table(prod.linear, range(l_out + 1), lambda l: (c, c))):
+            return False
+    return True
 
 
 class _Weights:
@@ -88,16 +144,18 @@ class ForceEngine:
 
     # ---------------------------------------------------------------- weights
     def _watch(self):
-        """Every module and parameter slot of the model with what it holds now: a replaced one is noticed by identity."""
-        slots, modules = [], list(self.model.modules())
+        """Every module and parameter slot of the model with what it holds now: a replaced one is noticed by identity, a new
+        one by the size of its table."""
+        slots, sizes, modules = [], [], list(self.model.modules())
         for module in modules:
             for table in (module._modules, module._parameters, module._buffers):
+                sizes.append((table, len(table)))
                 slots.extend((table, key, value) for key, value in table.items())
         params = list(self.model.parameters())
         inter = list(self.model.interactions)
         own = [module.__dict__ for module in modules]
         hooks = [d[name] for d in own for name in _HOOKS]
-        return slots, modules, params, inter, all(type(module) in _KNOWN for module in modules), own, hooks
+        return slots, sizes, params, inter, covers(self.model), own, hooks
 
     def _state(self):
         params, inter = self._watched[2:4]
@@ -106,14 +164,14 @@ class ForceEngine:
                 m.polynomial_cutoff_p, m.number_of_basis)
 
     def stands_for(self):
-        """Does the sweep compute what the model's own ``forward`` would?  Not with hooks, with modules of other types or
-        with a replaced ``forward``, with base coefficients that still require grad, or with other widths.  Returns the state of
-        the model for ``energy_and_forces``, or None."""
+        """Does the sweep compute what the model's own ``forward`` would?  Not with hooks, with other modules than those it was
+        written for (``covers``), with a replaced ``forward``, with base coefficients that still require grad, or with other
+        widths.  Returns the state of the model for ``energy_and_forces``, or None."""
         if self._watched is None or self._replaced():
             self._watched, self._weights, self._fit = self._watch(), None, None
-        _, modules, _, inter, known, own, hooks = self._watched
+        _, _, _, inter, covered, own, hooks = self._watched
         table = torch.nn.modules.module
-        if (not known or any(getattr(table, name) for name in _GLOBAL_HOOKS) or any(hooks)
+        if (not covered or any(getattr(table, name) for name in _GLOBAL_HOOKS) or any(hooks)
                 or any("forward" in d for d in own) or any(i.tp.weight.requires_grad for i in inter)):
             return None
         state, fit = self._state(), self._fit
@@ -122,19 +180,14 @@ class ForceEngine:
         return state if fit[1] else None
 
     def _sizes_fit(self):
-        m = self.model
-        if m.channels != 64 or len(m.interactions) != 2 or not 1 <= m.number_of_basis <= 8 or m.polynomial_cutoff_p < 2:
-            return False
-        if not m.max_radius > 0 or any(p.dtype != torch.float32 or p.device != self.dev for p in self._watched[2]):
-            return False
-        for inter in m.interactions:
-            shapes = [tuple(x.weight.shape) if type(x) is torch.nn.Linear and x.bias is None else None for x in inter.fc]
-            if shapes != [(64, m.number_of_basis), None, (64, 64), None, (64, 64), None, (inter.tp.num_paths * 64, 64)]:
-                return False
-        return True
+        m, index = self.model, self.model.atomic_number_to_index
+        return (type(m.number_of_basis) is int and 1 <= m.number_of_basis <= 8 and type(m.polynomial_cutoff_p) is int
+                and m.polynomial_cutoff_p >= 2 and m.max_radius > 0 and index.dtype == torch.int64 and index.device == self.dev
+                and index.is_contiguous() and all(p.dtype == torch.float32 and p.device == self.dev for p in self._watched[2]))
 
     def _replaced(self):
-        return any(table.get(key) is not value for table, key, value in self._watched[0])
+        return (any(table.get(key) is not value for table, key, value in self._watched[0])
+                or any(len(table) != size for table, size in self._watched[1]))
 
     def refresh(self, state=None):
         """(Re)build the GEMM-ready weight views when a parameter changed.  ``state``: what ``stands_for`` has just found."""
@@ -162,6 +215,10 @@ class ForceEngine:
         m, c, w = self.model, self.c, _Weights()
         if any(p.dtype != torch.float32 or p.device != self.dev for p in self._watched[2]):
             raise ValueError("the force engine needs float32 parameters on one CUDA device")
+        if not self._watched[4] or not self._sizes_fit():
+            raise ValueError("the force engine reproduces the forward of the stock model with a radial MLP num_basis (<= 8) -> 64 "
+                             "-> 64 -> 64 -> P*C and readouts without biases; a model with other modules runs on the "
+                             "autograd route (MolecularDynamics(..., use_engine=False))")
         w.keep, w.struct = [], _lib.Sweep()
 
         def hold(t):
@@ -173,9 +230,6 @@ class ForceEngine:
             w.nout = []
             for k, (inter, prod) in enumerate(zip(m.interactions, m.products)):
                 fc = [mod.weight.contiguous() for mod in inter.fc if isinstance(mod, torch.nn.Linear)]
-                if not (len(fc) == 4 and fc[0].shape[0] == 64 and fc[0].shape[1] <= 8 and tuple(fc[1].shape) == (64, 64)
-                        and tuple(fc[2].shape) == (64, 64) and fc[3].shape[1] == 64 and fc[3].shape[0] % 64 == 0):
-                    raise ValueError("the force engine needs the radial MLP num_basis (<= 8) -> 64 -> 64 -> 64 -> P*C")
                 L = w.struct.layer[k]
                 L.w0 = hold(fc[0])
                 L.hid = (hold(self._pack(fc[1], 0)), hold(self._pack(fc[2], 0)))

@@ -210,8 +210,8 @@ class MolecularDynamics:
     ``skin``: extra halo width of the decomposed run (see the module text).  ``chunk_rows``: owner rows per
     chunk of the force engine's streamed gate evaluation (None: whole tables) and ``stream_gates`` whether the
     gates themselves are streamed or only their gradient (``ForceEngine.stream_gates``).  ``use_engine``: None picks the
-    tape-free force engine for the 64-channel two-interaction model and autograd through the same kernels
-    otherwise.  ``watch_peers``: check before every block of steps that all ranks are still there.
+    tape-free force engine for the models it reproduces (``engine.covers``: 64 channels, two interactions, the stock modules)
+    and autograd through the same kernels otherwise.  ``watch_peers``: check before every block of steps that all ranks are still there.
     ``capture_collectives``: whether ``enable_graph`` of a decomposed run records the step, collectives included, as
     one CUDA graph.  On four ranks the replay of such a graph never completed with the collective library's defaults
     (every rank waiting in the host read after the replays; the same step run eagerly before it was fine; no GPU
@@ -281,10 +281,10 @@ class MolecularDynamics:
         self.species = species_all.index_select(0, mine)
         self.masses = torch.as_tensor(masses_all, dtype=torch.float32).to(dev).index_select(0, mine)
         self.inv_mass = (1.0 / self.masses).contiguous()
-        if use_engine is None:       # the tape-free engine exists for the 64-channel model; other widths differentiate
-            use_engine = model.channels == 64 and len(model.interactions) == 2      # through the same kernels by autograd
+        from .engine import ForceEngine, covers
+        if use_engine is None:       # the tape-free engine exists for the stock 64-channel model; other widths and modules
+            use_engine = covers(model)                                              # differentiate through the same kernels by autograd
         if use_engine:
-            from .engine import ForceEngine
             self.engine = ForceEngine(model, chunk_rows=chunk_rows, stream_gates=stream_gates)
         else:
             self.engine = None

@@ -111,6 +111,36 @@ def test_parameter_updates_replacement_copies_and_hooks():
     _close(energy_and_forces(model, *graph), _autograd(model, graph))
 
 
+def test_models_with_other_readouts_answer_through_their_own_forward():
+    from mace_ictc.hp import energy_and_forces
+    from mace_ictc.md import MolecularDynamics
+    from mace_ictc.model import MLPReadout
+    graph = _graph(np.random.default_rng(8), (45,), False)
+
+    def linear(rows, cols, bias):
+        return torch.nn.Linear(cols, rows, bias=bias, device="cuda")
+
+    changes = [lambda m: setattr(m.last_layer_energy_readout, "linear_2", linear(1, 16, True)),
+               lambda m: setattr(m.last_layer_energy_readout, "linear_1", linear(16, 64, True)),
+               lambda m: setattr(m.layer_energy_readouts[0], "readout", linear(1, 64, True)),
+               lambda m: setattr(m.last_layer_energy_readout, "linear_2", linear(3, 16, False)),
+               lambda m: setattr(m.last_layer_energy_readout, "activation", torch.nn.Sequential()),
+               lambda m: m.interactions[1].fc.__setitem__(1, torch.nn.Sequential()),
+               lambda m: m.layer_energy_readouts.__setitem__(0, MLPReadout(9 * 64).cuda())]
+    for change in changes:
+        model = _model()
+        stock = energy_and_forces(model, *graph)
+        change(model)
+        got, want = energy_and_forces(model, *graph), _autograd(model, graph)
+        _close(got, want)
+        assert float((got["atomic_energy"] - stock["atomic_energy"]).abs().max()) > 1e-3      # the change does something
+        box = np.full(3, 12.0)
+        md = MolecularDynamics(model, graph[0].cpu().numpy() % 12.0, graph[1].cpu().numpy(), box)
+        ref = MolecularDynamics(model, graph[0].cpu().numpy() % 12.0, graph[1].cpu().numpy(), box, use_engine=False)
+        md.compute_forces(), ref.compute_forces()
+        assert abs(float(md.energy) - float(ref.energy)) < TOL * abs(float(ref.energy))
+
+
 def test_weights_laid_out_on_another_stream():
     from mace_ictc.hp import energy_and_forces
     model = _model()
