@@ -427,10 +427,9 @@ class ForceEngine:
         return energy[0], grad, atomic
 
     @torch.no_grad()
-    def energy_and_forces(self, pos, numbers, batch, src, dst, shifts, cell, row_mask, check, state=None):
+    def energy_and_forces(self, pos, numbers, batch, src, dst, shifts, cell, row_mask, state=None):
         """(energy per graph, forces, per-atom energies) of a graph whose edges the caller has built, in any order.
-        ``check`` raises ValueError on an atomic number outside the model; a graph or edge index outside its range always
-        does."""
+        An atomic number that the model does not know and a graph or edge index outside its range raise ValueError."""
         if self._weights is not None and self._weights.tiles is None:
             self._weights = None
         w, dev = self.refresh(state), self.dev
@@ -458,8 +457,8 @@ class ForceEngine:
             bits, by_dst, by_src = flags.tolist()
         if bits & 4:                     # a parameter was written behind its version counter
             self._weights = None
-            return self.energy_and_forces(pos, numbers, batch, src, dst, shifts, cell, row_mask, check)
-        if bits & 1 and check:
+            return self.energy_and_forces(pos, numbers, batch, src, dst, shifts, cell, row_mask)
+        if bits & 1:
             raise ValueError(f"Encountered atomic numbers outside {self.model.atomic_numbers}")
         if bits & 2:
             raise ValueError(f"batch: graph index outside [0, {graphs})")

@@ -116,7 +116,7 @@ def energy_and_forces(model, positions, atomic_numbers, batch, edge_src, edge_ds
             energy, forces, per_atom = engine.energy_and_forces(
                 positions.detach().contiguous(), atomic_numbers.long().contiguous(), batch.long().contiguous(),
                 edge_src.long().contiguous(), edge_dst.long().contiguous(), edge_shifts.detach().to(dtype).contiguous(),
-                cell.detach().to(dtype).contiguous(), mask, not model.skip_input_validation, state)
+                cell.detach().to(dtype).contiguous(), mask, state)
             return {"energy": energy, "forces": forces, "atomic_energy": per_atom}
     with torch.enable_grad():
         coords = positions if positions.requires_grad else positions.detach().requires_grad_(True)

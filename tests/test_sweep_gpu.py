@@ -179,6 +179,18 @@ def test_unknown_atoms_and_bad_edges_raise_and_the_next_call_works():
     assert torch.equal(energy_and_forces(model, *graph)["forces"], good["forces"])
 
 
+@pytest.mark.parametrize("number", [7, 500])
+def test_unknown_atoms_raise_without_input_validation(number):
+    """The status word is read in any case: an unknown atom never counts as a known one."""
+    from mace_ictc.hp import energy_and_forces
+    model = _model()
+    model.skip_input_validation = True
+    graph = _graph(np.random.default_rng(4), (40,), False)
+    graph[1][5] = number
+    with pytest.raises(ValueError, match="atomic numbers"):
+        energy_and_forces(model, *graph)
+
+
 @pytest.mark.parametrize("chunk_rows", [None, 300])
 def test_stages_around_a_ghost_exchange(chunk_rows):
     """One rank that owns the whole box and sees its periodic images as ghost rows: same forces as the periodic list."""
