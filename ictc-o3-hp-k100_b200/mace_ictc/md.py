@@ -136,18 +136,14 @@ class StaticNeighborList:
 
     def __init__(self, num_atoms, box, cutoff, capacity, device, *, num_centres=None, lo=None, hi=None,
                  periodic=(1, 1, 1), pair_fraction=0.5, dummy_row=True):
-        self.n, self.cap, self.cutoff, self.dev = int(num_atoms), int(capacity), float(cutoff), device
+        self.n, self.cap, self.dev = int(num_atoms), int(capacity), device
         self.centres = self.n if num_centres is None else int(num_centres)
-        lib = _lib.load()
-        self.lo = _arr([0.0, 0.0, 0.0] if lo is None else [float(v) for v in lo], C.c_double)
-        self.hi = _arr([float(b) for b in box] if hi is None else [float(v) for v in hi], C.c_double)
-        self.box, self.per = _arr([float(b) for b in box], C.c_double), _arr([int(v) for v in periodic], C.c_int)
         # the position buffer of a recorded step carries one extra (dummy) row, the sender of the inert edges; a caller
         # that reads the edge count and uses the live edges alone needs none
         self.rows = self.n + (1 if dummy_row else 0)
         self.pad_src = self.n if dummy_row else 0
-        self.scratch = torch.empty(int(lib.ictc_neighbor_scratch_bytes(self.rows, self.lo, self.hi, self.cutoff)),
-                                   dtype=torch.uint8, device=device)
+        self.per = _arr([int(v) for v in periodic], C.c_int)
+        self.place(box, cutoff, lo, hi)
         # [row offsets | number of pairs | overflow flag] in one buffer, so that a host that wants all three copies once
         self._rows = torch.zeros(self.centres + 3, dtype=torch.int64, device=device)
         self.rowptr = self._rows[:self.centres + 1]
@@ -162,6 +158,15 @@ class StaticNeighborList:
         self.gate_row = torch.zeros(self.cap, dtype=torch.int64, device=device)
         self.rep = torch.zeros(self.ucap, dtype=torch.int64, device=device)
         self.other = torch.zeros(self.ucap, dtype=torch.int64, device=device)
+
+    def place(self, box, cutoff, lo=None, hi=None):
+        """Box, cutoff and cell grid of the next builds; the edge buffers stay."""
+        self.cutoff = float(cutoff)
+        self.lo = _arr([0.0, 0.0, 0.0] if lo is None else [float(v) for v in lo], C.c_double)
+        self.hi = _arr([float(b) for b in box] if hi is None else [float(v) for v in hi], C.c_double)
+        self.box = _arr([float(b) for b in box], C.c_double)
+        nbytes = int(_lib.load().ictc_neighbor_scratch_bytes(self.rows, self.lo, self.hi, self.cutoff))
+        self.scratch = torch.empty(nbytes, dtype=torch.uint8, device=self.dev)
 
     def build(self, pos):
         """pos [rows, 3]: the atoms, followed by the dummy row (far away from every atom) if there is one."""
@@ -322,26 +327,32 @@ class MolecularDynamics:
         self._forces_distributed()
         return self.forces
 
-    def _neighbors(self):
-        """This step's edge list in buffers that grow with the list: one build, one read-back."""
-        n, box = self.pos.shape[0], self.box.tolist()
+    def _neighbors(self, pos):
+        """This step's edge list in buffers that grow with the list: one build, one read-back.  The box, the cutoff and the
+        number of atoms are the present ones: a caller may change them between steps."""
+        n, box = pos.shape[0], self.box.tolist()
+        nl = self._eager_list
+        if nl is not None and nl.n != n:
+            nl = None
+        elif nl is not None and (list(nl.box) != box or nl.cutoff != self.cutoff):
+            nl.place(box, self.cutoff)
         while True:
-            if self._eager_list is None:
-                edges = count_edges(self.pos, n, [0, 0, 0], box, box, (1, 1, 1), self.cutoff)
-                self._eager_list = StaticNeighborList(n, box, self.cutoff, int(1.1 * edges) + 1024, self.device,
-                                                      dummy_row=False)
-            nl = self._eager_list
+            if nl is None:
+                edges = count_edges(pos, n, [0, 0, 0], box, box, (1, 1, 1), self.cutoff)
+                nl = self._eager_list = StaticNeighborList(n, box, self.cutoff, int(1.1 * edges) + 1024, self.device,
+                                                           dummy_row=False)
             with _lib.on_device(self.device):
-                nl.build(self.pos)
+                nl.build(pos)
             edges, pairs, over = nl.counts()
             if not over and pairs <= nl.ucap:
                 return nl, edges, pairs
-            self._eager_list = None         # the list outgrew its buffers
+            nl = self._eager_list = None         # the list outgrew its buffers
 
     def _forces_single(self):
-        n = self.pos.shape[0]
+        pos = self.pos.contiguous()
+        n = pos.shape[0]
         box = self.box.tolist()
-        nl, edges, num_pairs = self._neighbors()
+        nl, edges, num_pairs = self._neighbors(pos)
         src, dst, shifts, rowptr = nl.src[:edges], nl.dst[:edges], nl.shifts[:edges], nl.rowptr
         self.num_edges = edges
         if self.engine is not None:
@@ -349,14 +360,14 @@ class MolecularDynamics:
             self.num_gate_rows = num_pairs if pairs is not None else edges
             # a recorded graph reads and writes fixed buffers: an eager step in between keeps to them
             out = (self._static["energy"], self.forces) if self._static is not None else None
-            energy, forces, _ = self.engine.energy_and_gradient(self.pos, self.species, src, dst, shifts, box, n, rowptr,
+            energy, forces, _ = self.engine.energy_and_gradient(pos, self.species, src, dst, shifts, box, n, rowptr,
                                                                 pairs=pairs, src_csr=nl.sender_csr(), out=out, sign=-1.0)
             if out is None:
                 self.energy, self.forces = energy, forces
             return self.forces
         topo = Topology(src, dst, n, dst_sorted=True)
         topo._by_dst = (rowptr, None)
-        pos = self.pos.detach().requires_grad_(True)
+        pos = pos.detach().requires_grad_(True)
         batch = torch.zeros(n, dtype=torch.long, device=self.device)
         cell = torch.diag(self.box_f).unsqueeze(0)
         with torch.enable_grad():

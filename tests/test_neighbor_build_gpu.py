@@ -58,3 +58,40 @@ def test_capacity_that_does_not_fit_is_flagged():
     assert over and edges == 36
     for t, top in ((nl.src, 150), (nl.dst, 150), (nl.rev, 37), (nl.gate_row, nl.ucap), (nl.rep, 37)):
         assert int(t.min()) >= 0 and int(t.max()) < top
+
+
+@pytest.mark.parametrize("use_engine", [True, False])
+def test_eager_steps_follow_a_changed_box_cutoff_and_atom_count(use_engine):
+    """The buffers of the eager list outlive a step, what they were built for must not."""
+    from mace_ictc import synthetic as S
+    from mace_ictc.hp import create_model
+    from mace_ictc.md import MolecularDynamics, neighbor_list
+    torch.manual_seed(2)
+    model = create_model(channels=64, lmax=2, cutoff=CUTOFF, avg_num_neighbors=32.0)
+    pos, box, species = S.jittered_lattice(6, 7, 8, 2.15, 0.1, 3)
+    z = np.array([1, 6, 8])[species]
+    md = MolecularDynamics(model, pos, z, box, seed=1, use_engine=use_engine)
+    md.compute_forces()
+
+    def check():
+        fresh = MolecularDynamics(model, md.pos.cpu().numpy(), md.z.cpu().numpy(), md.box.numpy(), seed=1, sort_atoms=False,
+                                  use_engine=use_engine)
+        fresh.cutoff = md.cutoff
+        want = fresh.compute_forces()
+        assert md.compute_forces().shape == want.shape and md.num_edges == fresh.num_edges
+        assert torch.equal(md.forces, want) or not use_engine and float((md.forces - want).abs().max()) < 1e-4 * float(want.abs().max())
+
+    check()
+    for factor in (1.04, 0.97):                     # a barostat's changes, below and above the first box
+        md.box *= factor
+        md.box_f = md.box.to(md.device, torch.float32)
+        md.pos *= factor
+        check()
+    md.cutoff = 3.0
+    check()
+    md.pos, md.z, md.species = (t[:-9].contiguous() for t in (md.pos, md.z, md.species))
+    check()
+    md.pos = md.pos.t().contiguous().t()            # other strides
+    check()
+    rows = neighbor_list(md.pos, md.pos.shape[0], [0, 0, 0], md.box.tolist(), md.box.tolist(), (1, 1, 1), md.cutoff)
+    assert md.num_edges == rows[0].numel()
