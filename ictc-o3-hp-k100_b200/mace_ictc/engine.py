@@ -393,6 +393,9 @@ class ForceEngine:
         the gradient: a padding row has no edges).  ``src_csr`` = (row offsets, edge ids) of the senders where the caller
         has them.  ``out`` = (energy [1], gradient [N_local,3]) receives the results, the gradient times ``sign``."""
         w, dev = self.refresh(), self.dev
+        # read as plain words by the sweep: other types and strides are converted (these are no-ops for the MD drivers)
+        species = species.to(torch.int64).contiguous()
+        row_mask = None if row_mask is None else row_mask.to(torch.float32).contiguous()
         n_local, e = (pos.shape[0] if n_rows is None else int(n_rows)), int(src.numel())
         with _lib.on_device(dev):
             if src_csr is None:

@@ -191,6 +191,27 @@ def test_unknown_atoms_raise_without_input_validation(number):
         energy_and_forces(model, *graph)
 
 
+@pytest.mark.parametrize("dtype", [torch.bool, torch.int32, torch.float64])
+def test_engine_takes_masks_and_species_of_any_type_and_stride(dtype):
+    from mace_ictc.engine import ForceEngine
+    from ictc_o3.ops.topology import build_csr
+    model = _model()
+    pos, z, _, src, dst, shifts, cell = _graph(np.random.default_rng(6), (50,), False)
+    order = torch.argsort(dst, stable=True)
+    src, dst, shifts = src[order], dst[order], shifts[order].float()
+    species, engine = model.species_index(z), ForceEngine(model)
+    mask = torch.arange(50, device="cuda") % 3 != 1
+    args = (src, dst, shifts, cell[0].diag().tolist(), 50, build_csr(dst, 50, True)[0])
+    want = engine.energy_and_gradient(pos, species, *args, row_mask=mask.float())
+    wide = torch.zeros(50, 2, dtype=dtype, device="cuda")
+    wide[:, 0] = mask.to(dtype)
+    got = engine.energy_and_gradient(pos, species.to(torch.int32), *args, row_mask=wide[:, 0])
+    got2 = engine.energy_and_gradient(pos, species.repeat_interleave(2)[::2], *args, row_mask=mask.to(dtype))
+    for other in (got, got2):
+        assert torch.equal(other[1], want[1]) and torch.equal(other[2], want[2])
+        assert abs(float(other[0] - want[0])) <= 1e-6 * abs(float(want[0]))
+
+
 @pytest.mark.parametrize("chunk_rows", [None, 300])
 def test_stages_around_a_ghost_exchange(chunk_rows):
     """One rank that owns the whole box and sees its periodic images as ghost rows: same forces as the periodic list."""
