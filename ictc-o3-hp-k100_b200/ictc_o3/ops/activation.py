@@ -9,11 +9,25 @@ from .. import _lib
 
 def kernel_takes(x) -> bool:
     """The kernels take contiguous float32 CUDA tensors in eager reverse-mode differentiation; everything else stays with the
-    framework's operators."""
+    framework's operators: traced calls and dispatch modes, forward mode, tensors without a storage of their own (a batched
+    backward pass is not announced by any mode) and lazily negated ones."""
     return (type(x) in (torch.Tensor, torch.nn.Parameter) and x.is_cuda and x.dtype == torch.float32
-            and x.layout == torch.strided and x.is_contiguous() and not torch._C._are_functorch_transforms_active()
+            and x.layout == torch.strided and torch._C._has_storage(x) and x.is_contiguous() and not x.is_neg()
+            and not torch._C._are_functorch_transforms_active() and torch._C._len_torch_dispatch_stack() == 0
             and torch.autograd.forward_ad._current_level < 0 and not torch.compiler.is_compiling()
-            and not torch.is_autocast_enabled("cuda"))
+            and not torch.jit.is_tracing() and not torch.is_autocast_enabled("cuda"))
+
+
+def kernels_take(*tensors):
+    """The tensors made contiguous, or None when one of them is not for the kernels (looked at again in every backward pass:
+    what arrives there, cotangents and what saved-tensor hooks hand back, need not look like the forward's operands)."""
+    rows = [t.contiguous() if torch._C._has_storage(t) else t for t in tensors]
+    return rows if all(kernel_takes(t) for t in rows) else None
+
+
+def _first(x, scale):
+    s = torch.sigmoid(x)
+    return scale * s * (1 + x * (1 - s))
 
 
 def _launch(name, x, scale, *buffers):
@@ -34,7 +48,8 @@ class _Silu(torch.autograd.Function):
     @staticmethod
     def backward(ctx, grad):
         (x,) = ctx.saved_tensors
-        return _SiluGrad.apply(x, grad.contiguous(), ctx.scale), None
+        rows = kernels_take(x, grad)
+        return _SiluGrad.apply(*rows, ctx.scale) if rows else grad * _first(x, ctx.scale), None
 
 
 class _SiluGrad(torch.autograd.Function):
@@ -54,14 +69,15 @@ class _SiluGrad(torch.autograd.Function):
         if h is None:
             return None, None, None
         x, grad = ctx.saved_tensors
-        if torch.is_grad_enabled():                  # third order and above: plain operators
+        rows = None if torch.is_grad_enabled() else kernels_take(x, grad, h)
+        if rows is None:                             # third order and above, batched passes: plain operators
             s = torch.sigmoid(x)
-            first = ctx.scale * s * (1 + x * (1 - s))
             second = ctx.scale * s * (1 - s) * (2 + x * (1 - 2 * s))
-            return h * grad * second, h * first, None
+            return h * grad * second, h * _first(x, ctx.scale), None
+        x, grad, h = rows
         gx = torch.empty_like(x) if ctx.needs_input_grad[0] else None
         gg = torch.empty_like(x) if ctx.needs_input_grad[1] else None
-        _launch("ictc_silu_second", x, ctx.scale, grad, h.contiguous(), gx, gg)
+        _launch("ictc_silu_second", x, ctx.scale, grad, h, gx, gg)
         return gx, gg, None
 
 

@@ -28,3 +28,39 @@ def test_derivatives_up_to_third_order(n, shift):
     for a, b in zip(got, want):
         scale = max(1.0, float(b.detach().abs().max()))
         assert float((a.detach().double() - b.detach()).abs().max()) < TOL * scale
+
+
+def test_batched_traced_and_forward_mode_calls_keep_the_framework_operators():
+    """Forms in which no kernel can run, decided at the forward call or only in the backward pass."""
+    from ictc_o3 import normalized_silu
+    from torch.fx.experimental.proxy_tensor import make_fx
+    from torch.utils.flop_counter import FlopCounterMode
+    x = torch.randn(6, device="cuda", requires_grad=True)
+    v = torch.randn(4, 6, device="cuda")
+    ours, plain = (lambda t: normalized_silu(t, 1.7)), (lambda t: 1.7 * torch.nn.functional.silu(t))
+
+    def close(a, b):
+        assert a.shape == b.shape and float((a - b).detach().abs().max()) < 8 * TOL      # eight: double backward of sums
+
+    for f in (lambda g: torch.autograd.grad(g(x), x, v, is_grads_batched=True)[0],
+              lambda g: torch.autograd.grad(torch.autograd.grad(g(x), x, v[0], create_graph=True)[0], x, v, is_grads_batched=True)[0],
+              lambda g: torch.autograd.grad(torch.autograd.grad(g(x), x, v, create_graph=True, is_grads_batched=True)[0].sum(), x)[0],
+              lambda g: torch.autograd.functional.jacobian(g, x, vectorize=True),
+              lambda g: torch.autograd.functional.hessian(lambda t: g(t).sum(), x, vectorize=True),
+              lambda g: torch.func.vmap(lambda u, y=g(x): torch.autograd.grad(y, x, u, retain_graph=True)[0])(v),
+              lambda g: torch.func.jacfwd(g)(x.detach()), lambda g: torch.func.vmap(torch.func.grad(lambda t: g(t).sum()))(v),
+              lambda g: g(torch._neg_view(x.detach()))):
+        close(f(ours), f(plain))
+
+    def hooked(g):                                  # hooks that hand other strides back
+        turned = torch.randn(7, 5, device="cuda", generator=torch.Generator("cuda").manual_seed(1)).requires_grad_(True)
+        with torch.autograd.graph.saved_tensors_hooks(lambda t: t.t().contiguous(), lambda t: t.t()):
+            y = g(turned)
+        return torch.autograd.grad(y, turned, torch.ones_like(turned))[0]
+    close(hooked(ours), hooked(plain))
+
+    graph = make_fx(ours)(v)
+    close(graph(v + 1), ours(v + 1))
+    close(torch.jit.trace(ours, v)(v + 1), ours(v + 1))
+    with FlopCounterMode(display=False):
+        close(ours(v), plain(v))
