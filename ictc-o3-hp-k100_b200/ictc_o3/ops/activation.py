@@ -7,22 +7,25 @@ import torch
 from .. import _lib
 
 
-def kernel_takes(x) -> bool:
-    """The kernels take contiguous float32 CUDA tensors in eager reverse-mode differentiation; everything else stays with the
-    framework's operators: traced calls and dispatch modes, forward mode, tensors without a storage of their own (a batched
-    backward pass is not announced by any mode) and lazily negated ones."""
+def runs_eagerly(x) -> bool:
+    """A plain float32 CUDA tensor in eager reverse-mode differentiation.  Everything else stays with the framework's operators:
+    traced calls and dispatch modes, forward mode, tensors without a storage of their own (a batched backward pass is not
+    announced by any mode) and lazily negated ones."""
     return (type(x) in (torch.Tensor, torch.nn.Parameter) and x.is_cuda and x.dtype == torch.float32
-            and x.layout == torch.strided and torch._C._has_storage(x) and x.is_contiguous() and not x.is_neg()
+            and x.layout == torch.strided and torch._C._has_storage(x) and not x.is_neg()
             and not torch._C._are_functorch_transforms_active() and torch._C._len_torch_dispatch_stack() == 0
             and torch.autograd.forward_ad._current_level < 0 and not torch.compiler.is_compiling()
             and not torch.jit.is_tracing() and not torch.is_autocast_enabled("cuda"))
 
 
+def kernel_takes(x) -> bool:
+    return runs_eagerly(x) and x.is_contiguous()
+
+
 def kernels_take(*tensors):
     """The tensors made contiguous, or None when one of them is not for the kernels (looked at again in every backward pass:
     what arrives there, cotangents and what saved-tensor hooks hand back, need not look like the forward's operands)."""
-    rows = [t.contiguous() if torch._C._has_storage(t) else t for t in tensors]
-    return rows if all(kernel_takes(t) for t in rows) else None
+    return [t.contiguous() for t in tensors] if all(runs_eagerly(t) for t in tensors) else None
 
 
 def _first(x, scale):

@@ -5,7 +5,7 @@ from __future__ import annotations
 import torch
 
 from .. import _lib
-from .activation import kernel_takes
+from .activation import kernel_takes, runs_eagerly
 
 
 def narrow_takes(rows, weight) -> bool:
@@ -24,6 +24,11 @@ def _launch(name, *args):
         _lib.check(getattr(_lib.load(), name)(args[0], *[t.data_ptr() for t in args[1:]], _lib.stream(device)), name)
 
 
+def _may_run(*tensors):
+    """Looked at again in every backward pass, as in ``activation``; plain products otherwise."""
+    return all(runs_eagerly(t) for t in tensors)
+
+
 class NarrowLinear(torch.autograd.Function):
     """x [R, 8], w [64, 8] -> x w^T [R, 64]"""
 
@@ -37,8 +42,13 @@ class NarrowLinear(torch.autograd.Function):
     @staticmethod
     def backward(ctx, g):
         x, w = ctx.saved_tensors
-        return (_InputGrad.apply(g, w) if ctx.needs_input_grad[0] else None,
-                _WeightGrad.apply(g, x) if ctx.needs_input_grad[1] else None)
+        run = _may_run(x, w, g)
+        dx = dw = None
+        if ctx.needs_input_grad[0]:
+            dx = _InputGrad.apply(g, w) if run else g @ w
+        if ctx.needs_input_grad[1]:
+            dw = _WeightGrad.apply(g, x) if run else g.transpose(-2, -1) @ x
+        return dx, dw
 
 
 class _InputGrad(torch.autograd.Function):
@@ -54,8 +64,13 @@ class _InputGrad(torch.autograd.Function):
     @staticmethod
     def backward(ctx, h):
         g, w = ctx.saved_tensors
-        return (NarrowLinear.apply(h, w) if ctx.needs_input_grad[0] else None,
-                _WeightGrad.apply(g, h) if ctx.needs_input_grad[1] else None)
+        run = _may_run(g, w, h)
+        dg = dw = None
+        if ctx.needs_input_grad[0]:
+            dg = NarrowLinear.apply(h, w) if run else h @ w.transpose(-2, -1)
+        if ctx.needs_input_grad[1]:
+            dw = _WeightGrad.apply(g, h) if run else g.transpose(-2, -1) @ h
+        return dg, dw
 
 
 class _WeightGrad(torch.autograd.Function):
@@ -73,5 +88,10 @@ class _WeightGrad(torch.autograd.Function):
     @staticmethod
     def backward(ctx, h):
         g, x = ctx.saved_tensors
-        return (NarrowLinear.apply(x, h) if ctx.needs_input_grad[0] else None,
-                _InputGrad.apply(g, h) if ctx.needs_input_grad[1] else None)
+        run = _may_run(g, x, h)
+        dg = dx = None
+        if ctx.needs_input_grad[0]:
+            dg = NarrowLinear.apply(x, h) if run else x @ h.transpose(-2, -1)
+        if ctx.needs_input_grad[1]:
+            dx = _InputGrad.apply(g, h) if run else g @ h
+        return dg, dx

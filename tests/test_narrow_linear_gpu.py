@@ -28,3 +28,23 @@ def test_value_and_derivatives(rows, shift):
     # a sum of n terms in 32 bits is off by at most n half-units of that; random signs leave far less: 8 + sqrt(rows)
     for a, b, s in zip(got, want, size):
         assert float(((a.double() - b).abs() - (16 + rows ** 0.5) * EPS * s).max()) <= 0.0
+
+
+def test_batched_backward_passes_and_hooks_with_other_strides():
+    from ictc_o3.ops.narrow_linear import NarrowLinear
+    gen = torch.Generator("cuda").manual_seed(4)
+    make = lambda *s: torch.randn(*s, device="cuda", generator=gen)     # noqa: E731
+    x, w = make(33, 8).requires_grad_(True), make(64, 8).requires_grad_(True)
+    v, hx, hw = make(3, 33, 64), make(3, 33, 8), make(3, 64, 8)
+
+    def chain(f):
+        y = f(x, w)
+        first = torch.autograd.grad(y, [x, w], v, is_grads_batched=True, retain_graph=True)
+        single = torch.autograd.grad(y, [x, w], v[0], create_graph=True)
+        second = torch.autograd.grad(single, [x, w], [hx, hw], is_grads_batched=True)
+        with torch.autograd.graph.saved_tensors_hooks(lambda t: t.t().contiguous(), lambda t: t.t()):
+            y = f(x, w)
+        return [*first, *second, *torch.autograd.grad(y, [x, w], v[1])]
+
+    for a, b in zip(chain(NarrowLinear.apply), chain(lambda a, b: a @ b.t())):
+        assert a.shape == b.shape and float((a - b).abs().max()) < 64 * EPS * float(b.abs().max())      # sums of 64 terms
