@@ -42,6 +42,14 @@ def merge_irreps(blocks: Dict[int, torch.Tensor], channels: int, lmax: int) -> t
     return torch.cat([blocks[l].reshape(*blocks[l].shape[:-2], channels * (2 * l + 1)) for l in range(lmax + 1)], -1)
 
 
+def _calls_forward(module) -> bool:
+    """Does calling the module run its class's forward and nothing else (no hooks of its own or global ones, no replaced forward)?"""
+    table = nn.modules.module
+    return not ("forward" in module.__dict__ or module._forward_hooks or module._forward_pre_hooks or module._backward_hooks
+                or module._backward_pre_hooks or table._global_forward_hooks or table._global_forward_pre_hooks
+                or table._global_backward_hooks or table._global_backward_pre_hooks)
+
+
 class Normalize2MomSiLU(nn.Module):
     def forward(self, x):
         return normalized_silu(x, SILU_SCALE)
@@ -159,8 +167,7 @@ class InteractionBlock(nn.Module):
         for mod in self.fc:
             if isinstance(mod, nn.Linear) and _tc_eligible(h, mod.weight):
                 h = _RowsTimesWeight.apply(h, mod.weight)
-            elif (type(mod) is nn.Linear and mod.bias is None and narrow_takes(h, mod.weight)
-                  and not (mod._forward_hooks or mod._forward_pre_hooks or mod._backward_hooks or mod._backward_pre_hooks)):
+            elif type(mod) is nn.Linear and mod.bias is None and narrow_takes(h, mod.weight) and _calls_forward(mod):
                 h = NarrowLinear.apply(h, mod.weight)
             else:
                 h = mod(h)

@@ -48,3 +48,20 @@ def test_batched_backward_passes_and_hooks_with_other_strides():
 
     for a, b in zip(chain(NarrowLinear.apply), chain(lambda a, b: a @ b.t())):
         assert a.shape == b.shape and float((a - b).abs().max()) < 64 * EPS * float(b.abs().max())      # sums of 64 terms
+
+
+def test_the_first_radial_layer_honours_replaced_forwards_and_global_hooks():
+    from mace_ictc.model import MaceIctcModel
+    inter = MaceIctcModel(channels=64).cuda().interactions[0]
+    rows = torch.rand(40, 8, device="cuda")
+    plain = inter.radial_gates(rows)
+    inter.fc[0].forward = lambda t: 0.5 * torch.nn.functional.linear(t, inter.fc[0].weight)
+    halved = inter.radial_gates(rows)
+    del inter.fc[0].forward
+    assert float((halved - plain).abs().max()) > 0.01 * float(plain.abs().max())
+    seen = []
+    handle = torch.nn.modules.module.register_module_forward_hook(lambda module, *_: seen.append(module))
+    inter.radial_gates(rows)
+    handle.remove()
+    assert inter.fc[0] in seen
+    assert torch.equal(inter.radial_gates(rows), plain)
