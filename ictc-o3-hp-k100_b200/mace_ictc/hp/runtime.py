@@ -50,7 +50,8 @@ def create_model(*, channels=64, lmax=3, edge_lmax=None, num_interactions=2, cor
 def _force_engine(model, tensors, mask):
     """The tape-free engine for an inference call, or None where the autograd route has to answer: other widths or
     depths, hooks, tensors of another type, shape or device, stream capture (a recorded call reads the parameters at each
-    replay), forward-mode and functorch tracing, and autocast (which that route refuses)."""
+    replay), forward-mode and functorch tracing, dispatch modes and autocast (which that route sees or refuses), hooks on the
+    positions (which change the gradient) and lazily negated tensors (whose words have the other sign)."""
     if type(model) is not MaceIctcModel or model.channels != 64 or len(model.interactions) != 2:
         return None
     positions, numbers, batch, src, dst, shifts, cell = tensors
@@ -63,7 +64,9 @@ def _force_engine(model, tensors, mask):
             or shifts.dtype.is_complex or cell.dtype.is_complex
             or len(edges) != 1 or dst.shape != edges or tuple(shifts.shape) != (edges[0], 3)
             or edges[0] == 0 or positions.shape[0] == 0 or cell.shape[0] == 0
-            or mask is not None and (type(mask) is not torch.Tensor or mask.device != dev)
+            or mask is not None and (type(mask) is not torch.Tensor or mask.device != dev or mask.is_neg())
+            or any(t.is_neg() for t in (positions, shifts, cell)) or positions._backward_hooks
+            or torch._C._len_torch_dispatch_stack() > 0 or torch.jit.is_tracing()
             or torch.is_autocast_enabled("cuda") or torch._C._are_functorch_transforms_active()
             or torch.autograd.forward_ad._current_level >= 0 or torch.compiler.is_compiling()
             or torch.cuda.is_current_stream_capturing()):

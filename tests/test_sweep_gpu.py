@@ -191,6 +191,25 @@ def test_unknown_atoms_raise_without_input_validation(number):
         energy_and_forces(model, *graph)
 
 
+def test_traced_hooked_and_negated_calls_take_the_autograd_route():
+    from mace_ictc.hp import energy_and_forces
+    from torch.fx.experimental.proxy_tensor import make_fx
+    model = _model()
+    graph = _graph(np.random.default_rng(9), (30,), False)
+    want = _autograd(model, graph)
+    with pytest.raises((ValueError, RuntimeError)):         # tracing is refused, not recorded as a constant
+        make_fx(lambda p: energy_and_forces(model, p, *graph[1:])["forces"])(graph[0])
+    for k in (0, 5, 6):
+        other = list(graph)
+        other[k] = torch._neg_view(-graph[k].float())
+        _close(energy_and_forces(model, *other), want)
+    pinned = list(graph)                                    # an atom held in place by a hook on the positions
+    pinned[0] = graph[0].clone().requires_grad_(True)
+    pinned[0].register_hook(lambda g: g * (torch.arange(30, device="cuda") != 4).unsqueeze(1))
+    got = energy_and_forces(model, *pinned)["forces"]
+    assert bool((got[4] == 0).all()) and float((got[5:] - want["forces"][5:]).abs().max()) < TOL * float(want["forces"].abs().max())
+
+
 @pytest.mark.parametrize("dtype", [torch.bool, torch.int32, torch.float64])
 def test_engine_takes_masks_and_species_of_any_type_and_stride(dtype):
     from mace_ictc.engine import ForceEngine
