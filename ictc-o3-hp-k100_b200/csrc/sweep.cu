@@ -781,6 +781,36 @@ static int check(const ictc_sweep* p) {
   return ICTC_OK;
 }
 
+// Weights and buffers that are read in pieces of 8, 16 or 32 bytes.
+static int check_pointers(const ictc_sweep* p) {
+  uintptr_t bits = 0;
+  bool null = false;
+  const auto need = [&](const void* at, int bytes) {
+    null |= !at;
+    bits |= reinterpret_cast<uintptr_t>(at) & (bytes - 1);
+  };
+  const auto may = [&](const void* at, int bytes) { bits |= reinterpret_cast<uintptr_t>(at) & (bytes - 1); };
+  need(p->work, 32); may(p->features, 32); may(p->feature_grad, 32);
+  need(p->up0_table, 16); need(p->sc0_table, 4);
+  need(p->readout_rp, 8); need(p->readout_rs, 8); need(p->readout_ro0, 8); need(p->readout_w2, 4);
+  for (int k = 0; k < 2; ++k) {
+    const ictc_sweep_layer& L = p->layer[k];
+    need(L.w0, 4); need(L.w3, 16); need(L.w3t, 16); need(L.bank, 4);
+    for (int i = 0; i < 2; ++i) { need(L.hid[i], 16); need(L.hid_t[i], 16); }
+    for (int l = 0; l < 3; ++l) {
+      need(L.ml[l], 16); need(L.ml_b[l], 16);
+      need(k ? L.up[l] : L.pl[l], 16); need(k ? L.up_b[l] : L.pl_b[l], 16);
+    }
+  }
+  if (null || bits) {
+    set_error(null ? "sweep: NULL weights or workspace"
+                   : "sweep: workspace and feature buffers must be 32-byte, packed weights and up0_table 16-byte, the readout "
+                     "matrices 8-byte aligned");
+    return ICTC_ERR_BAD_ARG;
+  }
+  return ICTC_OK;
+}
+
 }  // namespace sweep
 }  // namespace ictc
 
@@ -817,6 +847,7 @@ int ictc_sweep_run(const ictc_sweep* p, int stages, void* stream) {
     set_error("sweep: NULL buffer");
     return ICTC_ERR_BAD_ARG;
   }
+  if (int rc = sweep::check_pointers(p)) return rc;
   if ((stages & 31) != 31 && (!p->features || !p->feature_grad)) {
     set_error("sweep: features and feature_grad are needed when the stages run one by one");
     return ICTC_ERR_BAD_ARG;

@@ -262,7 +262,8 @@ class ForceEngine:
             s.readout_rp = hold((w1 @ d(m.products[1].linear["0"]).t() / math.sqrt(c)).float().contiguous())
             s.readout_rs = hold(torch.einsum("ho,soi->shi", w1, d(last.self_connection.weights["0"])).float().contiguous())
             s.readout_w2 = hold(ro.linear_2.weight.reshape(-1).contiguous())
-            s.readout_ro0 = hold(m.layer_energy_readouts[0].readout.weight.reshape(-1).contiguous())
+            # a copy: read two floats at a time, and a parameter may stand at any word of a flattened buffer
+            s.readout_ro0 = hold(m.layer_energy_readouts[0].readout.weight.reshape(-1).clone())
             s.hidden, s.num_species = w1.shape[0], m.num_elements
             s.num_basis, s.poly_p, s.r_max = m.number_of_basis, m.polynomial_cutoff_p, m.max_radius
             w.tiles, w.copy = self._snapshot(w.keep)

@@ -415,7 +415,8 @@ int ictc_sc_second(int lmax, int target_lmax, int channels, int64_t num_nodes, i
  * Energy and position gradient of the two-interaction C64 / lmax 2 model as one launch sequence (the force path of
  * mace_ictc/hp/runtime.py:82-111).  All pointers are device pointers; edges need not be sorted when dst_order is given or
  * when both row-offset pointers are NULL (the sweep then builds both CSRs).  Weight matrices marked "packed" come from
- * ictc_gate_pack_weights. */
+ * ictc_gate_pack_weights.  Alignment (checked): work, features, feature_grad 32 bytes, packed weights and up0_table 16, readout_rp,
+ * readout_rs and readout_ro0 8. */
 typedef struct {
   const float* w0;              /* first radial layer [64, num_basis] */
   const float* hid[2];          /* packed hidden layers, forward and (hid_t) transposed use */

@@ -111,6 +111,24 @@ def test_parameter_updates_replacement_copies_and_hooks():
     _close(energy_and_forces(model, *graph), _autograd(model, graph))
 
 
+def test_parameters_at_any_word_of_a_flattened_buffer():
+    from mace_ictc.hp import energy_and_forces
+    model = _model()
+    graph = _graph(np.random.default_rng(11), (30,), False)
+    want = energy_and_forces(model, *graph)
+    params = list(model.parameters())
+    flat = torch.empty(sum(p.numel() + 2 for p in params) + 2, device="cuda")
+    at = 1
+    for p in params:
+        view = flat[at:at + p.numel()].view_as(p)
+        p.data = view.copy_(p.data)
+        at += p.numel() + 1 + (at + p.numel()) % 2        # every parameter at an odd word
+    assert all(p.data_ptr() % 8 == 4 for p in params)
+    got = energy_and_forces(model, *graph)
+    assert torch.equal(got["forces"], want["forces"]) and torch.equal(got["atomic_energy"], want["atomic_energy"])
+    _close(got, _autograd(model, graph))
+
+
 def test_models_with_other_readouts_answer_through_their_own_forward():
     from mace_ictc.hp import energy_and_forces
     from mace_ictc.md import MolecularDynamics

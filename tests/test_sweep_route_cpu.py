@@ -1,6 +1,7 @@
 """Which models the native force sweep may answer for (host logic, no GPU): the stock model, and none whose own forward computes
 something that the sweep does not read."""
 import copy
+import ctypes
 
 import pytest
 import torch
@@ -89,3 +90,41 @@ def test_the_stock_model_is_covered():
     biased.node_embedding = _biased(64, 3)
     biased.interactions[1].linear_up.adapters["1"] = _biased(64, 64)
     assert _stands_for(biased)
+
+
+def test_misaligned_weights_and_buffers_are_refused_before_any_launch():
+    """Made-up addresses, none of which is touched: the check comes before the first launch."""
+    from ictc_o3 import _lib
+    lib = _lib.load()
+
+    def sweep():
+        s = _lib.Sweep(n_local=4, n_owned=4, edges=8, pair_rows=8, num_species=3, graphs=1, num_basis=8, poly_p=5, hidden=16,
+                       r_max=4.5, work_bytes=0)
+        for name in ("pos", "src", "dst", "species", "energy", "atomic", "gradient", "status", "work", "up0_table", "sc0_table",
+                     "readout_rp", "readout_rs", "readout_w2", "readout_ro0"):
+            setattr(s, name, 4096)
+        for k in range(2):
+            for name in ("w0", "w3", "w3t", "bank"):
+                setattr(s.layer[k], name, 4096)
+            for name, count in (("hid", 2), ("hid_t", 2), ("up", 3), ("up_b", 3), ("ml", 3), ("ml_b", 3), ("pl", 3), ("pl_b", 3)):
+                setattr(s.layer[k], name, (4096,) * count)
+            s.layer[k].num_gates = 64 * (3, 11)[k]
+            s.layer[k].slots = ((1, 1, 1), (3, 4, 4))[k]
+        return s
+
+    def refused(s, text):
+        assert lib.ictc_sweep_run(ctypes.byref(s), 31, None) == -2 and text in _lib.last_error()
+
+    refused(sweep(), "too small")                         # everything in order, but the workspace has no room
+    for name, off in (("work", 16), ("features", 16), ("feature_grad", 4), ("up0_table", 8), ("readout_rp", 4), ("readout_rs", 4),
+                      ("readout_ro0", 4)):
+        s = sweep()
+        setattr(s, name, 4096 + off)
+        refused(s, "aligned")
+    for k, name in ((0, "w3"), (1, "w3t")):
+        s = sweep()
+        setattr(s.layer[k], name, 4096 + 8)
+        refused(s, "aligned")
+    s = sweep()
+    s.layer[1].up = (4096, 0, 4096)
+    refused(s, "NULL")
