@@ -152,7 +152,8 @@ __global__ void __launch_bounds__(kFwdThreads, 1) gate_gemm_forward_kernel(const
   Barriers* bar = reinterpret_cast<Barriers*>(offsets + 2 * kRows);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const unsigned tmem = enter(bar, 2, 4);
-  const Work work(a, pdl_enter());
+  const int zero = pdl_enter();
+  const Work work(a, zero);
   const unsigned tmem_a = tmem + 4 * kChunk;       // A operands start after the accumulator ring
 
   if (warp == 0) {
@@ -213,7 +214,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) gate_gemm_forward_kernel(const
       float* out = seg.out + (lane & 15) * 4;
       const int64_t step = int64_t(seg.out_cs) * kChunk;
       const float* add = (a.bias && s == 0 && valid && g < a.bias_nodes)
-                             ? a.bias + (a.bias_index ? ldg(a.bias_index + g) : g) * kK : nullptr;
+                             ? a.bias + (a.bias_index ? ldg(a.bias_index + g + zero) : g + zero) * kK : nullptr;
       for (int c = 0; c < chunks; ++c, ++it, out += step) {
         if (int(it & 1) != group) continue;
         const int d = int(it & 3);
@@ -383,7 +384,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) gate_gemm_backward_kernel(cons
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         const int64_t g = first + 4 * j + (lane >> 3);
-        const int64_t r = g < nrows ? (a.pair_a ? ldg(a.pair_a + g) : g) : -1;
+        const int64_t r = g < nrows ? (a.pair_a ? ldg(a.pair_a + work.base + g) : g) : -1;
         f_row[j] = r < 0 ? nullptr : seg.in + row_offset(r, seg.in_mm, seg.in_ld) + half * 32 + (lane & 7) * 4;
       }
     };
@@ -416,7 +417,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) gate_gemm_backward_kernel(cons
       const int s = work.segment(tile), chunks = a.seg[s].chunks;
       const Segment& seg = a.seg[s];
       const int64_t g = work.first_row(tile, s) + q * 32 + lane;
-      const int64_t rb = (a.pair_b && g < work.rows(a, s)) ? ldg(a.pair_b + g) : -1;
+      const int64_t rb = (a.pair_b && g < work.rows(a, s)) ? ldg(a.pair_b + work.base + g) : -1;
       for (int c = 0; c < chunks; ++c, ++it) {
         const int sa = int(it % kAStagesBwd);
         fetch();

@@ -29,8 +29,9 @@ inline int finish_launch(const char* what) {
 // of 216 atoms 298 -> 261 us, 10 recorded MD steps of 1,000 atoms 4.09 -> 4.02 ms (a graph's own gaps are short already).
 // Rules: every thread calls pdl_enter() before its first access to global memory that an earlier launch may have written or
 // still reads; a kernel that allocates tensor memory calls it behind the allocation (a later kernel's block must
-// not take the columns first and then wait for this one); addresses of read-only loads depend on the returned zero,
-// which keeps the compiler from moving them up.
+// not take the columns first and then wait for this one); an ordinary load cannot be moved above the wait (the clobber), a
+// non-coherent one (ldg) could be, as its memory counts as constant: its address depends on the returned zero, also in loops
+// and for weights and device scalars.
 __device__ __forceinline__ int pdl_enter() {
   int zero;
   asm volatile("griddepcontrol.launch_dependents;\n\tgriddepcontrol.wait;\n\tmov.u32 %0, 0;" : "=r"(zero) : : "memory");

@@ -55,7 +55,8 @@ __device__ __forceinline__ void stg256(float* p, const float* v) {
 }
 
 // Common prologue: barriers, TMEM, weights.  Returns the TMEM base address.
-__device__ __forceinline__ unsigned setup(const Args& a, const Stack& k, unsigned char* smem, Barriers* bar, float* w0s) {
+// `zero`: what pdl_enter() returned.
+__device__ __forceinline__ unsigned setup(const Args& a, const Stack& k, unsigned char* smem, Barriers* bar, float* w0s, int& zero) {
   const int warp = threadIdx.x >> 5;
   if (threadIdx.x == 0) {
     for (int i = 0; i < 2; ++i) {
@@ -77,7 +78,7 @@ __device__ __forceinline__ unsigned setup(const Args& a, const Stack& k, unsigne
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   __syncthreads();
-  const int zero = pdl_enter();
+  zero = pdl_enter();
   if (threadIdx.x == 0) {
     mbar_expect_tx(saddr(&bar->w_full), 2 * kWStageBytes);
     bulk_g2s(saddr(smem), k.wa, kWStageBytes, saddr(&bar->w_full));
@@ -133,10 +134,12 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_chain_forward_kernel(const __
   float* w0s = reinterpret_cast<float*>(chain_smem + 2 * kWStageBytes);
   Barriers* bar = reinterpret_cast<Barriers*>(chain_smem + kBarOffset);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const Share share(a);
+  Share share(a);
   const Stack& stack = a.stack[share.stack];
-  const unsigned tmem = setup(a, stack, chain_smem, bar, w0s);
-  const int64_t nrows = a.limit ? (ldg(a.limit) < a.E ? ldg(a.limit) : a.E) : a.E;
+  int zero;
+  const unsigned tmem = setup(a, stack, chain_smem, bar, w0s, zero);
+  share.first += zero;           // every row number, and so every address of a row, depends on it
+  const int64_t live = a.limit ? ldg(a.limit + zero) : a.E, nrows = live < a.E ? live : a.E;
   const int64_t tiles = (nrows + kRows - 1) / kRows;
   const int64_t my_tiles = share.first < tiles ? (tiles - share.first + share.step - 1) / share.step : 0;
 
@@ -208,10 +211,12 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_chain_backward_kernel(const _
   float* xchg = w0s + 64 * 8;                                         // [128][8] partial drb of the upper half
   Barriers* bar = reinterpret_cast<Barriers*>(chain_smem + kBarOffset);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const Share share(a);
+  Share share(a);
   const Stack& stack = a.stack[share.stack];
-  const unsigned tmem = setup(a, stack, chain_smem, bar, w0s);
-  const int64_t nrows = a.limit ? (ldg(a.limit) < a.E ? ldg(a.limit) : a.E) : a.E;
+  int zero;
+  const unsigned tmem = setup(a, stack, chain_smem, bar, w0s, zero);
+  share.first += zero;           // every row number, and so every address of a row, depends on it
+  const int64_t live = a.limit ? ldg(a.limit + zero) : a.E, nrows = live < a.E ? live : a.E;
   const int64_t tiles = (nrows + kRows - 1) / kRows;
   const int64_t my_tiles = share.first < tiles ? (tiles - share.first + share.step - 1) / share.step : 0;
 

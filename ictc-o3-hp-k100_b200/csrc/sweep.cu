@@ -303,14 +303,15 @@ static int tail_nodes(int64_t n) { return n <= kTailSlots ? 1 : 4; }
 __global__ void __launch_bounds__(kTailWarps * 32) tail_kernel(TailArgs a, int nodes) {
   __shared__ double block_energy[kTailWarps];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t first = (int64_t(blockIdx.x) * kTailWarps + warp) * nodes + pdl_enter();
-  const float2 ro = __ldg(reinterpret_cast<const float2*>(a.ro0) + lane);
+  const int zero = pdl_enter();
+  const int64_t first = (int64_t(blockIdx.x) * kTailWarps + warp) * nodes + zero;
+  const float2 ro = __ldg(reinterpret_cast<const float2*>(a.ro0 + zero) + lane);
   double sum = 0.0;
   int64_t graph = -1;
   for (int64_t n = first; n < first + nodes && n < a.n; ++n) {
     const float2 y = __ldg(reinterpret_cast<const float2*>(a.y + n * kC) + lane);
     const float2 h = __ldg(reinterpret_cast<const float2*>(a.h + n * a.h_ld) + lane);
-    const float2* rp = reinterpret_cast<const float2*>(a.rp) + lane;
+    const float2* rp = reinterpret_cast<const float2*>(a.rp + zero) + lane;
     const float2* rs = reinterpret_cast<const float2*>(a.rs + ldg(a.species + n) * a.H * kC) + lane;
     const float m = a.mask ? ldg(a.mask + n) : 1.f;
     float e = fmaf(h.x, ro.x, h.y * ro.y);
@@ -330,7 +331,7 @@ __global__ void __launch_bounds__(kTailWarps * 32) tail_kernel(TailArgs a, int n
       const float z = warp_reduce_scatter<16>(v, lane, idx, valid);        // hidden unit k sits on lane 2k
       float dz = 0.f;
       if (valid && k0 + idx < a.H) {
-        const float w = ldg(a.w2 + k0 + idx);
+        const float w = ldg(a.w2 + zero + k0 + idx);
         const float s = 1.f / (1.f + expf(-z));
         e = fmaf(w, z * s * kSilu, e);
         dz = w * m * kSilu * s * (1.f + z * (1.f - s));

@@ -101,10 +101,11 @@ struct TpTangents {
 };
 
 // Row of edge e, found at position `pos` of the owner's CSR walk, in the gate table.
-__device__ __forceinline__ int64_t gate_row_of(const TpArgs& a, int64_t e, int64_t pos) {
+// `zero`: what pdl_enter() returned, in kernels that may start early.
+__device__ __forceinline__ int64_t gate_row_of(const TpArgs& a, int64_t e, int64_t pos, int zero = 0) {
   int64_t r = a.g_by_pos ? pos : (a.grow ? ldg(a.grow + e) : e);
   if (a.g_base) {
-    r -= ldg(a.g_base);
+    r -= ldg(a.g_base + zero);
     r = r < 0 ? 0 : (r >= a.g_cap ? a.g_cap - 1 : r);
   }
   return r;

@@ -160,7 +160,8 @@ tp_graph_forward_tma_kernel(TpArgs a) {
   V acc[S::NO];
 #pragma unroll
   for (int k = 0; k < S::NO; ++k) acc[k] = V::dup(0.f);
-  n += pdl_enter();
+  const int zero = pdl_enter();
+  n += zero;
   int64_t begin = ldg(a.rowptr + n), end = ldg(a.rowptr + n + 1);
   if (SPLIT > 1) {
     const int64_t len = end - begin;
@@ -175,7 +176,7 @@ tp_graph_forward_tma_kernel(TpArgs a) {
       const unsigned bar = bars + slot * 8;
       unsigned char* dst = mine + slot * L::SLOT_BYTES;
       mbar_expect_tx(bar, L::SLOT_BYTES);
-      const int64_t gr = gate_row_of(a, e, pos);
+      const int64_t gr = gate_row_of(a, e, pos, zero);
       bulk_g2s(smem_addr(dst), a.g + gr * (S::NP * C), L::GATE_BYTES, bar);
       if (kStageRows) bulk_g2s(smem_addr(dst + L::GATE_BYTES), a.x + int64_t(s) * (S::NX * C), L::ROW_BYTES, bar);
     }
@@ -245,7 +246,7 @@ tp_graph_forward_tma_kernel(TpArgs a) {
 #pragma unroll
       for (int p = 0; p < S::NP; ++p) {
         ge[p] = vmul(ge[p], mu);
-        if (a.w) ge[p] = vmul(ge[p], V::load(a.w + p * C + lane * CPL));
+        if (a.w) ge[p] = vmul(ge[p], V::load(a.w + zero + p * C + lane * CPL));
       }
     }
     __syncwarp();   // geometry visible; every lane has read its slot data into registers
@@ -293,7 +294,8 @@ __global__ void __launch_bounds__(split_warps(SPLIT) * 32, kTmaMinWarpsAdj / spl
   BTerm bt[L::R];
 #pragma unroll
   for (int r = 0; r < L::R; ++r) bt[r] = (r * 32 + lane < F::NB) ? F::ap(r * 32 + lane) : BTerm{0, 0.f, 0, 0.f};
-  owner += pdl_enter();
+  const int zero = pdl_enter();
+  owner += zero;
   V x[S::NX], dx[S::NX];
   {
     const float* xp = a.x + owner * (S::NX * C) + lane * CPL;
@@ -320,7 +322,7 @@ __global__ void __launch_bounds__(split_warps(SPLIT) * 32, kTmaMinWarpsAdj / spl
       const unsigned bar = bars + slot * 8;
       unsigned char* dst = mine + slot * L::SLOT_BYTES;
       mbar_expect_tx(bar, L::SLOT_BYTES);
-      const int64_t gr = gate_row_of(a, e, pos);
+      const int64_t gr = gate_row_of(a, e, pos, zero);
       bulk_g2s(smem_addr(dst), a.g + gr * (S::NP * C), L::GATE_BYTES, bar);
       if (kStageRows) bulk_g2s(smem_addr(dst + L::GATE_BYTES), a.v + int64_t(d) * (S::NO * C), L::ROW_BYTES, bar);
     }
@@ -374,7 +376,7 @@ __global__ void __launch_bounds__(split_warps(SPLIT) * 32, kTmaMinWarpsAdj / spl
     const unsigned char* base = mine + slot * L::SLOT_BYTES + lane * (CPL * 4);
     const bool scaled = !PLAIN && (a.mask || a.w);
     const V mu = V::dup((scaled && a.mask) ? ldg(a.mask + e) : 1.f);
-    auto scale_of = [&](int p) -> V { return a.w ? vmul(mu, V::load(a.w + p * C + lane * CPL)) : mu; };
+    auto scale_of = [&](int p) -> V { return a.w ? vmul(mu, V::load(a.w + zero + p * C + lane * CPL)) : mu; };
     auto gate = [&](int p) -> V {
       const V g = lds_vec<CPL>(base + p * (C * 4));
       if (PLAIN) return g;
@@ -382,7 +384,7 @@ __global__ void __launch_bounds__(split_warps(SPLIT) * 32, kTmaMinWarpsAdj / spl
     };
     int dgr = e;            // row of this edge's gate gradient (negative: outside the caller's window, not stored)
     if (NEEDG && a.dg_base) {
-      const int64_t r = it - ldg(a.dg_base);
+      const int64_t r = it - ldg(a.dg_base + zero);
       dgr = (r >= 0 && r < a.dg_cap) ? int(r) : -1;
     }
     float* dgp = a.dg + int64_t(dgr < 0 ? 0 : dgr) * (S::NP * C) + lane * CPL;

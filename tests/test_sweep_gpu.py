@@ -197,6 +197,35 @@ def test_unknown_atoms_and_bad_edges_raise_and_the_next_call_works():
     assert torch.equal(energy_and_forces(model, *graph)["forces"], good["forces"])
 
 
+def test_small_sweeps_queued_behind_each_other_do_not_see_each_other():
+    """Launches of about one wave start before the previous one has ended: sweeps of other sizes (pair rows, CSR offsets, chunk
+    bounds, features) right behind each other give what each gives alone."""
+    from mace_ictc import synthetic as S
+    from mace_ictc.hp import energy_and_forces
+    from mace_ictc.md import MolecularDynamics
+    model = _model()
+    model.skip_input_validation = True
+    graphs = [_graph(np.random.default_rng(k), (n,), False) for k, n in enumerate((33, 150, 45, 90))]
+    runs = []
+    for k, (side, chunk) in enumerate(((6, None), (7, 64), (6, 100))):
+        pos, box, species = S.jittered_lattice(side, side, side, 2.15, 0.1, k)
+        md = MolecularDynamics(model, pos, np.array(ELEMENTS)[species], box, seed=k, chunk_rows=chunk, stream_gates=chunk == 64)
+        md.compute_forces()
+        runs.append(md)
+    alone = []
+    for graph in graphs:
+        alone.append(energy_and_forces(model, *graph)["forces"])
+        torch.cuda.synchronize()
+    steps = []
+    for md in runs:
+        steps.append(md.compute_forces().clone())
+        torch.cuda.synchronize()
+    for _ in range(10):
+        got = [energy_and_forces(model, *graph)["forces"] for graph in graphs]
+        forces = [md.compute_forces() for md in runs]
+        assert all(torch.equal(a, b) for a, b in zip(got + forces, alone + steps))
+
+
 @pytest.mark.parametrize("number", [7, 500])
 def test_unknown_atoms_raise_without_input_validation(number):
     """The status word is read in any case: an unknown atom never counts as a known one."""
