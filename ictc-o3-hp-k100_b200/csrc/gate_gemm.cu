@@ -78,7 +78,8 @@ __device__ __forceinline__ void give_up(Barriers* b, int* status, int code) {
   if (status) atomicExch(status, code);
 }
 
-// The weight stream of both kernels: chunk after chunk for every tile.  A segment with one chunk keeps it.
+// The weight stream of both kernels: chunk after chunk for every tile.  A segment with one chunk keeps it.  When the block has given
+// up, the copies in flight are waited for (again with a limit) before the lane leaves.
 __device__ __forceinline__ void stream_weights(const Args& a, const Work& work, Barriers* bar, unsigned char* w_buf, int code) {
   int64_t it = 0;
   int kept = -1;
@@ -86,15 +87,19 @@ __device__ __forceinline__ void stream_weights(const Args& a, const Work& work, 
     const int s = work.segment(tile);
     const Segment& seg = a.seg[s];
     if (s == kept) continue;
-    for (int c = 0; c < seg.chunks; ++c, ++it) {
+    for (int c = 0; c < seg.chunks && !bar->failed; ++c) {
       const int slot = int(it % kWStages);
-      if (!mbar_wait(saddr(&bar->w_empty[slot]), unsigned((it / kWStages) & 1) ^ 1u)) { give_up(bar, a.status, code); return; }
+      if (!mbar_wait(saddr(&bar->w_empty[slot]), unsigned((it / kWStages) & 1) ^ 1u)) { give_up(bar, a.status, code); break; }
       mbar_expect_tx(saddr(&bar->w_full[slot]), kWStageBytes);
       bulk_g2s(saddr(w_buf + slot * kWStageBytes), seg.w + int64_t(c) * (kWStageBytes / 4), kWStageBytes,
                saddr(&bar->w_full[slot]));
+      ++it;
     }
     kept = seg.chunks == 1 ? s : -1;
   }
+  if (bar->failed)
+    for (int64_t k = it > kWStages ? it - kWStages : 0; k < it; ++k)
+      mbar_wait(saddr(&bar->w_full[k % kWStages]), unsigned((k / kWStages) & 1));
 }
 
 // Barriers and all 512 TMEM columns; returns the TMEM base.
@@ -159,35 +164,33 @@ __global__ void __launch_bounds__(kFwdThreads, 1) gate_gemm_forward_kernel(const
   if (warp == 0) {
     if (lane == 0) stream_weights(a, work, bar, w_buf, 21);
   } else if (warp == 1) {
-    // ---- MMA issue
-    int64_t it = 0, wit = 0;
-    int t = 0, kept = -1;
-    bool ok = true;
-    for (int tile = blockIdx.x; tile < work.tiles() && ok && !bar->failed; tile += gridDim.x, ++t) {
-      const int s = work.segment(tile), chunks = a.seg[s].chunks;
-      const bool keep = chunks == 1 && tile + int(gridDim.x) < work.tiles() && work.segment(tile + gridDim.x) == s;
-      const int ab = t & 1;
-      if (!mbar_wait(saddr(&bar->a_full[ab]), unsigned((t >> 1) & 1))) { give_up(bar, a.status, 22); break; }
-      for (int c = 0; c < chunks; ++c, ++it) {
-        const int slot = int(wit % kWStages), d = int(it & 3);
-        if ((kept != s && !mbar_wait(saddr(&bar->w_full[slot]), unsigned((wit / kWStages) & 1))) ||
-            !mbar_wait(saddr(&bar->d_empty[d]), unsigned((it >> 2) & 1) ^ 1u)) {
-          give_up(bar, a.status, 23);
-          ok = false;
-          break;
-        }
-        tc_fence_after();
-        const unsigned w_big = saddr(w_buf + slot * kWStageBytes), w_small = w_big + kWPartBytes;
-        if (elect_one()) {
+    if (elect_one()) {           // ---- MMA issue: the role of one lane, its waits included
+      int64_t it = 0, wit = 0;
+      int t = 0, kept = -1;
+      bool ok = true;
+      for (int tile = blockIdx.x; tile < work.tiles() && ok && !bar->failed; tile += gridDim.x, ++t) {
+        const int s = work.segment(tile), chunks = a.seg[s].chunks;
+        const bool keep = chunks == 1 && tile + int(gridDim.x) < work.tiles() && work.segment(tile + gridDim.x) == s;
+        const int ab = t & 1;
+        if (!mbar_wait(saddr(&bar->a_full[ab]), unsigned((t >> 1) & 1))) { give_up(bar, a.status, 22); break; }
+        for (int c = 0; c < chunks; ++c, ++it) {
+          const int slot = int(wit % kWStages), d = int(it & 3);
+          if ((kept != s && !mbar_wait(saddr(&bar->w_full[slot]), unsigned((wit / kWStages) & 1))) ||
+              !mbar_wait(saddr(&bar->d_empty[d]), unsigned((it >> 2) & 1) ^ 1u)) {
+            give_up(bar, a.status, 23);
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          const unsigned w_big = saddr(w_buf + slot * kWStageBytes), w_small = w_big + kWPartBytes;
           issue_block(tmem + d * kChunk, tmem_a + ab * 2 * kK, w_big, w_small, true);
           if (!keep) umma_commit(saddr(&bar->w_empty[slot]));
           umma_commit(saddr(&bar->d_full[d]));
           if (c == chunks - 1) umma_commit(saddr(&bar->a_empty[ab]));
+          wit += !keep;
         }
-        __syncwarp();
-        wit += !keep;
+        kept = keep ? s : -1;
       }
-      kept = keep ? s : -1;
     }
   } else if (warp < kFwdProducer0) {
     // ---- epilogue, two groups of four warps that take alternate chunks: tcgen05.ld gives thread = row; the
@@ -202,8 +205,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) gate_gemm_forward_kernel(const
     int64_t* my_offset = offsets + group * kRows + row;
     const int64_t* offset = offsets + group * kRows + q * 32 + (lane >> 4);
     int64_t it = 0;
-    bool ok = true;
-    for (int tile = blockIdx.x; tile < work.tiles() && ok; tile += gridDim.x) {
+    for (int tile = blockIdx.x; tile < work.tiles(); tile += gridDim.x) {
       const int s = work.segment(tile);
       const Segment& seg = a.seg[s];
       const int chunks = seg.chunks;
@@ -218,11 +220,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) gate_gemm_forward_kernel(const
       for (int c = 0; c < chunks; ++c, ++it, out += step) {
         if (int(it & 1) != group) continue;
         const int d = int(it & 3);
-        if (bar->failed || !mbar_wait(saddr(&bar->d_full[d]), unsigned((it >> 2) & 1))) {
-          give_up(bar, a.status, 24);
-          ok = false;
-          break;
-        }
+        if (!bar->failed && !mbar_wait(saddr(&bar->d_full[d]), unsigned((it >> 2) & 1))) give_up(bar, a.status, 24);
         tc_fence_after();
         float v0[32], v1[32];
         const unsigned taddr = tmem + (unsigned(q * 32) << 16) + d * kChunk;
@@ -273,8 +271,7 @@ __global__ void __launch_bounds__(kFwdThreads, 1) gate_gemm_forward_kernel(const
 #pragma unroll
         for (int i = 0; i < 32; ++i) x[i] = silu_s(x[i]);
       }
-      if (bar->failed) break;
-      if (!mbar_wait(saddr(&bar->a_empty[ab]), unsigned((t >> 1) & 1) ^ 1u)) { give_up(bar, a.status, 25); break; }
+      if (!bar->failed && !mbar_wait(saddr(&bar->a_empty[ab]), unsigned((t >> 1) & 1) ^ 1u)) give_up(bar, a.status, 25);
       tc_fence_after();
       const unsigned t_big = tmem_a + (unsigned(q * 32) << 16) + ab * 2 * kK + half * 32;
       store_split_tmem(t_big, t_big + kK, x);
@@ -310,34 +307,33 @@ __global__ void __launch_bounds__(kBwdThreads, 1) gate_gemm_backward_kernel(cons
   if (warp == 0) {
     if (lane == 0) stream_weights(a, work, bar, w_buf, 31);
   } else if (warp == 1) {
-    int64_t it = 0, wit = 0;
-    int t = 0, kept = -1;
-    bool ok = true;
-    for (int tile = blockIdx.x; tile < work.tiles() && ok && !bar->failed; tile += gridDim.x, ++t) {
-      const int s = work.segment(tile), chunks = a.seg[s].chunks;
-      const bool keep = chunks == 1 && tile + int(gridDim.x) < work.tiles() && work.segment(tile + gridDim.x) == s;
-      const int d = t & 1;
-      if (!mbar_wait(saddr(&bar->d_empty[d]), unsigned((t >> 1) & 1) ^ 1u)) { give_up(bar, a.status, 32); break; }
-      for (int c = 0; c < chunks; ++c, ++it) {
-        const int slot = int(wit % kWStages), sa = int(it % kAStagesBwd);
-        if ((kept != s && !mbar_wait(saddr(&bar->w_full[slot]), unsigned((wit / kWStages) & 1))) ||
-            !mbar_wait(saddr(&bar->a_full[sa]), unsigned((it / kAStagesBwd) & 1))) {
-          give_up(bar, a.status, 33);
-          ok = false;
-          break;
-        }
-        tc_fence_after();
-        const unsigned w_big = saddr(w_buf + slot * kWStageBytes), w_small = w_big + kWPartBytes;
-        if (elect_one()) {
+    if (elect_one()) {           // ---- MMA issue
+      int64_t it = 0, wit = 0;
+      int t = 0, kept = -1;
+      bool ok = true;
+      for (int tile = blockIdx.x; tile < work.tiles() && ok && !bar->failed; tile += gridDim.x, ++t) {
+        const int s = work.segment(tile), chunks = a.seg[s].chunks;
+        const bool keep = chunks == 1 && tile + int(gridDim.x) < work.tiles() && work.segment(tile + gridDim.x) == s;
+        const int d = t & 1;
+        if (!mbar_wait(saddr(&bar->d_empty[d]), unsigned((t >> 1) & 1) ^ 1u)) { give_up(bar, a.status, 32); break; }
+        for (int c = 0; c < chunks; ++c, ++it) {
+          const int slot = int(wit % kWStages), sa = int(it % kAStagesBwd);
+          if ((kept != s && !mbar_wait(saddr(&bar->w_full[slot]), unsigned((wit / kWStages) & 1))) ||
+              !mbar_wait(saddr(&bar->a_full[sa]), unsigned((it / kAStagesBwd) & 1))) {
+            give_up(bar, a.status, 33);
+            ok = false;
+            break;
+          }
+          tc_fence_after();
+          const unsigned w_big = saddr(w_buf + slot * kWStageBytes), w_small = w_big + kWPartBytes;
           issue_block(tmem + d * kChunk, tmem_a + sa * 2 * kK, w_big, w_small, c == 0);
           if (!keep) umma_commit(saddr(&bar->w_empty[slot]));
           umma_commit(saddr(&bar->a_empty[sa]));
           if (c == chunks - 1) umma_commit(saddr(&bar->d_full[d]));
+          wit += !keep;
         }
-        __syncwarp();
-        wit += !keep;
+        kept = keep ? s : -1;
       }
-      kept = keep ? s : -1;
     }
   } else if (warp < kBwdProducer0) {
     const int q = warp & 3;
@@ -347,7 +343,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) gate_gemm_backward_kernel(cons
       const int s = work.segment(tile), d = t & 1;
       const Segment& seg = a.seg[s];
       const int64_t g = work.first_row(tile, s) + row;
-      if (bar->failed || !mbar_wait(saddr(&bar->d_full[d]), unsigned((t >> 1) & 1))) { give_up(bar, a.status, 34); break; }
+      if (!bar->failed && !mbar_wait(saddr(&bar->d_full[d]), unsigned((t >> 1) & 1))) give_up(bar, a.status, 34);
       tc_fence_after();
       float v0[32], v1[32];
       const unsigned taddr = tmem + (unsigned(q * 32) << 16) + d * kChunk;
@@ -412,8 +408,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) gate_gemm_backward_kernel(cons
     for (int k = 0; k < kRawStages - 1; ++k) fetch();
     int64_t it = 0;
     int slot = 0;
-    bool ok = true;
-    for (int tile = blockIdx.x; tile < work.tiles() && ok; tile += gridDim.x) {
+    for (int tile = blockIdx.x; tile < work.tiles(); tile += gridDim.x) {
       const int s = work.segment(tile), chunks = a.seg[s].chunks;
       const Segment& seg = a.seg[s];
       const int64_t g = work.first_row(tile, s) + q * 32 + lane;
@@ -440,11 +435,7 @@ __global__ void __launch_bounds__(kBwdThreads, 1) gate_gemm_backward_kernel(cons
 #pragma unroll
           for (int i = 0; i < 32; ++i) x[i] += y[i];
         }
-        if (bar->failed || !mbar_wait(saddr(&bar->a_empty[sa]), unsigned((it / kAStagesBwd) & 1) ^ 1u)) {
-          give_up(bar, a.status, 35);
-          ok = false;
-          break;
-        }
+        if (!bar->failed && !mbar_wait(saddr(&bar->a_empty[sa]), unsigned((it / kAStagesBwd) & 1) ^ 1u)) give_up(bar, a.status, 35);
         tc_fence_after();
         const unsigned t_big = tmem_a + (unsigned(q * 32) << 16) + sa * 2 * kK + half * 32;
         store_split_tmem(t_big, t_big + kK, x);

@@ -107,6 +107,7 @@ __device__ __forceinline__ void teardown(unsigned tmem) {
 // MMA issue of both kernels: per pair of tiles, layer A for slot 0 and 1, then layer B for slot 0 and 1.
 __device__ __forceinline__ void mma_loop(const Args& a, Barriers* bar, unsigned char* smem, unsigned tmem,
                                          int64_t my_tiles) {
+  if (!elect_one()) return;        // the role of one lane, its waits included
   if (!mbar_wait(saddr(&bar->w_full), 0)) { give_up(bar, a.status, 41); return; }
   unsigned phase[2] = {0, 0};
   for (int64_t i = 0; i < my_tiles && !bar->failed; i += 2) {
@@ -118,11 +119,8 @@ __device__ __forceinline__ void mma_loop(const Args& a, Barriers* bar, unsigned 
         ++phase[s];
         tc_fence_after();
         const unsigned base = tmem + s * kSlotCols;
-        if (elect_one()) {
-          issue_block(base + 2 * kK, base, w_big, w_small, true);
-          umma_commit(saddr(&bar->h_full[s]));
-        }
-        __syncwarp();
+        issue_block(base + 2 * kK, base, w_big, w_small, true);
+        umma_commit(saddr(&bar->h_full[s]));
       }
     }
   }
@@ -174,11 +172,10 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_chain_forward_kernel(const __
         acc = fmaf(rb[6], wh.z, acc);
         x[n] = fmaf(rb[7], wh.w, acc);
       }
-      bool ok = true;
 #pragma unroll 1
       for (int layer = 0; layer < 3; ++layer) {
         if (layer > 0) {
-          if (bar->failed || !mbar_wait(saddr(&bar->h_full[s]), phase & 1)) { give_up(bar, a.status, 43); ok = false; break; }
+          if (!bar->failed && !mbar_wait(saddr(&bar->h_full[s]), phase & 1)) give_up(bar, a.status, 43);
           ++phase;
           tc_fence_after();
           tmem_ld32(t_acc, x);
@@ -195,7 +192,6 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_chain_forward_kernel(const __
         tc_fence_before();
         mbar_arrive(saddr(&bar->a_ready[s]));
       }
-      if (!ok) break;
       tc_fence_before();
     }
   }
@@ -235,7 +231,6 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_chain_backward_kernel(const _
       const int64_t g = (share.first + i * share.step) * kRows + row;
       const bool valid = g < nrows;
       float x[32], z[32];
-      bool ok = true;
 #pragma unroll 1
       for (int layer = 0; layer < 3; ++layer) {
         // silu'(z) of this layer: issue the loads before waiting for the accumulator
@@ -265,7 +260,7 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_chain_backward_kernel(const _
             for (int n = 0; n < 32; ++n) x[n] = 0.f;
           }
         } else {
-          if (bar->failed || !mbar_wait(saddr(&bar->h_full[s]), phase & 1)) { give_up(bar, a.status, 44); ok = false; break; }
+          if (!bar->failed && !mbar_wait(saddr(&bar->h_full[s]), phase & 1)) give_up(bar, a.status, 44);
           ++phase;
           tc_fence_after();
           tmem_ld32(t_acc, x);
@@ -277,7 +272,6 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_chain_backward_kernel(const _
         tc_fence_before();
         mbar_arrive(saddr(&bar->a_ready[s]));
       }
-      if (!ok) break;
       tc_fence_before();
       // ---- drb[k] = sum_n t1[n] W0[n][k]: partial sums over this thread's 32 units, halves added through smem
       float p[8];
@@ -297,12 +291,12 @@ __global__ void __launch_bounds__(kThreads, 1) mlp_chain_backward_kernel(const _
         p[7] = fmaf(x[n], wh.w, p[7]);
       }
       if (half == 1) {
-        if (bar->failed || !mbar_wait(x_free, (xphase & 1) ^ 1u)) { give_up(bar, a.status, 45); break; }
+        if (!bar->failed && !mbar_wait(x_free, (xphase & 1) ^ 1u)) give_up(bar, a.status, 45);
         *reinterpret_cast<float4*>(slot_x) = make_float4(p[0], p[1], p[2], p[3]);
         *reinterpret_cast<float4*>(slot_x + 4) = make_float4(p[4], p[5], p[6], p[7]);
         mbar_arrive(x_full);
       } else {
-        if (bar->failed || !mbar_wait(x_full, xphase & 1)) { give_up(bar, a.status, 46); break; }
+        if (!bar->failed && !mbar_wait(x_full, xphase & 1)) give_up(bar, a.status, 46);
         const float4 lo = *reinterpret_cast<const float4*>(slot_x), hi = *reinterpret_cast<const float4*>(slot_x + 4);
         mbar_arrive(x_free);
         p[0] += lo.x; p[1] += lo.y; p[2] += lo.z; p[3] += lo.w;

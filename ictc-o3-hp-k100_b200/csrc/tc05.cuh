@@ -43,12 +43,20 @@ __device__ __forceinline__ bool mbar_try(unsigned bar, unsigned parity) {
       : "memory");
   return done != 0;
 }
-__device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity) {
+__device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity, long long limit = kWaitCycles) {
   if (mbar_try(bar, parity)) return true;
   const long long start = clock64();
   while (!mbar_try(bar, parity))
-    if (clock64() - start > kWaitCycles) return false;
+    if (clock64() - start > limit) return false;
   return true;
+}
+// In a role of a whole warp the lanes must stay together: tcgen05.ld / st and __syncwarp need all of them, and lanes that gave up
+// and left alone, by their own clocks, would leave the others waiting there without a limit.  So a lane whose wait ran out
+// raises the block's failure flag and goes on; with the flag up nobody waits any more, all roles run out their loops, and
+// the status word says that the results are void.  (A vote at every wait instead cost 1 to 2 % of the training step and of small
+// MD steps.)  A role of a single lane may leave.  This is a wait with a vote, for where it is not on the path of a loop.
+__device__ __forceinline__ bool warp_wait(unsigned bar, unsigned parity, const volatile int& failed, long long limit = kWaitCycles) {
+  return __all_sync(0xffffffffu, !failed && mbar_wait(bar, parity, limit));
 }
 __device__ __forceinline__ void bulk_g2s(unsigned dst, const void* src, unsigned bytes, unsigned bar) {
   asm volatile("cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),

@@ -1,6 +1,7 @@
 // C-ABI entry points of the tensor product / graph message kernels and library-wide helpers.
 #include <stdarg.h>
 #include <string.h>
+#include "tc05.cuh"
 #include "tp_chunk.cuh"
 #include "tp_tma_kernels.cuh"
 
@@ -51,8 +52,9 @@ int* kernel_status_word() {
   return cache[dev];
 }
 
-// A wait that nothing will ever satisfy: the same bounded polling loop as the kernels' mbarrier waits, with a short
-// limit.  It gives up, records `code` in the status word and returns normally.
+// A wait that nothing will ever satisfy: the tensor-core kernels' own bounded wait, with a short limit that half of the lanes reach
+// earlier than the others.  The warp gives up together, elects a lane, which records `code` in the status word, and returns
+// normally.
 __global__ void bounded_wait_selftest_kernel(long long limit_cycles, int* status, int code) {
   __shared__ __align__(8) unsigned long long bar;
   const unsigned addr = smem_addr(&bar);
@@ -61,10 +63,10 @@ __global__ void bounded_wait_selftest_kernel(long long limit_cycles, int* status
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
-  const long long start = clock64();
-  bool done = mbar_try(addr, 0);
-  while (!done && clock64() - start <= limit_cycles) done = mbar_try(addr, 0);
-  if (!done && threadIdx.x == 0 && status) atomicExch(status, code);
+  const volatile int failed = 0;
+  const bool done = tc::warp_wait(addr, 0, failed, threadIdx.x < 16 ? limit_cycles : limit_cycles / 2);
+  if (tc::elect_one() && !done && status) atomicExch(status, code);
+  __syncwarp();
 }
 
 static bool check(bool ok, const char* what) {

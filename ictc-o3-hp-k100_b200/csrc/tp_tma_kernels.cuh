@@ -28,6 +28,9 @@ __device__ __forceinline__ void mbar_init(unsigned bar, unsigned count) {
 __device__ __forceinline__ void mbar_expect_tx(unsigned bar, unsigned bytes) {
   asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
+__device__ __forceinline__ void mbar_arrive(unsigned bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
+}
 __device__ __forceinline__ void bulk_g2s(unsigned dst, const void* src, unsigned bytes, unsigned bar) {
   asm volatile("cp.async.bulk.shared::cta.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
                "l"(src), "r"(bytes), "r"(bar)
@@ -45,11 +48,11 @@ __device__ __forceinline__ bool mbar_try(unsigned bar, unsigned parity) {
   return done != 0;
 }
 // Bounded wait for the phase with the given parity; false when the time limit ran out.
-__device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity) {
+__device__ __forceinline__ bool mbar_wait(unsigned bar, unsigned parity, long long limit = kWaitCycles) {
   if (mbar_try(bar, parity)) return true;
   const long long start = clock64();
   while (!mbar_try(bar, parity))
-    if (clock64() - start > kWaitCycles) return false;
+    if (clock64() - start > limit) return false;
   return true;
 }
 
@@ -90,7 +93,7 @@ template <class S, class F, int CPL, int STAGES, bool ADJ> struct TmaLayout {
   static constexpr unsigned SLOT_BYTES = GATE_BYTES + ROW_BYTES;
   static constexpr unsigned GEO_BYTES = 2 * NBP * sizeof(Vec<CPL>);
   static constexpr unsigned BAR_OFF = STAGES * SLOT_BYTES;
-  static constexpr unsigned GEO_OFF = BAR_OFF + ((STAGES * 8 + 15) / 16) * 16;
+  static constexpr unsigned GEO_OFF = BAR_OFF + ((STAGES * 8 + 8 + 15) / 16) * 16;      // the last one: the row's barrier
   // adjoint only: per-lane harmonic-gradient partial sums of RED_EDGES edges, one padded row of 32 lanes per
   // (edge, harmonic); lane r later adds up row r
   static constexpr int RED_EDGES = 32 / S::NH, RED_PITCH = 36;
@@ -119,13 +122,20 @@ constexpr int64_t split_limit_adjoint() { return 2 * kResidentRows; }
 __host__ __device__ constexpr int split_warps(int split) { return split > 1 ? split : kTmaWarps; }
 
 // Sum of the warps' partial rows (`count` vectors per lane, parked at the start of every warp's slot memory), added
-// in warp order; warp w finishes the vectors w, w + SPLIT, ...
+// in warp order; warp w finishes the vectors w, w + SPLIT, ...  The threads of the row meet at a barrier with a time limit (`bar`,
+// `warps x 32` arrivals): a lane whose own wait ran out has left, and nobody may wait for it for ever.  The limit is longer than a
+// copy's, since the parts of a row differ by a few edges' time at most.
 template <int SPLIT, int COUNT, unsigned WARP_BYTES, class V, class Put>
-__device__ __forceinline__ void add_parts(unsigned char* smem, const V (&mine)[COUNT], int warp, int lane, Put put) {
+__device__ __forceinline__ void add_parts(unsigned char* smem, unsigned bar, int* status, const V (&mine)[COUNT], int warp,
+                                          int lane, Put put) {
   V* part = reinterpret_cast<V*>(smem + warp * WARP_BYTES) + lane;
 #pragma unroll
   for (int k = 0; k < COUNT; ++k) part[k * 32] = mine[k];
-  __syncthreads();
+  mbar_arrive(bar);
+  if (!mbar_wait(bar, 0, 4 * kWaitCycles)) {
+    if (status) atomicExch(status, 5);
+    return;
+  }
   for (int k = warp; k < COUNT; k += SPLIT) {
     V sum = reinterpret_cast<const V*>(smem)[k * 32 + lane];
 #pragma unroll
@@ -146,14 +156,16 @@ tp_graph_forward_tma_kernel(TpArgs a) {
   int64_t n = SPLIT > 1 ? int64_t(blockIdx.x) : int64_t(blockIdx.x) * kTmaWarps + warp;
   if (n >= a.N) return;
   unsigned char* mine = tma_smem + warp * L::WARP_BYTES;
-  const unsigned bars = smem_addr(mine + L::BAR_OFF);
+  const unsigned bars = smem_addr(mine + L::BAR_OFF), row_bar = smem_addr(tma_smem + L::BAR_OFF) + STAGES * 8;
   V* geo = reinterpret_cast<V*>(mine + L::GEO_OFF);
   if (lane == 0) {
 #pragma unroll
     for (int s = 0; s < STAGES; ++s) mbar_init(bars + s * 8, 1);
+    if (SPLIT > 1 && warp == 0) mbar_init(row_bar, SPLIT * 32);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  __syncwarp();
+  if (SPLIT > 1) __syncthreads();
+  else __syncwarp();
   BTerm bt[L::R];
 #pragma unroll
   for (int r = 0; r < L::R; ++r) bt[r] = (r * 32 + lane < F::NB) ? F::fb(r * 32 + lane) : BTerm{0, 0.f, 0, 0.f};
@@ -231,7 +243,6 @@ tp_graph_forward_tma_kernel(TpArgs a) {
         const int64_t owner = it - slot + s + (refilled ? STAGES : 0);
         if (owner < end) mbar_wait(bars + s * 8, refilled ? parity ^ 1u : parity);
       }
-      if (SPLIT > 1) break;       // the row's other warps wait for this one at the block's barrier
       return;
     }
     const unsigned char* base = mine + slot * L::SLOT_BYTES + lane * (CPL * 4);
@@ -264,7 +275,7 @@ tp_graph_forward_tma_kernel(TpArgs a) {
   if constexpr (SPLIT > 1) {
     static_assert(S::NO <= STAGES * S::NP, "the partial row has to fit the slots");
     __syncwarp();
-    add_parts<SPLIT, S::NO, L::WARP_BYTES>(tma_smem, acc, warp, lane, [&](int k, V v) { v.store(op + k * C); });
+    add_parts<SPLIT, S::NO, L::WARP_BYTES>(tma_smem, row_bar, a.status, acc, warp, lane, [&](int k, V v) { v.store(op + k * C); });
     return;
   }
 #pragma unroll
@@ -283,14 +294,16 @@ __global__ void __launch_bounds__(split_warps(SPLIT) * 32, kTmaMinWarpsAdj / spl
   int64_t owner = SPLIT > 1 ? int64_t(blockIdx.x) : int64_t(blockIdx.x) * kTmaWarps + warp;
   if (owner >= (GRAPH ? a.N : a.E)) return;
   unsigned char* mine = tma_smem + warp * L::WARP_BYTES;
-  const unsigned bars = smem_addr(mine + L::BAR_OFF);
+  const unsigned bars = smem_addr(mine + L::BAR_OFF), row_bar = smem_addr(tma_smem + L::BAR_OFF) + STAGES * 8;
   V* geo = reinterpret_cast<V*>(mine + L::GEO_OFF);
   if (lane == 0) {
 #pragma unroll
     for (int s = 0; s < STAGES; ++s) mbar_init(bars + s * 8, 1);
+    if (SPLIT > 1 && warp == 0) mbar_init(row_bar, SPLIT * 32);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  __syncwarp();
+  if (SPLIT > 1) __syncthreads();
+  else __syncwarp();
   BTerm bt[L::R];
 #pragma unroll
   for (int r = 0; r < L::R; ++r) bt[r] = (r * 32 + lane < F::NB) ? F::ap(r * 32 + lane) : BTerm{0, 0.f, 0, 0.f};
@@ -370,7 +383,6 @@ __global__ void __launch_bounds__(split_warps(SPLIT) * 32, kTmaMinWarpsAdj / spl
         const int64_t owner = it - slot + s + (refilled ? STAGES : 0);
         if (owner < end) mbar_wait(bars + s * 8, refilled ? parity ^ 1u : parity);
       }
-      if (SPLIT > 1) break;
       return;
     }
     const unsigned char* base = mine + slot * L::SLOT_BYTES + lane * (CPL * 4);
@@ -444,7 +456,7 @@ __global__ void __launch_bounds__(split_warps(SPLIT) * 32, kTmaMinWarpsAdj / spl
     if constexpr (SPLIT > 1) {
       static_assert(S::NX <= STAGES * S::NP, "the partial row has to fit the slots");
       __syncwarp();
-      add_parts<SPLIT, S::NX, L::WARP_BYTES>(tma_smem, dx, warp, lane, [&](int i, V v) { v.store(dxp + i * C); });
+      add_parts<SPLIT, S::NX, L::WARP_BYTES>(tma_smem, row_bar, a.status, dx, warp, lane, [&](int i, V v) { v.store(dxp + i * C); });
       return;
     }
 #pragma unroll

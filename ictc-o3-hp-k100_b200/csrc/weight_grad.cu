@@ -117,14 +117,9 @@ __global__ void __launch_bounds__(kThreads, 1) weight_grad_kernel(Args a) {
 
   if (warp == 0) {
     // ---- MMA issue: per operand stage ks_n K = 8 steps, three products per feature tile
-    bool ok = true;
-    for (int64_t it = 0; it < mine && !bar->failed; ++it) {
+    for (int64_t it = 0; it < mine; ++it) {
       const int s = int(it % kOpStages);
-      if (!mbar_wait(saddr(&bar->op_full[s]), unsigned((it / kOpStages) & 1))) {
-        give_up(bar, a.status, 41);
-        ok = false;
-        break;
-      }
+      if (!bar->failed && !mbar_wait(saddr(&bar->op_full[s]), unsigned((it / kOpStages) & 1))) give_up(bar, a.status, 41);
       tc_fence_after();
       if (elect_one()) {
         for (int ks = 0; ks < ks_n; ++ks) {
@@ -144,21 +139,20 @@ __global__ void __launch_bounds__(kThreads, 1) weight_grad_kernel(Args a) {
       }
       __syncwarp();
     }
-    if (ok && mine > 0 && !bar->failed && elect_one()) umma_commit(saddr(&bar->done));
+    if (mine > 0 && elect_one()) umma_commit(saddr(&bar->done));
     __syncwarp();
   } else if (warp == 1) {
     // ---- row stream: lane r copies rows r, r + 32, ... of the stage (one bulk copy per row and operand)
-    for (int64_t it = 0; it < mine && !bar->failed; ++it) {
+    bool ok = true;
+    int64_t it = 0;
+    for (; it < mine; ++it) {
       const int s = int(it % kRawStages);
-      if (!mbar_wait(saddr(&bar->raw_empty[s]), unsigned((it / kRawStages) & 1) ^ 1u)) {
-        give_up(bar, a.status, 44);
-        break;
-      }
+      if (bar->failed || !mbar_wait(saddr(&bar->raw_empty[s]), unsigned((it / kRawStages) & 1) ^ 1u)) { give_up(bar, a.status, 44); ok = false; }
       const int64_t r0 = (s0 + it) * stage_rows;
       const int valid = int(min(int64_t(stage_rows), a.R - r0));
       const unsigned fb = saddr(&bar->raw_full[s]);
-      if (lane == 0) mbar_expect_tx(fb, unsigned(valid) * unsigned(pitch));
-      __syncwarp();
+      if (lane == 0 && ok) mbar_expect_tx(fb, unsigned(valid) * unsigned(pitch));
+      if (!__all_sync(0xffffffffu, ok)) break;
       // raw stage = [stage_rows x NO] block of grad, then [stage_rows x 64] block of rows; an operand stored without
       // row padding arrives as ONE copy (small per-row copies are bound by the copy engine's request rate)
       const unsigned gdst = saddr(raw + s * raw_b), xdst = gdst + unsigned(stage_rows) * unsigned(a.NO) * 4u;
@@ -175,6 +169,9 @@ __global__ void __launch_bounds__(kThreads, 1) weight_grad_kernel(Args a) {
           bulk_g2s(xdst + unsigned(r) * kK * 4u, a.rows + (r0 + r) * a.rows_ld, kK * 4u, fb);
       }
     }
+    if (it < mine && lane == 0)        // given up: the copies in flight are waited for (again with a limit) before the warp leaves
+      for (int64_t k = it > kRawStages ? it - kRawStages : 0; k < it; ++k)
+        mbar_wait(saddr(&bar->raw_full[k % kRawStages]), unsigned((k / kRawStages) & 1));
   } else {
     // ---- transform: thread = up to kItemsMax 16-byte chunks (K step, feature, four consecutive rows) per stage
     const int pt = threadIdx.x - 64;
@@ -199,11 +196,8 @@ __global__ void __launch_bounds__(kThreads, 1) weight_grad_kernel(Args a) {
     }
     for (int64_t it = 0; it < mine; ++it) {
       const int rs = int(it % kRawStages), os = int(it % kOpStages);
-      if (bar->failed || !mbar_wait(saddr(&bar->raw_full[rs]), unsigned((it / kRawStages) & 1)) ||
-          !mbar_wait(saddr(&bar->op_empty[os]), unsigned((it / kOpStages) & 1) ^ 1u)) {
-        give_up(bar, a.status, 42);
-        break;
-      }
+      if (!bar->failed && (!mbar_wait(saddr(&bar->raw_full[rs]), unsigned((it / kRawStages) & 1)) ||
+                           !mbar_wait(saddr(&bar->op_empty[os]), unsigned((it / kOpStages) & 1) ^ 1u))) give_up(bar, a.status, 42);
       const int valid = int(min(int64_t(stage_rows), a.R - (s0 + it) * stage_rows));
       const unsigned char* in = raw + rs * raw_b;
       unsigned char* out = ops + os * op_b;
@@ -234,7 +228,7 @@ __global__ void __launch_bounds__(kThreads, 1) weight_grad_kernel(Args a) {
       const int qd = warp & 3;
       float* outp = a.partial + int64_t(blockIdx.x) * tiles * kRows * kK;
       bool have = mine > 0;
-      if (have && (bar->failed || !mbar_wait(saddr(&bar->done), 0u))) {
+      if (have && !warp_wait(saddr(&bar->done), 0u, bar->failed)) {
         give_up(bar, a.status, 43);
         have = false;
       }
