@@ -479,6 +479,7 @@ int launch_forward(Args a, cudaStream_t st) {
   if (attr != cudaSuccess) { set_error("gate gemm smem: %s", cudaGetErrorString(attr)); return ICTC_ERR_LAUNCH; }
   bool one_wave;
   const int grid = prepare(a, one_wave);
+  if (grid == 0) return ICTC_OK;          // no rows
   launch_if(one_wave, gate_gemm_forward_kernel, grid, kFwdThreads, kFwdSmem, st, a);
   return finish_launch("gate_gemm_forward");
 }
@@ -489,6 +490,7 @@ int launch_backward(Args a, cudaStream_t st) {
   if (attr != cudaSuccess) { set_error("gate gemm smem: %s", cudaGetErrorString(attr)); return ICTC_ERR_LAUNCH; }
   bool one_wave;
   const int grid = prepare(a, one_wave);
+  if (grid == 0) return ICTC_OK;          // no rows
   launch_if(one_wave, gate_gemm_backward_kernel, grid, kBwdThreads, kBwdSmem, st, a);
   return finish_launch("gate_gemm_backward");
 }

@@ -486,6 +486,14 @@ class Runner {
     call(stage, label(kLinear, layer), 1, [&] { return deep ? gg::launch_backward(a, st) : gg::launch_forward(a, st); });
   }
 
+  // messages and feature gradients of a list without edges
+  void clear(int stage, float* out, int64_t count) {
+    call(stage, -1, 1, [&] {
+      if (count > 0) cudaMemsetAsync(out, 0, count * sizeof(float), st);
+      return finish_launch("sweep_clear");
+    });
+  }
+
   // Chunk bounds of a sweep over `rows` owner rows.
   int64_t chunk_rows(int64_t rows) const { return p.chunk_rows > 0 && p.chunk_rows < rows ? p.chunk_rows : rows; }
 
@@ -503,7 +511,7 @@ class Runner {
 };
 
 int Runner::run() {
-  const int64_t n = p.n_owned, N = p.n_local, E = p.edges, U = p.rep ? p.pair_rows : E;
+  const int64_t n = p.n_owned, N = p.n_local, E = p.edges, U = p.rep && E > 0 ? p.pair_rows : E;
   const ictc_sweep_layer &L0 = p.layer[0], &L1 = p.layer[1];
   const int spec[2] = {ictc_tp_spec(0, 2, 2), ictc_tp_spec(2, 2, 2)};
   const int64_t W0 = 9 * kC, W1 = 35 * kC;
@@ -597,6 +605,7 @@ int Runner::run() {
   auto graph_forward = [&](int stage, int layer, const float* x, float* out) {
     const ictc_sweep_layer& L = p.layer[layer];
     const int64_t width = layer == 0 ? W0 : W1;
+    if (E == 0) return clear(stage, out, n * width);
     if (table) {
       gate_table[layer] = buffer(U * L.num_gates);
       if (U > 0) gates(stage, layer, pre[layer][2], gate_table[layer], U, nullptr, nullptr, p.live);
@@ -675,6 +684,10 @@ int Runner::run() {
   const int64_t* gates_by_position = nullptr;
   auto graph_adjoint = [&](int stage, int layer, const float* x, const float* cot, float* dx, float* dsh, float* da3) {
     const ictc_sweep_layer& L = p.layer[layer];
+    if (E == 0) {
+      if (dx) clear(stage, dx, N * W0);
+      return;
+    }
     const int64_t xw = layer == 0 ? kC : W0, step = chunk_rows(N);
     const int64_t cap = step < N ? p.chunk_capacity_src : (E > 0 ? E : 1);
     float* dg = buffer(cap * L.num_gates);
@@ -843,7 +856,7 @@ int64_t ictc_sweep_workspace(const ictc_sweep* p) {
 
 int ictc_sweep_run(const ictc_sweep* p, int stages, void* stream) {
   if (int rc = sweep::check(p)) return rc;
-  if (!p->pos || !p->species || !p->energy || !p->atomic || !p->gradient || !p->status ||
+  if (!p->pos || !p->species || !p->energy || (p->n_owned > 0 && !p->atomic) || !p->gradient || !p->status ||
       !p->work || (p->edges > 0 && (!p->src || !p->dst))) {
     set_error("sweep: NULL buffer");
     return ICTC_ERR_BAD_ARG;

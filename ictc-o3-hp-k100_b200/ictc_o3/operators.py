@@ -450,6 +450,8 @@ def _tc_weight_grad(grad, rows):
         return _tc_weight_grad(rows, grad).t()
     grad, rows = grad.contiguous(), rows.contiguous()
     r = grad.shape[0]
+    if r == 0:
+        return torch.zeros(cout, 64, dtype=torch.float32, device=grad.device)
     out = torch.empty(cout, 64, dtype=torch.float32, device=grad.device)
     lib = _lib.load()
     with _lib.on_device(grad.device):

@@ -226,6 +226,41 @@ def test_small_sweeps_queued_behind_each_other_do_not_see_each_other():
         assert all(torch.equal(a, b) for a, b in zip(got + forces, alone + steps))
 
 
+@pytest.mark.parametrize("share_gates,chunk_rows,stream_gates", [(True, None, None), (False, None, None), (True, 1, True)])
+def test_atoms_without_any_neighbour(share_gates, chunk_rows, stream_gates):
+    from mace_ictc.hp import energy_and_forces
+    from mace_ictc.md import MolecularDynamics
+    model = _model()
+    pos, z = np.array([[1.0, 1.0, 1.0], [9.0, 9.0, 9.0], [1.0, 9.0, 17.0]]), np.array([1, 6, 8])
+    md = MolecularDynamics(model, pos, z, np.full(3, 24.0), velocities=np.zeros((3, 3)), share_gates=share_gates,
+                           chunk_rows=chunk_rows, stream_gates=stream_gates)
+    assert md.engine is not None and bool((md.compute_forces() == 0).all()) and md.num_edges == 0
+    empty = torch.zeros(0, dtype=torch.int64, device="cuda")
+    graph = [torch.as_tensor(pos, dtype=torch.float32).cuda(), torch.as_tensor(z).cuda(), torch.zeros(3, dtype=torch.int64, device="cuda"),
+             empty, empty, torch.zeros(0, 3, device="cuda"), 24.0 * torch.eye(3, device="cuda").unsqueeze(0)]
+    alone = energy_and_forces(model, *graph)
+    assert bool((alone["forces"] == 0).all()) and torch.isfinite(alone["energy"]).all()
+    assert abs(float(md.energy) - float(alone["energy"])) < 1e-5 * abs(float(alone["energy"]))
+    tape = energy_and_forces(model, *graph, training=True)
+    tape["energy"].sum().backward()
+    assert all(p.grad is None or torch.isfinite(p.grad).all() for p in model.parameters())
+    md.step()
+    md.enable_graph()
+    md.run(2)
+    assert bool((md.forces == 0).all()) and abs(float(md.energy) - float(alone["energy"])) < 1e-5 * abs(float(alone["energy"]))
+
+
+def test_a_rank_without_owned_rows():
+    """Ghost rows alone: nothing to sum up, no launch without rows."""
+    from mace_ictc.engine import ForceEngine
+    model = _model()
+    pos = torch.rand(5, 3, device="cuda")
+    empty = torch.zeros(0, dtype=torch.int64, device="cuda")
+    energy, grad, atomic = ForceEngine(model).energy_and_gradient(pos, empty.new_zeros(5), empty, empty, None, [9.0, 9.0, 9.0], 0,
+                                                                  empty.new_zeros(1))
+    assert float(energy) == 0.0 and atomic.numel() == 0 and bool((grad == 0).all())
+
+
 @pytest.mark.parametrize("number", [7, 500])
 def test_unknown_atoms_raise_without_input_validation(number):
     """The status word is read in any case: an unknown atom never counts as a known one."""
