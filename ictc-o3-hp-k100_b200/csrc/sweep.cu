@@ -32,7 +32,7 @@ struct EmbedArgs {
   int64_t* species;
   const float* up;             // [S, 64] embedding times linear_up
   float* u0;                   // [n, 64]
-  double* energy;              // [graphs], cleared here
+  double* energy;              // [graphs], cleared here (several graphs)
   int64_t graphs, n;
   const int64_t* batch;        // or null
   int* status;                 // bit 0: an atomic number outside the model, bit 1: a graph index outside [0, graphs)
@@ -216,14 +216,33 @@ struct GradArgs {
   const float4* dvec;
   float sign;
   float* out;
-  const double* energy_sum;    // [graphs] -> energy (float)
+  const double* energy_sum;    // sums per graph, or (parts > 0) the readout blocks' sums of the one graph
   float* energy;
-  int64_t graphs;
+  int64_t graphs, parts;
 };
 
-__global__ void position_gradient8_kernel(GradArgs a) {
+// The one graph's energy: the first block adds the readout blocks' sums, every thread its own and then a tree, in an order that
+// depends on their number alone (the sweep is repeatable bit by bit).  131,072 atoms have 4,096 of them.
+constexpr int kGradThreads = 256;
+__device__ __forceinline__ void add_energy(const GradArgs& a) {
+  __shared__ double part[kGradThreads];
+  double s = 0.0;
+  for (int64_t k = threadIdx.x; k < a.parts; k += kGradThreads) s += a.energy_sum[k];
+  part[threadIdx.x] = s;
+  for (int half = kGradThreads / 2; half > 0; half >>= 1) {
+    __syncthreads();
+    if (threadIdx.x < half) part[threadIdx.x] += part[threadIdx.x + half];
+  }
+  if (threadIdx.x == 0) a.energy[0] = float(part[0]);
+}
+
+__global__ void __launch_bounds__(kGradThreads) position_gradient8_kernel(GradArgs a) {
   const int64_t t = int64_t(blockIdx.x) * blockDim.x + threadIdx.x + pdl_enter();
-  if (t < a.graphs) a.energy[t] = float(a.energy_sum[t]);
+  if (a.parts > 0) {
+    if (blockIdx.x == 0) add_energy(a);
+  } else if (t < a.graphs) {
+    a.energy[t] = float(a.energy_sum[t]);
+  }
   const int64_t i = t >> 3;
   const int sub = int(t & 7);
   float x = 0.f, y = 0.f, z = 0.f;
@@ -287,7 +306,7 @@ struct TailArgs {
   int64_t graphs;
   int mask_atomic;
   float* atomic;               // [n]
-  double* energy;              // [graphs]
+  double* energy;              // [graphs], added to; without a batch [blocks], written
   float* dy;                   // [n, 64]
   float* dh;                   // [n, 64]
   int64_t n;
@@ -299,6 +318,7 @@ struct TailArgs {
 constexpr int kTailWarps = 8;
 constexpr int64_t kTailSlots = 148 * 64;
 static int tail_nodes(int64_t n) { return n <= kTailSlots ? 1 : 4; }
+static int64_t tail_blocks(int64_t n) { return (n + kTailWarps * tail_nodes(n) - 1) / (kTailWarps * tail_nodes(n)); }
 
 __global__ void __launch_bounds__(kTailWarps * 32) tail_kernel(TailArgs a, int nodes) {
   __shared__ double block_energy[kTailWarps];
@@ -371,7 +391,7 @@ __global__ void __launch_bounds__(kTailWarps * 32) tail_kernel(TailArgs a, int n
   if (threadIdx.x == 0) {
     double total = 0.0;
     for (int w = 0; w < kTailWarps; ++w) total += block_energy[w];
-    atomicAdd(a.energy, total);
+    a.energy[blockIdx.x] = total;
   }
 }
 
@@ -523,7 +543,10 @@ int Runner::run() {
   const bool merged_back = merged && E <= (int64_t(4) << 20);
 
   // ---------------------------------------------------------------- stage 1
-  double* energy = buffer<double>(p.graphs);
+  // one graph: the readout's blocks leave their sums; several: they add to the graphs' sums
+  const int64_t* batch = p.graphs > 1 ? p.batch : nullptr;
+  const int64_t parts = batch ? 0 : tail_blocks(n);
+  double* energy = buffer<double>(parts > p.graphs ? parts : p.graphs);
   float* u0 = buffer(N * kC);
   call(1, -1, 1, [&] {
     EmbedArgs a{p.numbers, p.species_table, p.species_table_size, p.species, p.up0_table, u0, energy, p.graphs, N, p.batch, p.status};
@@ -664,10 +687,8 @@ int Runner::run() {
   contraction(4, 1, m1, y1);
   call(4, -1, 1, [&] {
     TailArgs a{y1, features, W0, p.species, p.readout_rp, p.readout_rs, p.readout_w2, p.readout_ro0, int(p.hidden),
-               p.row_mask, p.batch, p.graphs, int(p.mask_atomic), p.atomic, energy, dy1, dh, n};
-    const int nodes = tail_nodes(n);
-    if (n > 0)
-      launch_after(tail_kernel, (unsigned)((n + kTailWarps * nodes - 1) / (kTailWarps * nodes)), kTailWarps * 32, 0, st, a, nodes);
+               p.row_mask, batch, p.graphs, int(p.mask_atomic), p.atomic, energy, dy1, dh, n};
+    if (n > 0) launch_after(tail_kernel, (unsigned)tail_blocks(n), kTailWarps * 32, 0, st, a, tail_nodes(n));
     return finish_launch("sweep_tail");
   });
   float* dm = buffer(n * W0);
@@ -777,9 +798,10 @@ int Runner::run() {
   });
   call(16, -1, 1, [&] {
     GradArgs a{N, n, dst_rowptr, dst_order, src_rowptr, src_order, dvec, float(p.gradient_sign), p.gradient, energy,
-               p.energy, p.graphs};
+               p.energy, p.graphs, parts};
     const int64_t threads = 8 * N > p.graphs ? 8 * N : p.graphs;
-    if (threads > 0) launch_after(position_gradient8_kernel, (unsigned)((threads + 255) / 256), 256, 0, st, a);
+    if (threads > 0)
+      launch_after(position_gradient8_kernel, (unsigned)((threads + kGradThreads - 1) / kGradThreads), kGradThreads, 0, st, a);
     return finish_launch("sweep_position_gradient");
   });
   return rc;

@@ -16,7 +16,8 @@ gates of a chunk's edges from the 64-wide hidden state, consumes them and reuses
 recomputes the chunk's gates, lets the tensor-product adjoint write the chunk's gate gradients and contracts
 them back to the hidden width at once.  No tensor wider than 64 floats per edge outlives a chunk.  Without
 chunking the gate table of the (edge, reverse edge) pairs is kept for both sweeps and only the gate gradient is
-per edge.  Both modes run the same arithmetic per edge in the same order, so their results agree bit for bit.
+per edge.  Both modes run the same arithmetic per edge in the same order, so their results agree bit for bit (the energy of
+one graph included; those of a batch are added up with double-precision atomics).
 """
 from __future__ import annotations
 

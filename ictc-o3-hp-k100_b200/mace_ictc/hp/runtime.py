@@ -51,7 +51,8 @@ def _force_engine(model, tensors, mask):
     """The tape-free engine for an inference call, or None where the autograd route has to answer: other widths or
     depths, hooks, tensors of another type, shape or device, stream capture (a recorded call reads the parameters at each
     replay), forward-mode and functorch tracing, dispatch modes and autocast (which that route sees or refuses), hooks on the
-    positions (which change the gradient) and lazily negated tensors (whose words have the other sign)."""
+    positions (which change the gradient), lazily negated tensors (whose words have the other sign), and several graphs under
+    deterministic algorithms (the sweep adds a batch's energies with atomics)."""
     if type(model) is not MaceIctcModel or model.channels != 64 or len(model.interactions) != 2:
         return None
     positions, numbers, batch, src, dst, shifts, cell = tensors
@@ -67,6 +68,7 @@ def _force_engine(model, tensors, mask):
             or mask is not None and (type(mask) is not torch.Tensor or mask.device != dev or mask.is_neg())
             or any(t.is_neg() for t in (positions, shifts, cell)) or positions._backward_hooks
             or torch._C._len_torch_dispatch_stack() > 0 or torch.jit.is_tracing()
+            or cell.shape[0] > 1 and torch.are_deterministic_algorithms_enabled()
             or torch.is_autocast_enabled("cuda") or torch._C._are_functorch_transforms_active()
             or torch.autograd.forward_ad._current_level >= 0 or torch.compiler.is_compiling()
             or torch.cuda.is_current_stream_capturing()):

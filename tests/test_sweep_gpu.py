@@ -261,6 +261,41 @@ def test_a_rank_without_owned_rows():
     assert float(energy) == 0.0 and atomic.numel() == 0 and bool((grad == 0).all())
 
 
+@pytest.mark.parametrize("side,chunk_rows", [(6, None), (22, None), (22, 4000)])
+def test_energies_repeat_bit_by_bit(side, chunk_rows):
+    """Below and above the sizes where a warp of the readout takes several atoms; an order of additions that changed from run to
+    run would show in the last bit of some of these sums."""
+    from mace_ictc import synthetic as S
+    from mace_ictc.hp import energy_and_forces
+    from mace_ictc.md import MolecularDynamics
+    model = _model()
+    with torch.no_grad():
+        model.layer_energy_readouts[0].readout.weight.mul_(1e3)         # large terms of both signs
+    pos, box, species = S.jittered_lattice(side, side, side, 2.15, 0.1, 5)
+    z = np.array(ELEMENTS)[species]
+    md = MolecularDynamics(model, pos, z, box, seed=2, chunk_rows=chunk_rows)
+    md.compute_forces()
+    first = md.energy.clone()
+    whole = MolecularDynamics(model, pos, z, box, seed=2)
+    whole.compute_forces()
+    assert torch.equal(first, whole.energy)
+    exact = float(whole.engine.energy_and_gradient(whole.pos, whole.species, *_edges(whole))[2].double().sum())
+    assert abs(float(first) - exact) <= 1e-7 * abs(exact)              # the blocks' sums are in double precision
+    for _ in range(5):
+        md.compute_forces()
+        assert torch.equal(md.energy, first)
+    src, dst, shifts = whole._eager_list.src, whole._eager_list.dst, whole._eager_list.shifts
+    graph = [whole.pos, whole.z, torch.zeros_like(whole.z), src[:whole.num_edges], dst[:whole.num_edges], shifts[:whole.num_edges],
+             torch.diag(whole.box_f).unsqueeze(0)]
+    energies = {float(energy_and_forces(model, *graph)["energy"]) for _ in range(5)}
+    assert len(energies) == 1
+
+
+def _edges(md):
+    nl, e = md._eager_list, md.num_edges
+    return nl.src[:e], nl.dst[:e], nl.shifts[:e], md.box.tolist(), md.pos.shape[0], nl.rowptr
+
+
 @pytest.mark.parametrize("number", [7, 500])
 def test_unknown_atoms_raise_without_input_validation(number):
     """The status word is read in any case: an unknown atom never counts as a known one."""
