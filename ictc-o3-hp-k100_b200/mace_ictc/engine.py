@@ -39,7 +39,6 @@ _ALL, _STAGES = 31, (1, 2, 4, 8, 16)
 _LABELS = ("radial_mlp_hidden_forward_{nout}", "gate_gemm_forward_{nout}", "graph_forward_l{layer}",
            "graph_adjoint_l{layer}", "gate_gemm_backward_{nout}", "radial_mlp_hidden_backward_{nout}",
            "channel_linear_tc", "symmetric_contraction_l{layer}")
-_MARKS = 1024            # timed launches of one sweep (eager steps of a benchmark)
 _WATCH_WORDS = 2048      # words of a parameter that one block of the sweep compares
 _HOOKS = ("_forward_hooks", "_forward_pre_hooks", "_backward_hooks", "_backward_pre_hooks")
 _GLOBAL_HOOKS = ("_global_forward_hooks", "_global_forward_pre_hooks", "_global_backward_hooks", "_global_backward_pre_hooks")
@@ -351,12 +350,15 @@ class ForceEngine:
         counts = (C.c_int64 * 2)()
         s.host_counts = C.addressof(counts)
         if self.profile is not None:
-            events = [torch.cuda.Event(enable_timing=True) for _ in range(2 * _MARKS)]
+            # room for every timed launch: some 40 of a sweep, per chunk and interaction two receiver and three sender launches
+            chunks = 1 if not s.chunk_rows else -(-max(s.n_owned, s.n_local) // s.chunk_rows)
+            marks = 64 + 10 * chunks
+            events = [torch.cuda.Event(enable_timing=True) for _ in range(2 * marks)]
             for e in events:
                 e.record()
-            handles = (C.c_void_p * (2 * _MARKS))(*[e.cuda_event for e in events])
-            labels = (C.c_int64 * _MARKS)()
-            s.host_marks, s.host_marks_capacity, s.host_mark_labels = C.addressof(handles), _MARKS, C.addressof(labels)
+            handles = (C.c_void_p * (2 * marks))(*[e.cuda_event for e in events])
+            labels = (C.c_int64 * marks)()
+            s.host_marks, s.host_marks_capacity, s.host_mark_labels = C.addressof(handles), marks, C.addressof(labels)
         st = _lib.stream(self.dev)
 
         def stages(mask):

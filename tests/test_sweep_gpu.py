@@ -296,6 +296,24 @@ def _edges(md):
     return nl.src[:e], nl.dst[:e], nl.shifts[:e], md.box.tolist(), md.pos.shape[0], nl.rowptr
 
 
+@pytest.mark.parametrize("chunk_rows", [None, 3])
+def test_a_profile_names_every_heavy_launch(chunk_rows):
+    from mace_ictc import synthetic as S
+    from mace_ictc.md import MolecularDynamics
+    pos, box, species = S.jittered_lattice(9, 9, 9, 2.15, 0.1, 5)
+    md = MolecularDynamics(_model(), pos, np.array(ELEMENTS)[species], box, chunk_rows=chunk_rows, stream_gates=True)
+    md.engine.profile = profile = []
+    md.compute_forces()
+    torch.cuda.synchronize()
+    names = [name for name, start, end in profile if start.elapsed_time(end) >= 0]
+    chunks = 1 if chunk_rows is None else 243
+    for layer, gates in ((0, 192), (1, 704)):
+        assert names.count(f"graph_forward_l{layer}") == names.count(f"graph_adjoint_l{layer}") == chunks
+        assert names.count(f"gate_gemm_backward_{gates}") == chunks
+        assert names.count(f"gate_gemm_forward_{gates}") == (1 if chunk_rows is None else 2 * chunks)
+        assert names.count(f"radial_mlp_hidden_backward_{gates}") == 1
+
+
 @pytest.mark.parametrize("number", [7, 500])
 def test_unknown_atoms_raise_without_input_validation(number):
     """The status word is read in any case: an unknown atom never counts as a known one."""
