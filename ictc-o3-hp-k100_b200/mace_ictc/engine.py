@@ -24,6 +24,7 @@ from __future__ import annotations
 import ctypes as C
 import math
 import threading
+import weakref
 
 import torch
 
@@ -113,16 +114,17 @@ class ForceEngine:
     """``chunk_rows``: owner rows per chunk of the streamed gate evaluation (None: one pass over everything).
     ``chunk_margin``: a chunk buffer holds ``chunk_rows x mean degree x chunk_margin`` edges; a chunk with more
     edges than that raises ``overflow`` (device flag) and its surplus edges are dropped, never written out of
-    bounds.  ``stream_gates``: see the attribute."""
+    bounds.  ``stream_gates``: see the attribute.  ``owned``: the model keeps this engine, which then holds no reference to it
+    (a cycle would keep the laid-out weights of a deleted model until the next garbage collection)."""
 
     def __init__(self, model: MaceIctcModel, chunk_rows: int | None = None, chunk_margin: float = 1.3,
-                 stream_gates: bool | None = None, lay_out: bool = True):
+                 stream_gates: bool | None = None, lay_out: bool = True, owned: bool = False):
         if len(model.interactions) != 2:
             raise ValueError("the force engine covers the two-interaction model")
         if model.channels != 64:
             raise ValueError("the force engine runs on the 64-channel tensor-core kernels; other widths use the "
                              "autograd route (MolecularDynamics(..., use_engine=False))")
-        self.model = model
+        self._model, self._held = weakref.ref(model), None if owned else model
         self.c = model.channels
         self.dev = next(model.parameters()).device
         self.lib = _lib.load()
@@ -142,6 +144,10 @@ class ForceEngine:
         if lay_out:
             self.refresh()
 
+    @property
+    def model(self) -> MaceIctcModel:
+        return self._model()
+
     # ---------------------------------------------------------------- weights
     def _watch(self):
         """Every module and parameter slot of the model with what it holds now: a replaced one is noticed by identity, a new
@@ -153,8 +159,8 @@ class ForceEngine:
                 slots.extend((table, key, value) for key, value in table.items())
         params = list(self.model.parameters())
         inter = list(self.model.interactions)
-        own = [module.__dict__ for module in modules]
-        hooks = [d[name] for d in own for name in _HOOKS]
+        hooks = [module.__dict__[name] for module in modules for name in _HOOKS]
+        own = [module.__dict__ for module in modules[1:]]           # without the model's own, where this engine may be kept
         return slots, sizes, params, inter, covers(self.model), own, hooks
 
     def _state(self):
@@ -172,7 +178,7 @@ class ForceEngine:
         _, _, _, inter, covered, own, hooks = self._watched
         table = torch.nn.modules.module
         if (not covered or any(getattr(table, name) for name in _GLOBAL_HOOKS) or any(hooks)
-                or any("forward" in d for d in own) or any(i.tp.weight.requires_grad for i in inter)):
+                or "forward" in self.model.__dict__ or any("forward" in d for d in own) or any(i.tp.weight.requires_grad for i in inter)):
             return None
         state, fit = self._state(), self._fit
         if fit is None or fit[0] != state:

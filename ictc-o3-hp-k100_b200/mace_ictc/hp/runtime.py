@@ -78,7 +78,7 @@ def _force_engine(model, tensors, mask):
         from ..engine import ForceEngine
         if model.node_embedding.weight.device != dev:
             return None
-        engine = ForceEngine(model, lay_out=False)
+        engine = ForceEngine(model, lay_out=False, owned=True)
         model.__dict__["_force_engine"] = engine
     state = engine.stands_for()
     return None if state is None else (engine, state)

@@ -296,6 +296,29 @@ def _edges(md):
     return nl.src[:e], nl.dst[:e], nl.shifts[:e], md.box.tolist(), md.pos.shape[0], nl.rowptr
 
 
+def test_a_deleted_model_gives_its_memory_back_at_once():
+    import gc
+    import weakref
+    from mace_ictc.engine import ForceEngine
+    from mace_ictc.hp import energy_and_forces
+    graph = _graph(np.random.default_rng(1), (20,), False)
+    model = _model()
+    energy_and_forces(model, *graph)
+    before = torch.cuda.memory_allocated()
+    gc.disable()
+    try:
+        model = _model()
+        energy_and_forces(model, *graph)
+        seen, engine = weakref.ref(model), weakref.ref(model.__dict__["_force_engine"])
+        del model
+        assert seen() is None and engine() is None
+        assert torch.cuda.memory_allocated() <= before
+    finally:
+        gc.enable()
+    engine = ForceEngine(_model())                  # an engine of its own keeps its model
+    assert engine.model is not None and engine.stands_for() is not None
+
+
 @pytest.mark.parametrize("chunk_rows", [None, 3])
 def test_a_profile_names_every_heavy_launch(chunk_rows):
     from mace_ictc import synthetic as S

@@ -59,6 +59,10 @@ OTHER_MODELS = {
     "contraction of the other layout": lambda m: setattr(m.products[0].symmetric_contractions, "ir_mul", True),
     "a fractional cutoff order": lambda m: setattr(m, "polynomial_cutoff_p", 5.5),
     "double precision": lambda m: m.double(),
+    "a forward of its own on the model": lambda m: setattr(m, "forward", lambda *a, **k: None),
+    "a forward of its own on a block": lambda m: setattr(m.products[1], "forward", lambda *a, **k: None),
+    "a hook": lambda m: m.interactions[0].linear_up.register_forward_hook(lambda *_: None),
+    "a hook on the model": lambda m: m.register_forward_pre_hook(lambda *_: None),
     "trainable base coefficients": lambda m: m.interactions[0].tp.weight.requires_grad_(True),
 }
 
