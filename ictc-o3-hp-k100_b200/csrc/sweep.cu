@@ -45,7 +45,8 @@ __global__ void embed_kernel(EmbedArgs a) {
   if (row >= a.n) return;
   int64_t s;
   if (a.numbers) {
-    const int64_t z = ldg(a.numbers + row);
+    int64_t z = ldg(a.numbers + row);
+    if (z < 0) z += a.table_size;            // as an index of the table counts from its end in the model's forward
     s = z >= 0 && z < a.table_size ? ldg(a.table + z) : -1;
     if ((i & 15) == 0) {
       if (s < 0) atomicOr(a.status, 1);

@@ -337,7 +337,15 @@ def test_a_profile_names_every_heavy_launch(chunk_rows):
         assert names.count(f"radial_mlp_hidden_backward_{gates}") == 1
 
 
-@pytest.mark.parametrize("number", [7, 500])
+def test_negative_numbers_index_the_species_table_as_in_the_forward():
+    from mace_ictc.hp import energy_and_forces
+    model = _model()
+    graph = _graph(np.random.default_rng(4), (40,), False)
+    graph[1][5], graph[1][6] = -1, -3                         # of a table of nine: 8 and 6
+    _close(energy_and_forces(model, *graph), _autograd(model, graph))
+
+
+@pytest.mark.parametrize("number", [7, 500, -2, -10])
 def test_unknown_atoms_raise_without_input_validation(number):
     """The status word is read in any case: an unknown atom never counts as a known one."""
     from mace_ictc.hp import energy_and_forces
