@@ -52,10 +52,6 @@ __global__ void nb_bin_fill_kernel(const float* __restrict__ pos, int64_t n, con
   atoms[cell_start[w.x] + w.y] = make_float4(pos[3 * i], pos[3 * i + 1], pos[3 * i + 2], __int_as_float(int(i)));
 }
 
-__device__ __forceinline__ int64_t nb_key(int64_t j, int sx, int sy, int sz) {
-  return j * 27 + ((sx + 1) * 3 + (sy + 1)) * 3 + (sz + 1);
-}
-
 // One warp per centre.  The 27 cells around it are one list of candidates (lane l describes cell l; prefix sums in
 // shared memory), which the lanes walk 32 at a time: about 8 rounds for 250 candidates.  One thread per centre, the
 // former split, left 8 of 148 SMs busy at 1,000 atoms and spent its time on dependent loads.  f(hit, key) is called by
