@@ -38,7 +38,9 @@ __device__ __forceinline__ int pdl_enter() {
   return zero;
 }
 // Only for launches of about one wave: blocks that wait early take room from the running kernel's own, and a long kernel gains
-// nothing (2 steps of 131,072 atoms: 51.5 ms with ordinary launches, 53.1 with every launch early).
+// nothing (2 steps of 131,072 atoms: 51.5 ms with ordinary launches, 53.1 with every launch early).  Where the line lies
+// matters little: recorded MD step with half, this and twice the limit 216 atoms 262 / 262 / 262 us, 1,000 397 / 394 / 395, 2,744
+// 771 / 774 / 775, 8,000 1,817 / 1,816 / 1,813, 10,164 2,312 / 2,277 / 2,295, larger systems within the runs' spread of 1 %.
 constexpr int64_t kEarlyBlocks = 148 * 8;
 template <class... P, class... A>
 inline void launch_if(bool early, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {

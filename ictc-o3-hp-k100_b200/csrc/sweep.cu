@@ -313,9 +313,9 @@ struct TailArgs {
   int64_t n;
 };
 
-// A warp goes through four atoms, which saves energy atomics; while the atoms do not fill the chip's warp slots (148 SMs x 64) one
-// each is faster.  10 recorded MD steps of 1,000 atoms
-// 4.02 -> 3.92 ms, energy_and_forces of 216 atoms 261 -> 250 us.
+// While the atoms do not fill the chip's warp slots (148 SMs x 64) a warp has one atom, beyond that four, which quarters the sums
+// that the last kernel adds up (and a batch's atomics).  Recorded MD step with one atom / four: 216 atoms 262 / 267 us, 1,000
+// 394 / 403, 2,744 774 / 780, 8,000 1,812 / 1,829; 17,576 3,891 / 3,850, larger systems within the runs' spread of 1 %.
 constexpr int kTailWarps = 8;
 constexpr int64_t kTailSlots = 148 * 64;
 static int tail_nodes(int64_t n) { return n <= kTailSlots ? 1 : 4; }
@@ -539,7 +539,9 @@ int Runner::run() {
   const bool paired = p.rep != nullptr;
   const bool table = !(p.chunk_rows > 0 && p.chunk_rows < (n > N ? n : N) && p.stream_gates);
   // The interactions share launches when all stages run together; with timing every launch is one interaction's.  Both
-  // reverse sweeps' hidden gradients are then alive together: not for lists beyond 4 M edges.
+  // reverse sweeps' hidden gradients (256 bytes an edge) are then alive together: not for lists beyond 4 M edges, where the time is
+  // the same and the memory counts.  Recorded MD step, shared against separate: 216 atoms 262 / 276 us, 1,000 394 / 402, 2,744
+  // 774 / 785, 8,000 1,816 / 1,831; from 10,164 atoms to 262,144 (8.4 M edges) within the runs' spread of 1 %.
   const bool merged = stages == 31 && !p.host_marks;
   const bool merged_back = merged && E <= (int64_t(4) << 20);
 
