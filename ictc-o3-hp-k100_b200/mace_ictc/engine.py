@@ -65,7 +65,8 @@ def covers(m):
     """Is every module at its place the one whose forward the sweep reproduces, with the shapes that the layout reads and
     nothing (a bias, another activation, a further output) that it does not read?"""
     c, species = 64, getattr(m, "num_elements", None)
-    if not (_has(m, MaceIctcModel, channels=c, lmax=2, num_interaction=2) and _linear(m.node_embedding, c, species, bias=True)
+    if not (isinstance(m, MaceIctcModel) and type(m).forward is MaceIctcModel.forward and _has(m, type(m), channels=c, lmax=2, num_interaction=2)
+            and _linear(m.node_embedding, c, species, bias=True)
             and all(_has(x, torch.nn.ModuleList) for x in (m.interactions, m.products, m.layer_energy_readouts))
             and len(m.interactions) == len(m.products) == 2 and len(m.layer_energy_readouts) >= 1):
         return False

@@ -96,6 +96,20 @@ def test_the_stock_model_is_covered():
     assert _stands_for(biased)
 
 
+def test_subclasses_with_the_stock_forward_keep_the_engine():
+    from mace_ictc.engine import covers
+    from mace_ictc.model import MaceIctcModel
+
+    class Named(MaceIctcModel):
+        name = "mine"
+
+    class Other(MaceIctcModel):
+        def forward(self, *args, **kwargs):
+            return 2 * super().forward(*args, **kwargs)
+
+    assert covers(Named()) and not covers(Other()) and not covers(torch.nn.Linear(2, 2))
+
+
 def test_misaligned_weights_and_buffers_are_refused_before_any_launch():
     """Made-up addresses, none of which is touched: the check comes before the first launch."""
     from ictc_o3 import _lib
