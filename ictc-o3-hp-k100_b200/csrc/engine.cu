@@ -136,8 +136,7 @@ __global__ void __launch_bounds__(256) silu_kernel(int64_t n, bool wide, float s
 }
 
 // Whole-row layout conversion between mul_ir (block [C][m]) and ir_mul (block [m][C]) for a row made of
-// degree blocks, each holding `count` path slots.  One thread per output element: writes are coalesced,
-// reads are strided by at most 2l+1 floats and stay inside one cache line group.
+// degree blocks, each holding `count` path slots.
 constexpr int kLayoutBlocks = 8;
 struct LayoutArgs {
   int64_t rows;

@@ -270,7 +270,7 @@ class PackedGraphMessage(torch.nn.Module):
     """Gather at the sender, tensor product, sum at the receiver, on packed ir_mul rows.
 
     Same call contract as the reference (ictc_o3/operators.py:343-409).  The receiver sum always walks a
-    receiver CSR with one warp per row (no float atomics, bitwise repeatable), so ``reduction`` and the K100
+    receiver CSR in a fixed order (no float atomics, bitwise repeatable), so ``reduction`` and the K100
     tuning arguments (``edge_chunk_size``, ``topology_backend``, ``csr_accumulator_limit``,
     ``csr_slice_search``, ``geometry_schedule``) are checked for validity and otherwise unused.
     """
